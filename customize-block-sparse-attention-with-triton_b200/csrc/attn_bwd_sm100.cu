@@ -726,10 +726,10 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   const void* str0 = kDKDV ? q : k;
   const void* str1 = kDKDV ? dout : v;
   CUtensorMap tm_a0, tm_a1, tm_b0, tm_b1;
-  if ((rc = make_qkv_tmap(&tm_a0, stat0, strides, B, H, N, dtype, 64)) != BSA_OK) return rc;
-  if ((rc = make_qkv_tmap(&tm_a1, stat1, strides, B, H, N, dtype, 64)) != BSA_OK) return rc;
-  if ((rc = make_qkv_tmap(&tm_b0, str0, strides, B, H, N, dtype, 64)) != BSA_OK) return rc;
-  if ((rc = make_qkv_tmap(&tm_b1, str1, strides, B, H, N, dtype, 64)) != BSA_OK) return rc;
+  if ((rc = make_qkv_tmap(&tm_a0, stat0, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
+  if ((rc = make_qkv_tmap(&tm_a1, stat1, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
+  if ((rc = make_qkv_tmap(&tm_b0, str0, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
+  if ((rc = make_qkv_tmap(&tm_b1, str1, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
 
   BwdParams prm;
   prm.list_ptr = list_ptr;

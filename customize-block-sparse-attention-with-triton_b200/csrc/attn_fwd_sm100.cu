@@ -5,53 +5,64 @@
 // optional work counter (or walks a fixed stride).  The list is taken FOUR key tiles at a time
 // ("supersteps": tiles a, b, c, d in list order).  The 128 TMEM lanes are split between the
 // tiles: lanes 0..63 own tiles a and c, lanes 64..127 own tiles b and d, so that every SM
-// sub-partition (32 lanes) has the same amount of exp2 work whatever the sparsity pattern, and a
-// softmax warp works through 128 logits per row between two barrier round trips.
+// sub-partition (32 lanes) has the same amount of exp2 work whatever the sparsity pattern.
 //
-// The query block sits in shared memory once, between blocks of zero rows: [Z; Q; Z].  The
-// 128-row A operand [Q; Z] (Q in rows 0..63) multiplied with [K_a; K_c]^T fills lanes 0..63 of an
-// S slot with the logits of tiles a (columns 0..63) and c (columns 64..127) and lanes 64..127 with
-// zeros; the operand [Z; Q] with [K_b; K_d]^T then adds the logits of tiles b and d to lanes
-// 64..127 (and zeros to the others): eight M=128, N=128, K=16 MMAs per superstep, none of whose
-// 128 x 128 outputs is thrown away.
+// S of a superstep is ONE product of 64 query rows with 256 keys: the M = 64 "weight stationary"
+// form of the MMA puts columns [0, 128) of its result into lanes 0..63 and columns [128, 256) into
+// lanes 64..127 of the same 128 TMEM columns, which is just the split above.  (An M = 128
+// instruction can only fill the lanes that way with half of its rows multiplied by zeros.)  P V
+// writes the accumulator rows of the lanes that own the tile and leaves the others alone, so the
+// other lanes' P columns need no zeros either.  Measured on one SM, in cycles per tile: S 80 (128
+// with the M = 128 form, both bound by the operand reads from shared memory at 128 B per cycle),
+// P V 128 (any form), S and P V issued together 210 (259).
+//
+// The supersteps alternate between two softmax teams of four warps, each with its own accumulator,
+// so that one team exponentiates while the other waits for its products.  Three S slots rotate;
+// the probabilities go over the logits of their slot, which is held from the S product until P V
+// is complete.
+//
+// What bounds it: with everything listed a tile takes about 335 SM cycles, of which the exp2 unit
+// is busy 256 (4096 exponentials at 16 per cycle; a loop of nothing but loads, exponentials and
+// stores, two warps per sub-partition, measures 281); what is left are hand-overs between the
+// roles, about 140 cycles each.  With short lists the instruction cache comes first: all roles run
+// at the same time, and 2.5 KB more in the softmax loop made everything 10 % slower.  So what is
+// executed per item or per superstep is kept short, waits included.
+// B200, fp16, D = 64, against the form with M = 128 products and both teams on every superstep:
+// N = 17536 with one head, all blocks 136 -> 110 us, a tenth of them 27.0 -> 23.7 us; 8 heads, a
+// tenth 133 -> 110 us; bf16 N = 32000, 32 heads, a tenth 1.53 -> 1.31 ms.
 //
 // Roles (16 warps); every role walks the same item sequence, so set-up of item i+1 and write-out
 // of item i-1 overlap the arithmetic of item i:
-//   warp 8      : producer — lists the CTA's first item, then TMA-loads Q and the listed K tiles of
-//                 every item into a 2-deep ring of superstages (4 tiles, held until S is
-//                 complete), one lane per tile, and tells the lister when to set up the next item
-//   warp 14     : lister (also a write-out warp) — draws the next item, lists its key blocks (from
-//                 the mask row, or copies the CSR row) into the other list buffer and publishes it
-//   warp 15     : V producer — TMA-loads the listed V tiles into a 3-deep ring (held until P V is
-//                 complete), one lane per tile.  Only listed tiles are ever loaded.
+//   warps 0..7  : online softmax (team = warp / 4, TMEM lane quarter = warp % 4; superstep g is team
+//                 g % 2's).  A warp loads its tiles' 128 logits, exponentiates them, packs P to 16 bit
+//                 and stores it over the logits (first tile in columns [0, 32) of the slot, second
+//                 one in [32, 64)).
+//   warp 8      : K producer — lists the CTA's first item, then TMA-loads Q and the listed K tiles of
+//                 every item into a 3-deep ring of superstages (4 tiles, held until S is complete),
+//                 one lane per tile, and tells the lister when to set up the next item
 //   warp 9      : S issuer and TMEM owner
-//   warp 10     : P V issuer — O[T] += P_t V_t for the tiles t of the superstep: tiles a, b into the
-//                 accumulator of softmax team 0, tiles c, d into that of team 1.  P is read from
-//                 TMEM, V is an MN-major shared-memory operand.  The lanes that do not own tile t
-//                 hold zeros in t's P columns, so row r of an accumulator only sums products of
-//                 the tile owned by lanes 0..63 and row r+64 only of the other one.
-//   warps 0..7  : online softmax in two teams of four warps (team = warp / 4, TMEM lane quarter =
-//                 warp % 4).  Every warp works on every superstep: team 0 on tiles a, b (columns
-//                 0..63 of the slot), team 1 on tiles c, d (columns 64..127); each team has its own
-//                 accumulator and (m, l) per lane.  Three S slots (128 TMEM columns) rotate over
-//                 the supersteps; a slot is held from the S MMAs until the P V MMAs that read the
-//                 probabilities, which overwrite the logits in place, are complete, so while one
-//                 slot is with the softmax warps the next already holds its logits and the
-//                 previous one is being multiplied with V.  A warp loads its tile's 64 logits,
-//                 takes the row maximum, moves the lane's reference maximum if need be (rescaling
-//                 its accumulator rows), exponentiates, and stores P (16-bit, 32 columns) over one
-//                 half of the tile's columns and zeros over the other half, where the other 64
-//                 lanes' P goes: tile t's P ends up in columns [32 t, +32) of the slot.
-//   warps 11..14: write-out — merge the four partial results (m, l, O) of every query row (teams x
-//                 lanes r / r+64), normalise, store O, LSE and the row maximum.
+//   warp 10     : P V issuer — O[team] += P_t V_t for the tiles t of the superstep.  P is read from
+//                 TMEM, V is an MN-major shared-memory operand.  Row r of an accumulator sums products
+//                 of tiles a and c, row r+64 of tiles b and d.
+//   warp 11     : V producer — TMA-loads the listed V tiles in pairs into a 5-deep ring (held until
+//                 their P V is complete).  Only listed tiles are ever loaded.
+//   warps 12..15: write-out — merge the four partial results (m, l, O) of every query row (teams x
+//                 lanes r / r+64), normalise, store O, LSE and the row maximum
+//   warp 15     : also the lister — draws the next item, lists its key blocks (from the mask row, or
+//                 copies the CSR row) into the next of three list buffers and publishes it
 // TMEM (512 columns): S/P slots 3 x 128, accumulators 2 x 64.
+//
+// Head dimensions 16 and 32 run on the same 128-byte rows: the tensor maps are D wide, so TMA fills
+// the other columns of a tile with zeros without reading them, S takes D / 16 K steps instead of
+// four, and P V is D columns wide.
 //
 // Numerics follow the reference's loop (fa2_custom_mask/fa2_fwd.py:150-196): logits scaled by
 // sm_scale*log2(e), exp2 domain, fp32 row sums of the fp32 probabilities, P rounded to the input
-// dtype before P V.  The running maximum is only advanced when it grew by more than 8 (a factor
-// 256), which leaves O = acc / l unchanged because both use the same reference maximum.  Which
-// partial result a tile goes into depends on its position in the row's list alone, so results do
-// not depend on which CTA computes an item.
+// dtype before P V.  The reference maximum of a row is the maximum of its first tiles and moves only
+// when later logits would make probabilities too large for 16 bit (sum of a superstep above 4096),
+// which leaves O = acc / l unchanged because both use the same reference.  Which partial result a
+// tile goes into depends on its position in the row's list alone, so results do not depend on which
+// CTA computes an item.
 //
 // Every wait is bounded; a wait that gives up raises a CTA-wide flag, every role then falls
 // through its loops without touching barriers' data again, and TMEM is always released.  Every
@@ -65,51 +76,60 @@
 
 namespace bsa {
 
-constexpr int kKStages = 2;     // K superstages (4 tiles) in flight: held from load to S complete
-constexpr int kVStages = 3;     // V superstages (4 tiles) in flight: held from load to P V complete
+constexpr int kKStages = 3;     // K superstages (4 tiles) in flight: held from load to S complete
+constexpr int kVStages = 5;     // pairs of V tiles in flight: held from load to P V complete
 constexpr int kSlots = 3;       // S/P slots (128 TMEM columns): held from S issue to P V complete
+constexpr int kLists = 3;       // items set up at a time: one being worked on, one written out, one to come
+constexpr int kSoftmaxWarps = 8;
+constexpr int kTeamWarps = kSoftmaxWarps / 2;
+constexpr int kProducerWarp = 8, kSWarp = 9, kPvWarp = 10, kVProducerWarp = 11;
+constexpr int kListerWarp = 15;      // the last of the write-out warps 12..15: also sets up the items
 constexpr int kFwdThreads = 512;
-constexpr int kSoftmaxWarps = 8, kProducerWarp = 8, kSWarp = 9, kPvWarp = 10;  // warps 11..14 write out
-constexpr int kVProducerWarp = 15;  // = the last warp
-constexpr int kListerWarp = 14;     // the write-out warp that also sets up the items
-constexpr int kGoBefore = 2;         // ordered hand-out: K superstages before an item's end at which the next is drawn
+constexpr int kGoBefore = 2;         // ordered hand-out: supersteps before an item's end at which the next is drawn
 constexpr uint32_t kTileBytes = 64 * 64 * 2;       // one Q, K or V tile
 constexpr uint32_t kFwdTmemCols = 512;
 // TMEM columns: slot r at 128 r; accumulator of softmax team T at 384 + 64 T.
 constexpr uint32_t kTmemO = 384;
 constexpr float kRescaleThreshold = 8.0f;
+// Largest sum of a row's probabilities in a superstep (hence largest probability) that may go into P
+// against a reference maximum that was not checked: far below fp16's 65504.
+constexpr float kMaxRowSum = 4096.0f;
 constexpr int kFwdMaxTiles = 2048;  // key blocks per row that a CTA can list (N <= 131072)
 constexpr int kMaxSorted = 320;     // items beyond the first round that a CTA can put in order
 constexpr uint16_t kColPartial = 0x8000;  // list entry in shared memory: the tile has masked elements
 constexpr uint16_t kColIndex = 0x7fff;
 
 struct FwdSmem {
-  uint8_t qz[5][kTileBytes];                  // Z, Q (even items), Z, Q (odd items), Z
+  uint8_t q[2][kTileBytes];                   // by parity of the non-empty items
   uint8_t k[kKStages][4][kTileBytes];         // tiles in the order a, c, b, d
-  uint8_t v[kVStages][4][kTileBytes];         // tiles in the order a, b, c, d
-  float xfer[32][65];                         // write-out: lanes 64..127 hand over, [col][row]
-  uint16_t cols[2][kFwdMaxTiles];             // by item parity: the item's key-block list (| kColPartial)
+  uint8_t v[kVStages][2][kTileBytes];
+  // write-out: what lanes 0..63 and 64..127 hand to each other, 16 columns of 64 rows at a time (rows
+  // of 20 floats: eight lanes' 16-byte accesses then fall into different banks)
+  float xfer[2][64][20];
+  uint16_t cols[kLists][kFwdMaxTiles];        // ring over the items: the item's key-block list (| kColPartial)
   alignas(16) int cnt[kMaxSorted];            // sort keys (tile count, item) of the items beyond the first round
   int order[kMaxSorted];                      // those items, longest first
-  int ntiles[2];
-  int item[2];                                // by item parity: the work item, -1 = no more work
+  int4 item[kLists];                          // the item: batch (-1 = no more work), head, query block, tile count
+  int first_team[2];                          // by item parity: the team with the item's first superstep
   float mref[2][2][128];                      // by item parity, softmax team, lane
   float lsum[2][2][128];
   float mtrue[2][2][128];
   uint64_t order_full;                        // `order` is ready
-  uint64_t list_full[2];                      // lister -> everyone: list and tile count ready
+  uint64_t list_full[kLists];                 // lister -> everyone: list and header ready
+  uint64_t list_free[kLists];                 // producers and issuers are through with list and header
   uint64_t setup_go[2];                       // producer -> lister: time to set up the next item
   uint64_t q_full[2], q_free[2];
   uint64_t k_full[kKStages];
   uint64_t k_empty[kKStages];                 // S of the superstep complete
   uint64_t v_full[kVStages];
-  uint64_t v_empty[kVStages];                 // P V of the superstep complete
-  uint64_t s_full[kSlots];                    // S of the superstep complete
-  uint64_t p_full[kSlots][2];                 // by team: its four warps stored P of the superstep
+  uint64_t v_empty[kVStages];                 // P V of the pair complete
+  uint64_t s_full[2 * kSlots];                // S of the superstep complete; one per (team, slot), so
+                                              // that the team that waits on it sees each phase
+  uint64_t p_full[kSlots];                    // the team's four warps stored P of the superstep
   uint64_t pv_done[kSlots];                   // P V of the superstep complete: slot free, O current
   uint64_t o_full[2];                         // last P V of the item done
   uint64_t stats_full[2];                     // softmax warps published (m, l) of the item
-  uint64_t o_free[2];                         // write-out holds accumulators/stats/header in registers
+  uint64_t o_free[2];                         // write-out has read accumulators, stats and header
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -126,7 +146,7 @@ struct FwdParams {
   int64_t o_sb, o_sh, o_sn;
   float* lse2;
   float* rowmax;
-  int B, H, N, nb;
+  int B, H, N, D, nb;
   int row_begin, nrows;     // the query-block rows [row_begin, row_begin + nrows) of every head
   int list_b_stride, list_h_stride;
   int items;                // B * H * nrows
@@ -143,14 +163,13 @@ __device__ __forceinline__ void fwd_give_up(FwdSmem* sm, int32_t* status, int co
   report_status(status, code);
 }
 
-// exp2 of one 32-column chunk of S against the row's reference maximum; returns the packed
-// 16-bit probabilities and adds their fp32 sum to l.  The scale-and-subtract and the running sums
-// take two columns per instruction.
+// exp2 of 32 columns of S against the row's reference maximum: packs the probabilities to 16 bit and
+// adds them (fp32) to two pairs of running sums.  The scale-and-subtract and the sums take two
+// columns per instruction.
 template <bool kBf16>
 __device__ __forceinline__ void exp_chunk(const uint32_t* sr, float c, float neg_m, uint32_t* pk,
-                                          float& l) {
+                                          uint64_t& l0, uint64_t& l1) {
   const uint64_t c2 = pack_f32x2(c, c), m2 = pack_f32x2(neg_m, neg_m);
-  uint64_t l01 = pack_f32x2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < 32; i += 4) {
     float z0, z1, z2, z3;
@@ -160,13 +179,11 @@ __device__ __forceinline__ void exp_chunk(const uint32_t* sr, float c, float neg
         fma_f32x2(pack_f32x2(__uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3])), c2, m2), z2,
         z3);
     const float p0 = ex2_approx(z0), p1 = ex2_approx(z1), p2 = ex2_approx(z2), p3 = ex2_approx(z3);
-    l01 = add_f32x2(add_f32x2(l01, pack_f32x2(p0, p1)), pack_f32x2(p2, p3));
+    l0 = add_f32x2(l0, pack_f32x2(p0, p1));
+    l1 = add_f32x2(l1, pack_f32x2(p2, p3));
     pk[i / 2] = pack_2x16<kBf16>(p0, p1);
     pk[i / 2 + 1] = pack_2x16<kBf16>(p2, p3);
   }
-  float a0, a1;
-  unpack_f32x2(l01, a0, a1);
-  l += a0 + a1;
 }
 
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -183,6 +200,58 @@ __device__ __forceinline__ float max_chunk(const uint32_t* sr) {
     mx1 = max3(mx1, __uint_as_float(sr[i + 2]), __uint_as_float(sr[i + 3]));
   }
   return max3(mx0, mx1, fmaxf(__uint_as_float(sr[30]), __uint_as_float(sr[31])));
+}
+
+// 32 logits of one row: those whose mask byte is zero become -inf, so that they take no part in the
+// maximum and exponentiate to 0.
+__device__ __forceinline__ void mask_chunk(uint32_t* sr, const uint8_t* mask) {
+  uint4 mw[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) mw[j] = __ldg(reinterpret_cast<const uint4*>(mask) + j);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t w4[4] = {mw[j].x, mw[j].y, mw[j].z, mw[j].w};
+#pragma unroll
+    for (int q4 = 0; q4 < 4; ++q4) {
+      const uint32_t nz = __vcmpne4(w4[q4], 0u);  // 0xff in every byte that keeps its element
+#pragma unroll
+      for (int bb = 0; bb < 4; ++bb) {
+        const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
+        const int i = 16 * j + 4 * q4 + bb;
+        sr[i] = (sr[i] & keep) | (0xff800000u & ~keep);
+      }
+    }
+  }
+}
+
+// Takes a superstep's scaled row maximum into a lane's running ones; returns the factor by which the lane's
+// rows of O have to be rescaled (1: not at all).  (A row with nothing kept so far keeps m_ref = -inf:
+// its logits are all -inf, and against a zero in place of the maximum they exponentiate to 0 instead
+// of NaN.)
+__device__ __forceinline__ float fwd_new_max(float zmax, float& m_ref, float& m_true, float& l) {
+  float alpha = 1.f;
+  m_true = fmaxf(m_true, zmax);
+  if (m_ref == -INFINITY) {
+    m_ref = zmax;  // first tile of this lane in this item: O and l are still zero
+  } else if (zmax > m_ref + kRescaleThreshold) {
+    alpha = ex2_approx(m_ref - zmax);
+    l *= alpha;
+    m_ref = zmax;
+  }
+  return alpha;
+}
+
+// Multiplies the warp's rows of an accumulator (64 columns) with a factor per lane.
+__device__ __forceinline__ void fwd_rescale(uint32_t o_addr, float alpha) {
+#pragma unroll 1
+  for (int part = 0; part < 4; ++part) {
+    uint32_t orow[16];
+    tmem_ld_32x32b_x16(o_addr + 16 * part, orow);
+    tc_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) orow[j] = __float_as_uint(__uint_as_float(orow[j]) * alpha);
+    tmem_st_32x32b_x16(o_addr + 16 * part, orow);
+  }
 }
 
 // Work item w -> (batch, head, query block); late (long, if causal) query blocks of a head first.
@@ -275,13 +344,12 @@ __device__ __forceinline__ void fwd_build_order(FwdSmem* sm, const FwdParams& p,
   if (tid == 0) mbar_arrive(smem_u32(&sm->order_full));
 }
 
-// Lists the key blocks of work item w into the list buffer of parity par (one warp) and publishes
-// list, tile count and item.
+// Lists the key blocks of work item w into list buffer `at` (one warp) and publishes list and item.
 template <bool kElementMask>
-__device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, int w, int par,
+__device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, int w, int at,
                                               int lane) {
   const FwdItem it = fwd_item(w, p);
-  uint16_t* cols = sm->cols[par];
+  uint16_t* cols = sm->cols[at];
   int n_tiles = 0;
   if (p.block != nullptr) {
     // mask mode: ordered compaction of the kept blocks of mask row (b, h, mb)
@@ -323,11 +391,24 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
   }
   __syncwarp();
   if (lane == 0) {
-    sm->ntiles[par] = n_tiles;
-    sm->item[par] = w;
-    mbar_arrive(smem_u32(&sm->list_full[par]));  // release: count and list are visible
+    sm->item[at] = make_int4(it.b, it.h, it.mb, n_tiles);
+    mbar_arrive(smem_u32(&sm->list_full[at]));  // release: list and item are visible
   }
 }
+
+// A role's walk over the items: waits for the next one to be published and reads its header.
+struct FwdWalk {
+  int at = 0, ph = 0;  // list buffer, phase of its barrier
+  int4 it;             // batch (< 0: no more work), head, query block, tile count
+  __device__ __forceinline__ bool wait(FwdSmem* sm, volatile int* abort_flag) {
+    if (!mbar_wait_warp(smem_u32(&sm->list_full[at]), ph, abort_flag)) return false;
+    it = sm->item[at];
+    return true;
+  }
+  __device__ __forceinline__ void next() {
+    if (++at == kLists) { at = 0; ph ^= 1; }
+  }
+};
 
 // kElementMask: the instantiation that applies a dense mask inside the tiles marked partial; the
 // plain one carries none of that code.
@@ -351,7 +432,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // ---- set-up ----
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sm->list_full[i]), 1);
       mbar_init(smem_u32(&sm->setup_go[i]), 1);
       mbar_init(smem_u32(&sm->q_full[i]), 1);
       mbar_init(smem_u32(&sm->q_free[i]), 1);
@@ -367,24 +447,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(smem_u32(&sm->v_full[s]), 1);
       mbar_init(smem_u32(&sm->v_empty[s]), 1);
     }
+    for (int s = 0; s < 2 * kSlots; ++s) mbar_init(smem_u32(&sm->s_full[s]), 1);
     for (int s = 0; s < kSlots; ++s) {
-      mbar_init(smem_u32(&sm->s_full[s]), 1);
-      mbar_init(smem_u32(&sm->p_full[s][0]), kSoftmaxWarps / 2);
-      mbar_init(smem_u32(&sm->p_full[s][1]), kSoftmaxWarps / 2);
+      mbar_init(smem_u32(&sm->p_full[s]), kTeamWarps);
       mbar_init(smem_u32(&sm->pv_done[s]), 1);
+    }
+    for (int s = 0; s < kLists; ++s) {
+      mbar_init(smem_u32(&sm->list_full[s]), 1);
+      mbar_init(smem_u32(&sm->list_free[s]), 4);  // two producers, two issuers
     }
     mbar_init(smem_u32(&sm->order_full), 1);
     sm->abort_flag = 0;
     mbar_fence_init();
-  }
-  {
-    // the three blocks of zero rows around the two query buffers; the MMAs read them through the
-    // async proxy
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    constexpr int kVecs = kTileBytes / 16;
-    for (int i = threadIdx.x; i < 3 * kVecs; i += kFwdThreads)
-      reinterpret_cast<uint4*>(sm->qz[2 * (i / kVecs)])[i % kVecs] = z;
-    fence_proxy_async_smem();
   }
   if (warp == kSWarp) {
     tmem_alloc(smem_u32(&sm->tmem_base), kFwdTmemCols);
@@ -401,27 +475,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
 
+  // 512 threads are launched with 128 registers: the softmax warps, which hold 128 logits each, take
+  // what the others do without (2 x 160 + 80 + 112 = 4 x 128).
+  if (warp >= kSoftmaxWarps && warp < kSoftmaxWarps + 4) {
+  give_registers<80>();
   if (warp == kProducerWarp) {
-    // =========================== producer ===========================
+    // =========================== K producer ===========================
     bool ok = true;
     // Loads Q and the K tiles of the listed key blocks from the list the lister published, and
     // tells the lister when to set up the next item.  A set-up takes 3-4 thousand cycles (the draw
     // from the work counter, the mask row, the ballots in a warp that shares its scheduler with
-    // two softmax warps), about two supersteps.  With many items per CTA it is started as soon as
-    // an item begins; with the few items of the ordered hand-out, where it matters that a CTA
-    // draws its next item only when it is about to need it, kGoBefore superstages before the end.
-    int gs = 0;  // supersteps issued so far by this CTA (ring position)
-    int qi = 0;  // non-empty items so far (Q buffer position)
+    // the softmax warps), about three supersteps.  With many items per CTA it is started as soon as an
+    // item begins; with the few items of the ordered hand-out, where it matters that a CTA draws
+    // its next item only when it is about to need it, kGoBefore supersteps of loads before the end.
+    int ks = 0, kph = 1;  // ring position, parity to wait for
+    int qi = 0;           // non-empty items so far (Q buffer position)
     fwd_list_item<kElementMask>(sm, p, blockIdx.x, 0, lane);  // the CTA's own first item
-    for (int i = 0; ok; ++i) {
+    FwdWalk walk;
+    for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->list_full[par]), (i >> 1) & 1, abort_flag);
-      if (!ok) break;
-      const int w = *const_cast<volatile int*>(&sm->item[par]);
-      if (w < 0) break;  // no more work
-      const FwdItem it = fwd_item(w, p);
-      const int n_tiles = *const_cast<volatile int*>(&sm->ntiles[par]);
-      const uint16_t* cols = sm->cols[par];
+      ok = walk.wait(sm, abort_flag);
+      if (!ok || walk.it.x < 0) break;  // (no more work)
+      const int n_tiles = walk.it.w;
+      const uint16_t* cols = sm->cols[walk.at];
       const int n_super = (n_tiles + 3) >> 2;
       if (n_super > 0) {
         const int qpar = qi & 1;
@@ -430,131 +506,133 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (lane == 0) {
           const uint32_t bar = smem_u32(&sm->q_full[qpar]);
           mbar_expect_tx(bar, kTileBytes);
-          tma_load_4d(smem_u32(sm->qz[1 + 2 * qpar]), &tm_q, bar, 0, it.mb * 64, it.h, it.b);
+          tma_load_4d(smem_u32(sm->q[qpar]), &tm_q, bar, 0, walk.it.z * 64, walk.it.y, walk.it.x);
         }
         ++qi;
       }
       const int u_go = sorted ? max(n_super - kGoBefore, 0) : 0;
       if (n_super == 0 && lane == 0) mbar_arrive(smem_u32(&sm->setup_go[par]));
       // One lane per tile issues its load: a single thread can start a tile load only every couple
-      // of hundred cycles, which four loads in a row would turn into the kernel's bound.
+      // of hundred cycles.
       for (int u = 0; u < n_super; ++u) {
         if (u == u_go && lane == 0) mbar_arrive(smem_u32(&sm->setup_go[par]));
-        const int g = gs + u, ks = g % kKStages;
         const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->k_empty[ks]), ((g / kKStages) & 1) ^ 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->k_empty[ks]), kph, abort_flag);
         if (!ok) break;
         const uint32_t bar = smem_u32(&sm->k_full[ks]);
         if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
         __syncwarp();
-        if (lane < nt)  // shared-memory order a, c, b, d
-          tma_load_4d(smem_u32(sm->k[ks][((lane & 1) << 1) | (lane >> 1)]), &tm_k, bar, 0,
-                      static_cast<int>(cols[4 * u + lane] & kColIndex) * 64, it.h, it.b);
+        if (lane < nt) {  // in shared memory a, c, b, d; only a, b: next to each other
+          const int at = nt > 2 ? ((lane & 1) << 1) | (lane >> 1) : lane;
+          tma_load_4d(smem_u32(sm->k[ks][at]), &tm_k, bar, 0,
+                      static_cast<int>(cols[4 * u + lane] & kColIndex) * 64, walk.it.y, walk.it.x);
+        }
+        if (++ks == kKStages) { ks = 0; kph ^= 1; }
       }
-      gs += n_super;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
     }
     if (!ok) fwd_give_up(sm, p.status, kFailProducer);
   } else if (warp == kVProducerWarp) {
     // =========================== V producer ===========================
-    // Loads the V tiles of the listed key blocks, one lane per tile, from the list the producer
-    // published; a warp of its own, so that waiting for a free V stage (P V complete) never holds
-    // back the K tiles of a later superstep.
+    // Loads the V tiles of the listed key blocks, one lane per tile; a warp of its own, so that
+    // waiting for a free V stage (P V complete) never holds back the K tiles of a later superstep.
     bool ok = true;
-    int gs = 0;
-    for (int i = 0; ok; ++i) {
-      const int par = i & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->list_full[par]), (i >> 1) & 1, abort_flag);
-      if (!ok) break;
-      const int w = *const_cast<volatile int*>(&sm->item[par]);
-      if (w < 0) break;  // no more work
-      const FwdItem it = fwd_item(w, p);
-      const int n_tiles = *const_cast<volatile int*>(&sm->ntiles[par]);
-      const int n_super = (n_tiles + 3) >> 2;
-      const uint16_t* cols = sm->cols[par];
-      for (int u = 0; u < n_super; ++u, ++gs) {
-        const int vs = gs % kVStages;
-        const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->v_empty[vs]), ((gs / kVStages) & 1) ^ 1, abort_flag);
+    int vs = 0, vph = 1;
+    FwdWalk walk;
+    for (; ok; walk.next()) {
+      ok = walk.wait(sm, abort_flag);
+      if (!ok || walk.it.x < 0) break;  // (no more work)
+      const int n_tiles = walk.it.w;
+      const int n_pairs = (n_tiles + 1) >> 1;
+      const uint16_t* cols = sm->cols[walk.at];
+      for (int u = 0; u < n_pairs; ++u) {
+        const int nt = min(2, n_tiles - 2 * u);
+        ok = mbar_wait_warp(smem_u32(&sm->v_empty[vs]), vph, abort_flag);
         if (!ok) break;
         const uint32_t bar = smem_u32(&sm->v_full[vs]);
         if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
         __syncwarp();
         if (lane < nt)
           tma_load_4d(smem_u32(sm->v[vs][lane]), &tm_v, bar, 0,
-                      static_cast<int>(cols[4 * u + lane] & kColIndex) * 64, it.h, it.b);
+                      static_cast<int>(cols[2 * u + lane] & kColIndex) * 64, walk.it.y, walk.it.x);
+        if (++vs == kVStages) { vs = 0; vph ^= 1; }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
     }
     if (!ok) fwd_give_up(sm, p.status, kFailProducer);
   } else if (warp == kSWarp) {
     // =========================== S issuer ===========================
-    constexpr uint32_t idesc_n128 = umma_idesc(kBf16, 0, 0, 128, 128);
-    constexpr uint32_t idesc_n64 = umma_idesc(kBf16, 0, 0, 128, 64);
+    constexpr uint32_t idesc_s4 = umma_idesc(kBf16, 0, 0, 64, 256);
+    constexpr uint32_t idesc_s2 = umma_idesc(kBf16, 0, 0, 64, 128);
     const bool leader = elect_one();
-    const uint64_t desc_qz = smem_desc_sw128(smem_u32(sm->qz[0]), 16, 1024);
+    const uint64_t desc_q0 = smem_desc_sw128(smem_u32(sm->q[0]), 16, 1024);
     const uint64_t desc_k0 = smem_desc_sw128(smem_u32(sm->k[0][0]), 16, 1024);
     constexpr uint64_t kTileDesc = kTileBytes >> 4;  // one tile further, in descriptor units
+    const int k_steps = p.D >> 4;
     bool ok = true;
-    int gs = 0, qi = 0;
-    for (int i = 0; ok; ++i) {
-      const int par = i & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->list_full[par]), (i >> 1) & 1, abort_flag);
-      if (!ok) break;
-      if (*const_cast<volatile int*>(&sm->item[par]) < 0) break;  // no more work
-      const int n_tiles = *const_cast<volatile int*>(&sm->ntiles[par]);
+    int ks = 0, kph = 0, qi = 0;
+    int slot = 0, slot_ph = 1, bar_s = 0;  // (bar_s: superstep number mod 2 kSlots)
+    FwdWalk walk;
+    for (; ok; walk.next()) {
+      ok = walk.wait(sm, abort_flag);
+      if (!ok || walk.it.x < 0) break;  // (no more work)
+      const int n_tiles = walk.it.w;
       const int n_super = (n_tiles + 3) >> 2;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
       if (n_super == 0) continue;
       const int qpar = qi & 1;
       ok = mbar_wait_warp(smem_u32(&sm->q_full[qpar]), (qi >> 1) & 1, abort_flag);
       if (!ok) break;
-      // [Z; Q] starts at the zero block in front of the query buffer, [Q; Z] at the buffer itself
-      const uint64_t desc_bot = desc_qz + static_cast<uint64_t>(2 * qpar) * kTileDesc;
-      const uint64_t desc_top = desc_bot + kTileDesc;
-      for (int u = 0; u < n_super; ++u, ++gs) {
-        const int ks = gs % kKStages, slot = gs % kSlots;
-        const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->k_full[ks]), (gs / kKStages) & 1, abort_flag);
+      const uint64_t desc_q = desc_q0 + static_cast<uint64_t>(qpar) * kTileDesc;
+      for (int u = 0; u < n_super; ++u) {
+        ok = mbar_wait_warp(smem_u32(&sm->k_full[ks]), kph, abort_flag);
         if (!ok) break;
-        // the slot's previous user, three supersteps ago, must have had its P V completed
-        if (gs >= kSlots)
-          ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), ((gs - kSlots) / kSlots) & 1,
-                              abort_flag);
+        // the slot's previous user, three supersteps ago, must have had its P V completed (for the
+        // first users this asks for the phase before the first one, which counts as complete)
+        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), slot_ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (leader) {
+          // an odd number of tiles multiplies with whatever the rest of the stage holds: those
+          // logits are nobody's
           const uint32_t d = tmem + 128 * slot;
-          const uint64_t desc_ac = desc_k0 + static_cast<uint64_t>(ks * 4) * kTileDesc;
-          const uint64_t desc_bd = desc_ac + 2 * kTileDesc;
-          const uint32_t id_ac = nt >= 3 ? idesc_n128 : idesc_n64;
-          const uint32_t id_bd = nt >= 4 ? idesc_n128 : idesc_n64;
+          const uint64_t desc_k = desc_k0 + static_cast<uint64_t>(ks * 4) * kTileDesc;
+          const uint32_t idesc = n_tiles - 4 * u > 2 ? idesc_s4 : idesc_s2;
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk) umma_ss(d, desc_top + 2 * kk, desc_ac + 2 * kk, id_ac, kk > 0);
-          if (nt >= 2) {
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) umma_ss(d, desc_bot + 2 * kk, desc_bd + 2 * kk, id_bd, 1);
-          }
-          tc_commit(smem_u32(&sm->s_full[slot]));
+          for (int kk = 0; kk < 4; ++kk)
+            if (kk < k_steps) umma_ws_ss(d, desc_q + 2 * kk, desc_k + 2 * kk, idesc, kk > 0);
+          tc_commit(smem_u32(&sm->s_full[bar_s]));
           tc_commit(smem_u32(&sm->k_empty[ks]));
           if (u == n_super - 1) tc_commit(smem_u32(&sm->q_free[qpar]));  // Q buffer reusable
         }
+        if (++ks == kKStages) { ks = 0; kph ^= 1; }
+        if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
+        if (++bar_s == 2 * kSlots) bar_s = 0;
       }
       ++qi;
     }
     if (!ok) fwd_give_up(sm, p.status, kFailMma);
   } else if (warp == kPvWarp) {
     // =========================== P V issuer ===========================
-    constexpr uint32_t idesc_pv = umma_idesc(kBf16, 0, 1, 128, 64);  // P (TMEM) x V (MN-major)
+    const uint32_t idesc_pv = umma_idesc(kBf16, 0, 1, 128, p.D);  // P (TMEM) x V (MN-major)
     const bool leader = elect_one();
     const uint64_t desc_v0 = smem_desc_sw128(smem_u32(sm->v[0][0]), 8192, 1024);
     bool ok = true;
-    int gs = 0;
-    for (int i = 0; ok; ++i) {
+    int vs = 0, vph = 0;
+    int slot = 0, slot_ph = 0, team = 0;
+    FwdWalk walk;
+    for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->list_full[par]), (i >> 1) & 1, abort_flag);
-      if (!ok) break;
-      if (*const_cast<volatile int*>(&sm->item[par]) < 0) break;  // no more work
-      const int n_tiles = *const_cast<volatile int*>(&sm->ntiles[par]);
+      ok = walk.wait(sm, abort_flag);
+      if (!ok || walk.it.x < 0) break;  // (no more work)
+      const int n_tiles = walk.it.w;
       const int n_super = (n_tiles + 3) >> 2;
-      // the accumulators are free once the previous item has been written out; the softmax warps
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
+      // the accumulators are free once the previous item has been read out; the softmax warps
       // meanwhile work ahead
       if (i >= 1)
         ok = mbar_wait_warp(smem_u32(&sm->o_free[par ^ 1]), ((i - 1) >> 1) & 1, abort_flag);
@@ -563,173 +641,165 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (leader) mbar_arrive(smem_u32(&sm->o_full[par]));
         continue;
       }
-      for (int u = 0; u < n_super; ++u, ++gs) {
-        const int vs = gs % kVStages, slot = gs % kSlots;
+      for (int u = 0; u < n_super && ok; ++u, team ^= 1) {
         const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->v_full[vs]), (gs / kVStages) & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph, abort_flag);
         if (!ok) break;
-        // Tiles a, b go to the accumulator of team 0 as soon as that team has stored their P, tiles
-        // c, d to that of team 1; the first product of an item into an accumulator starts it
-        // afresh.  Keys [16 kk, +16) of tile t sit at column 32 t + 8 kk of the slot; the lanes
-        // that do not own the tile hold zeros there.
-        const uint32_t p_slot = tmem + 128 * slot;
-        for (int team = 0; team < 2 && ok; ++team) {
-          ok = mbar_wait_warp(smem_u32(&sm->p_full[slot][team]), (gs / kSlots) & 1, abort_flag);
+        tc_fence_after();
+        // Tiles a and b have their P in columns [0, 32) of the slot, a in lanes 0..63 and b in lanes
+        // 64..127; c and d in columns [32, 64).  Each product writes the lanes of its tile only.  A
+        // lane half's first product of an item starts its accumulator afresh.
+        const uint32_t o_acc = tmem + kTmemO + 64 * team;
+        for (int pair = 0; pair < 2; ++pair) {
+          if (2 * pair >= nt) break;
+          ok = mbar_wait_warp(smem_u32(&sm->v_full[vs]), vph, abort_flag);
           if (!ok) break;
           tc_fence_after();
           if (leader) {
-            const uint32_t o_acc = tmem + kTmemO + 64 * team;
-            for (int t = 2 * team; t < min(nt, 2 * team + 2); ++t) {
-              const uint64_t desc_v = desc_v0 + static_cast<uint64_t>((vs * 4 + t) * (kTileBytes >> 4));
+            const uint32_t p_cols = tmem + 128 * slot + 32 * pair;
+            const uint64_t desc_v = desc_v0 + static_cast<uint64_t>(vs * 2) * (kTileBytes >> 4);
+            const uint32_t started = u > 1 || pair > 0;
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_ts_half(o_acc, p_cols + 8 * kk, desc_v + 128 * kk, idesc_pv, started | (kk > 0), 0);
+            if (nt > 2 * pair + 1) {
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
-                umma_ts(o_acc, p_slot + 32 * t + 8 * kk, desc_v + 128 * kk, idesc_pv,
-                        (u > 0) || (t & 1) || (kk > 0));
+                umma_ts_half(o_acc, p_cols + 8 * kk, desc_v + (kTileBytes >> 4) + 128 * kk, idesc_pv,
+                             started | (kk > 0), 1);
             }
+            tc_commit(smem_u32(&sm->v_empty[vs]));
           }
+          if (++vs == kVStages) { vs = 0; vph ^= 1; }
         }
         if (!ok) break;
         if (leader) {
-          tc_commit(smem_u32(&sm->v_empty[vs]));
           tc_commit(smem_u32(&sm->pv_done[slot]));
           if (u == n_super - 1) tc_commit(smem_u32(&sm->o_full[par]));
         }
+        if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
       }
     }
     if (!ok) fwd_give_up(sm, p.status, kFailMma);
+  }
   } else if (warp < kSoftmaxWarps) {
     // =========================== softmax ===========================
-    const int team = warp >> 2;       // team 0 takes tiles a, b of every superstep, team 1 tiles c, d
+    take_registers<160>();
+    const int team = warp >> 2;
     const int quarter = warp & 3;     // TMEM lane quarter this warp may touch
     const int half = quarter >> 1;    // lanes 0..63 own tiles a, c of a superstep, 64..127 b, d
-    const int t_mine = 2 * team + half, t_other = 2 * team + (half ^ 1);
     const int lane_row = quarter * 32 + lane;  // TMEM lane
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t o_addr = tmem + lane_base + kTmemO + 64 * team;
-    // columns of a slot: the team's logits at [64 team, +64); this warp's P over the first or the
-    // second half of them, zeros over the other half (where the other lanes' P goes)
-    const uint32_t col_s = 64u * team;
-    const uint32_t col_p = col_s + 32u * half, col_z = col_s + 32u * (half ^ 1);
     const float c = p.scale_log2;
     bool ok = true;
-    int g0 = 0;  // supersteps of all earlier items of this CTA
-    for (int i = 0; ok; ++i) {
+    int g = 0;        // supersteps of earlier items; this team takes those with g % 2 == team
+    int next = team;  // its next one, with the slot next % kSlots and the barrier next % (2 kSlots)
+    int slot = team, bar_s = team, bar_ph = 0;
+    FwdWalk walk;
+    for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->list_full[par]), (i >> 1) & 1, abort_flag);
-      if (!ok) break;
-      const int w_item = *const_cast<volatile int*>(&sm->item[par]);
-      if (w_item < 0) break;  // no more work
-      const int n_tiles = *const_cast<volatile int*>(&sm->ntiles[par]);
+      ok = walk.wait(sm, abort_flag);
+      if (!ok || walk.it.x < 0) break;  // (no more work)
+      const int n_tiles = walk.it.w;
       const int n_super = (n_tiles + 3) >> 2;
-      const uint16_t* cols = sm->cols[par];
+      const uint16_t* cols = sm->cols[walk.at];
       float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
-      bool next_ready = false;  // the S barrier of the coming superstep has been seen complete
       // this lane's row of the element-level mask, if there is one
       const uint8_t* mask_row = nullptr;
-      if constexpr (kElementMask) {
-        const FwdItem it = fwd_item(w_item, p);
-        mask_row = p.dense + it.b * p.ds0 + it.h * p.ds1 +
-                   static_cast<int64_t>(it.mb * 64 + (quarter & 1) * 32 + lane) * p.ds2;
-      }
+      if constexpr (kElementMask)
+        mask_row = p.dense + walk.it.x * p.ds0 + walk.it.y * p.ds1 +
+                   static_cast<int64_t>(walk.it.z * 64 + (quarter & 1) * 32 + lane) * p.ds2;
 
-      for (int u = 0; u < n_super; ++u) {
-        const int g = g0 + u;
-        const int slot = g % kSlots;
+      for (; next < g + n_super; next += 2) {
+        const int u = next - g;
         const uint32_t s_addr = tmem + lane_base + 128 * slot;
-        const int nt = min(4, n_tiles - 4 * u);
-        // A tile with masked elements inside: fetch this row's 64 mask bytes while S is on its way
-        uint16_t entry = 0;
-        if constexpr (kElementMask) entry = t_mine < nt ? cols[4 * u + t_mine] : 0;
-        const bool partial = kElementMask && (entry & kColPartial) != 0;  // warp-uniform
-        uint4 mw[4];
-        if (partial) {
-          const uint4* mp = reinterpret_cast<const uint4*>(mask_row + (entry & kColIndex) * 64);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) mw[j] = __ldg(mp + j);
-        }
-        if (!next_ready) {
-          ok = mbar_wait_warp(smem_u32(&sm->s_full[slot]), (g / kSlots) & 1, abort_flag);
-          if (!ok) break;
-        }
+        const int mine = n_tiles - 4 * u - half;  // > 0: this lane's first tile exists, > 2: both
+        ok = mbar_wait_warp(smem_u32(&sm->s_full[bar_s]), bar_ph, abort_flag);
+        if (!ok) break;
         tc_fence_after();
-        if (t_mine < nt) {
-          uint32_t sr[64];
-          tmem_ld_32x32b_x32(s_addr + col_s, sr);
-          tmem_ld_32x32b_x32(s_addr + col_s + 32, sr + 32);
-          tc_wait_ld();
-          // the other lanes' tile of this team reads these lanes too: zeros (the logits are in
-          // registers now); stored first, so that it drains under the arithmetic
-          if (t_other < nt) tmem_st_zero_32x32b_x32(s_addr + col_z);
-          if (partial) {
-            // masked elements become -inf: they take no part in the maximum and exponentiate to 0
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t w4[4] = {mw[j].x, mw[j].y, mw[j].z, mw[j].w};
-#pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4) {
-                const uint32_t nz = __vcmpne4(w4[q4], 0u);  // 0xff in every byte that keeps its element
-#pragma unroll
-                for (int bb = 0; bb < 4; ++bb) {
-                  const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
-                  const int i = 16 * j + 4 * q4 + bb;
-                  sr[i] = (sr[i] & keep) | (0xff800000u & ~keep);
-                }
+        // The row maximum is looked up only where it is needed: for the item's first superstep of
+        // the team (and when the caller wants it, or with element masks, under which a row may have
+        // nothing yet).  Otherwise the logits are exponentiated against the reference maximum as it
+        // is; a row whose sum shows that this was too low (or not finite) makes the warp do the
+        // superstep again with the maximum.  S is still in tensor memory then: P goes over it last.
+        bool with_max = kElementMask || u < 2 || p.rowmax != nullptr;
+        if (mine > 0) {
+          const bool two = mine > 2;  // both tiles exist (warp-uniform)
+          const auto masked = [&](uint32_t* sr, int col) {
+            if constexpr (kElementMask) {
+              const uint16_t entry = cols[4 * u + (col >> 6) * 2 + half];
+              if (entry & kColPartial)
+                mask_chunk(sr, mask_row + (entry & kColIndex) * 64 + (col & 32));
+            }
+          };
+          uint32_t pk[64];
+          float sum;
+          while (true) {
+            uint32_t sa[32], sb[32];
+            if (with_max) {
+              float zmax = -INFINITY;
+#pragma unroll 1
+              for (int col = 0; col < (two ? 128 : 64); col += 32) {
+                tmem_ld_32x32b_x32(s_addr + col, sa);
+                tc_wait_ld();
+                masked(sa, col);
+                zmax = fmaxf(zmax, max_chunk(sa));
+              }
+              const float alpha = fwd_new_max(zmax * c, m_ref, m_true, l);
+              if (__any_sync(0xffffffffu, alpha != 1.f)) {
+                // the previous product of this team, two supersteps ago, must be in O
+                const int prev = slot == 2 ? 0 : slot + 1;  // (slot - 2) % 3
+                ok = mbar_wait_warp(smem_u32(&sm->pv_done[prev]),
+                                    static_cast<uint32_t>((next - 2) / kSlots) & 1u, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                fwd_rescale(o_addr, alpha);
               }
             }
-          }
-          const float zmax = fmaxf(max_chunk(sr), max_chunk(sr + 32)) * c;
-          m_true = fmaxf(m_true, zmax);
-          float alpha = 1.f;
-          bool rescale = false;
-          if (m_ref == -INFINITY) {
-            m_ref = zmax;  // first tile of this lane in this item: O and l are still zero
-          } else if (zmax > m_ref + kRescaleThreshold) {
-            alpha = ex2_approx(m_ref - zmax);
-            l *= alpha;
-            m_ref = zmax;
-            rescale = true;
-          }
-          if (__any_sync(0xffffffffu, rescale)) {
-            // this warp's O rows must hold the team's previous product (the superstep before) first
-            ok = mbar_wait_warp(smem_u32(&sm->pv_done[(g - 1) % kSlots]), ((g - 1) / kSlots) & 1,
-                                abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-#pragma unroll 1
-            for (int part = 0; part < 4; ++part) {
-              uint32_t orow[16];
-              tmem_ld_32x32b_x16(o_addr + 16 * part, orow);
+            const float neg_m = (kElementMask && m_ref == -INFINITY) ? 0.f : -m_ref;
+            uint64_t l0 = pack_f32x2(0.f, 0.f), l1 = l0;
+            tmem_ld_32x32b_x32(s_addr, sa);
+            tmem_ld_32x32b_x32(s_addr + 32, sb);
+            tc_wait_ld();
+            masked(sa, 0);
+            masked(sb, 32);
+            exp_chunk<kBf16>(sa, c, neg_m, pk, l0, l1);
+            if (two) {
+              tmem_ld_32x32b_x32(s_addr + 64, sa);
+              exp_chunk<kBf16>(sb, c, neg_m, pk + 16, l0, l1);
+              tmem_ld_32x32b_x32(s_addr + 96, sb);
               tc_wait_ld();
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                orow[j] = __float_as_uint(__uint_as_float(orow[j]) * alpha);
-              tmem_st_32x32b_x16(o_addr + 16 * part, orow);
+              masked(sa, 64);
+              masked(sb, 96);
+              exp_chunk<kBf16>(sa, c, neg_m, pk + 32, l0, l1);
+              exp_chunk<kBf16>(sb, c, neg_m, pk + 48, l0, l1);
+            } else {
+              exp_chunk<kBf16>(sb, c, neg_m, pk + 16, l0, l1);
             }
+            float a0, a1;
+            unpack_f32x2(add_f32x2(l0, l1), a0, a1);
+            sum = a0 + a1;
+            if (with_max || !__any_sync(0xffffffffu, !(sum <= kMaxRowSum))) break;
+            with_max = true;
           }
-          // (a row with nothing kept so far has m_ref = -inf: its logits are all -inf, and with a
-          // zero in place of the maximum they exponentiate to 0 instead of NaN)
-          const float neg_m = (kElementMask && m_ref == -INFINITY) ? 0.f : -m_ref;
-          uint32_t pk[16];
-          exp_chunk<kBf16>(sr, c, neg_m, pk, l);
-          tmem_st_32x32b_x16(s_addr + col_p, pk);
-          exp_chunk<kBf16>(sr + 32, c, neg_m, pk, l);
-          tmem_st_32x32b_x16(s_addr + col_p + 16, pk);
-        } else if (t_other < nt) {
-          tmem_st_zero_32x32b_x32(s_addr + col_z);
+          if (!ok) break;
+          l += sum;
+          // this lane's first tile in columns [0, 32) of the slot, its second one in [32, 64)
+          tmem_st_32x32b_x32(s_addr, pk);
+          if (two) tmem_st_32x32b_x32(s_addr + 32, pk + 32);
         }
-        // Look at the next superstep's S barrier now: the round trip to it runs under the drain of
-        // the stores, and if S is there (it normally is: three slots) the wait at the top of the
-        // loop is skipped.
-        bool polled = false;
-        if (u + 1 < n_super)
-          polled = mbar_test(smem_u32(&sm->s_full[(g + 1) % kSlots]), ((g + 1) / kSlots) & 1);
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->p_full[slot][team]));
-        next_ready = __all_sync(0xffffffffu, polled);
+        if (lane == 0) mbar_arrive(smem_u32(&sm->p_full[slot]));
+        slot = slot >= 1 ? slot - 1 : kSlots - 1;  // (slot + 2) % 3
+        bar_s += 2;
+        if (bar_s >= 2 * kSlots) { bar_s -= 2 * kSlots; bar_ph ^= 1; }
       }
       if (!ok) break;
+      const int first_team = g & 1;
+      g += n_super;
 
       // publish this item's (m, l) of the warp's lanes; the slots of item i-2 must have been read
       if (i >= 2) ok = mbar_wait_warp(smem_u32(&sm->o_free[par]), ((i - 2) >> 1) & 1, abort_flag);
@@ -737,37 +807,49 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       sm->mref[par][team][lane_row] = m_ref;
       sm->lsum[par][team][lane_row] = l;
       sm->mtrue[par][team][lane_row] = m_true;
+      if (warp == 0 && lane == 0) sm->first_team[par] = first_team;
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->stats_full[par]));
-      g0 += n_super;
     }
     if (!ok) fwd_give_up(sm, p.status, kFailSoftmax);
   } else {
     // =========================== write-out ===========================
-    // Merges the four partial results of every query row (teams 0 / 1 x lanes r / r+64).
-    // A warp reads both accumulators of its own lanes from TMEM; lanes 64..127 hand their weighted
-    // rows to lanes 0..63 through shared memory, 32 columns at a time.  All named barriers of an
-    // iteration are always executed, also after a give-up, and the last one carries the give-up
-    // vote, so that no warp of this role can be left waiting at one.
+    // Merges the four partial results of every query row (first / second team of the item x lanes
+    // r / r+64).  A warp reads both accumulators of its own lanes from TMEM; lanes 64..127 hand
+    // their weighted rows to each other through shared memory, 16 columns at a time.  All named
+    // barriers of an iteration are always executed, also after a give-up, and the last one carries
+    // the give-up vote, so that no warp of this role can be left waiting at one.
     //
     // One of the four warps is also the lister: it sets up item i+1 when the producer says so
     // during item i, i.e. between its write-outs of items i-1 and i (the producer lists the
-    // CTA's first item itself, which nothing can overlap).  The draw
-    // from the work counter, the mask row and the ballots take a couple of thousand cycles, which
-    // in the producer's own instruction stream held back the K tiles of the current item.
+    // CTA's first item itself, which nothing can overlap).  The draw from the work counter, the mask
+    // row and the ballots take a couple of thousand cycles, which in the producer's own instruction
+    // stream held back the K tiles of the current item.
+    give_registers<112>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
     const bool lister = warp == kListerWarp;
     bool ok = true;
     bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
     int lw = blockIdx.x;
-    // Lister (one of the four warps): draws item j >= 1, lists its key blocks into the list buffer
-    // of j's parity and publishes them, or publishes that there is no further item.  A wait that
-    // gives up leaves ok = false and nothing published.
-    auto set_up = [&](int j) {
-      const int par = j & 1;
-      {
-        // next item: the following ticket when items are handed out dynamically, else a fixed stride
-        if (p.ticket != nullptr) {
+    if (sorted) fwd_build_order(sm, p, quarter * 32 + lane, stride, n2);
+    const int half = quarter >> 1;
+    const int lane_row = quarter * 32 + lane;
+    const int r_blk = (quarter & 1) * 32 + lane;  // row of the query block
+    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    FwdWalk walk;
+    for (int i = 0;; ++i, walk.next()) {
+      const int par = i & 1;
+      if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag, 256);
+      walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
+      if (walk.it.x < 0) break;  // no more work: the same for all four warps
+      const int n_tiles = walk.it.w;
+      if (lister && ok) {
+        // Sets up the next item, or publishes that there is none; a wait that gives up leaves ok =
+        // false and nothing published.  The next ticket when items are handed out dynamically, else
+        // a fixed stride.
+        ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1, abort_flag);
+        const int at = walk.at + 1 < kLists ? walk.at + 1 : 0;
+        if (ok && p.ticket != nullptr) {
           int t = 0;
           if (lane == 0) {
             t = atomicAdd(p.ticket, 1);
@@ -778,54 +860,34 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           t = __shfl_sync(0xffffffffu, t, 0);
           terminal = t >= n2;
           if (sorted && t < n2) {
-            if (j == 1) ok = mbar_wait_warp(smem_u32(&sm->order_full), 0, abort_flag);
-            if (!ok) return;
+            if (i == 0) ok = mbar_wait_warp(smem_u32(&sm->order_full), 0, abort_flag);
             t = *const_cast<volatile int*>(&sm->order[t]);
           }
           lw = stride + t;
         } else {
           lw += stride;
         }
-      }
-      // the list buffer (and the tile count) of item j-2 must have been read by everyone
-      if (j >= 2)
-        ok = mbar_wait_warp_idle(smem_u32(&sm->o_free[par]), ((j - 2) >> 1) & 1, abort_flag, 128);
-      if (!ok) return;
-      if (lw >= p.items) {
-        if (lane == 0) {
-          sm->item[par] = -1;
-          mbar_arrive(smem_u32(&sm->list_full[par]));
+        // The list buffer was that of item i-2, which these warps have written out (and the softmax
+        // warps with them are through with); the producers and issuers may lag behind.
+        if (ok && i >= 2)
+          ok = mbar_wait_warp_idle(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag, 128);
+        if (ok) {
+          if (lw < p.items) {
+            fwd_list_item<kElementMask>(sm, p, lw, at, lane);
+          } else if (lane == 0) {
+            sm->item[at].x = -1;
+            mbar_arrive(smem_u32(&sm->list_full[at]));
+          }
         }
-        return;
       }
-      fwd_list_item<kElementMask>(sm, p, lw, par, lane);
-    };
-
-    if (sorted) fwd_build_order(sm, p, quarter * 32 + lane, stride, n2);
-    const int half = quarter >> 1;
-    const int lane_row = quarter * 32 + lane;
-    const int r_blk = (quarter & 1) * 32 + lane;  // row of the query block
-    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    bool ahead = false;  // lister: item i+1 was set up during the write-out of item i-1 already
-    for (int i = 0;; ++i) {
-      const int par = i & 1;
-      if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[par]), (i >> 1) & 1, abort_flag, 256);
-      const int w = ok ? *const_cast<volatile int*>(&sm->item[par]) : 0;
-      if (w < 0) break;  // no more work: the same for all four warps
-      const FwdItem it = fwd_item(w, p);
-      const int n_tiles = ok ? *const_cast<volatile int*>(&sm->ntiles[par]) : 0;
-      if (lister && ok && !ahead) {
-        ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1, abort_flag);
-        if (ok) set_up(i + 1);
-      }
-      ahead = false;
       if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->stats_full[par]), (i >> 1) & 1, abort_flag, 128);
       // The weights of the four partial results need the statistics only, which the softmax warps
-      // publish before the item's last P V is complete: work them out before waiting for that, so
-      // that the accumulators are given back (o_free) as soon as they have been read.
-      float acc[64];
+      // publish before the item's last P V is complete.
+      int t0 = 0;  // the team with the item's first superstep
+      uint64_t acc[32];  // 64 columns in pairs
       float m_all = -INFINITY, l_all = 0.f, mt = -INFINITY, w0 = 0.f, w1 = 0.f;
       if (ok) {
+        t0 = *const_cast<volatile int*>(&sm->first_team[par]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           m_all = fmaxf(m_all, sm->mref[par][j & 1][r_blk + 64 * (j >> 1)]);
@@ -833,89 +895,99 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float mi = sm->mref[par][j & 1][r_blk + 64 * (j >> 1)];
+          const int tj = (j & 1) ^ t0, lj = r_blk + 64 * (j >> 1);
+          const float mi = sm->mref[par][tj][lj];
           if (mi != -INFINITY)
-            l_all += ex2_approx(mi - m_all) * sm->lsum[par][j & 1][r_blk + 64 * (j >> 1)];
+            l_all += ex2_approx(mi - m_all) * sm->lsum[par][tj][lj];
         }
         const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
-        const float m0 = sm->mref[par][0][lane_row], m1 = sm->mref[par][1][lane_row];
+        const float m0 = sm->mref[par][t0][lane_row], m1 = sm->mref[par][t0 ^ 1][lane_row];
         w0 = m0 == -INFINITY ? 0.f : ex2_approx(m0 - m_all) * inv;
         w1 = m1 == -INFINITY ? 0.f : ex2_approx(m1 - m_all) * inv;
       }
       if (ok) ok = mbar_wait_warp(smem_u32(&sm->o_full[par]), (i >> 1) & 1, abort_flag);
       if (ok) {
         if (n_tiles > 0) {  // warp-uniform
-          // team 1's accumulator holds this item's sums only if the item has a tile c
-          const bool live1 = n_tiles > 2;
+          // An accumulator holds sums of this item only if the item has a tile for these lanes of it
+          // (warp-uniform).
+          const bool live0 = n_tiles > half, live1 = n_tiles > 4 + half;
+          const uint64_t w0w0 = pack_f32x2(w0, w0), w1w1 = pack_f32x2(w1, w1);
           tc_fence_after();
 #pragma unroll
-          for (int part = 0; part < 4; ++part) {
+          for (int q = 0; q < 4; ++q) {
             uint32_t a0[16], a1[16];
-            tmem_ld_32x32b_x16(tmem + lane_base + kTmemO + 16 * part, a0);
-            tmem_ld_32x32b_x16(tmem + lane_base + kTmemO + 64 + 16 * part, a1);
+            const uint32_t o_cols = tmem + lane_base + kTmemO + 16 * q;
+            tmem_ld_32x32b_x16(o_cols + 64 * t0, a0);
+            tmem_ld_32x32b_x16(o_cols + 64 * (t0 ^ 1), a1);
             tc_wait_ld();
+            if (live1) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const float x0 = __uint_as_float(a0[j]) * w0;
-              acc[16 * part + j] = live1 ? fmaf(__uint_as_float(a1[j]), w1, x0) : x0;
+              for (int j = 0; j < 8; ++j)
+                acc[8 * q + j] = fma_f32x2(
+                    pack_f32x2(__uint_as_float(a1[2 * j]), __uint_as_float(a1[2 * j + 1])), w1w1,
+                    mul_f32x2(pack_f32x2(__uint_as_float(a0[2 * j]), __uint_as_float(a0[2 * j + 1])), w0w0));
+            } else {
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                acc[8 * q + j] =
+                    live0 ? mul_f32x2(pack_f32x2(__uint_as_float(a0[2 * j]), __uint_as_float(a0[2 * j + 1])), w0w0)
+                          : 0ull;
             }
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < 64; ++j) acc[j] = 0.f;
+          for (int j = 0; j < 32; ++j) acc[j] = 0ull;
         }
         // Accumulators, statistics and the item's header are in registers now: the next item may
         // use them, while this one is still being merged and stored.
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm->o_free[par]));
-        // Lister: this item's list buffer is free now.  When the next item is already under way
-        // and has asked for its successor (many items per CTA: it asks at once), set that one up
-        // before merging and storing this item's rows: the write-out of an item ends late in the
-        // next one, and a set-up that waited for it would itself be late for the one after.
-        if (lister) {
-          const int j = i + 1;
-          if (__all_sync(0xffffffffu, mbar_test(smem_u32(&sm->setup_go[j & 1]), (j >> 1) & 1))) {
-            set_up(j + 1);
-            ahead = true;
-          }
-        }
       }
-      const int row = it.mb * 64 + r_blk;
-      uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.o) + it.b * p.o_sb +
-                                            it.h * p.o_sh + static_cast<int64_t>(row) * p.o_sn);
+      // Lanes 0..63 finish columns [0, 32) of their rows, lanes 64..127 columns [32, 64) of the same
+      // rows; each hands the other its sums of the other columns.
+      const int row = walk.it.z * 64 + r_blk;
+      uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.o) + walk.it.x * p.o_sb +
+                                            walk.it.y * p.o_sh + static_cast<int64_t>(row) * p.o_sn);
       bool any_failed = false;
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
-        if (ok && half == 1) {
+        if (ok) {
+          ulonglong2* out = reinterpret_cast<ulonglong2*>(sm->xfer[half][r_blk]);
 #pragma unroll
-          for (int j = 0; j < 32; ++j) sm->xfer[j][r_blk] = acc[32 * part + j];
+          for (int j = 0; j < 4; ++j)
+            out[j] = half ? make_ulonglong2(acc[8 * part + 2 * j], acc[8 * part + 2 * j + 1])
+                          : make_ulonglong2(acc[16 + 8 * part + 2 * j], acc[16 + 8 * part + 2 * j + 1]);
         }
         named_barrier_sync(2, 128);
-        if (ok && half == 0) {
+        const int col = 32 * half + 16 * part;
+        if (ok && col < p.D) {
+          const ulonglong2* in = reinterpret_cast<const ulonglong2*>(sm->xfer[half ^ 1][r_blk]);
+          uint32_t pkd[8];
 #pragma unroll
-          for (int v8 = 0; v8 < 2; ++v8) {
-            uint32_t pkd[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const int col = 16 * v8 + 2 * j;
-              pkd[j] = pack_2x16<kBf16>(acc[32 * part + col] + sm->xfer[col][r_blk],
-                                        acc[32 * part + col + 1] + sm->xfer[col + 1][r_blk]);
-            }
-            // whole 32-byte sectors when the rows start on such boundaries
-            if (p.wide_stores) {
-              st_global_v8(dst + 4 * part + 2 * v8, pkd);
-            } else {
-              dst[4 * part + 2 * v8] = make_uint4(pkd[0], pkd[1], pkd[2], pkd[3]);
-              dst[4 * part + 2 * v8 + 1] = make_uint4(pkd[4], pkd[5], pkd[6], pkd[7]);
-            }
+          for (int j = 0; j < 4; ++j) {
+            const ulonglong2 x = in[j];
+            float f0, f1, f2, f3;
+            unpack_f32x2(add_f32x2(half ? acc[16 + 8 * part + 2 * j] : acc[8 * part + 2 * j], x.x), f0, f1);
+            unpack_f32x2(
+                add_f32x2(half ? acc[16 + 8 * part + 2 * j + 1] : acc[8 * part + 2 * j + 1], x.y), f2, f3);
+            pkd[2 * j] = pack_2x16<kBf16>(f0, f1);
+            pkd[2 * j + 1] = pack_2x16<kBf16>(f2, f3);
+          }
+          // whole 32-byte sectors when the rows start on such boundaries
+          if (p.wide_stores) {
+            st_global_v8(dst + (col >> 3), pkd);
+          } else {
+            dst[col >> 3] = make_uint4(pkd[0], pkd[1], pkd[2], pkd[3]);
+            dst[(col >> 3) + 1] = make_uint4(pkd[4], pkd[5], pkd[6], pkd[7]);
           }
         }
         // xfer may be overwritten now; all four warps leave together if any gave up
         any_failed = named_barrier_or(2, 128, !ok);
+        if (any_failed) break;
       }
       if (ok && half == 0) {
-        const int64_t ri = (static_cast<int64_t>(it.b) * p.H + it.h) * p.N + row;
+        const int64_t ri = (static_cast<int64_t>(walk.it.x) * p.H + walk.it.y) * p.N + row;
         p.lse2[ri] = l_all > 0.f ? m_all + lg2_approx(l_all) : -INFINITY;
         if (p.rowmax) p.rowmax[ri] = mt;
       }
@@ -949,7 +1021,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 struct TmapKey {
   const void* base;
   int64_t s[4];
-  int B, H, N, dtype;
+  int B, H, N, D, dtype;
 };
 struct TmapEntry {
   TmapKey key;
@@ -958,7 +1030,7 @@ struct TmapEntry {
 };
 
 static int cached_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B, int H,
-                           int N, int dtype) {
+                           int N, int D, int dtype) {
   constexpr int kEntries = 12;
   static thread_local TmapEntry cache[kEntries];
   static thread_local int next = 0;
@@ -969,13 +1041,14 @@ static int cached_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4
   key.B = B;
   key.H = H;
   key.N = N;
+  key.D = D;
   key.dtype = dtype;
   for (int i = 0; i < kEntries; ++i)
     if (cache[i].valid && memcmp(&cache[i].key, &key, sizeof(key)) == 0) {
       *out = cache[i].map;
       return BSA_OK;
     }
-  const int rc = make_qkv_tmap(out, base, s, B, H, N, dtype, 64);
+  const int rc = make_qkv_tmap(out, base, s, B, H, N, D, dtype, 64);
   if (rc != BSA_OK) return rc;
   TmapEntry& e = cache[next];
   next = (next + 1) % kEntries;
@@ -993,7 +1066,8 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
                       float sm_scale, int dtype, int B, int H, int N, int D, int row_begin,
                       int row_end, const uint8_t* dense, const int64_t* dense_strides,
                       int32_t* status, int32_t* ticket, void* stream) {
-  if (B <= 0 || H <= 0 || N <= 0 || (N % kBlock) != 0 || D != kHeadDim) return BSA_ERR_BAD_SHAPE;
+  if (B <= 0 || H <= 0 || N <= 0 || (N % kBlock) != 0 || !head_dim_ok(D))
+    return BSA_ERR_BAD_SHAPE;
   if (!(sm_scale >= 0.f)) return BSA_ERR_BAD_SHAPE;  // the row maximum is taken before scaling
   if (dtype != BSA_F16 && dtype != BSA_BF16) return BSA_ERR_BAD_DTYPE;
   if (!lse2 || (block == nullptr && (!row_ptr || !col_idx))) return BSA_ERR_BAD_POINTER;
@@ -1021,9 +1095,9 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
   if (static_cast<int64_t>(B) * H * nrows > 0x7fffffffLL) return BSA_ERR_TOO_LARGE;
 
   CUtensorMap tm_q, tm_k, tm_v;
-  if ((rc = cached_qkv_tmap(&tm_q, q, q_strides, B, H, N, dtype)) != BSA_OK) return rc;
-  if ((rc = cached_qkv_tmap(&tm_k, k, k_strides, B, H, N, dtype)) != BSA_OK) return rc;
-  if ((rc = cached_qkv_tmap(&tm_v, v, v_strides, B, H, N, dtype)) != BSA_OK) return rc;
+  if ((rc = cached_qkv_tmap(&tm_q, q, q_strides, B, H, N, D, dtype)) != BSA_OK) return rc;
+  if ((rc = cached_qkv_tmap(&tm_k, k, k_strides, B, H, N, D, dtype)) != BSA_OK) return rc;
+  if ((rc = cached_qkv_tmap(&tm_v, v, v_strides, B, H, N, D, dtype)) != BSA_OK) return rc;
 
   FwdParams prm;
   prm.row_ptr = row_ptr;
@@ -1046,6 +1120,7 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
   prm.B = B;
   prm.H = H;
   prm.N = N;
+  prm.D = D;
   prm.nb = nb;
   prm.row_begin = row_begin;
   prm.nrows = nrows;

@@ -92,13 +92,13 @@ static encode_tiled_fn resolve_encode() {
 }
 
 int make_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B, int H, int N,
-                  int dtype, int box_rows) {
+                  int D, int dtype, int box_rows) {
   encode_tiled_fn enc = resolve_encode();
   if (!enc) return BSA_ERR_NO_DRIVER;
   const CUtensorMapDataType dt =
       dtype == BSA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   // innermost first: (d, n, h, b)
-  cuuint64_t dims[4] = {static_cast<cuuint64_t>(kHeadDim), static_cast<cuuint64_t>(N),
+  cuuint64_t dims[4] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(N),
                         static_cast<cuuint64_t>(H), static_cast<cuuint64_t>(B)};
   cuuint64_t strides[3] = {static_cast<cuuint64_t>(s[2]) * 2, static_cast<cuuint64_t>(s[1]) * 2,
                            static_cast<cuuint64_t>(s[0]) * 2};
@@ -117,7 +117,7 @@ extern "C" int bsa_version(void) { return BSA_VERSION; }
 extern "C" const char* bsa_strerror(int status) {
   switch (status) {
     case BSA_OK: return "ok";
-    case BSA_ERR_BAD_SHAPE: return "bad shape (N must be a positive multiple of 64, D must be 64)";
+    case BSA_ERR_BAD_SHAPE: return "bad shape (N must be a positive multiple of 64, D must be 16, 32 or 64)";
     case BSA_ERR_BAD_DTYPE: return "bad dtype (fp16 or bf16 only)";
     case BSA_ERR_BAD_STRIDE:
       return "bad stride (innermost stride must be 1, outer strides multiples of 16 bytes)";

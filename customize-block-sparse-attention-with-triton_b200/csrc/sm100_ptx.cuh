@@ -30,6 +30,17 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Register split between the warpgroups of a block: executed by all four warps of one.  The shares
+// must add up to no more than the registers the block was launched with.
+template <int kRegs>
+__device__ __forceinline__ void give_registers() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void take_registers() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+
 // Named barrier that also ORs a predicate over the participating threads.
 __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool pred) {
   uint32_t out;
@@ -124,20 +135,21 @@ __device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t pari
 #ifndef BSA_WAIT_LIMIT_NS
 #define BSA_WAIT_LIMIT_NS 2000000000ull
 #endif
+// (32 bits of the timer and one small loop on purpose: this code is inlined at every wait of every
+// role, and the instruction cache is what the roles of a persistent kernel share most tightly.)
+__device__ __forceinline__ uint32_t global_timer_lo_ns() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+  return t;
+}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
                                           volatile int* abort_flag) {
   if (mbar_try_wait(bar, parity)) return true;
-  uint64_t t0 = 0;
-  uint32_t spins = 0;
-  while (true) {
-    if (mbar_try_wait_parked(bar, parity, 2000u)) return true;
-    if ((++spins & 255u) == 0u) {
-      if (*abort_flag) return false;
-      uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > BSA_WAIT_LIMIT_NS) return false;
-    }
-  }
+  const uint32_t t0 = global_timer_lo_ns();
+#pragma unroll 1
+  while (!mbar_try_wait_parked(bar, parity, 2000u))
+    if (*abort_flag || global_timer_lo_ns() - t0 > static_cast<uint32_t>(BSA_WAIT_LIMIT_NS)) return false;
+  return true;
 }
 
 // Same wait made by a whole (converged) warp; the verdict is made warp-uniform so that the
@@ -154,18 +166,15 @@ __device__ __forceinline__ bool mbar_wait_warp_idle(uint32_t bar, uint32_t parit
                                                     volatile int* abort_flag, unsigned sleep_ns) {
   bool ok = true;
   if (!mbar_try_wait(bar, parity)) {
-    uint64_t t0 = 0;
-    uint32_t spins = 0;
-    while (true) {
+    const uint32_t t0 = global_timer_lo_ns();
+#pragma unroll 1
+    do {
       __nanosleep(sleep_ns);
-      if (mbar_try_wait(bar, parity)) break;
-      if ((++spins & 63u) == 0u) {
-        if (*abort_flag) { ok = false; break; }
-        const uint64_t now = global_timer_ns();
-        if (t0 == 0) t0 = now;
-        else if (now - t0 > BSA_WAIT_LIMIT_NS) { ok = false; break; }
+      if (*abort_flag || global_timer_lo_ns() - t0 > static_cast<uint32_t>(BSA_WAIT_LIMIT_NS)) {
+        ok = false;
+        break;
       }
-    }
+    } while (!mbar_try_wait(bar, parity));
   }
   return __all_sync(0xffffffffu, ok);
 }
@@ -251,6 +260,18 @@ __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same with M = 64 rows of A in the "weight stationary" form: columns [0, N/2) of the result
+// go to TMEM lanes 0..63, columns [N/2, N) to lanes 64..127 of the same N/2 TMEM columns, so all
+// lanes are used (the ordinary M = 64 form runs at half rate).
+__device__ __forceinline__ void umma_ws_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // D[tmem] (+)= A[tmem] * B[smem desc]
 __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
                                         uint32_t idesc, uint32_t accumulate) {
@@ -259,6 +280,19 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// D[tmem] (+)= A[tmem] * B[smem desc] for lanes 0..63 (half = 0) or 64..127 (half = 1) only: the other
+// lanes of D keep what they hold, whatever their rows of A are.  Same rate as the full form.
+__device__ __forceinline__ void umma_ts_half(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                             uint32_t idesc, uint32_t accumulate, int half) {
+  const uint32_t off_lo = half != 0 ? 0xffffffffu : 0u, off_hi = ~off_lo;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %6, %6}, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(off_lo), "r"(off_hi)
       : "memory");
 }
 
@@ -312,16 +346,6 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t* r) 
       : "r"(taddr)
       : "memory");
 }
-// Stores zeros to 32 columns of the warp's 32 lanes.
-__device__ __forceinline__ void tmem_st_zero_32x32b_x32(uint32_t taddr) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
-      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
-      ::"r"(taddr), "r"(0u)
-      : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -330,6 +354,18 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t* r) 
         "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+      "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
+      "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]),
+      "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+      "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
 __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t* r) {
