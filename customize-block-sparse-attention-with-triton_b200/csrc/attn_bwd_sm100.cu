@@ -1,20 +1,23 @@
 // Backward block-sparse attention for sm_100a: one kernel template, two instantiations.
 //
-//   dK/dV (kDKDV = true):  a CTA owns ONE key block (64 keys), keeps its K and V in shared memory,
-//       each loaded twice (rows 0..63 and 64..127 of the tcgen05 A operands), and walks the
-//       block's list of query blocks (the column lists of the mask) two at a time ("supersteps"):
-//         S^T = [K;K] [Q_a;Q_b]^T, dP^T = [V;V] [dO_a;dO_b]^T   (SS MMAs, M=128, N=128)
-//       so that TMEM lanes 0..63 hold query tile a (columns 0..63) and lanes 64..127 query tile b
-//       (columns 64..127): every SM sub-partition has exponentials to do whatever the mask is.
-//         P^T = exp2(S^T c - LSE2[q]), dS^T = P^T (dP^T - delta[q])     (one thread per key row)
-//         dV += P^T_a dO_a + P^T_b dO_b,  dK += dS^T_a Q_a + dS^T_b Q_b (TS MMAs: A from TMEM, B
-//       MN-major from shared memory).  The half of the lanes that does not own a tile holds zeros
-//       where that tile's P^T / dS^T live, so lane r sums the tile-a products of key r and lane
-//       r+64 its tile-b products; the two are added when the block is written out.
-//   dQ    (kDKDV = false): a CTA owns one query block, keeps Q and dO resident (twice) and walks the
-//       row list of key blocks two at a time:
-//         S = [Q;Q] [K_a;K_b]^T, dP = [dO;dO] [V_a;V_b]^T;  dS = exp2(S c - LSE2[row]) (dP - delta[row]);
+//   dK/dV (kDKDV = true):  a CTA owns ONE key block (64 keys), keeps its K and V in shared memory and
+//       walks the block's list of query blocks (the column lists of the mask) two at a time
+//       ("supersteps", tiles a and b):
+//         S^T = K [Q_a;Q_b]^T, dP^T = V [dO_a;dO_b]^T                     (SS MMAs, M=64, N=128)
+//         P^T = exp2(S^T c - LSE2[q]), dS^T = P^T (dP^T - delta[q])       (one thread per key row)
+//         dV += P^T_a dO_a + P^T_b dO_b,  dK += dS^T_a Q_a + dS^T_b Q_b   (TS MMAs: A from TMEM, B
+//       MN-major from shared memory).
+//   dQ    (kDKDV = false): a CTA owns one query block, keeps Q and dO resident and walks the row list
+//       of key blocks two at a time:
+//         S = Q [K_a;K_b]^T, dP = dO [V_a;V_b]^T;  dS = exp2(S c - LSE2[row]) (dP - delta[row]);
 //         dQ += dS_a K_a + dS_b K_b
+//
+// The M = 64 "weight stationary" form of the MMA puts the columns of tile a into TMEM lanes 0..63 and
+// those of tile b into lanes 64..127 of the same 64 columns, so every SM sub-partition has
+// exponentials to do whatever the mask is, and no operand is multiplied twice.  The accumulating
+// products write the accumulator rows of the lanes that own the tile and leave the others alone: lane
+// r sums the tile-a products of row r, lane r+64 its tile-b products; the two are added when the block
+// is written out.
 //
 // Formulas are those of the reference's backward (fa2_custom_mask/fa2_bwd.py:56-74, 116-130) with
 // M replaced by a true base-2 log-sum-exp; the iteration space is the tile lists, not the
@@ -22,13 +25,22 @@
 //
 // Persistent: one CTA per SM starts with block blockIdx.x and draws further blocks from an
 // optional work counter (or walks a fixed stride); long lists first when the mask is causal.
-// Roles: warps 0..15 compute (lane quarter = warp % 4, 16 of a tile's 64 columns = warp / 4: four
-// warps per SM sub-partition, so that one warp's TMEM loads, stores and barrier round trips hide
-// behind the others' arithmetic), warp 16 TMA producer, warp 17 issues the S/dP MMAs and owns
-// TMEM, warp 18 issues the accumulating MMAs (two issuers, so neither waits behind the other's
-// barrier round trips; both run warp-wide with one elected lane issuing), warps 19..22 write a
-// block's sums out while the compute warps are already at work on the next block.  S/dP are released as soon as the compute warps hold them in registers;
-// P^T/dS^T live in their own TMEM buffers until the accumulating MMAs that read them are complete.
+// Roles (25 warps):
+//   warps 0..15 : compute, two teams of eight warps on alternate supersteps (team = warp / 8, TMEM lane
+//                 quarter = warp % 4, 32 of a tile's 64 columns = (warp / 4) % 2), each team with its
+//                 own S/dP and P/dS columns, so that one team's barrier round trips and products run
+//                 under the other one's arithmetic
+//   warps 16, 19: TMA producers, one for Q and K (and LSE2), one for dO and V (and delta): an SM starts a
+//                 copy only every 190 cycles or so from one warp, and four tiles and four vectors a
+//                 superstep from a single one (1,270 cycles) were what the whole kernel waited for
+//   warps 17, 24: issue the S/dP MMAs, one for each team (a wait, eight MMAs and their commit take an
+//                 issuer longer than the superstep); warp 17 owns TMEM
+//   warp 18     : issues the accumulating MMAs (all issuers run warp-wide with one elected lane issuing)
+//   warps 20..23: take a block's sums out of tensor memory and store them while the compute warps are
+//                 already at work on the next block
+// A block's own operands are double-buffered: the next block's are loaded while this one is at work.
+// Head dimensions 16 and 32: zero-filled on load by D-wide tensor maps, D / 16 K steps for S and dP,
+// D-wide accumulating products.
 // Every wait is bounded and every barrier is waited on by warps that see each of its phases.
 #include <math.h>
 
@@ -37,39 +49,46 @@
 
 namespace bsa {
 
-constexpr int kBwdStages = 4;
-constexpr int kCW = 16;                    // compute warps: 4 lane quarters x (kCW / 4) column parts
-constexpr int kChunk = 64 / (kCW / 4);     // columns of a tile per compute warp
-constexpr int kProdWarp = kCW, kXWarp = kCW + 1, kAccWarp = kCW + 2;
-constexpr int kBwdThreads = 32 * (kCW + 7);  // ... and four write-out warps (lane quarter = warp % 4)
+// The streamed tiles: ten places of two tiles (16 KB), split into a ring for Q (dK/dV) or K (dQ) and one
+// for dO or V.  What an accumulating product reads (Q and dO; K) is held from its load to the end of
+// that product, about 5,000 cycles with the arithmetic in between; V only until dP is complete.  With
+// rings too short for that the issuers wait for operands (four places each: a third of the time).
+constexpr int kRing = 10;
+template <bool kDKDV> constexpr int kRing0 = kDKDV ? 5 : 7;
+template <bool kDKDV> constexpr int kRing1 = kRing - kRing0<kDKDV>;
+constexpr int kCW = 16;                    // compute warps: 2 teams x 4 lane quarters x 2 column halves
+constexpr int kTeamW = kCW / 2;
+constexpr int kProdWarp = kCW, kXWarp = kCW + 1, kAccWarp = kCW + 2, kProd2Warp = kCW + 3;
+constexpr int kX2Warp = kCW + 8;           // (warps kCW + 4 .. kCW + 7 write out: lane quarter = warp % 4)
+constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: three warps at the end only fill one
 constexpr uint32_t kBwdTile = 64 * 64 * 2;
 constexpr uint32_t kBwdTmemCols = 512;
 constexpr int kListIndex = BSA_LIST_PARTIAL_FLAG - 1;  // a list entry without its flag
-// TMEM columns: X0 = S (or S^T), X1 = dP (or dP^T), 128 each (tile a in columns 0..63 of lanes
-// 0..63, tile b in columns 64..127 of lanes 64..127); P and dS as 16-bit pairs, 32 columns per
-// tile; two fp32 accumulators.
-constexpr uint32_t kTmX0 = 0, kTmX1 = 128, kTmP = 256, kTmDS = 320, kTmAcc0 = 384, kTmAcc1 = 448;
+// TMEM columns: S (or S^T) of team T at 128 T, its dP (or dP^T) at 128 T + 64; P and dS as 16-bit
+// pairs, 32 columns each, at 256 + 64 T; two fp32 accumulators.
+constexpr uint32_t kTmP = 256, kTmAcc0 = 384, kTmAcc1 = 448;
 
 struct BwdSmem {
-  uint8_t stat0[2][kBwdTile];               // the CTA's own block, twice: K (dK/dV) or Q (dQ)
-  uint8_t stat1[2][kBwdTile];               // V or dO, twice
-  uint8_t str0[kBwdStages][2][kBwdTile];    // streamed tiles a, b: Q (dK/dV) or K (dQ)
-  uint8_t str1[kBwdStages][2][kBwdTile];    // dO or V
-  float lse[kBwdStages][2][64];             // dK/dV: LSE2 and delta of the streamed query tiles
-  float delta[kBwdStages][2][64];
-  // write-out hand-over, [col][row]: 0 = lanes 64..127 of the first (or only) accumulator, 1 =
-  // lanes 64..127 of the second, 2 = lanes 0..63 of the second
-  float xfer[3][64][65];
+  uint8_t stat[2][2][kBwdTile];             // by block parity: the CTA's own K, V (dK/dV) or Q, dO (dQ)
+  uint8_t ring[kRing][2][kBwdTile];         // streamed tiles a, b: Q (dK/dV) or K (dQ), then dO or V
+  float lse[kRing0<true>][2][64];           // dK/dV: LSE2 and delta of the streamed query tiles
+  float delta[kRing1<true>][2][64];
+  // write-out: what lanes 0..63 and 64..127 hand to each other, 32 columns of 64 rows at a time (rows of
+  // 36 floats: eight lanes' 16-byte accesses then fall into different banks)
+  float xfer[2][64][36];
   int item[2];                              // by item parity: the work item, -1 = no more work
   int item_tiles[2], item_begin[2];         // ... its list length and where its list begins
-  uint64_t item_full[2], item_free[2];      // header published; header read by all ten readers
-  uint64_t stat_full, stat_free;            // own operands loaded; their S/dP instructions complete
+  uint64_t item_full[2], item_free[2];      // header published; header read by all its readers
+  uint64_t stat_full[2], stat_free[2];      // own operands loaded; their S/dP instructions complete
   uint64_t acc_done;                        // all accumulating MMAs of the block complete
   uint64_t acc_free;                        // the write-out warps have read the accumulators
-  uint64_t in_full[kBwdStages];
-  uint64_t in_empty[kBwdStages];            // accumulating MMAs of the superstep complete
-  uint64_t x_full, x_free;                  // S/dP complete; S/dP in the compute warps' registers
-  uint64_t d_full, d_free;                  // P/dS stored; accumulating MMAs that read them complete
+  // a place's tiles have landed: one barrier for each place and team, so that the team's issuer and
+  // compute warps, which wait on it, see each of its phases
+  uint64_t in_full0[2 * kRing0<false>], in_full1[2 * kRing1<true>];
+  uint64_t in_empty0[kRing0<false>];        // accumulating MMAs of the superstep complete
+  uint64_t in_empty1[kRing1<true>];         // ... (dQ: dP complete)
+  uint64_t x_full[2], x_free[2];            // by team: S/dP complete; S/dP in the compute warps' registers
+  uint64_t d_full[2], d_free[2];            // P/dS stored; accumulating MMAs that read them complete
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -79,14 +98,15 @@ static_assert(sizeof(BwdSmem) + 1024 <= 232448, "BwdSmem exceeds the shared memo
 struct BwdParams {
   const int32_t* list_ptr;  // dK/dV: column lists (col_ptr/row_idx); dQ: row lists (row_ptr/col_idx)
   const int32_t* list_idx;
+  int list_places;          // 0: list_ptr holds offsets; else counts, list u at list_idx + u * list_places
   const uint8_t* dense;     // optional element-level mask for the tiles whose list entry is flagged
   int64_t ds0, ds1, ds2;
   const float* lse2;
   const float* delta;
   void* out0;  // dV (dK/dV kernel only)
   void* out1;  // dK or dQ
-  int64_t sb, sh, sn;
-  int B, H, N, nb;
+  int64_t sb0, sh0, sn0, sb1, sh1, sn1;  // their element strides
+  int B, H, N, D, nb;
   int items;  // B * H * nb
   int list_b_stride, list_h_stride;
   float scale_log2;
@@ -99,31 +119,6 @@ struct BwdParams {
 __device__ __forceinline__ void bwd_give_up(BwdSmem* sm, int32_t* status, int code) {
   sm->abort_flag = 1;
   report_status(status, code);
-}
-
-// Stores 32 columns of one output row: (own[c] + other[c]) * scale as 16-bit; `other` walks the
-// hand-over buffer ([col][row], 65 floats per column).
-// (wide: the rows start on 32-byte boundaries, so 16 columns go out as one whole sector)
-template <bool kBf16>
-__device__ __forceinline__ void store_cols32(void* base, int64_t elem_off, const uint32_t* own,
-                                             const float* other, float scale, bool wide) {
-  uint16_t* dst = static_cast<uint16_t*>(base) + elem_off;
-#pragma unroll
-  for (int v = 0; v < 2; ++v) {
-    uint32_t w[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const int c = 16 * v + 2 * t;
-      w[t] = pack_2x16<kBf16>((__uint_as_float(own[c]) + other[c * 65]) * scale,
-                              (__uint_as_float(own[c + 1]) + other[(c + 1) * 65]) * scale);
-    }
-    if (wide) {
-      st_global_v8(dst + 16 * v, w);
-    } else {
-      reinterpret_cast<uint4*>(dst + 16 * v)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-      reinterpret_cast<uint4*>(dst + 16 * v)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    }
-  }
 }
 
 // Readers of the item header: wait for item i, read it (the producer looked the list up, so the
@@ -159,13 +154,99 @@ __device__ __forceinline__ BwdItem bwd_item(int w, const BwdParams& p, int n_til
   if (n_tiles < 0) {
     const int64_t li =
         static_cast<int64_t>(it.b * p.list_b_stride + it.h * p.list_h_stride) * p.nb + it.blk;
-    begin = __ldg(p.list_ptr + li);
-    n_tiles = __ldg(p.list_ptr + li + 1) - begin;
+    if (p.list_places > 0) {
+      begin = static_cast<int>(li * p.list_places);
+      n_tiles = __ldg(p.list_ptr + li);
+    } else {
+      begin = __ldg(p.list_ptr + li);
+      n_tiles = __ldg(p.list_ptr + li + 1) - begin;
+    }
   }
   it.n_tiles = n_tiles;
   it.ents = p.list_idx + begin;
   it.vec_base = (static_cast<int64_t>(it.b) * p.H + it.h) * p.N;
   return it;
+}
+
+// A producer's share of an item's supersteps: the listed tiles a, b of one tensor into its half of the
+// ring (and, dK/dV, the tiles' part of one of the two vectors), one lane per copy, copies of one kind in
+// one instruction.
+template <int kPlaces, bool kVector>
+__device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, uint64_t* empty,
+                                               const CUtensorMap* map, float* vec_ring, const float* vec,
+                                               const BwdItem& it, int n_super, int lane,
+                                               volatile int* abort_flag, int* gs) {
+  for (int j = 0; j < n_super; ++j, ++*gs) {
+    const int s = *gs % kPlaces;
+    const int nt = min(2, it.n_tiles - 2 * j), t = lane & 1;
+    const int nj = t < nt ? (__ldg(it.ents + 2 * j + t) & kListIndex) : 0;
+    if (!mbar_wait_warp(smem_u32(empty + s), ((*gs / kPlaces) & 1) ^ 1, abort_flag)) return false;
+    const uint32_t bar = smem_u32(full + *gs % (2 * kPlaces));
+    if (lane == 0) mbar_expect_tx(bar, nt * (kBwdTile + (kVector ? 256u : 0u)));
+    __syncwarp();
+    if (lane < 2 && t < nt)
+      tma_load_4d(smem_u32(ring) + (2 * s + t) * kBwdTile, map, bar, 0, nj * 64, it.h, it.b);
+    if (kVector && (lane & 30) == 2 && t < nt)
+      bulk_load_1d(smem_u32(vec_ring + (2 * s + t) * 64), vec + it.vec_base + nj * 64, 256, bar);
+  }
+  return true;
+}
+
+// The S/dP instructions of one team's supersteps (one warp).
+template <bool kBf16, bool kDKDV>
+__device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uint32_t tmem, int team,
+                                            int lane, volatile int* abort_flag) {
+  constexpr uint32_t idesc_x = umma_idesc(kBf16, 0, 0, 64, 128);
+  const bool leader = elect_one();
+  const uint64_t desc_a0 = smem_desc_sw128(smem_u32(sm->stat[0][0]), 16, 1024);
+  const uint64_t desc_b0 = smem_desc_sw128(smem_u32(sm->ring[0][0]), 16, 1024);
+  const uint64_t desc_b1 = smem_desc_sw128(smem_u32(sm->ring[kRing0<kDKDV>][0]), 16, 1024);
+  constexpr int kR0 = kRing0<kDKDV>, kR1 = kRing1<kDKDV>;
+  constexpr uint64_t kTileDesc = kBwdTile >> 4;  // one tile further, in descriptor units
+  const int k_steps = p.D >> 4;
+  const uint32_t x_full = smem_u32(&sm->x_full[team]), x_free = smem_u32(&sm->x_free[team]);
+  bool ok = true;
+  int gs = 0, ni = 0;
+  for (int i = 0; ok; ++i) {
+    int w, w_tiles, w_begin;
+    ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+    if (!ok || w < 0) break;
+    const int n_super = (w_tiles + 1) >> 1;
+    if (n_super == 0) continue;
+    const int own = ni & 1;
+    ok = mbar_wait_warp(smem_u32(&sm->stat_full[own]), (ni >> 1) & 1, abort_flag);
+    const uint64_t a0 = desc_a0 + static_cast<uint64_t>(2 * own) * kTileDesc;
+    int g = gs + ((gs ^ team) & 1);
+    gs += n_super;
+    for (; ok && g < gs; g += 2) {
+      ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, abort_flag) &&
+           mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, abort_flag);
+      if (!ok) break;
+      // the team must have its previous S/dP in registers (for the first one this asks for the
+      // phase before the first one, which counts as complete)
+      ok = mbar_wait_warp(x_free, ((g >> 1) & 1) ^ 1, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      if (leader) {
+        // (a superstep with one tile multiplies with whatever the second tile's place holds: nobody
+        // reads those lanes)
+        const uint64_t b0 = desc_b0 + static_cast<uint64_t>(2 * (g % kR0)) * kTileDesc;
+        const uint64_t b1 = desc_b1 + static_cast<uint64_t>(2 * (g % kR1)) * kTileDesc;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          if (kk < k_steps) umma_ws_ss(tmem + 128 * team, a0 + 2 * kk, b0 + 2 * kk, idesc_x, kk > 0);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          if (kk < k_steps)
+            umma_ws_ss(tmem + 128 * team + 64, a0 + kTileDesc + 2 * kk, b1 + 2 * kk, idesc_x, kk > 0);
+        tc_commit(x_full);
+        if constexpr (!kDKDV) tc_commit(smem_u32(&sm->in_empty1[g % kR1]));  // V is not needed any more
+      }
+    }
+    if (ok && leader) tc_commit(smem_u32(&sm->stat_free[own]));  // this issuer is through with the operands
+    ++ni;
+  }
+  if (!ok) bwd_give_up(sm, p.status, 2);
 }
 
 // Persistent: one CTA per SM.  The producer starts with item blockIdx.x and then draws further
@@ -192,18 +273,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->item_full[i]), 1);
-      mbar_init(smem_u32(&sm->item_free[i]), kCW + 6);  // compute warps, two issuers, four write-out warps
+      mbar_init(smem_u32(&sm->item_free[i]), kCW + 8);  // all roles but the first producer
+      mbar_init(smem_u32(&sm->stat_full[i]), 2);  // two producers
+      mbar_init(smem_u32(&sm->stat_free[i]), 2);  // two S/dP issuers
+      mbar_init(smem_u32(&sm->x_full[i]), 1);
+      mbar_init(smem_u32(&sm->x_free[i]), kTeamW);  // one arrival per warp of the team
+      mbar_init(smem_u32(&sm->d_full[i]), kTeamW);
+      mbar_init(smem_u32(&sm->d_free[i]), 1);
     }
-    mbar_init(smem_u32(&sm->stat_full), 1);
-    mbar_init(smem_u32(&sm->stat_free), 1);
-    for (int s = 0; s < kBwdStages; ++s) {
-      mbar_init(smem_u32(&sm->in_full[s]), 1);
-      mbar_init(smem_u32(&sm->in_empty[s]), 1);
-    }
-    mbar_init(smem_u32(&sm->x_full), 1);
-    mbar_init(smem_u32(&sm->x_free), kCW);  // one arrival per compute warp
-    mbar_init(smem_u32(&sm->d_full), kCW);
-    mbar_init(smem_u32(&sm->d_free), 1);
+    for (int s = 0; s < 2 * kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_full0[s]), 1);
+    for (int s = 0; s < 2 * kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_full1[s]), 1);
+    for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), 1);
+    for (int s = 0; s < kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
     mbar_init(smem_u32(&sm->acc_done), 1);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
     sm->abort_flag = 0;
@@ -225,247 +306,209 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
 
-  if (warp == kProdWarp) {
-    // =========================== TMA producer ===========================
-    bool ok = true;
-    bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
-    int gs = 0, ni = 0;
-    for (int i = 0, w = blockIdx.x; ok; ++i) {
-      const int par = i & 1;
-      if (i > 0) {
-        if (p.ticket != nullptr) {
-          int t = 0;
+  // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
+  // issuers do without (56 + 104 + 56 = 3 x 72).
+  if (warp >= kCW && warp < kCW + 4) {
+    give_registers<56>();
+    if (warp == kProdWarp) {
+      // =========================== TMA producer ===========================
+      bool ok = true;
+      bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
+      int gs = 0, ni = 0;
+      for (int i = 0, w = blockIdx.x; ok; ++i) {
+        const int par = i & 1;
+        if (i > 0) {
+          if (p.ticket != nullptr) {
+            int t = 0;
+            if (lane == 0) {
+              t = atomicAdd(p.ticket, 1);
+              // every CTA draws until its first ticket past the end, so the launch draws exactly
+              // `items` tickets in all; whoever draws the last one leaves the counter at zero
+              if (t == p.items - 1) atomicExch(p.ticket, 0);
+            }
+            w = stride + __shfl_sync(0xffffffffu, t, 0);
+            terminal = w >= p.items;
+          } else {
+            w += stride;
+          }
+        }
+        // the header slot of item i-2 must have been read by everyone
+        if (i >= 2)
+          ok = mbar_wait_warp(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1, abort_flag);
+        if (!ok) break;
+        BwdItem it;
+        it.n_tiles = 0;
+        if (w < p.items) it = bwd_item<kDKDV>(w, p);
+        if (lane == 0) {
+          sm->item[par] = w < p.items ? w : -1;
+          sm->item_tiles[par] = it.n_tiles;
+          sm->item_begin[par] = w < p.items ? static_cast<int>(it.ents - p.list_idx) : 0;
+          mbar_arrive(smem_u32(&sm->item_full[par]));  // release: the header is visible
+        }
+        if (w >= p.items) break;
+        const int n_super = (it.n_tiles + 1) >> 1;
+        if (n_super == 0) continue;
+        // the block's own operands: the S/dP instructions of the block before the previous one must
+        // be complete
+        const int own = ni & 1;
+        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1, abort_flag);
+        if (!ok) break;
+        {
+          const uint32_t bar = smem_u32(&sm->stat_full[own]);
           if (lane == 0) {
-            t = atomicAdd(p.ticket, 1);
-            // every CTA draws until its first ticket past the end, so the launch draws exactly
-            // `items` tickets in all; whoever draws the last one leaves the counter at zero
-            if (t == p.items - 1) atomicExch(p.ticket, 0);
-          }
-          w = stride + __shfl_sync(0xffffffffu, t, 0);
-          terminal = w >= p.items;
-        } else {
-          w += stride;
-        }
-      }
-      // the header slot of item i-2 must have been read by everyone
-      if (i >= 2)
-        ok = mbar_wait_warp(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1, abort_flag);
-      if (!ok) break;
-      BwdItem it;
-      it.n_tiles = 0;
-      if (w < p.items) it = bwd_item<kDKDV>(w, p);
-      if (lane == 0) {
-        sm->item[par] = w < p.items ? w : -1;
-        sm->item_tiles[par] = it.n_tiles;
-        sm->item_begin[par] = w < p.items ? static_cast<int>(it.ents - p.list_idx) : 0;
-        mbar_arrive(smem_u32(&sm->item_full[par]));  // release: the header is visible
-      }
-      if (w >= p.items) break;
-      const int n_super = (it.n_tiles + 1) >> 1;
-      if (n_super == 0) continue;
-      // the block's own operands: the previous item's S/dP instructions must be complete
-      if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->stat_free), (ni - 1) & 1, abort_flag);
-      if (!ok) break;
-      // One lane per copy: a single thread can start a tile load only every couple of hundred
-      // cycles, which up to eight copies in a row would turn into the kernel's bound.
-      {
-        const uint32_t bar = smem_u32(&sm->stat_full);
-        if (lane == 0) mbar_expect_tx(bar, 4 * kBwdTile);
-        __syncwarp();
-        if (lane < 2)
-          tma_load_4d(smem_u32(sm->stat0[lane]), &tm_stat0, bar, 0, it.blk * 64, it.h, it.b);
-        else if (lane < 4)
-          tma_load_4d(smem_u32(sm->stat1[lane - 2]), &tm_stat1, bar, 0, it.blk * 64, it.h, it.b);
-      }
-      for (int j = 0; j < n_super; ++j, ++gs) {
-        const int s = gs % kBwdStages;
-        const int nt = min(2, it.n_tiles - 2 * j);
-        const int tl = (lane >> 1) & 1;  // lanes 0, 1, 4, 5 serve tile a, lanes 2, 3, 6, 7 tile b
-        const int nj = tl < nt ? (__ldg(it.ents + 2 * j + tl) & kListIndex) : 0;
-        ok = mbar_wait_warp(smem_u32(&sm->in_empty[s]), ((gs / kBwdStages) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        const uint32_t bar = smem_u32(&sm->in_full[s]);
-        if (lane == 0) mbar_expect_tx(bar, nt * (2 * kBwdTile + (kDKDV ? 512u : 0u)));
-        __syncwarp();
-        if (tl < nt) {
-          if (lane < 4) {
-            if (lane & 1)
-              tma_load_4d(smem_u32(sm->str1[s][tl]), &tm_str1, bar, 0, nj * 64, it.h, it.b);
-            else
-              tma_load_4d(smem_u32(sm->str0[s][tl]), &tm_str0, bar, 0, nj * 64, it.h, it.b);
-          } else if (kDKDV && lane < 8) {
-            if (lane & 1)
-              bulk_load_1d(smem_u32(sm->delta[s][tl]), p.delta + it.vec_base + nj * 64, 256, bar);
-            else
-              bulk_load_1d(smem_u32(sm->lse[s][tl]), p.lse2 + it.vec_base + nj * 64, 256, bar);
+            mbar_expect_tx(bar, kBwdTile);
+            tma_load_4d(smem_u32(sm->stat[own][0]), &tm_stat0, bar, 0, it.blk * 64, it.h, it.b);
           }
         }
+        ok = bwd_load_tiles<kRing0<kDKDV>, kDKDV>(sm->ring[0][0], sm->in_full0, sm->in_empty0, &tm_str0,
+                                                  sm->lse[0][0], p.lse2, it, n_super, lane, abort_flag,
+                                                  &gs);
+        ++ni;
       }
-      ++ni;
-    }
-    if (!ok) bwd_give_up(sm, p.status, 1);
-    if (!terminal && lane == 0) {
-      // gave up before the last draw: draw on (without working) until this CTA's first ticket past
-      // the end, so that the launch still draws `items` tickets and the counter returns to zero
-      int t;
-      do {
-        t = atomicAdd(p.ticket, 1);
-        if (t == p.items - 1) atomicExch(p.ticket, 0);
-      } while (stride + t < p.items);
-    }
-  } else if (warp == kXWarp) {
-    // =========================== S / dP issuer ===========================
-    constexpr uint32_t idesc_x128 = umma_idesc(kBf16, 0, 0, 128, 128);
-    constexpr uint32_t idesc_x64 = umma_idesc(kBf16, 0, 0, 128, 64);  // odd tail: one tile
-    const bool leader = elect_one();
-    const uint64_t desc_a0 = smem_desc_sw128(smem_u32(sm->stat0[0]), 16, 1024);
-    const uint64_t desc_a1 = smem_desc_sw128(smem_u32(sm->stat1[0]), 16, 1024);
-    const uint64_t desc_b0 = smem_desc_sw128(smem_u32(sm->str0[0][0]), 16, 1024);
-    const uint64_t desc_b1 = smem_desc_sw128(smem_u32(sm->str1[0][0]), 16, 1024);
-    bool ok = true;
-    int gs = 0, ni = 0;
-    for (int i = 0; ok; ++i) {
-      int w, w_tiles, w_begin;
-      ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
-      if (!ok || w < 0) break;
-      const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
-      const int n_super = (it.n_tiles + 1) >> 1;
-      if (n_super == 0) continue;
-      ok = mbar_wait_warp(smem_u32(&sm->stat_full), ni & 1, abort_flag);
-      for (int j = 0; ok && j < n_super; ++j, ++gs) {
-        const int s = gs % kBwdStages;
-        const int nt = min(2, it.n_tiles - 2 * j);
-        ok = mbar_wait_warp(smem_u32(&sm->in_full[s]), (gs / kBwdStages) & 1, abort_flag);
+      if (!ok) bwd_give_up(sm, p.status, 1);
+      if (!terminal && lane == 0) {
+        // gave up before the last draw: draw on (without working) until this CTA's first ticket past
+        // the end, so that the launch still draws `items` tickets and the counter returns to zero
+        int t;
+        do {
+          t = atomicAdd(p.ticket, 1);
+          if (t == p.items - 1) atomicExch(p.ticket, 0);
+        } while (stride + t < p.items);
+      }
+    } else if (warp == kProd2Warp) {
+      // =========================== second TMA producer ===========================
+      bool ok = true;
+      int gs = 0, ni = 0;
+      for (int i = 0; ok; ++i) {
+        int w, w_tiles, w_begin;
+        ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+        if (!ok || w < 0) break;
+        const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
+        const int n_super = (w_tiles + 1) >> 1;
+        if (n_super == 0) continue;
+        const int own = ni & 1;
+        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1, abort_flag);
         if (!ok) break;
-        // S/dP of the previous superstep must be in the compute warps' registers (for the first
-        // one this asks for the phase before the first one, which counts as complete)
-        ok = mbar_wait_warp(smem_u32(&sm->x_free), (gs & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        if (leader) {
-          const uint64_t b0 = desc_b0 + static_cast<uint64_t>(s * ((2 * kBwdTile) >> 4));
-          const uint64_t b1 = desc_b1 + static_cast<uint64_t>(s * ((2 * kBwdTile) >> 4));
-          const uint32_t idesc = nt == 2 ? idesc_x128 : idesc_x64;
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ss(tmem + kTmX0, desc_a0 + 2 * kk, b0 + 2 * kk, idesc, kk > 0);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ss(tmem + kTmX1, desc_a1 + 2 * kk, b1 + 2 * kk, idesc, kk > 0);
-          tc_commit(smem_u32(&sm->x_full));
-          if (j == n_super - 1) tc_commit(smem_u32(&sm->stat_free));  // own operands reusable
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(&sm->stat_full[own]);
+          mbar_expect_tx(bar, kBwdTile);
+          tma_load_4d(smem_u32(sm->stat[own][1]), &tm_stat1, bar, 0, it.blk * 64, it.h, it.b);
         }
+        ok = bwd_load_tiles<kRing1<kDKDV>, kDKDV>(sm->ring[kRing0<kDKDV>][0], sm->in_full1,
+                                                  sm->in_empty1, &tm_str1, sm->delta[0][0], p.delta, it,
+                                                  n_super, lane, abort_flag, &gs);
+        ++ni;
       }
-      ++ni;
-    }
-    if (!ok) bwd_give_up(sm, p.status, 2);
-  } else if (warp == kAccWarp) {
-    // =========================== accumulating-MMA issuer ===========================
-    constexpr uint32_t idesc_acc = umma_idesc(kBf16, 0, 1, 128, 64);
-    const bool leader = elect_one();
-    const uint64_t desc_m0 = smem_desc_sw128(smem_u32(sm->str0[0][0]), 8192, 1024);
-    const uint64_t desc_m1 = smem_desc_sw128(smem_u32(sm->str1[0][0]), 8192, 1024);
-    bool ok = true;
-    int gs = 0, ni = 0;
-    for (int i = 0; ok; ++i) {
-      int w, w_tiles, w_begin;
-      ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
-      if (!ok || w < 0) break;
-      const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
-      const int n_super = (it.n_tiles + 1) >> 1;
-      if (n_super == 0) continue;
-      // the write-out warps must have read the previous block's accumulators
-      if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1, abort_flag);
-      for (int j = 0; ok && j < n_super; ++j, ++gs) {
-        const int s = gs % kBwdStages;
-        const int nt = min(2, it.n_tiles - 2 * j);
-        ok = mbar_wait_warp(smem_u32(&sm->d_full), gs & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        if (leader) {
-          // keys/queries [16 kk, +16) of tile t sit at column 32 t + 8 kk of the P / dS buffers
-          for (int t = 0; t < nt; ++t) {
-            const uint32_t first = (j > 0 || t > 0) ? 1u : 0u;
-            if constexpr (kDKDV) {
-              const uint64_t bmn = desc_m1 + static_cast<uint64_t>((2 * s + t) * (kBwdTile >> 4));
+      if (!ok) bwd_give_up(sm, p.status, 1);
+    } else if (warp == kXWarp) {
+      bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, 0, lane, abort_flag);
+    } else if (warp == kAccWarp) {
+      // =========================== accumulating-MMA issuer ===========================
+      const uint32_t idesc_acc = umma_idesc(kBf16, 0, 1, 128, p.D);
+      const bool leader = elect_one();
+      const uint64_t desc_m0 = smem_desc_sw128(smem_u32(sm->ring[0][0]), 8192, 1024);
+      const uint64_t desc_m1 = smem_desc_sw128(smem_u32(sm->ring[kRing0<kDKDV>][0]), 8192, 1024);
+      bool ok = true;
+      int gs = 0, ni = 0;
+      for (int i = 0; ok; ++i) {
+        int w, w_tiles, w_begin;
+        ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+        if (!ok || w < 0) break;
+        const int n_super = (w_tiles + 1) >> 1;
+        if (n_super == 0) continue;
+        // the write-out warps must have read the previous block's accumulators
+        if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1, abort_flag);
+        for (int j = 0; ok && j < n_super; ++j, ++gs) {
+          const int s0 = gs % kRing0<kDKDV>, s1 = gs % kRing1<kDKDV>, team = gs & 1;
+          const int nt = min(2, w_tiles - 2 * j);
+          ok = mbar_wait_warp(smem_u32(&sm->d_full[team]), (gs >> 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (leader) {
+            // keys/queries [16 kk, +16) of a tile sit at column 8 kk of the P / dS columns, tile a's in
+            // lanes 0..63, tile b's in lanes 64..127; each product writes the lanes of its tile only
+            const uint32_t p_cols = tmem + kTmP + 64 * team, ds_cols = p_cols + 32;
+            for (int t = 0; t < nt; ++t) {
+              if constexpr (kDKDV) {
+                const uint64_t bmn = desc_m1 + static_cast<uint64_t>((2 * s1 + t) * (kBwdTile >> 4));
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                  umma_ts_half(tmem + kTmAcc0, p_cols + 8 * kk, bmn + 128 * kk, idesc_acc,
+                               (j > 0) || (kk > 0), t);
+              }
+              const uint64_t bmn = desc_m0 + static_cast<uint64_t>((2 * s0 + t) * (kBwdTile >> 4));
 #pragma unroll
               for (int kk = 0; kk < 4; ++kk)
-                umma_ts(tmem + kTmAcc0, tmem + kTmP + 32 * t + 8 * kk, bmn + 128 * kk, idesc_acc,
-                        first | (kk > 0));
+                umma_ts_half(tmem + kTmAcc1, ds_cols + 8 * kk, bmn + 128 * kk, idesc_acc,
+                             (j > 0) || (kk > 0), t);
             }
-            const uint64_t bmn = desc_m0 + static_cast<uint64_t>((2 * s + t) * (kBwdTile >> 4));
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              umma_ts(tmem + kTmAcc1, tmem + kTmDS + 32 * t + 8 * kk, bmn + 128 * kk, idesc_acc,
-                      first | (kk > 0));
+            tc_commit(smem_u32(&sm->in_empty0[s0]));  // places free
+            if constexpr (kDKDV) tc_commit(smem_u32(&sm->in_empty1[s1]));
+            tc_commit(smem_u32(&sm->d_free[team]));  // P/dS columns free; accumulators updated
+            if (j == n_super - 1) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
           }
-          tc_commit(smem_u32(&sm->in_empty[s]));  // stage free
-          tc_commit(smem_u32(&sm->d_free));       // P/dS buffers free; accumulators updated
-          if (j == n_super - 1) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
         }
+        ++ni;
       }
-      ++ni;
+      if (!ok) bwd_give_up(sm, p.status, 2);
     }
-    if (!ok) bwd_give_up(sm, p.status, 2);
   } else if (warp < kCW) {
     // =========================== compute warps ===========================
+    const int team = warp >> 3;
+    const int ch = (warp >> 2) & 1;     // which 32 of the tile's 64 columns
     const int quarter = warp & 3;
-    const int ch = warp >> 2;           // which kChunk of the tile's 64 columns
     const int t_mine = quarter >> 1;    // lanes 0..63 own tile a of a superstep, 64..127 tile b
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the CTA's block
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t s_at = tmem + lane_base + 128 * team + 32 * ch, dp_at = s_at + 64;
+    const uint32_t p_at = tmem + lane_base + kTmP + 64 * team + 16 * ch, ds_at = p_at + 32;
     const float c = p.scale_log2;
-    {
-      // The accumulating MMAs of a tile sweep all 128 lanes: the half of the lanes that does not
-      // own the tile holds zeros where that tile's P / dS live.  Nothing else ever writes there.
-      uint32_t z[kChunk / 2];
-#pragma unroll
-      for (int i = 0; i < kChunk / 2; ++i) z[i] = 0u;
-      if constexpr (kDKDV)
-        tmem_st_cols<kChunk / 2>(tmem + lane_base + kTmP + 32 * (1 - t_mine) + (kChunk / 2) * ch, z);
-      tmem_st_cols<kChunk / 2>(tmem + lane_base + kTmDS + 32 * (1 - t_mine) + (kChunk / 2) * ch, z);
-      tc_wait_st();
-    }
     bool ok = true;
-    int gs = 0;
+    int gs = 0;  // supersteps of earlier items; this team takes those with gs % 2 == team
     for (int i = 0; ok; ++i) {
       int w, w_tiles, w_begin;
       ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
       if (!ok || w < 0) break;
-      const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
-      const int n_super = (it.n_tiles + 1) >> 1;
-      const int row = it.blk * 64 + r_blk;
+      const int n_super = (w_tiles + 1) >> 1;
       if (n_super == 0) continue;  // (the write-out warps store the zero gradients)
       float my_lse = 0.f, my_delta = 0.f;
-      if constexpr (!kDKDV) {
-        // (a row whose elements are all masked has LSE = -inf; every logit it meets is -inf too,
-        // and against a finite stand-in it exponentiates to 0 instead of NaN)
-        my_lse = __ldg(p.lse2 + it.vec_base + row);
-        if constexpr (kElementMask) my_lse = fmaxf(my_lse, -3.0e38f);
-        my_delta = __ldg(p.delta + it.vec_base + row);
-      }
-      // element-level mask: where this lane's mask bytes of a tile start (dQ: its query row, 32
-      // consecutive keys; dK/dV: its key column, 32 consecutive query rows)
       const uint8_t* mask_at = nullptr;
-      if constexpr (kElementMask)
-        mask_at = p.dense + it.b * p.ds0 + it.h * p.ds1 +
-                  (kDKDV ? static_cast<int64_t>(row) : static_cast<int64_t>(row) * p.ds2);
-      for (int j = 0; ok && j < n_super; ++j, ++gs) {
-        const int s = gs % kBwdStages;
-        const int nt = min(2, it.n_tiles - 2 * j);
-        const bool active = t_mine < nt;  // warp-uniform
+      const int32_t* ents = nullptr;
+      if constexpr (!kDKDV || kElementMask) {
+        const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
+        const int row = it.blk * 64 + r_blk;
+        ents = it.ents + t_mine;
+        if constexpr (!kDKDV) {
+          // (a row whose elements are all masked has LSE = -inf; every logit it meets is -inf too,
+          // and against a finite stand-in it exponentiates to 0 instead of NaN)
+          my_lse = __ldg(p.lse2 + it.vec_base + row);
+          if constexpr (kElementMask) my_lse = fmaxf(my_lse, -3.0e38f);
+          my_delta = __ldg(p.delta + it.vec_base + row);
+        }
+        // element-level mask: where this lane's mask bytes of a tile start (dQ: its query row, 32
+        // consecutive keys; dK/dV: its key column, 32 consecutive query rows)
+        if constexpr (kElementMask)
+          mask_at = p.dense + it.b * p.ds0 + it.h * p.ds1 +
+                    (kDKDV ? static_cast<int64_t>(row) : static_cast<int64_t>(row) * p.ds2);
+      }
+      int j = (gs ^ team) & 1;
+      int g = gs + j;
+      gs += n_super;
+      for (; ok && j < n_super; j += 2, g += 2) {
+        const bool active = 2 * j + t_mine < w_tiles;  // this lane's tile exists (warp-uniform)
+        const uint32_t ph = (g >> 1) & 1;
         // A tile with masked elements inside: fetch this lane's 32 mask bytes while S is on its way
-        uint32_t mw[kChunk / 4];
+        uint32_t mw[8];
         bool partial = false;
         if (kElementMask && active) {
-          const int e = __ldg(it.ents + 2 * j + t_mine);
+          const int e = __ldg(ents + 2 * j);
           partial = (e & BSA_LIST_PARTIAL_FLAG) != 0;  // warp-uniform
           if (partial) {
-            const int64_t other = static_cast<int64_t>((e & kListIndex) * 64 + kChunk * ch);
+            const int64_t other = static_cast<int64_t>((e & kListIndex) * 64 + 32 * ch);
             if constexpr (kDKDV) {
               const uint8_t* mp = mask_at + other * p.ds2;
 #pragma unroll
-              for (int q4 = 0; q4 < kChunk / 4; ++q4) {
+              for (int q4 = 0; q4 < 8; ++q4) {
                 uint32_t w4 = 0;
 #pragma unroll
                 for (int bb = 0; bb < 4; ++bb)
@@ -475,7 +518,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
             } else {
               const uint4* mp = reinterpret_cast<const uint4*>(mask_at + other);
 #pragma unroll
-              for (int q16 = 0; q16 < kChunk / 16; ++q16) {
+              for (int q16 = 0; q16 < 2; ++q16) {
                 const uint4 a = __ldg(mp + q16);
                 mw[4 * q16] = a.x; mw[4 * q16 + 1] = a.y; mw[4 * q16 + 2] = a.z; mw[4 * q16 + 3] = a.w;
               }
@@ -484,123 +527,131 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         }
         if constexpr (kDKDV) {
           // the LSE2/delta vectors of this stage arrive through the async proxy
-          ok = mbar_wait_warp(smem_u32(&sm->in_full[s]), (gs / kBwdStages) & 1, abort_flag);
+          constexpr int kR0 = kRing0<true>, kR1 = kRing1<true>;
+          ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, abort_flag) &&
+               mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, abort_flag);
           if (!ok) break;
         }
-        ok = mbar_wait_warp(smem_u32(&sm->x_full), gs & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->x_full[team]), ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        uint32_t xs[kChunk], xd[kChunk];
         if (active) {
-          tmem_ld_cols<kChunk>(tmem + lane_base + kTmX0 + 64 * t_mine + kChunk * ch, xs);
-          tmem_ld_cols<kChunk>(tmem + lane_base + kTmX1 + 64 * t_mine + kChunk * ch, xd);
-        }
-        tc_wait_ld();
-        // S/dP are in registers: the next superstep's may be issued
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->x_free));
-        if (partial) {
-          // masked elements: logit -inf, so P = 0 and with it dS = 0
+          const float4* lse4 = reinterpret_cast<const float4*>(&sm->lse[g % kRing0<true>][t_mine][32 * ch]);
+          const ulonglong2* del4 = reinterpret_cast<const ulonglong2*>(&sm->delta[g % kRing1<true>][t_mine][32 * ch]);
+          // 16 columns at a time in a loop: half the code, and no more than 32 logits in registers
 #pragma unroll
-          for (int q4 = 0; q4 < kChunk / 4; ++q4) {
-            const uint32_t nz = __vcmpne4(mw[q4], 0u);
-#pragma unroll
-            for (int bb = 0; bb < 4; ++bb) {
-              const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
-              xs[4 * q4 + bb] = (xs[4 * q4 + bb] & keep) | (0xff800000u & ~keep);
+          for (int half16 = 0; half16 < 2; ++half16) {
+            uint32_t xs[16], xd[16], pk_p[8], pk_ds[8];
+            tmem_ld_32x32b_x16(s_at + 16 * half16, xs);
+            tmem_ld_32x32b_x16(dp_at + 16 * half16, xd);
+            tc_wait_ld();
+            if (half16 == 1) {  // S/dP are in registers: the team's next ones may be issued
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(smem_u32(&sm->x_free[team]));
             }
-          }
-        }
-        uint32_t pk_p[kChunk / 2], pk_ds[kChunk / 2];
-        if (active) {
-          const float4* lse4 = reinterpret_cast<const float4*>(&sm->lse[s][t_mine][kChunk * ch]);
-          const float4* del4 = reinterpret_cast<const float4*>(&sm->delta[s][t_mine][kChunk * ch]);
+            if (partial) {
+              // masked elements: logit -inf, so P = 0 and with it dS = 0
 #pragma unroll
-          for (int i = 0; i < kChunk; i += 4) {
-            float l[4], d[4];
-            if constexpr (kDKDV) {
-              const float4 lv = lse4[i / 4], dv = del4[i / 4];
-              // (-inf = a query row with every element masked: see my_lse above)
-              l[0] = lv.x; l[1] = lv.y; l[2] = lv.z; l[3] = lv.w;
-              if constexpr (kElementMask) {
+              for (int q4 = 0; q4 < 4; ++q4) {
+                const uint32_t nz = __vcmpne4(mw[4 * half16 + q4], 0u);
 #pragma unroll
-                for (int t = 0; t < 4; ++t) l[t] = fmaxf(l[t], -3.0e38f);
+                for (int bb = 0; bb < 4; ++bb) {
+                  const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
+                  xs[4 * q4 + bb] = (xs[4 * q4 + bb] & keep) | (0xff800000u & ~keep);
+                }
               }
-              d[0] = dv.x; d[1] = dv.y; d[2] = dv.z; d[3] = dv.w;
-            } else {
-              l[0] = l[1] = l[2] = l[3] = my_lse;
-              d[0] = d[1] = d[2] = d[3] = my_delta;
             }
-            // two columns per instruction where the operands allow it (same rounding as scalar)
-            float pv[4], dsv[4];
 #pragma unroll
-            for (int t = 0; t < 4; t += 2) {
-              const uint64_t dp2 =
-                  pack_f32x2(__uint_as_float(xd[i + t]), __uint_as_float(xd[i + t + 1]));
-              uint64_t diff2;
+            for (int q = 0; q < 16; q += 4) {
+              // two columns per instruction where the operands allow it
+              float pv[4], dsv[4], nl[4];
+              uint64_t d2[2];
               if constexpr (kDKDV) {
                 // LSE and delta differ from column to column here
-                pv[t] = ex2_approx(fmaf(__uint_as_float(xs[i + t]), c, -l[t]));
-                pv[t + 1] = ex2_approx(fmaf(__uint_as_float(xs[i + t + 1]), c, -l[t + 1]));
-                diff2 = fma_f32x2(pack_f32x2(d[t], d[t + 1]), pack_f32x2(-1.f, -1.f), dp2);
-              } else {
-                float z0, z1;
-                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(xs[i + t]),
-                                                  __uint_as_float(xs[i + t + 1])),
-                                       pack_f32x2(c, c), pack_f32x2(-my_lse, -my_lse)),
-                             z0, z1);
-                pv[t] = ex2_approx(z0);
-                pv[t + 1] = ex2_approx(z1);
-                diff2 = add_f32x2(dp2, pack_f32x2(-my_delta, -my_delta));
+                // (-inf = a query row with every element masked: see my_lse above)
+                const float4 lv = lse4[4 * half16 + q / 4];
+                const ulonglong2 dv = del4[4 * half16 + q / 4];
+                nl[0] = lv.x; nl[1] = lv.y; nl[2] = lv.z; nl[3] = lv.w;
+                if constexpr (kElementMask) {
+#pragma unroll
+                  for (int t = 0; t < 4; ++t) nl[t] = fmaxf(nl[t], -3.0e38f);
+                }
+                d2[0] = dv.x; d2[1] = dv.y;
               }
-              unpack_f32x2(mul_f32x2(pack_f32x2(pv[t], pv[t + 1]), diff2), dsv[t], dsv[t + 1]);
+#pragma unroll
+              for (int t = 0; t < 4; t += 2) {
+                const uint64_t dp2 =
+                    pack_f32x2(__uint_as_float(xd[q + t]), __uint_as_float(xd[q + t + 1]));
+                uint64_t diff2;
+                if constexpr (kDKDV) {
+                  pv[t] = ex2_approx(fmaf(__uint_as_float(xs[q + t]), c, -nl[t]));
+                  pv[t + 1] = ex2_approx(fmaf(__uint_as_float(xs[q + t + 1]), c, -nl[t + 1]));
+                  diff2 = fma_f32x2(d2[t / 2], pack_f32x2(-1.f, -1.f), dp2);
+                } else {
+                  float z0, z1;
+                  unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(xs[q + t]),
+                                                    __uint_as_float(xs[q + t + 1])),
+                                         pack_f32x2(c, c), pack_f32x2(-my_lse, -my_lse)),
+                               z0, z1);
+                  pv[t] = ex2_approx(z0);
+                  pv[t + 1] = ex2_approx(z1);
+                  diff2 = add_f32x2(dp2, pack_f32x2(-my_delta, -my_delta));
+                }
+                unpack_f32x2(mul_f32x2(pack_f32x2(pv[t], pv[t + 1]), diff2), dsv[t], dsv[t + 1]);
+              }
+              pk_p[q / 2] = pack_2x16<kBf16>(pv[0], pv[1]);
+              pk_p[q / 2 + 1] = pack_2x16<kBf16>(pv[2], pv[3]);
+              pk_ds[q / 2] = pack_2x16<kBf16>(dsv[0], dsv[1]);
+              pk_ds[q / 2 + 1] = pack_2x16<kBf16>(dsv[2], dsv[3]);
             }
-            pk_p[i / 2] = pack_2x16<kBf16>(pv[0], pv[1]);
-            pk_p[i / 2 + 1] = pack_2x16<kBf16>(pv[2], pv[3]);
-            pk_ds[i / 2] = pack_2x16<kBf16>(dsv[0], dsv[1]);
-            pk_ds[i / 2 + 1] = pack_2x16<kBf16>(dsv[2], dsv[3]);
+            if (half16 == 0) {
+              // the accumulating MMAs of the team's previous superstep must be through with the P/dS
+              // columns
+              ok = mbar_wait_warp(smem_u32(&sm->d_free[team]), ph ^ 1, abort_flag);
+              tc_fence_after();
+            }
+            if (!ok) break;
+            if constexpr (kDKDV) tmem_st_32x32b_x8(p_at + 8 * half16, pk_p);
+            tmem_st_32x32b_x8(ds_at + 8 * half16, pk_ds);
           }
+          tc_wait_st();
+        } else {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sm->x_free[team]));
+          ok = mbar_wait_warp(smem_u32(&sm->d_free[team]), ph ^ 1, abort_flag);
         }
-        // the accumulating MMAs of the previous superstep still read the P/dS buffers
-        ok = mbar_wait_warp(smem_u32(&sm->d_free), (gs & 1) ^ 1, abort_flag);
         if (!ok) break;
-        if (active) {
-          tc_fence_after();
-          if constexpr (kDKDV)
-            tmem_st_cols<kChunk / 2>(tmem + lane_base + kTmP + 32 * t_mine + (kChunk / 2) * ch, pk_p);
-          tmem_st_cols<kChunk / 2>(tmem + lane_base + kTmDS + 32 * t_mine + (kChunk / 2) * ch, pk_ds);
-        }
-        tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->d_full));
+        if (lane == 0) mbar_arrive(smem_u32(&sm->d_full[team]));
       }
       // (the block's sums are merged and stored by the write-out warps; these warps go straight
       // on to the next block, whose first S/dP is usually complete already)
     }
     if (!ok) bwd_give_up(sm, p.status, 3);
-  } else {
+  } else if (warp < kCW + 8) {
     // =========================== write-out ===========================
-    // Lane r of an accumulator holds the tile-a sums of row r of the CTA's block, lane r+64 its
-    // tile-b sums (never unwritten, even for a single-tile list: the first accumulate-off MMA
-    // sweeps all lanes, and theirs hold zeros for tile a).  These four warps (lane quarter = warp
-    // % 4) take the sums out of tensor memory as soon as the block's last MMAs are complete, so
-    // that the next block can start accumulating, then add the two halves, scale, round and
-    // store, while the compute warps are already at work on the next block.  Lanes 64..127 pass
-    // everything on through shared memory; for dK/dV lanes 0..63 pass their second accumulator
-    // on as well, and the warps of lanes 64..127 merge and store that one.
+    // Lane r of an accumulator holds the tile-a sums of row r of the CTA's block, lane r+64 its tile-b
+    // sums (unwritten when the list has a single tile).  These four warps (lane quarter = warp % 4)
+    // take the sums out of tensor memory as soon as the block's last MMAs are complete, so that the
+    // next block can start accumulating, then add the two halves, scale, round and store, while the
+    // compute warps are already at work on the next block.  dK/dV: lanes 0..63 finish dV and hand
+    // over their sums of dK, lanes 64..127 the other way round; dQ: lanes 0..63 finish columns
+    // [0, 32), lanes 64..127 columns [32, 64).
     // Both named barriers of an iteration are always executed, also after a give-up, and the
     // last one carries the give-up vote, so that no warp of this role is left waiting at one.
+    take_registers<104>();
     const int quarter = warp & 3;
     const int half = quarter >> 1;
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the CTA's block
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t tm_first = tmem + lane_base + (kDKDV ? kTmAcc0 : kTmAcc1);
-    const uint32_t tm_second = tmem + lane_base + kTmAcc1;  // dK (dK/dV kernel only)
-    void* const out_first = kDKDV ? p.out0 : p.out1;
-    const float scale_first = kDKDV ? 1.0f : p.sm_scale;
-    const bool wide = p.wide_stores != 0;
+    constexpr int kKeep = kDKDV ? 64 : 32;        // columns a lane finishes, and hands over
+    const uint32_t tm_keep = tmem + lane_base + (kDKDV ? (half ? kTmAcc1 : kTmAcc0) : kTmAcc1 + 32 * half);
+    const uint32_t tm_send = tmem + lane_base + (kDKDV ? (half ? kTmAcc0 : kTmAcc1) : kTmAcc1 + 32 - 32 * half);
+    const bool first_out = kDKDV && half == 0;    // dV; else dK or dQ
+    const float scale = first_out ? 1.0f : p.sm_scale;
+    const int col0 = kDKDV ? 0 : 32 * half;
     bool ok = true;
     int ni = 0;
     for (int i = 0;; ++i) {
@@ -608,80 +659,84 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       if (ok) ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
       if (ok && w < 0) break;  // no more work: the same for all four warps
       const BwdItem it = bwd_item<kDKDV>(ok ? w : 0, p, ok ? w_tiles : 1, 0);
-      const int n_super = (it.n_tiles + 1) >> 1;
-      const int64_t off =
-          it.b * p.sb + it.h * p.sh + static_cast<int64_t>(it.blk * 64 + r_blk) * p.sn;
-      if (n_super == 0) {
+      const int64_t row = it.blk * 64 + r_blk;
+      uint16_t* dst = first_out
+                          ? static_cast<uint16_t*>(p.out0) + it.b * p.sb0 + it.h * p.sh0 + row * p.sn0
+                          : static_cast<uint16_t*>(p.out1) + it.b * p.sb1 + it.h * p.sh1 + row * p.sn1;
+      if (ok && w_tiles == 0) {
         // a block with an empty list: zero gradients (the same decision in all four warps)
-        if (half == 0 || kDKDV) {
-          uint4* dst = reinterpret_cast<uint4*>(
-              static_cast<uint16_t*>(half == 0 ? out_first : p.out1) + off);
-#pragma unroll
-          for (int v = 0; v < 8; ++v) dst[v] = make_uint4(0u, 0u, 0u, 0u);
-        }
+#pragma unroll 1
+        for (int v = col0; v < min(col0 + kKeep, p.D); v += 8)
+          *reinterpret_cast<uint4*>(dst + v) = make_uint4(0u, 0u, 0u, 0u);
         continue;
       }
       if (ok) ok = mbar_wait_warp(smem_u32(&sm->acc_done), ni & 1, abort_flag);
       ++ni;
-      uint32_t own[32];
-      if (ok) {
-        tc_fence_after();
-        if (half == 1) {
+      const bool live = half == 0 || w_tiles > 1;  // warp-uniform
+      bool any_failed = false;
+#pragma unroll 1
+      for (int q = 0; q < kKeep; q += 32) {
+        uint32_t keep[32];
+        if (ok) {
+          uint4* to = reinterpret_cast<uint4*>(sm->xfer[half][r_blk]);
+          if (live) {
+            uint32_t send[32];
+            tc_fence_after();
+            tmem_ld_32x32b_x32(tm_send + q, send);
+            tmem_ld_32x32b_x32(tm_keep + q, keep);
+            tc_wait_ld();
 #pragma unroll
-          for (int a = 0; a < (kDKDV ? 2 : 1); ++a) {
+            for (int k = 0; k < 8; ++k)
+              to[k] = make_uint4(send[4 * k], send[4 * k + 1], send[4 * k + 2], send[4 * k + 3]);
+          } else {
 #pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-              tmem_ld_32x32b_x32((a == 0 ? tm_first : tm_second) + 32 * h2, own);
-              tc_wait_ld();
+            for (int k = 0; k < 32; ++k) keep[k] = 0u;
 #pragma unroll
-              for (int c = 0; c < 32; ++c) sm->xfer[a][32 * h2 + c][r_blk] = __uint_as_float(own[c]);
+            for (int k = 0; k < 8; ++k) to[k] = make_uint4(0u, 0u, 0u, 0u);
+          }
+          if (q + 32 == kKeep) {
+            // the accumulators are out of tensor memory: the next block may start accumulating
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sm->acc_free));
+          }
+        }
+        named_barrier_sync(2, 128);
+        if (ok) {
+          const float4* from = reinterpret_cast<const float4*>(sm->xfer[half ^ 1][r_blk]);
+          const int col = col0 + q;
+#pragma unroll
+          for (int v = 0; v < 32; v += 16) {
+            if (col + v < p.D) {
+              uint32_t o[8];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float4 x = from[v / 4 + k];
+                o[2 * k] = pack_2x16<kBf16>((__uint_as_float(keep[v + 4 * k]) + x.x) * scale,
+                                            (__uint_as_float(keep[v + 4 * k + 1]) + x.y) * scale);
+                o[2 * k + 1] = pack_2x16<kBf16>((__uint_as_float(keep[v + 4 * k + 2]) + x.z) * scale,
+                                                (__uint_as_float(keep[v + 4 * k + 3]) + x.w) * scale);
+              }
+              // 16 columns go out as one whole sector when the rows start on such boundaries
+              if (p.wide_stores) {
+                st_global_v8(dst + col + v, o);
+              } else {
+                reinterpret_cast<uint4*>(dst + col + v)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                reinterpret_cast<uint4*>(dst + col + v)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+              }
             }
           }
-        } else {
-          if constexpr (kDKDV) {
-#pragma unroll
-            for (int h2 = 0; h2 < 2; ++h2) {
-              tmem_ld_32x32b_x32(tm_second + 32 * h2, own);
-              tc_wait_ld();
-#pragma unroll
-              for (int c = 0; c < 32; ++c) sm->xfer[2][32 * h2 + c][r_blk] = __uint_as_float(own[c]);
-            }
-          }
-          tmem_ld_32x32b_x32(tm_first, own);
-          tc_wait_ld();
         }
-        if (half == 1) {
-          // everything of these lanes is out of tensor memory
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sm->acc_free));
-        }
+        // xfer may be overwritten now; all four warps leave together on a give-up
+        any_failed = named_barrier_or(2, 128, !ok);
+        if (any_failed) break;
       }
-      named_barrier_sync(2, 128);
-      if (ok) {
-        if (half == 0) {
-          store_cols32<kBf16>(out_first, off, own, &sm->xfer[0][0][r_blk], scale_first, wide);
-          tmem_ld_32x32b_x32(tm_first + 32, own);
-          tc_wait_ld();
-          // the accumulators are out of tensor memory: the next block may start accumulating
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sm->acc_free));
-          store_cols32<kBf16>(out_first, off + 32, own, &sm->xfer[0][32][r_blk], scale_first, wide);
-        } else if constexpr (kDKDV) {
-#pragma unroll
-          for (int h2 = 0; h2 < 2; ++h2) {
-#pragma unroll
-            for (int c = 0; c < 32; ++c) own[c] = __float_as_uint(sm->xfer[2][32 * h2 + c][r_blk]);
-            store_cols32<kBf16>(p.out1, off + 32 * h2, own, &sm->xfer[1][32 * h2][r_blk],
-                                p.sm_scale, wide);
-          }
-        }
-      }
-      // xfer may be overwritten by the next block now; all four warps leave together on a give-up
-      if (named_barrier_or(2, 128, !ok)) break;
+      if (any_failed) break;
     }
     if (!ok) bwd_give_up(sm, p.status, 3);
+  } else {
+    give_registers<56>();
+    if (warp == kX2Warp) bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, 1, lane, abort_flag);
   }
 
   tc_fence_before();
@@ -693,14 +748,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   }
 }
 
+struct BwdOperand {
+  const void* p;
+  const int64_t* strides;
+};
+
+// q, k, v, dO and the one or two outputs with strides of their own; out0 = dV (dK/dV only), out1 = dK
+// or dQ.
 template <bool kDKDV>
-static int launch_bwd(const void* q, const void* k, const void* v, const void* dout,
-                      const int64_t strides[4], const float* lse2, const float* delta, void* out0,
-                      void* out1, const int32_t* list_ptr, const int32_t* list_idx,
-                      int list_b_stride, int list_h_stride, float sm_scale, int dtype, int B, int H,
-                      int N, int D, const uint8_t* dense, const int64_t* dense_strides,
-                      int32_t* ticket, int32_t* status, void* stream) {
-  if (B <= 0 || H <= 0 || N <= 0 || (N % kBlock) != 0 || D != kHeadDim) return BSA_ERR_BAD_SHAPE;
+static int launch_bwd(BwdOperand q, BwdOperand k, BwdOperand v, BwdOperand dout, const float* lse2,
+                      const float* delta, BwdOperand out0, BwdOperand out1, const int32_t* list_ptr,
+                      const int32_t* list_idx, int list_places, int list_b_stride, int list_h_stride,
+                      float sm_scale, int dtype, int B, int H, int N, int D, const uint8_t* dense,
+                      const int64_t* dense_strides, int32_t* ticket, int32_t* status, void* stream) {
+  if (B <= 0 || H <= 0 || N <= 0 || (N % kBlock) != 0 || !head_dim_ok(D)) return BSA_ERR_BAD_SHAPE;
   if (dense != nullptr) {
     if (!dense_strides || !is_aligned(dense, 16)) return BSA_ERR_BAD_POINTER;
     if (dense_strides[3] != 1 || dense_strides[2] <= 0 || (dense_strides[2] % 16) != 0 ||
@@ -713,41 +774,43 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   if (!lse2 || !delta || !list_ptr || !list_idx || !is_aligned(lse2, 16) || !is_aligned(delta, 16))
     return BSA_ERR_BAD_POINTER;
   int rc;
-  const void* ops[6] = {q, k, v, dout, out1, kDKDV ? out0 : out1};
-  for (const void* op : ops)
-    if ((rc = check_qkv_operand(op, strides)) != BSA_OK) return rc;
+  if (!kDKDV) out0 = out1;
+  for (const BwdOperand& op : {q, k, v, dout, out0, out1})
+    if ((rc = check_qkv_operand(op.p, op.strides)) != BSA_OK) return rc;
   if ((rc = check_device_sm100()) != BSA_OK) return rc;
   const int nb = N / kBlock;
+  if (list_places != 0 && list_places != nb) return BSA_ERR_BAD_SHAPE;
   if (static_cast<int64_t>(B) * H * nb > 0x7fffffffLL) return BSA_ERR_TOO_LARGE;
 
   // dK/dV: K, V resident; Q, dO streamed.   dQ: Q, dO resident; K, V streamed.
-  const void* stat0 = kDKDV ? k : q;
-  const void* stat1 = kDKDV ? v : dout;
-  const void* str0 = kDKDV ? q : k;
-  const void* str1 = kDKDV ? dout : v;
-  CUtensorMap tm_a0, tm_a1, tm_b0, tm_b1;
-  if ((rc = make_qkv_tmap(&tm_a0, stat0, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
-  if ((rc = make_qkv_tmap(&tm_a1, stat1, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
-  if ((rc = make_qkv_tmap(&tm_b0, str0, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
-  if ((rc = make_qkv_tmap(&tm_b1, str1, strides, B, H, N, D, dtype, 64)) != BSA_OK) return rc;
+  CUtensorMap tm_q, tm_k, tm_v, tm_do;
+  if ((rc = cached_qkv_tmap(&tm_q, q.p, q.strides, B, H, N, D, dtype)) != BSA_OK) return rc;
+  if ((rc = cached_qkv_tmap(&tm_k, k.p, k.strides, B, H, N, D, dtype)) != BSA_OK) return rc;
+  if ((rc = cached_qkv_tmap(&tm_v, v.p, v.strides, B, H, N, D, dtype)) != BSA_OK) return rc;
+  if ((rc = cached_qkv_tmap(&tm_do, dout.p, dout.strides, B, H, N, D, dtype)) != BSA_OK) return rc;
 
   BwdParams prm;
   prm.list_ptr = list_ptr;
   prm.list_idx = list_idx;
+  prm.list_places = list_places;
   prm.dense = dense;
   prm.ds0 = dense ? dense_strides[0] : 0;
   prm.ds1 = dense ? dense_strides[1] : 0;
   prm.ds2 = dense ? dense_strides[2] : 0;
   prm.lse2 = lse2;
   prm.delta = delta;
-  prm.out0 = out0;
-  prm.out1 = out1;
-  prm.sb = strides[0];
-  prm.sh = strides[1];
-  prm.sn = strides[2];
+  prm.out0 = const_cast<void*>(out0.p);
+  prm.out1 = const_cast<void*>(out1.p);
+  prm.sb0 = out0.strides[0];
+  prm.sh0 = out0.strides[1];
+  prm.sn0 = out0.strides[2];
+  prm.sb1 = out1.strides[0];
+  prm.sh1 = out1.strides[1];
+  prm.sn1 = out1.strides[2];
   prm.B = B;
   prm.H = H;
   prm.N = N;
+  prm.D = D;
   prm.nb = nb;
   prm.items = B * H * nb;
   prm.list_b_stride = list_b_stride;
@@ -757,10 +820,12 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   prm.status = status;
   prm.ticket = ticket;
   {
-    // a thread's 16 output columns are one 32-byte sector when every row starts on such a boundary
-    const uintptr_t bits = reinterpret_cast<uintptr_t>(out0) | reinterpret_cast<uintptr_t>(out1);
-    const int64_t sbits = (strides[0] | strides[1] | strides[2]) * 2;
-    prm.wide_stores = ((bits | static_cast<uintptr_t>(sbits)) & 31u) == 0 ? 1 : 0;
+    // 16 output columns are one 32-byte sector when every row starts on such a boundary
+    uintptr_t bits = 0;
+    for (const BwdOperand& op : {out0, out1})
+      bits |= reinterpret_cast<uintptr_t>(op.p) |
+              static_cast<uintptr_t>((op.strides[0] | op.strides[1] | op.strides[2]) * 2);
+    prm.wide_stores = (bits & 31u) == 0 ? 1 : 0;
   }
 
   const size_t smem_bytes = sizeof(BwdSmem) + 1024;
@@ -773,12 +838,27 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   int sms = 0;
   if ((rc = sm_count(&sms)) != BSA_OK) return rc;
   const dim3 grid(static_cast<unsigned>(prm.items < sms ? prm.items : sms));  // one CTA per SM
-  kern<<<grid, kBwdThreads, smem_bytes, static_cast<cudaStream_t>(stream)>>>(tm_a0, tm_a1, tm_b0,
-                                                                             tm_b1, prm);
+  kern<<<grid, kBwdThreads, smem_bytes, static_cast<cudaStream_t>(stream)>>>(
+      kDKDV ? tm_k : tm_q, kDKDV ? tm_v : tm_do, kDKDV ? tm_q : tm_k, kDKDV ? tm_do : tm_v, prm);
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 
 }  // namespace bsa
+
+extern "C" int bsa_attn_bwd_dkdv_strided(
+    const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4],
+    const void* v, const int64_t v_strides[4], const void* dout, const int64_t do_strides[4],
+    const float* lse2, const float* delta, void* dk, const int64_t dk_strides[4], void* dv,
+    const int64_t dv_strides[4], const int32_t* col_ptr, const int32_t* row_idx, int list_places,
+    int list_b_stride, int list_h_stride, float sm_scale, int dtype, int B, int H, int N, int D, const uint8_t* dense,
+    const int64_t dense_strides[4], int32_t* work_counter, int32_t* status, void* stream) {
+  if (!q_strides || !k_strides || !v_strides || !do_strides || !dk_strides || !dv_strides)
+    return BSA_ERR_BAD_POINTER;
+  return bsa::launch_bwd<true>({q, q_strides}, {k, k_strides}, {v, v_strides}, {dout, do_strides},
+                               lse2, delta, {dv, dv_strides}, {dk, dk_strides}, col_ptr, row_idx,
+                               list_places, list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D, dense,
+                               dense_strides, work_counter, status, stream);
+}
 
 extern "C" int bsa_attn_bwd_dkdv(const void* q, const void* k, const void* v, const void* dout,
                                  const int64_t strides[4], const float* lse2, const float* delta,
@@ -787,9 +867,24 @@ extern "C" int bsa_attn_bwd_dkdv(const void* q, const void* k, const void* v, co
                                  float sm_scale, int dtype, int B, int H, int N, int D,
                                  const uint8_t* dense, const int64_t dense_strides[4],
                                  int32_t* work_counter, int32_t* status, void* stream) {
-  return bsa::launch_bwd<true>(q, k, v, dout, strides, lse2, delta, dv, dk, col_ptr, row_idx,
-                               list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D, dense,
-                               dense_strides, work_counter, status, stream);
+  return bsa_attn_bwd_dkdv_strided(q, strides, k, strides, v, strides, dout, strides, lse2, delta, dk,
+                                   strides, dv, strides, col_ptr, row_idx, 0, list_b_stride,
+                                   list_h_stride, sm_scale, dtype, B, H, N, D, dense, dense_strides,
+                                   work_counter, status, stream);
+}
+
+extern "C" int bsa_attn_bwd_dq_strided(
+    const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4],
+    const void* v, const int64_t v_strides[4], const void* dout, const int64_t do_strides[4],
+    const float* lse2, const float* delta, void* dq, const int64_t dq_strides[4],
+    const int32_t* row_ptr, const int32_t* col_idx, int list_places, int list_b_stride, int list_h_stride,
+    float sm_scale, int dtype, int B, int H, int N, int D, const uint8_t* dense,
+    const int64_t dense_strides[4], int32_t* work_counter, int32_t* status, void* stream) {
+  if (!q_strides || !k_strides || !v_strides || !do_strides || !dq_strides) return BSA_ERR_BAD_POINTER;
+  return bsa::launch_bwd<false>({q, q_strides}, {k, k_strides}, {v, v_strides}, {dout, do_strides},
+                                lse2, delta, {nullptr, nullptr}, {dq, dq_strides}, row_ptr, col_idx,
+                                list_places, list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D, dense,
+                                dense_strides, work_counter, status, stream);
 }
 
 extern "C" int bsa_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dout,
@@ -799,7 +894,7 @@ extern "C" int bsa_attn_bwd_dq(const void* q, const void* k, const void* v, cons
                                int B, int H, int N, int D, const uint8_t* dense,
                                const int64_t dense_strides[4], int32_t* work_counter,
                                int32_t* status, void* stream) {
-  return bsa::launch_bwd<false>(q, k, v, dout, strides, lse2, delta, nullptr, dq, row_ptr,
-                                col_idx, list_b_stride, list_h_stride, sm_scale, dtype, B, H, N,
-                                D, dense, dense_strides, work_counter, status, stream);
+  return bsa_attn_bwd_dq_strided(q, strides, k, strides, v, strides, dout, strides, lse2, delta, dq,
+                                 strides, row_ptr, col_idx, 0, list_b_stride, list_h_stride, sm_scale,
+                                 dtype, B, H, N, D, dense, dense_strides, work_counter, status, stream);
 }

@@ -69,7 +69,6 @@
 // barrier is waited on only by warps that see each of its phases, or that know the barrier to be
 // at most one phase behind (a parity wait cannot tell a phase from the one two before it).
 #include <math.h>
-#include <string.h>
 
 #include "host_common.h"
 #include "sm100_ptx.cuh"
@@ -1014,48 +1013,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem, kFwdTmemCols);
   }
-}
-
-// Tensor maps of recent operands.  Encoding one takes the driver about a microsecond, and a
-// forward call needs three; a model calls the op with the same few buffers over and over.
-struct TmapKey {
-  const void* base;
-  int64_t s[4];
-  int B, H, N, D, dtype;
-};
-struct TmapEntry {
-  TmapKey key;
-  CUtensorMap map;
-  bool valid;
-};
-
-static int cached_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B, int H,
-                           int N, int D, int dtype) {
-  constexpr int kEntries = 12;
-  static thread_local TmapEntry cache[kEntries];
-  static thread_local int next = 0;
-  TmapKey key;
-  memset(&key, 0, sizeof(key));
-  key.base = base;
-  for (int i = 0; i < 4; ++i) key.s[i] = s[i];
-  key.B = B;
-  key.H = H;
-  key.N = N;
-  key.D = D;
-  key.dtype = dtype;
-  for (int i = 0; i < kEntries; ++i)
-    if (cache[i].valid && memcmp(&cache[i].key, &key, sizeof(key)) == 0) {
-      *out = cache[i].map;
-      return BSA_OK;
-    }
-  const int rc = make_qkv_tmap(out, base, s, B, H, N, D, dtype, 64);
-  if (rc != BSA_OK) return rc;
-  TmapEntry& e = cache[next];
-  next = (next + 1) % kEntries;
-  e.key = key;
-  e.map = *out;
-  e.valid = true;
-  return BSA_OK;
 }
 
 static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,

@@ -37,29 +37,34 @@ __device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {
   return acc;
 }
 
-template <bool kBf16>
+// A row of D elements takes D / 8 lanes, 16 bytes each; four rows of a lane are in flight.  O and dO have
+// strides of their own.
+template <bool kBf16, int kD>
 __global__ void __launch_bounds__(kDeltaThreads)
-bwd_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ dout, int64_t sb,
-                 int64_t sh, int64_t sn, float* __restrict__ delta, int H, int N, int64_t rows) {
+bwd_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int64_t o_sn,
+                 const uint16_t* __restrict__ dout, int64_t d_sb, int64_t d_sh, int64_t d_sn,
+                 float* __restrict__ delta, int H, int N, int64_t rows) {
+  constexpr int kLanes = kD / 8, kStep = 32 / kLanes;  // lanes of a row, rows of a warp at a time
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane >> 3, chunk = lane & 7;
-  // A warp's 16 rows lie in one (batch, head): N is a multiple of 64 and the warp starts at a
-  // multiple of 16, so the division is done once per thread, not once per row.
-  const int64_t warp_row = static_cast<int64_t>(blockIdx.x) * kDeltaRowsPerCta + warp * 16;
+  const int sub = lane / kLanes, chunk = lane % kLanes;
+  // A warp's rows (16, 32 or 64) lie in one (batch, head): N is a multiple of 64 and the warp starts at
+  // a multiple of their number, so the division is done once per thread, not once per row.
+  const int64_t warp_row =
+      (static_cast<int64_t>(blockIdx.x) * (kDeltaThreads / 32) + warp) * (4 * kStep);
   const int64_t row0 = warp_row + sub;
   const int64_t bh = warp_row / N;
   const int64_t n0 = warp_row - bh * N + sub;
-  const int64_t b = bh / H;
-  const int64_t base = b * sb + (bh - b * H) * sh + chunk * 8;
+  const int64_t b = bh / H, h = bh - b * H;
+  const uint16_t* po = o + b * o_sb + h * o_sh + chunk * 8;
+  const uint16_t* pd = dout + b * d_sb + h * d_sh + chunk * 8;
   uint4 xo[4], xd[4];
   bool live[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    live[i] = row0 + 4 * i < rows;
+    live[i] = row0 + kStep * i < rows;
     if (live[i]) {
-      const int64_t off = base + (n0 + 4 * i) * sn;
-      xo[i] = __ldg(reinterpret_cast<const uint4*>(o + off));
-      xd[i] = __ldg(reinterpret_cast<const uint4*>(dout + off));
+      xo[i] = __ldg(reinterpret_cast<const uint4*>(po + (n0 + kStep * i) * o_sn));
+      xd[i] = __ldg(reinterpret_cast<const uint4*>(pd + (n0 + kStep * i) * d_sn));
     } else {
       xo[i] = make_uint4(0, 0, 0, 0);
       xd[i] = make_uint4(0, 0, 0, 0);
@@ -68,11 +73,21 @@ bwd_delta_kernel(const uint16_t* __restrict__ o, const uint16_t* __restrict__ do
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float acc = dot8<kBf16>(xo[i], xd[i]);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-    if (chunk == 0 && live[i]) delta[row0 + 4 * i] = acc;
+#pragma unroll
+    for (int x = 1; x < kLanes; x *= 2) acc += __shfl_xor_sync(0xffffffffu, acc, x);
+    if (chunk == 0 && live[i]) delta[row0 + kStep * i] = acc;
   }
+}
+
+template <int kD>
+static void launch_delta(bool bf16, const void* o, const int64_t* os, const void* dout, const int64_t* ds,
+                         float* delta, int H, int N, int64_t rows, cudaStream_t stream) {
+  constexpr int64_t kRows = kDeltaThreads / 32 * 4 * (32 / (kD / 8));  // of a CTA
+  const unsigned blocks = static_cast<unsigned>((rows + kRows - 1) / kRows);
+  auto kern = bf16 ? bwd_delta_kernel<true, kD> : bwd_delta_kernel<false, kD>;
+  kern<<<blocks, kDeltaThreads, 0, stream>>>(static_cast<const uint16_t*>(o), os[0], os[1], os[2],
+                                             static_cast<const uint16_t*>(dout), ds[0], ds[1], ds[2],
+                                             delta, H, N, rows);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -207,28 +222,29 @@ static int launch_reorder(const void* in, const int64_t s[4], void* out, const i
 
 }  // namespace bsa
 
+extern "C" int bsa_attn_bwd_delta_strided(const void* o, const int64_t o_strides[4], const void* dout,
+                                          const int64_t do_strides[4], float* delta, int dtype, int B,
+                                          int H, int N, int D, void* stream) {
+  using namespace bsa;
+  if (B <= 0 || H <= 0 || N <= 0 || !head_dim_ok(D)) return BSA_ERR_BAD_SHAPE;
+  if (dtype != BSA_F16 && dtype != BSA_BF16) return BSA_ERR_BAD_DTYPE;
+  if (!delta || !o_strides || !do_strides) return BSA_ERR_BAD_POINTER;
+  int rc;
+  if ((rc = check_qkv_operand(o, o_strides)) != BSA_OK) return rc;
+  if ((rc = check_qkv_operand(dout, do_strides)) != BSA_OK) return rc;
+  const int64_t rows = static_cast<int64_t>(B) * H * N;
+  if (rows / 128 >= 0x7fffffffLL) return BSA_ERR_TOO_LARGE;
+  const bool bf16 = dtype == BSA_BF16;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (D == 64) launch_delta<64>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
+  else if (D == 32) launch_delta<32>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
+  else launch_delta<16>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
+  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
+
 extern "C" int bsa_attn_bwd_delta(const void* o, const void* dout, const int64_t s[4], float* delta,
                                   int dtype, int B, int H, int N, int D, void* stream) {
-  using namespace bsa;
-  if (B <= 0 || H <= 0 || N <= 0 || D != kHeadDim) return BSA_ERR_BAD_SHAPE;
-  if (dtype != BSA_F16 && dtype != BSA_BF16) return BSA_ERR_BAD_DTYPE;
-  if (!delta) return BSA_ERR_BAD_POINTER;
-  int rc;
-  if ((rc = check_qkv_operand(o, s)) != BSA_OK) return rc;
-  if ((rc = check_qkv_operand(dout, s)) != BSA_OK) return rc;
-  const int64_t rows = static_cast<int64_t>(B) * H * N;
-  const int64_t blocks = (rows + kDeltaRowsPerCta - 1) / kDeltaRowsPerCta;
-  if (blocks > 0x7fffffffLL) return BSA_ERR_TOO_LARGE;
-  cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  const uint16_t* po = static_cast<const uint16_t*>(o);
-  const uint16_t* pd = static_cast<const uint16_t*>(dout);
-  if (dtype == BSA_BF16)
-    bwd_delta_kernel<true><<<static_cast<unsigned>(blocks), kDeltaThreads, 0, cs>>>(
-        po, pd, s[0], s[1], s[2], delta, H, N, rows);
-  else
-    bwd_delta_kernel<false><<<static_cast<unsigned>(blocks), kDeltaThreads, 0, cs>>>(
-        po, pd, s[0], s[1], s[2], delta, H, N, rows);
-  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+  return bsa_attn_bwd_delta_strided(o, s, dout, s, delta, dtype, B, H, N, D, stream);
 }
 
 extern "C" int bsa_reorder(const void* in, void* out, const int64_t strides[4],

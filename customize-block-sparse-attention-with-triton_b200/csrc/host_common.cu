@@ -110,6 +110,39 @@ int make_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B,
   return r == CUDA_SUCCESS ? BSA_OK : BSA_ERR_CUDA;
 }
 
+int cached_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B, int H, int N, int D,
+                    int dtype) {
+  struct Entry {
+    const void* base;  // nullptr: empty
+    int64_t s[3];
+    int B, H, N, D, dtype;
+    CUtensorMap map;
+  };
+  constexpr int kEntries = 32;
+  static thread_local Entry cache[kEntries];
+  static thread_local int next = 0;
+  for (const Entry& e : cache)
+    if (e.base == base && e.s[0] == s[0] && e.s[1] == s[1] && e.s[2] == s[2] && e.N == N && e.H == H &&
+        e.B == B && e.D == D && e.dtype == dtype) {
+      *out = e.map;
+      return BSA_OK;
+    }
+  Entry& e = cache[next];
+  e.base = nullptr;
+  const int rc = make_qkv_tmap(&e.map, base, s, B, H, N, D, dtype, 64);
+  if (rc != BSA_OK) return rc;
+  next = (next + 1) % kEntries;
+  e.base = base;
+  for (int i = 0; i < 3; ++i) e.s[i] = s[i];
+  e.B = B;
+  e.H = H;
+  e.N = N;
+  e.D = D;
+  e.dtype = dtype;
+  *out = e.map;
+  return BSA_OK;
+}
+
 }  // namespace bsa
 
 extern "C" int bsa_version(void) { return BSA_VERSION; }

@@ -29,6 +29,12 @@ int check_qkv_operand(const void* p, const int64_t s[4]);
 int make_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B, int H, int N,
                   int D, int dtype, int box_rows);
 
+// The same with 64-row boxes out of a small per-thread cache of recent operands: encoding a map takes
+// the driver about a microsecond, a forward and backward need seven, and a model calls the op with the
+// same few buffers over and over.
+int cached_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int B, int H, int N, int D,
+                    int dtype);
+
 // Number of SMs of the current device (cached per device).
 int sm_count(int* out);
 

@@ -40,6 +40,7 @@ SIGNATURES = {
     "bsa_mask_reduce": [_vp, _s4, _i, _i, _i, _vp, _vp, _i, _vp],
     "bsa_tile_list_sizes": [_i, _i, _i, ctypes.POINTER(ListSizes)],
     "bsa_tile_lists_build": [_vp, _s4, _i, _i, _i] + [_vp] * 6 + [_vp],
+    "bsa_tile_lists_places": [_vp, _s4, _i, _i, _i] + [_vp] * 4 + [_vp],
     "bsa_attn_fwd": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _vp, _i, _i, _f, _i,
                      _i, _i, _i, _i, _vp, _vp, _vp],
     "bsa_attn_fwd_block_mask": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _s4, _i, _i,
@@ -53,6 +54,11 @@ SIGNATURES = {
                           _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
     "bsa_attn_bwd_dq": [_vp, _vp, _vp, _vp, _s4, _vp, _vp, _vp, _vp, _vp, _i, _i, _f, _i,
                         _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
+    "bsa_attn_bwd_delta_strided": [_vp, _s4, _vp, _s4, _vp, _i, _i, _i, _i, _i, _vp],
+    "bsa_attn_bwd_dkdv_strided": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _s4, _vp, _s4,
+                                  _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
+    "bsa_attn_bwd_dq_strided": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _s4,
+                                _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
     "bsa_reorder": [_vp, _vp, _s4, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_inv_reorder": [_vp, _vp, _s4, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_reorder_strided": [_vp, _s4, _vp, _s4, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
@@ -81,6 +87,25 @@ def load():
         fn.restype = ctypes.c_char_p if name == "bsa_strerror" else ctypes.c_int
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The native host path (csrc/native.cpp), loaded once; raises if it has not been built."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise ImportError(f"the native host path cannot be loaded ({e}): build it with `python "
+                              "build.py` in the package directory; there is no fallback path") from e
+        from .fa2_custom_mask import _raise_native
+        module.set_raise(_raise_native)
+        _native = module
+    return _native
 
 
 def check(fn: str, status: int):

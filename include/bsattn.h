@@ -106,6 +106,15 @@ int bsa_tile_lists_build(const uint8_t* block, const int64_t block_strides[4], i
                          int32_t* groups, int32_t* meta, void* stream);
 
 /*
+ * Row and column lists with places instead of offsets, in one launch: list u (of Bm*Hm*nb) has its
+ * row_cnt[u] entries at col_idx[u*nb ...], and col_cnt[u] at row_idx[u*nb ...].  The backward entry
+ * points take them with list_places = nb.
+ */
+int bsa_tile_lists_places(const uint8_t* block, const int64_t block_strides[4], int Bm, int Hm, int nb,
+                          int32_t* row_cnt, int32_t* col_idx, int32_t* col_cnt, int32_t* row_idx,
+                          void* stream);
+
+/*
  * Forward attention over the listed tiles; replaces the _attn_fwd launch
  * (fa2_custom_mask/fa2_custom_mask.py:77-87, kernel fa2_custom_mask/fa2_fwd.py:108-206).
  *   q,k,v,o : [B,H,N,64] fp16/bf16, element strides *_strides[4]; last stride 1, others multiples
@@ -197,6 +206,11 @@ int bsa_attn_fwd_block_mask_rows(const void* q, const int64_t q_strides[4], cons
 int bsa_attn_bwd_delta(const void* o, const void* dout, const int64_t o_strides[4], float* delta,
                        int dtype, int B, int H, int N, int D, void* stream);
 
+/* The same with strides of their own for o and dout. */
+int bsa_attn_bwd_delta_strided(const void* o, const int64_t o_strides[4], const void* dout,
+                               const int64_t do_strides[4], float* delta, int dtype, int B, int H,
+                               int N, int D, void* stream);
+
 /*
  * dK and dV; replaces _attn_bwd_dkdv
  * (fa2_custom_mask/fa2_bwd.py:23-81, driven from fa2_custom_mask/fa2_bwd.py:199-234).
@@ -215,6 +229,20 @@ int bsa_attn_bwd_dkdv(const void* q, const void* k, const void* v, const void* d
                       int N, int D, const uint8_t* dense, const int64_t dense_strides[4],
                       int32_t* work_counter, int32_t* status, void* stream);
 
+/* The same with strides of their own for every operand: q, k, v, dout, dk, dv [B,H,N,D], each with a
+ * unit innermost stride and 16-byte-aligned base and outer strides.  list_places = 0: lists of
+ * bsa_tile_lists_build; nb: counts and entries of bsa_tile_lists_places. */
+int bsa_attn_bwd_dkdv_strided(const void* q, const int64_t q_strides[4], const void* k,
+                              const int64_t k_strides[4], const void* v,
+                              const int64_t v_strides[4], const void* dout,
+                              const int64_t do_strides[4], const float* lse2, const float* delta,
+                              void* dk, const int64_t dk_strides[4], void* dv,
+                              const int64_t dv_strides[4], const int32_t* col_ptr,
+                              const int32_t* row_idx, int list_places, int list_b_stride,
+                              int list_h_stride, float sm_scale, int dtype, int B, int H, int N, int D,
+                              const uint8_t* dense, const int64_t dense_strides[4],
+                              int32_t* work_counter, int32_t* status, void* stream);
+
 /*
  * dQ over the row lists (row_ptr/col_idx, as in bsa_attn_fwd); replaces _attn_bwd_dq
  * (fa2_custom_mask/fa2_bwd.py:85-137, driven from fa2_custom_mask/fa2_bwd.py:237-285).
@@ -225,6 +253,16 @@ int bsa_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dou
                     int list_h_stride, float sm_scale, int dtype, int B, int H, int N, int D,
                     const uint8_t* dense, const int64_t dense_strides[4], int32_t* work_counter,
                     int32_t* status, void* stream);
+
+/* The same with strides of their own for every operand (see bsa_attn_bwd_dkdv_strided). */
+int bsa_attn_bwd_dq_strided(const void* q, const int64_t q_strides[4], const void* k,
+                            const int64_t k_strides[4], const void* v, const int64_t v_strides[4],
+                            const void* dout, const int64_t do_strides[4], const float* lse2,
+                            const float* delta, void* dq, const int64_t dq_strides[4],
+                            const int32_t* row_ptr, const int32_t* col_idx, int list_places,
+                            int list_b_stride, int list_h_stride, float sm_scale, int dtype, int B, int H, int N,
+                            int D, const uint8_t* dense, const int64_t dense_strides[4],
+                            int32_t* work_counter, int32_t* status, void* stream);
 
 /*
  * Head-wise token reorder; replaces reorder_kernel (fa2_custom_mask/permute.py:5-58, launched from
