@@ -1,0 +1,290 @@
+// Native host path of the public op: checks, workspaces, launches and the autograd node in C++, so that
+// a call costs a few microseconds of host time instead of forty (the kernels of a short sequence take
+// less than ten).  Everything on the device is done by the C-ABI library (include/bsattn.h); this file
+// only knows torch tensors.
+//
+// A call that is out of the ordinary in any way (wrong types or shapes, no mask, a library call that
+// refuses) is answered with None, and the Python layer takes it, which also raises the errors.
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/extension.h>
+
+#include <mutex>
+#include <unordered_map>
+
+#include "../../include/bsattn.h"
+
+namespace {
+
+using at::Tensor;
+constexpr int64_t kBlock = 64;
+
+// ---------------------------------------------------------------------------------------------
+// Per (device, stream): the zeroed work counter of the persistent kernels (they leave it at zero, also
+// after a bounded wait gave up), and a status word in pinned host memory, which the device can write
+// and the host can read without a synchronisation.
+// ---------------------------------------------------------------------------------------------
+struct StreamState {
+  Tensor counter, status;
+  int32_t* counter_ptr;
+  volatile int32_t* word;
+};
+
+struct StreamKey {
+  int device;
+  cudaStream_t stream;
+  bool operator==(const StreamKey& o) const { return device == o.device && stream == o.stream; }
+};
+struct StreamHash {
+  size_t operator()(const StreamKey& k) const {
+    return std::hash<void*>()(k.stream) * 31u + static_cast<size_t>(k.device);
+  }
+};
+
+// nullptr: the stream is being captured and has no state yet (nothing is allocated inside a capture:
+// fixed-stride hand-out, no report).  `device` is the current device.
+StreamState* stream_state(int device, cudaStream_t stream) {
+  thread_local StreamKey last_key{-1, nullptr};
+  thread_local StreamState* last = nullptr;
+  const StreamKey key{device, stream};
+  if (last != nullptr && last_key == key) return last;
+  static std::mutex mutex;
+  static auto* states = new std::unordered_map<StreamKey, StreamState*, StreamHash>();  // never torn down
+  std::lock_guard<std::mutex> lock(mutex);
+  auto it = states->find(key);
+  if (it == states->end()) {
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
+    auto* st = new StreamState;
+    // zeroed on the stream that will use it, so no cross-stream ordering is needed
+    st->counter = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+    st->status = at::zeros({1}, at::TensorOptions().dtype(at::kInt)).pin_memory();
+    st->counter_ptr = st->counter.data_ptr<int32_t>();
+    st->word = st->status.data_ptr<int32_t>();
+    it = states->emplace(key, st).first;
+  }
+  last_key = key;
+  return last = it->second;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Arguments
+// ---------------------------------------------------------------------------------------------
+// TMA needs a unit inner stride, 16-byte aligned base and outer strides.
+Tensor tma_ready(const Tensor& t) {
+  bool ok = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.const_data_ptr()) % 16 == 0;
+  for (int i = 0; ok && i < 3; ++i) ok = t.stride(i) > 0 && t.stride(i) % 8 == 0;
+  return ok ? t : t.contiguous();
+}
+
+struct Mask {
+  Tensor block;         // bytes [Bm,Hm,nb,nb]
+  Tensor dense;         // bytes [Bm,Hm,N,N], or undefined
+  int64_t dense_strides[4];
+  const uint8_t* dense_ptr = nullptr;
+};
+
+// The op's mask argument as 4-D bytes; false when it is nothing that this path takes.
+bool read_mask(const Tensor& mask, int64_t B, int64_t H, int64_t N, const Tensor& q, void* stream, Mask* out) {
+  const int64_t dims = mask.dim(), nb = N / kBlock;
+  if (dims < 2 || dims > 4 || mask.device() != q.device()) return false;
+  if (mask.scalar_type() != at::kBool && mask.scalar_type() != at::kByte) return false;
+  Tensor m = mask.scalar_type() == at::kBool ? mask.view(at::kByte) : mask;
+  while (m.dim() < 4) m = m.unsqueeze(0);
+  if ((m.size(0) != 1 && m.size(0) != B) || (m.size(1) != 1 && m.size(1) != H)) return false;
+  if (m.size(2) == nb && m.size(3) == nb) {
+    out->block = m;
+    return true;
+  }
+  if (m.size(2) != N || m.size(3) != N) return false;
+  // a dense mask: reduced to blocks, the partly kept ones marked 2, and applied inside those
+  bool ok = m.stride(3) == 1 && reinterpret_cast<uintptr_t>(m.const_data_ptr()) % 16 == 0;
+  for (int i = 0; ok && i < 3; ++i) ok = m.stride(i) % 16 == 0;
+  out->dense = ok ? m : m.contiguous();
+  out->block = at::empty({m.size(0), m.size(1), nb, nb}, m.options());
+  out->dense_ptr = out->dense.const_data_ptr<uint8_t>();
+  for (int i = 0; i < 4; ++i) out->dense_strides[i] = out->dense.stride(i);
+  if (bsa_mask_reduce(out->dense_ptr, out->dense_strides, m.size(0), m.size(1), N,
+                      out->block.mutable_data_ptr<uint8_t>(), nullptr, 1, stream) != 0)
+    return false;
+  for (int i = 0; i < 2; ++i)
+    if (m.size(i) == 1) out->dense_strides[i] = 0;  // broadcast
+  return true;
+}
+
+int dtype_code(const Tensor& t) { return t.scalar_type() == at::kHalf ? BSA_F16 : BSA_BF16; }
+
+// Runs the forward; false when the library refused.
+bool run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& m, double scale,
+                 StreamState* state, void* stream, Tensor* o, Tensor* lse2) {
+  const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
+  *o = at::empty({B, H, N, D}, q.options());
+  *lse2 = at::empty({B, H, N}, q.options().dtype(at::kFloat));
+  return bsa_attn_fwd_block_mask_rows(
+             q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
+             v.const_data_ptr(), v.strides().data(), o->mutable_data_ptr(), o->strides().data(),
+             lse2->mutable_data_ptr<float>(), nullptr, m.block.const_data_ptr<uint8_t>(),
+             m.block.strides().data(), m.block.size(0), m.block.size(1), static_cast<float>(scale),
+             dtype_code(q), B, H, N, D, 0, N / kBlock, m.dense_ptr,
+             m.dense_ptr ? m.dense_strides : nullptr, state ? state->counter_ptr : nullptr,
+             state ? const_cast<int32_t*>(state->word) : nullptr, stream) == 0;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Errors of the backward: raised by the Python layer's function (fn, status), on whatever thread
+// ---------------------------------------------------------------------------------------------
+PyObject* raise_error = nullptr;
+
+[[noreturn]] void raise_in_python(const char* fn, int status) {
+  pybind11::gil_scoped_acquire gil;
+  PyObject* r = PyObject_CallFunction(raise_error, "si", fn, status);
+  Py_XDECREF(r);  // (it always raises)
+  python_error err;
+  err.persist();
+  throw err;
+}
+void check(const char* fn, int rc) {
+  if (rc != 0) raise_in_python(fn, rc);
+}
+
+// ---------------------------------------------------------------------------------------------
+// Autograd
+// ---------------------------------------------------------------------------------------------
+struct Refused {};  // the forward cannot be done here
+
+// The tile lists of one call in one buffer of words: counts of the row and column lists, then their
+// entries, every list in a place of nb words.
+struct Lists {
+  int64_t col_cnt, col_idx, row_idx, words;
+  Lists(int64_t Bm, int64_t Hm, int64_t nb) {
+    const int64_t rows = Bm * Hm * nb;
+    col_cnt = rows;
+    col_idx = (2 * rows + 3) & ~int64_t{3};
+    row_idx = col_idx + rows * nb;
+    words = row_idx + rows * nb;
+  }
+};
+
+struct Attention : torch::autograd::Function<Attention> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q0, const Tensor& k0,
+                        const Tensor& v0, const Mask* m, double scale, StreamState* state, void* stream) {
+    const Tensor q = tma_ready(q0), k = tma_ready(k0), v = tma_ready(v0);
+    Tensor o, lse2;
+    if (!run_forward(q, k, v, *m, scale, state, stream, &o, &lse2)) throw Refused();
+    // the forward lists each mask row inside the kernel; only the backward needs lists as data
+    const int64_t Bm = m->block.size(0), Hm = m->block.size(1), nb = m->block.size(2);
+    const Lists at(Bm, Hm, nb);
+    Tensor lists = at::empty({at.words}, q.options().dtype(at::kInt));
+    int32_t* p = lists.mutable_data_ptr<int32_t>();
+    if (bsa_tile_lists_places(m->block.const_data_ptr<uint8_t>(), m->block.strides().data(), Bm, Hm, nb, p,
+                              p + at.col_idx, p + at.col_cnt, p + at.row_idx, stream) != 0)
+      throw Refused();
+    ctx->save_for_backward({q0, k0, v0, o});
+    ctx->saved_data["lse2"] = lse2;
+    ctx->saved_data["lists"] = lists;
+    // the caller's mask (or an aligned copy of it): not to be changed before backward
+    if (m->dense.defined()) ctx->saved_data["dense"] = m->dense;
+    ctx->saved_data["mask"] = std::vector<int64_t>{Bm, Hm, nb};
+    ctx->saved_data["scale"] = scale;
+    return o;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor q = tma_ready(saved[0]), k = tma_ready(saved[1]), v = tma_ready(saved[2]), &o = saved[3];
+    const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
+    const Tensor dout = tma_ready(grads[0].defined() ? grads[0].to(q.scalar_type()) : at::zeros_like(o));
+    const Tensor lse2 = ctx->saved_data["lse2"].toTensor(), lists = ctx->saved_data["lists"].toTensor();
+    const auto shape = ctx->saved_data["mask"].toIntVector();
+    const int64_t Bm = shape[0], Hm = shape[1];
+    const Lists at(Bm, Hm, shape[2]);
+    const float scale = static_cast<float>(ctx->saved_data["scale"].toDouble());
+    const uint8_t* dense = nullptr;
+    int64_t strides[4] = {0, 0, 0, 0};
+    const auto dense_it = ctx->saved_data.find("dense");
+    if (dense_it != ctx->saved_data.end()) {
+      const Tensor t = dense_it->second.toTensor();
+      dense = t.const_data_ptr<uint8_t>();
+      for (int i = 0; i < 4; ++i) strides[i] = i < 2 && t.size(i) == 1 ? 0 : t.stride(i);
+    }
+    const int64_t* dense_strides = dense ? strides : nullptr;
+    const c10::cuda::CUDAGuard guard(q.device());
+    const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
+    StreamState* state = stream_state(q.device().index(), stream);
+    if (state != nullptr && *state->word != 0) raise_in_python("flash_attention_custom_mask", -9);
+    int32_t* counter = state ? state->counter_ptr : nullptr;
+    int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
+    // the gradients are laid out like the tensors they belong to, gaps included
+    const auto like = [](const Tensor& t) { return at::empty_strided(t.sizes(), t.strides(), t.options()); };
+    Tensor dq = like(q), dk = like(k), dv = like(v);
+    const Tensor delta = at::empty({B, H, N}, lse2.options());
+    const float* lse_p = lse2.const_data_ptr<float>();
+    float* delta_p = delta.mutable_data_ptr<float>();
+    const int32_t* p = lists.const_data_ptr<int32_t>();
+    const int code = dtype_code(q), sb = Bm > 1 ? Hm : 0, sh = Hm > 1 ? 1 : 0;
+    check("bsa_attn_bwd_delta_strided",
+          bsa_attn_bwd_delta_strided(o.const_data_ptr(), o.strides().data(), dout.const_data_ptr(),
+                                     dout.strides().data(), delta_p, code, B, H, N, D, stream));
+    check("bsa_attn_bwd_dkdv_strided",
+          bsa_attn_bwd_dkdv_strided(
+              q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
+              v.const_data_ptr(), v.strides().data(), dout.const_data_ptr(), dout.strides().data(), lse_p,
+              delta_p, dk.mutable_data_ptr(), dk.strides().data(), dv.mutable_data_ptr(),
+              dv.strides().data(), p + at.col_cnt, p + at.row_idx, shape[2], sb, sh, scale, code, B, H, N, D, dense,
+              dense_strides, counter, status, stream));
+    check("bsa_attn_bwd_dq_strided",
+          bsa_attn_bwd_dq_strided(q.const_data_ptr(), q.strides().data(), k.const_data_ptr(),
+                                  k.strides().data(), v.const_data_ptr(), v.strides().data(),
+                                  dout.const_data_ptr(), dout.strides().data(), lse_p, delta_p,
+                                  dq.mutable_data_ptr(), dq.strides().data(), p, p + at.col_idx, shape[2], sb, sh,
+                                  scale, code, B, H, N, D, dense, dense_strides, counter, status, stream));
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v,
+                                const std::optional<Tensor>& mask, double scale) {
+  if (!mask.has_value() || !q.is_cuda() || q.dim() != 4 || k.sizes() != q.sizes() || v.sizes() != q.sizes())
+    return std::nullopt;
+  const auto type = q.scalar_type();
+  if ((type != at::kHalf && type != at::kBFloat16) || k.scalar_type() != type || v.scalar_type() != type ||
+      k.device() != q.device() || v.device() != q.device())
+    return std::nullopt;
+  const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
+  if ((D != 16 && D != 32 && D != 64) || B == 0 || H == 0 || N == 0 || N % kBlock != 0) return std::nullopt;
+  const c10::cuda::CUDAGuard guard(q.device());
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
+  StreamState* state = stream_state(q.device().index(), stream);
+  if (state != nullptr && *state->word != 0) return std::nullopt;  // a report of an earlier kernel
+  Mask m;
+  if (!read_mask(*mask, B, H, N, q, stream, &m)) return std::nullopt;
+  if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
+    try {
+      return Attention::apply(q, k, v, &m, scale, state, static_cast<void*>(stream));
+    } catch (const Refused&) {
+      return std::nullopt;
+    }
+  }
+  Tensor o, lse2;
+  if (!run_forward(tma_ready(q), tma_ready(k), tma_ready(v), m, scale, state, stream, &o, &lse2))
+    return std::nullopt;
+  return o;
+}
+
+std::optional<std::pair<Tensor, Tensor>> state_tensors(int64_t device, int64_t stream) {
+  const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
+  StreamState* st = stream_state(static_cast<int>(device), reinterpret_cast<cudaStream_t>(stream));
+  if (st == nullptr) return std::nullopt;
+  return std::make_pair(st->counter, st->status);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  m.def("attention", &attention);
+  m.def("state_tensors", &state_tensors);
+  m.def("set_raise", [](pybind11::object f) { raise_error = f.release().ptr(); });
+}

@@ -232,15 +232,13 @@ def check_status(status: torch.Tensor):
 
 
 class _StreamState:
-    """What the public op keeps per (device, stream): the zeroed work counter of the persistent
-    kernels (they leave it at zero, also after a bounded wait gave up), and a status word in
-    pinned host memory, which the device can write and the host can read without a
+    """What the public op keeps per (device, stream), here and in the native host path: the zeroed work
+    counter of the persistent kernels (they leave it at zero, also after a bounded wait gave up), and a
+    status word in pinned host memory, which the device can write and the host can read without a
     synchronisation.  The kernels only ever touch the status word when a wait gave up."""
 
-    def __init__(self, device):
-        # zeroed on the stream that will use it, so no cross-stream ordering is needed
-        self.counter = torch.zeros(1, dtype=torch.int32, device=device)
-        self.status = torch.zeros(1, dtype=torch.int32).pin_memory()
+    def __init__(self, counter, status):
+        self.counter, self.status = counter, status
 
     def raise_if_reported(self):
         """Looks at the status word as it is now.  A report means that some earlier call on this
@@ -261,11 +259,19 @@ def _stream_state(device: torch.device, stream: int) -> Optional[_StreamState]:
     key = (device.index, stream)
     st = _stream_states.get(key)
     if st is None:
-        if torch.cuda.is_current_stream_capturing():
-            return None  # no allocation inside a graph capture: fixed-stride hand-out, no report
-        st = _StreamState(device)
-        _stream_states[key] = st
+        tensors = _lib.native().state_tensors(device.index, stream)
+        if tensors is None:
+            return None  # inside a graph capture: fixed-stride hand-out, no report
+        st = _stream_states[key] = _StreamState(*tensors)
     return st
+
+
+def _raise_native(fn: str, status: int):
+    """Raises what a step of the native host path reported."""
+    if status == -9:
+        for st in list(_stream_states.values()):
+            st.raise_if_reported()
+    raise _lib.BsaError(fn, status, _lib.load().bsa_strerror(status).decode())
 
 
 def _row_range(rows, nb):
@@ -349,34 +355,32 @@ def attention_backward(q, k, v, o, lse2, dout, lists: TileLists, sm_scale: float
     mask the forward was given, if any."""
     lib = _lib.load()
     B, H, N, D = q.shape
-    # the three kernels take one stride set for q, k, v, o, dO and the gradients
-    same = q.stride() == k.stride() == v.stride() == o.stride() == dout.stride()
-    if not same or _tma_ready(q) is not q:
-        q, k, v, o, dout = (t.contiguous() for t in (q, k, v, o, dout))
-    # the gradients are written with q's strides: allocate them with exactly those (empty_like
+    q, k, v, o, dout = (_tma_ready(t) for t in (q, k, v, o, dout))
+    # a gradient is written with the strides of its tensor: allocate it with exactly those (empty_like
     # would hand back a compact tensor for a view with gaps, e.g. a slice of a fused qkv buffer)
-    dq, dk, dv = (torch.empty_strided(q.shape, q.stride(), dtype=q.dtype, device=q.device)
-                  for _ in range(3))
+    dq, dk, dv = (torch.empty_strided(t.shape, t.stride(), dtype=t.dtype, device=t.device)
+                  for t in (q, k, v))
     delta = torch.empty((B, H, N), dtype=torch.float32, device=q.device)
     sb, sh = lists.list_strides(B, H)
     code = _lib.dtype_code(q.dtype)
-    st = _lib.strides4(q)
+    qs, ks, vs, ds = (_lib.strides4(t) for t in (q, k, v, dout))
     d4, dst = _dense_args(dense, B, H)
     with _on_device(q.device):
         stream = _lib.stream_ptr(q.device)
         state = _stream_state(q.device, stream.value or 0)
         counter = state.counter if state else None
-        _lib.check("bsa_attn_bwd_delta", lib.bsa_attn_bwd_delta(
-            _lib.ptr(o), _lib.ptr(dout), st, _lib.ptr(delta), code, B, H, N, D, stream))
-        _lib.check("bsa_attn_bwd_dkdv", lib.bsa_attn_bwd_dkdv(
-            _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dout), st, _lib.ptr(lse2),
-            _lib.ptr(delta), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(lists.col_ptr),
-            _lib.ptr(lists.row_idx), sb, sh, float(sm_scale), code, B, H, N, D, _lib.ptr(d4), dst,
+        _lib.check("bsa_attn_bwd_delta_strided", lib.bsa_attn_bwd_delta_strided(
+            _lib.ptr(o), _lib.strides4(o), _lib.ptr(dout), ds, _lib.ptr(delta), code, B, H, N, D,
+            stream))
+        _lib.check("bsa_attn_bwd_dkdv_strided", lib.bsa_attn_bwd_dkdv_strided(
+            _lib.ptr(q), qs, _lib.ptr(k), ks, _lib.ptr(v), vs, _lib.ptr(dout), ds, _lib.ptr(lse2),
+            _lib.ptr(delta), _lib.ptr(dk), ks, _lib.ptr(dv), vs, _lib.ptr(lists.col_ptr),
+            _lib.ptr(lists.row_idx), 0, sb, sh, float(sm_scale), code, B, H, N, D, _lib.ptr(d4), dst,
             _lib.ptr(counter), _lib.ptr(status), stream))
-        _lib.check("bsa_attn_bwd_dq", lib.bsa_attn_bwd_dq(
-            _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(dout), st, _lib.ptr(lse2),
-            _lib.ptr(delta), _lib.ptr(dq), _lib.ptr(lists.row_ptr), _lib.ptr(lists.col_idx),
-            sb, sh, float(sm_scale), code, B, H, N, D, _lib.ptr(d4), dst, _lib.ptr(counter),
+        _lib.check("bsa_attn_bwd_dq_strided", lib.bsa_attn_bwd_dq_strided(
+            _lib.ptr(q), qs, _lib.ptr(k), ks, _lib.ptr(v), vs, _lib.ptr(dout), ds, _lib.ptr(lse2),
+            _lib.ptr(delta), _lib.ptr(dq), qs, _lib.ptr(lists.row_ptr), _lib.ptr(lists.col_idx),
+            0, sb, sh, float(sm_scale), code, B, H, N, D, _lib.ptr(d4), dst, _lib.ptr(counter),
             _lib.ptr(status), stream))
     return dq, dk, dv
 
@@ -402,9 +406,8 @@ class _attention(torch.autograd.Function):
         B, H, N, D = q.shape
         assert q.shape[-1] == k.shape[-1] == v.shape[-1]
         assert D in {16, 32, 64, 128, 256}  # the reference's own check (fa2_custom_mask.py:58)
-        if D != 64:
-            raise NotImplementedError("the kernels are built for head dimension 64 (16 and 32 are "
-                                      "zero-padded to it by flash_attention_custom_mask)")
+        if D > 64:
+            raise NotImplementedError("the kernels are built for head dimensions up to 64")
         if N % BLOCK:
             raise AssertionError("sequence length must be a multiple of 64")
         if not q.is_cuda:
@@ -438,13 +441,11 @@ class _attention(torch.autograd.Function):
 
 def flash_attention_custom_mask(q, k, v, mask=None, sm_scale=1.3):
     """The reference's public op (fa2_custom_mask/fa2_custom_mask.py:157, `_attention.apply`), same
-    positional arguments.  Head dimensions 16 and 32 run on the D = 64 kernels with zero columns
-    appended to q, k, v (Q K^T is unchanged, the extra columns of P V are zero and are cut off
-    again; autograd slices the gradients); 128 and 256, which the reference also lists, are not
-    built."""
-    D = q.shape[-1] if q.dim() == 4 else 0
-    if D in (16, 32) and k.shape == q.shape and v.shape == q.shape:
-        pad = (0, 64 - D)
-        qp, kp, vp = (torch.nn.functional.pad(t, pad) for t in (q, k, v))
-        return _attention.apply(qp, kp, vp, mask, sm_scale)[..., :D].contiguous()
+    positional arguments.  Head dimensions 16, 32 and 64; 128 and 256, which the reference also lists,
+    are not built.  An ordinary call is made by the native host path; what that does not take (no mask,
+    a report of an earlier kernel, anything that is refused) goes through `_attention`."""
+    if isinstance(q, torch.Tensor) and q.is_cuda:
+        out = _lib.native().attention(q, k, v, mask, sm_scale)
+        if out is not None:
+            return out
     return _attention.apply(q, k, v, mask, sm_scale)
