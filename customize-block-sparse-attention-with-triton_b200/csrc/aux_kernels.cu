@@ -4,6 +4,9 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <atomic>
+#include <string.h>
+
 #include "host_common.h"
 
 namespace bsa {
@@ -220,6 +223,146 @@ static int launch_reorder(const void* in, const int64_t s[4], void* out, const i
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 
+// ---------------------------------------------------------------------------------------------
+// head-wise token reorder in place
+// ---------------------------------------------------------------------------------------------
+// One cluster of CTAs reorders one column chunk (64 bytes or more of every row) of one head: every CTA
+// gathers its share of the destination rows into registers, the cluster waits until all of it has been
+// read, and every CTA stores its share.  Bound by HBM: each byte is read once and written once, where a
+// gather into a second tensor and a copy back move it twice and allocate that tensor.  Registers hold
+// 72 KB a CTA, so that two CTAs share an SM and one's loads run under the other's stores; a cluster of
+// 16 holds 17,550 rows of 64 bytes (the reference's 13 x 30 x 45 grid at D = 64, 16 bit).
+// B200, q, k, v and output of 2 x 48 such heads (1.7 GB to move): 0.69 -> 0.36 ms.
+constexpr int kPermThreads = 512;
+constexpr int kPermPieces = 9;  // 16-byte pieces a thread holds
+constexpr int kPermTensors = 3;
+
+struct PermuteArgs {
+  uint8_t* base[kPermTensors];
+  int64_t sb[kPermTensors], sh[kPermTensors], st[kPermTensors];  // bytes
+  const void* plan;       // the axis order of a head, as an index into the six of permute_order()
+  int64_t plan_stride;    // in elements
+  int plan_is_64;
+  int B, heads, T, chunks, chunk_bytes, pieces_per_cta;
+  int ext[3];             // F, Hh, W
+  // floor(n / d) = umulhi(n, m) for n * d < 2^32: m = floor(2^32 / d) + 1
+  uint32_t m_vec;         // d = pieces of a row's chunk
+  uint32_t m_ext[3];      // d = ext[i]
+  uint32_t m_plane[3];    // d = product of the other two extents
+};
+
+__device__ __forceinline__ uint32_t div_by(uint32_t n, uint32_t d, uint32_t m) {
+  return d == 1 ? n : __umulhi(n, m);
+}
+
+// (indexing of PermuteArgs with constants only, so that nothing goes through local memory)
+__device__ __forceinline__ uint32_t pick3u(int sel, uint32_t v0, uint32_t v1, uint32_t v2) {
+  return sel == 0 ? v0 : (sel == 1 ? v1 : v2);
+}
+
+template <bool kInverse>
+__global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_constant__ PermuteArgs a) {
+  int unit = blockIdx.y;
+  const int chunk = unit % a.chunks;
+  unit /= a.chunks;
+  const int h = unit % a.heads;
+  unit /= a.heads;
+  const int b = unit % a.B, which = unit / a.B;
+  int64_t order = a.plan_is_64 ? static_cast<const int64_t*>(a.plan)[h * a.plan_stride]
+                               : static_cast<const int32_t*>(a.plan)[h * a.plan_stride];
+  if (order < 0) order += 6;
+  // nothing to do for the order (0,1,2); an index that is none leaves the head alone.  The same for
+  // every CTA of the cluster.
+  if (order <= 0 || order > 5) return;
+  // axis orders 1..5: (0,2,1), (1,2,0), (1,0,2), (2,1,0), (2,0,1)
+  const int p0 = order >= 4 ? 2 : (order == 1 ? 0 : 1);
+  const int p1 = order == 1 || order == 2 ? 2 : (order == 4 ? 1 : 0);
+  const int p2 = 3 - p0 - p1;
+  const uint32_t e0 = a.ext[0], e1 = a.ext[1], e2 = a.ext[2];
+  const uint32_t d1 = pick3u(p1, e0, e1, e2), d2 = pick3u(p2, e0, e1, e2);
+  // the destination is walked in its own axis order; its token splits into coordinates along the axes
+  // q0, q1, q2 (the permuted ones, or, laying back, the grid's own)
+  const uint32_t g1 = kInverse ? e1 : d1, g2 = kInverse ? e2 : d2;
+  const uint32_t m_plane = kInverse ? a.m_plane[0] : pick3u(p0, a.m_plane[0], a.m_plane[1], a.m_plane[2]);
+  const uint32_t m_last = kInverse ? a.m_ext[2] : pick3u(p2, a.m_ext[0], a.m_ext[1], a.m_ext[2]);
+  // weight of each of those coordinates in the source token
+  uint32_t w0, w1, w2;
+  if (kInverse) {  // source: grid in the order (p0, p1, p2)
+    const uint32_t s0 = d1 * d2, s1 = d2;
+    w0 = p0 == 0 ? s0 : (p1 == 0 ? s1 : 1u);
+    w1 = p0 == 1 ? s0 : (p1 == 1 ? s1 : 1u);
+    w2 = p0 == 2 ? s0 : (p1 == 2 ? s1 : 1u);
+  } else {         // source: the grid's own order
+    w0 = pick3u(p0, e1 * e2, e2, 1u);
+    w1 = pick3u(p1, e1 * e2, e2, 1u);
+    w2 = pick3u(p2, e1 * e2, e2, 1u);
+  }
+  const int64_t st = which == 0 ? a.st[0] : (which == 1 ? a.st[1] : a.st[2]);
+  uint8_t* const base =
+      (which == 0 ? a.base[0] + b * a.sb[0] + h * a.sh[0]
+                  : (which == 1 ? a.base[1] + b * a.sb[1] + h * a.sh[1] : a.base[2] + b * a.sb[2] + h * a.sh[2])) +
+      static_cast<int64_t>(chunk) * a.chunk_bytes;
+  const uint32_t vec = static_cast<uint32_t>(a.chunk_bytes) >> 4;
+  const uint32_t first = blockIdx.x * a.pieces_per_cta + threadIdx.x;
+  const uint32_t end = min(static_cast<uint32_t>(a.T) * vec, (blockIdx.x + 1) * a.pieces_per_cta);
+  uint4 val[kPermPieces];
+#pragma unroll
+  for (int i = 0; i < kPermPieces; ++i) {
+    const uint32_t idx = first + i * kPermThreads;
+    if (idx < end) {
+      const uint32_t t = div_by(idx, vec, a.m_vec), piece = idx - t * vec;
+      const uint32_t c0 = div_by(t, g1 * g2, m_plane), rem = t - c0 * (g1 * g2);
+      const uint32_t c1 = div_by(rem, g2, m_last), c2 = rem - c1 * g2;
+      const uint32_t from = c0 * w0 + c1 * w1 + c2 * w2;
+      val[i] = *reinterpret_cast<const uint4*>(base + from * st + piece * 16u);
+    }
+  }
+  // every CTA of the cluster has read its share before any of them stores
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < kPermPieces; ++i) {
+    const uint32_t idx = first + i * kPermThreads;
+    if (idx < end) {
+      const uint32_t t = div_by(idx, vec, a.m_vec), piece = idx - t * vec;
+      *reinterpret_cast<uint4*>(base + t * st + piece * 16u) = val[i];
+    }
+  }
+}
+
+template <bool kInverse>
+static int launch_permute(PermuteArgs& a, int n_tensors, int cluster, cudaStream_t stream) {
+  auto kern = permute_kernel<kInverse>;
+  static std::atomic<int> ready[64];  // per device: 0 unknown, 1 clusters of 16 fit, 2 they do not
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BSA_ERR_CUDA;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  const int64_t units = static_cast<int64_t>(n_tensors) * a.B * a.heads * a.chunks;
+  if (units > 65535) return BSA_ERR_TOO_LARGE;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(cluster), static_cast<unsigned>(units), 1);
+  cfg.blockDim = dim3(kPermThreads, 1, 1);
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cluster > 8) {
+    int r = ready[dev].load(std::memory_order_relaxed);
+    if (r == 0) {
+      int n = 0;
+      const bool ok = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                      cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0;
+      if (!ok) (void)cudaGetLastError();
+      r = ok ? 1 : 2;
+      ready[dev].store(r, std::memory_order_relaxed);
+    }
+    if (r == 2) return BSA_ERR_TOO_LARGE;
+  }
+  return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
+
 }  // namespace bsa
 
 extern "C" int bsa_attn_bwd_delta_strided(const void* o, const int64_t o_strides[4], const void* dout,
@@ -245,6 +388,64 @@ extern "C" int bsa_attn_bwd_delta_strided(const void* o, const int64_t o_strides
 extern "C" int bsa_attn_bwd_delta(const void* o, const void* dout, const int64_t s[4], float* delta,
                                   int dtype, int B, int H, int N, int D, void* stream) {
   return bsa_attn_bwd_delta_strided(o, s, dout, s, delta, dtype, B, H, N, D, stream);
+}
+
+extern "C" int bsa_permute_in_place(void* const tensors[], const int64_t* strides, int n_tensors,
+                                    const void* plan, int plan_elem_bytes, int64_t plan_stride,
+                                    int inverse, int B, int heads, int T, int D, int F, int Hh, int W,
+                                    int elem_bytes, void* stream) {
+  using namespace bsa;
+  if (B <= 0 || heads <= 0 || T <= 0 || D <= 0 || F <= 0 || Hh <= 0 || W <= 0 || n_tensors < 1 ||
+      n_tensors > kPermTensors || static_cast<int64_t>(F) * Hh * W != T)
+    return BSA_ERR_BAD_SHAPE;
+  if ((elem_bytes != 1 && elem_bytes != 2 && elem_bytes != 4 && elem_bytes != 8) ||
+      (plan_elem_bytes != 4 && plan_elem_bytes != 8))
+    return BSA_ERR_BAD_DTYPE;
+  if (!tensors || !strides || !plan) return BSA_ERR_BAD_POINTER;
+  PermuteArgs a;
+  memset(&a, 0, sizeof(a));
+  for (int i = 0; i < n_tensors; ++i) {
+    const int64_t* s = strides + 4 * i;
+    if (s[3] != 1) return BSA_ERR_BAD_STRIDE;
+    for (int k = 0; k < 3; ++k)
+      if (s[k] < 0 || (s[k] * elem_bytes) % 16 != 0) return BSA_ERR_BAD_STRIDE;
+    if (!tensors[i] || !is_aligned(tensors[i], 16)) return BSA_ERR_BAD_POINTER;
+    a.base[i] = static_cast<uint8_t*>(tensors[i]);
+    a.sb[i] = s[0] * elem_bytes;
+    a.sh[i] = s[1] * elem_bytes;
+    a.st[i] = s[2] * elem_bytes;
+  }
+  const int64_t row_bytes = static_cast<int64_t>(D) * elem_bytes;
+  if (row_bytes % 16 != 0 || row_bytes > (1 << 20)) return BSA_ERR_BAD_STRIDE;
+  // As few column chunks as a cluster of 16 can hold, none below 64 bytes (two DRAM sectors) unless the
+  // row is; then the smallest cluster that holds one.
+  constexpr int64_t kCapacity = kPermThreads * kPermPieces * 16;
+  int64_t chunk = row_bytes;
+  while (T * chunk > 16 * kCapacity && chunk % 32 == 0 && chunk >= 128) chunk /= 2;
+  const int64_t pieces = T * (chunk / 16);
+  if (pieces * 16 > 16 * kCapacity || pieces * (chunk / 16) >= (1ll << 32) || T >= 65536) return BSA_ERR_TOO_LARGE;
+  int cluster = 1;
+  while (cluster * kCapacity < pieces * 16) cluster *= 2;
+  a.plan = plan;
+  a.plan_stride = plan_stride;
+  a.plan_is_64 = plan_elem_bytes == 8;
+  a.B = B;
+  a.heads = heads;
+  a.T = T;
+  a.chunk_bytes = static_cast<int>(chunk);
+  a.chunks = static_cast<int>(row_bytes / chunk);
+  a.pieces_per_cta = static_cast<int>((pieces + cluster - 1) / cluster);
+  a.ext[0] = F;
+  a.ext[1] = Hh;
+  a.ext[2] = W;
+  const auto magic = [](int64_t d) { return static_cast<uint32_t>((1ll << 32) / d + 1); };
+  a.m_vec = magic(chunk / 16);
+  for (int i = 0; i < 3; ++i) {
+    a.m_ext[i] = magic(a.ext[i]);
+    a.m_plane[i] = magic(T / a.ext[i]);
+  }
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return inverse ? launch_permute<true>(a, n_tensors, cluster, st) : launch_permute<false>(a, n_tensors, cluster, st);
 }
 
 extern "C" int bsa_reorder(const void* in, void* out, const int64_t strides[4],

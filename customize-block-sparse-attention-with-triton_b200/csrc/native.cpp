@@ -274,6 +274,40 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
   return o;
 }
 
+// The image tokens (those behind the first n_text) of one to three tensors [B,heads,tokens,D] reordered in
+// place; false when the tensors, the plan or the grid are nothing that one launch takes.
+bool permute_tokens(const std::vector<Tensor>& tensors, const Tensor& plan, int64_t F, int64_t Hh, int64_t W,
+                    int64_t n_text, bool inverse) {
+  const Tensor& t0 = tensors[0];
+  if (tensors.size() > 3 || !t0.is_cuda() || t0.dim() != 4 || plan.device() != t0.device() || plan.dim() != 1 ||
+      (plan.scalar_type() != at::kLong && plan.scalar_type() != at::kInt) || plan.size(0) != t0.size(1) ||
+      n_text < 0 || t0.size(2) - n_text != F * Hh * W)
+    return false;
+  void* ptrs[3];
+  int64_t strides[12];
+  for (size_t i = 0; i < tensors.size(); ++i) {
+    const Tensor& t = tensors[i];
+    if (t.sizes() != t0.sizes() || t.scalar_type() != t0.scalar_type() || t.device() != t0.device() ||
+        (t.requires_grad() && at::GradMode::is_enabled()))
+      return false;
+    for (size_t j = 0; j < i; ++j)
+      if (t.is_alias_of(tensors[j])) return false;  // shared storage: one after the other
+    ptrs[i] = static_cast<char*>(t.mutable_data_ptr()) + n_text * t.stride(2) * t.element_size();
+    for (int d = 0; d < 4; ++d) strides[4 * i + d] = t.stride(d);
+    // rows that overlap (expanded tensors) cannot be reordered in place
+    for (int d = 0; d < 3; ++d)
+      if (t.size(d) > 1 && t.stride(d) < t.size(3)) return false;
+  }
+  const c10::cuda::CUDAGuard guard(t0.device());
+  const cudaStream_t stream = at::cuda::getCurrentCUDAStream(t0.device().index());
+  if (bsa_permute_in_place(ptrs, strides, tensors.size(), plan.const_data_ptr(), plan.element_size(),
+                           plan.stride(0), inverse ? 1 : 0, t0.size(0), t0.size(1), F * Hh * W, t0.size(3), F,
+                           Hh, W, t0.element_size(), stream) != 0)
+    return false;
+  for (const Tensor& t : tensors) t.unsafeGetTensorImpl()->bump_version();
+  return true;
+}
+
 std::optional<std::pair<Tensor, Tensor>> state_tensors(int64_t device, int64_t stream) {
   const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device));
   StreamState* st = stream_state(static_cast<int>(device), reinterpret_cast<cudaStream_t>(stream));
@@ -285,6 +319,7 @@ std::optional<std::pair<Tensor, Tensor>> state_tensors(int64_t device, int64_t s
 
 PYBIND11_MODULE(_native, m) {
   m.def("attention", &attention);
+  m.def("permute_tokens", &permute_tokens);
   m.def("state_tensors", &state_tensors);
   m.def("set_raise", [](pybind11::object f) { raise_error = f.release().ptr(); });
 }

@@ -63,6 +63,8 @@ SIGNATURES = {
     "bsa_inv_reorder": [_vp, _vp, _s4, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_reorder_strided": [_vp, _s4, _vp, _s4, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_inv_reorder_strided": [_vp, _s4, _vp, _s4, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
+    "bsa_permute_in_place": [ctypes.POINTER(_vp), _s4, _i, _vp, _i, ctypes.c_int64, _i, _i, _i, _i, _i, _i,
+                             _i, _i, _i, _vp],
     "bsa_attn_fwd_block_mask_static": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _s4, _i,
                                        _i, _f, _i, _i, _i, _i, _i, _vp],
     "bsa_static_warmup": [],

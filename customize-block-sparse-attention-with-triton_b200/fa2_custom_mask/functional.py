@@ -79,11 +79,21 @@ def apply_head_wise_reorder(tensor, permute_orders, F, H, W):
     return output
 
 
+def _in_place(tensors, idx, F, H, W, n_text_tokens, inverse):
+    """The reorder of all the tensors in one launch, each byte read and written once; False when the
+    tensors are not made for that (a token row that is no multiple of 16 bytes, a grid that the registers
+    of 16 CTAs do not hold, a plan that is not on the device), with nothing done."""
+    return (isinstance(idx, torch.Tensor) and all(isinstance(t, torch.Tensor) and t.is_cuda for t in tensors)
+            and _lib.native().permute_tokens(tensors, idx, F, H, W, n_text_tokens, inverse))
+
+
 def permute_qkv_triton(query, key, value, permute_plan, i_block, F=13, H=30, W=45, n_text_tokens=226):
     """Reorders the image tokens of q, k, v in place (text tokens stay) and returns the same three
     tensors, like the reference (fa2_custom_mask/functional.py:22-43)."""
-    permutations, _ = _tables(query.device)
     idx = permute_plan['permute'][i_block]  # [N_head]
+    if _in_place((query, key, value), idx, F, H, W, n_text_tokens, False):
+        return query, key, value
+    permutations, _ = _tables(query.device)
     permute_orders = permutations[idx]      # [N_head, 3]
     for t in (query, key, value):
         image = t[:, :, n_text_tokens:, :]
@@ -110,8 +120,10 @@ def apply_inv_reorder(tensor, permute_orders, inv_permute_orders, F, H, W):
 def inv_permute_attn_triton(attn_out, permute_plan, i_block, F=13, H=30, W=45, n_text_tokens=226):
     """Lays the image tokens of the attention output back in place and returns attn_out
     (fa2_custom_mask/functional.py:64-84)."""
-    permutations, permutations_inv = _tables(attn_out.device)
     idx = permute_plan['permute'][i_block]
+    if _in_place((attn_out,), idx, F, H, W, n_text_tokens, True):
+        return attn_out
+    permutations, permutations_inv = _tables(attn_out.device)
     permute_orders = permutations[idx]
     inv_permute_orders = permutations_inv[idx]
     attn_image = attn_out[:, :, n_text_tokens:, :]

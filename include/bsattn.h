@@ -302,6 +302,21 @@ int bsa_inv_reorder_strided(const void* in, const int64_t in_strides[4], void* o
                             int W, int elem_bytes, void* stream);
 
 /*
+ * The token reorder of one to three tensors in place, in one launch: what permute_qkv_triton and
+ * inv_permute_attn_triton (fa2_custom_mask/functional.py:22-43, 64-84) do to the image tokens.
+ *   tensors  : n_tensors (1..3) tensors [B,heads,T=F*Hh*W,D]; strides: four element strides for each
+ *              (last one 1, the others multiples of 16 bytes; bases 16-byte aligned)
+ *   plan     : device array of the head's axis orders, as indexes (4- or 8-byte integers, plan_stride
+ *              elements apart) into (0,1,2), (0,2,1), (1,2,0), (1,0,2), (2,1,0), (2,0,1)
+ *   inverse  : 0 lays the tokens out in that order, 1 lays them back
+ * BSA_ERR_TOO_LARGE or BSA_ERR_BAD_STRIDE: use the reorder calls above with a second tensor.
+ */
+int bsa_permute_in_place(void* const tensors[], const int64_t* strides, int n_tensors,
+                         const void* plan, int plan_elem_bytes, int64_t plan_stride, int inverse,
+                         int B, int heads, int T, int D, int F, int Hh, int W, int elem_bytes,
+                         void* stream);
+
+/*
  * Forward attention directly from a block mask, allocating nothing.  It has no counterpart in the
  * reference; it exists for hosts that cannot hand the library device buffers at call time, such as
  * an inference-engine plugin whose workspace was sized when the engine was built, or a process
