@@ -9,7 +9,9 @@
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
-#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <torch/extension.h>
 
 #include <mutex>
@@ -152,8 +154,6 @@ void check(const char* fn, int rc) {
 // ---------------------------------------------------------------------------------------------
 // Autograd
 // ---------------------------------------------------------------------------------------------
-struct Refused {};  // the forward cannot be done here
-
 // The tile lists of one call in one buffer of words: counts of the row and column lists, then their
 // entries, every list in a place of nb words.
 struct Lists {
@@ -167,50 +167,41 @@ struct Lists {
   }
 };
 
-struct Attention : torch::autograd::Function<Attention> {
-  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& q0, const Tensor& k0,
-                        const Tensor& v0, const Mask* m, double scale, StreamState* state, void* stream) {
-    const Tensor q = tma_ready(q0), k = tma_ready(k0), v = tma_ready(v0);
-    Tensor o, lse2;
-    if (!run_forward(q, k, v, *m, scale, state, stream, &o, &lse2)) throw Refused();
-    // the forward lists each mask row inside the kernel; only the backward needs lists as data
-    const int64_t Bm = m->block.size(0), Hm = m->block.size(1), nb = m->block.size(2);
-    const Lists at(Bm, Hm, nb);
-    Tensor lists = at::empty({at.words}, q.options().dtype(at::kInt));
-    int32_t* p = lists.mutable_data_ptr<int32_t>();
-    if (bsa_tile_lists_places(m->block.const_data_ptr<uint8_t>(), m->block.strides().data(), Bm, Hm, nb, p,
-                              p + at.col_idx, p + at.col_cnt, p + at.row_idx, stream) != 0)
-      throw Refused();
-    ctx->save_for_backward({q0, k0, v0, o});
-    ctx->saved_data["lse2"] = lse2;
-    ctx->saved_data["lists"] = lists;
-    // the caller's mask (or an aligned copy of it): not to be changed before backward
-    if (m->dense.defined()) ctx->saved_data["dense"] = m->dense;
-    ctx->saved_data["mask"] = std::vector<int64_t>{Bm, Hm, nb};
-    ctx->saved_data["scale"] = scale;
-    return o;
+// (A node of its own and not torch::autograd::Function: that keeps what is saved in a map of boxed values,
+// which costs a small call another 10 us.)
+struct AttentionBackward : torch::autograd::Node {
+  torch::autograd::SavedVariable q_, k_, v_, o_;
+  Tensor lse2, lists;
+  Tensor dense;  // the caller's mask (or an aligned copy of it): not to be changed before backward
+  int64_t Bm, Hm, nb;
+  float scale;
+
+  std::string name() const override { return "AttentionBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (auto* s : {&q_, &k_, &v_, &o_}) s->reset_data();
+    lse2.reset();
+    lists.reset();
+    dense.reset();
   }
 
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
-                                                 torch::autograd::variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor q = tma_ready(saved[0]), k = tma_ready(saved[1]), v = tma_ready(saved[2]), &o = saved[3];
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    // (unpacking raises when the buffers have been released or an input was modified in place)
+    const Tensor q = tma_ready(q_.unpack()), k = tma_ready(k_.unpack()), v = tma_ready(v_.unpack());
+    const Tensor o = o_.unpack(shared_from_this());
+    at::AutoDispatchBelowADInplaceOrView no_autograd;
     const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
-    const Tensor dout = tma_ready(grads[0].defined() ? grads[0].to(q.scalar_type()) : at::zeros_like(o));
-    const Tensor lse2 = ctx->saved_data["lse2"].toTensor(), lists = ctx->saved_data["lists"].toTensor();
-    const auto shape = ctx->saved_data["mask"].toIntVector();
-    const int64_t Bm = shape[0], Hm = shape[1];
-    const Lists at(Bm, Hm, shape[2]);
-    const float scale = static_cast<float>(ctx->saved_data["scale"].toDouble());
-    const uint8_t* dense = nullptr;
+    if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
+    const Tensor dout = tma_ready(grads[0].to(q.scalar_type()));
+    const Lists at(Bm, Hm, nb);
+    const uint8_t* dense_ptr = nullptr;
     int64_t strides[4] = {0, 0, 0, 0};
-    const auto dense_it = ctx->saved_data.find("dense");
-    if (dense_it != ctx->saved_data.end()) {
-      const Tensor t = dense_it->second.toTensor();
-      dense = t.const_data_ptr<uint8_t>();
-      for (int i = 0; i < 4; ++i) strides[i] = i < 2 && t.size(i) == 1 ? 0 : t.stride(i);
+    if (dense.defined()) {
+      dense_ptr = dense.const_data_ptr<uint8_t>();
+      for (int i = 0; i < 4; ++i) strides[i] = i < 2 && dense.size(i) == 1 ? 0 : dense.stride(i);
     }
-    const int64_t* dense_strides = dense ? strides : nullptr;
+    const int64_t* dense_strides = dense_ptr ? strides : nullptr;
     const c10::cuda::CUDAGuard guard(q.device());
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
     StreamState* state = stream_state(q.device().index(), stream);
@@ -233,17 +224,49 @@ struct Attention : torch::autograd::Function<Attention> {
               q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
               v.const_data_ptr(), v.strides().data(), dout.const_data_ptr(), dout.strides().data(), lse_p,
               delta_p, dk.mutable_data_ptr(), dk.strides().data(), dv.mutable_data_ptr(),
-              dv.strides().data(), p + at.col_cnt, p + at.row_idx, shape[2], sb, sh, scale, code, B, H, N, D, dense,
-              dense_strides, counter, status, stream));
+              dv.strides().data(), p + at.col_cnt, p + at.row_idx, nb, sb, sh, scale, code, B, H, N, D,
+              dense_ptr, dense_strides, counter, status, stream));
     check("bsa_attn_bwd_dq_strided",
           bsa_attn_bwd_dq_strided(q.const_data_ptr(), q.strides().data(), k.const_data_ptr(),
                                   k.strides().data(), v.const_data_ptr(), v.strides().data(),
                                   dout.const_data_ptr(), dout.strides().data(), lse_p, delta_p,
-                                  dq.mutable_data_ptr(), dq.strides().data(), p, p + at.col_idx, shape[2], sb, sh,
-                                  scale, code, B, H, N, D, dense, dense_strides, counter, status, stream));
-    return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+                                  dq.mutable_data_ptr(), dq.strides().data(), p, p + at.col_idx, nb, sb, sh,
+                                  scale, code, B, H, N, D, dense_ptr, dense_strides, counter, status,
+                                  stream));
+    return {dq, dk, dv};
   }
 };
+
+// The forward with its node; undefined when the library refused.
+Tensor forward_with_grad(const Tensor& q0, const Tensor& k0, const Tensor& v0, const Mask& m, double scale,
+                         StreamState* state, void* stream) {
+  std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(q0, k0, v0));
+  Tensor o;
+  {
+    at::AutoDispatchBelowADInplaceOrView no_autograd;
+    if (!run_forward(tma_ready(q0), tma_ready(k0), tma_ready(v0), m, scale, state, stream, &o, &node->lse2))
+      return Tensor();
+    // the forward lists each mask row inside the kernel; only the backward needs lists as data
+    node->Bm = m.block.size(0);
+    node->Hm = m.block.size(1);
+    node->nb = m.block.size(2);
+    const Lists at(node->Bm, node->Hm, node->nb);
+    node->lists = at::empty({at.words}, q0.options().dtype(at::kInt));
+    int32_t* p = node->lists.mutable_data_ptr<int32_t>();
+    if (bsa_tile_lists_places(m.block.const_data_ptr<uint8_t>(), m.block.strides().data(), node->Bm, node->Hm,
+                              node->nb, p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, stream) != 0)
+      return Tensor();
+  }
+  node->dense = m.dense;
+  node->scale = static_cast<float>(scale);
+  node->q_ = torch::autograd::SavedVariable(q0, false);
+  node->k_ = torch::autograd::SavedVariable(k0, false);
+  node->v_ = torch::autograd::SavedVariable(v0, false);
+  torch::autograd::set_history(o, node);
+  node->o_ = torch::autograd::SavedVariable(o, true);
+  return o;
+}
 
 std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& v,
                                 const std::optional<Tensor>& mask, double scale) {
@@ -262,11 +285,8 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
   Mask m;
   if (!read_mask(*mask, B, H, N, q, stream, &m)) return std::nullopt;
   if (at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad())) {
-    try {
-      return Attention::apply(q, k, v, &m, scale, state, static_cast<void*>(stream));
-    } catch (const Refused&) {
-      return std::nullopt;
-    }
+    Tensor o = forward_with_grad(q, k, v, m, scale, state, stream);
+    return o.defined() ? std::optional<Tensor>(o) : std::nullopt;
   }
   Tensor o, lse2;
   if (!run_forward(tma_ready(q), tma_ready(k), tma_ready(v), m, scale, state, stream, &o, &lse2))
