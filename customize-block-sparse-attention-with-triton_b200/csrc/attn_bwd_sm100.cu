@@ -305,6 +305,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
+  grid_dependency_wait();
 
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
   // issuers do without (56 + 104 + 56 = 3 x 72).
@@ -739,6 +740,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     if (warp == kX2Warp) bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, 1, lane, abort_flag);
   }
 
+  // (not before: CTAs of the next kernel that wait on free SMs slowed the working ones down by 3 %)
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   if (warp == kXWarp) {
@@ -838,9 +841,9 @@ static int launch_bwd(BwdOperand q, BwdOperand k, BwdOperand v, BwdOperand dout,
   int sms = 0;
   if ((rc = sm_count(&sms)) != BSA_OK) return rc;
   const dim3 grid(static_cast<unsigned>(prm.items < sms ? prm.items : sms));  // one CTA per SM
-  kern<<<grid, kBwdThreads, smem_bytes, static_cast<cudaStream_t>(stream)>>>(
-      kDKDV ? tm_k : tm_q, kDKDV ? tm_v : tm_do, kDKDV ? tm_q : tm_k, kDKDV ? tm_do : tm_v, prm);
-  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+  return launch_dependent(kern, grid, kBwdThreads, smem_bytes, static_cast<cudaStream_t>(stream),
+                          kDKDV ? tm_k : tm_q, kDKDV ? tm_v : tm_do, kDKDV ? tm_q : tm_k,
+                          kDKDV ? tm_do : tm_v, prm);
 }
 
 }  // namespace bsa

@@ -473,6 +473,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
+  grid_dependency_wait();
 
   // 512 threads are launched with 128 registers: the softmax warps, which hold 128 logits each, take
   // what the others do without (2 x 160 + 80 + 112 = 4 x 128).
@@ -1006,6 +1007,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
 
   // ---- tear-down: every role arrives here, also after a give-up ----
+  // (not before: CTAs of the next kernel that wait on free SMs slowed the working ones down by 3 %)
+  grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   if (warp == kSWarp) {
@@ -1100,9 +1103,8 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
   if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes)) != BSA_OK)
     return rc;
   const dim3 grid(static_cast<unsigned>(prm.items < sms ? prm.items : sms));  // one CTA per SM
-  kern<<<grid, kFwdThreads, smem_bytes, static_cast<cudaStream_t>(stream)>>>(tm_q, tm_k, tm_v, prm);
-  if (cudaGetLastError() != cudaSuccess) return BSA_ERR_CUDA;
-  return BSA_OK;
+  return launch_dependent(kern, grid, kFwdThreads, smem_bytes, static_cast<cudaStream_t>(stream), tm_q, tm_k,
+                          tm_v, prm);
 }
 
 }  // namespace bsa

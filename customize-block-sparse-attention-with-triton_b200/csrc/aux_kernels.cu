@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include "host_common.h"
+#include "sm100_ptx.cuh"
 
 namespace bsa {
 
@@ -60,6 +61,8 @@ bwd_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int
   const int64_t b = bh / H, h = bh - b * H;
   const uint16_t* po = o + b * o_sb + h * o_sh + chunk * 8;
   const uint16_t* pd = dout + b * d_sb + h * d_sh + chunk * 8;
+  grid_dependents_launch();
+  grid_dependency_wait();
   uint4 xo[4], xd[4];
   bool live[4];
 #pragma unroll
@@ -83,14 +86,14 @@ bwd_delta_kernel(const uint16_t* __restrict__ o, int64_t o_sb, int64_t o_sh, int
 }
 
 template <int kD>
-static void launch_delta(bool bf16, const void* o, const int64_t* os, const void* dout, const int64_t* ds,
+static int launch_delta(bool bf16, const void* o, const int64_t* os, const void* dout, const int64_t* ds,
                          float* delta, int H, int N, int64_t rows, cudaStream_t stream) {
   constexpr int64_t kRows = kDeltaThreads / 32 * 4 * (32 / (kD / 8));  // of a CTA
   const unsigned blocks = static_cast<unsigned>((rows + kRows - 1) / kRows);
   auto kern = bf16 ? bwd_delta_kernel<true, kD> : bwd_delta_kernel<false, kD>;
-  kern<<<blocks, kDeltaThreads, 0, stream>>>(static_cast<const uint16_t*>(o), os[0], os[1], os[2],
-                                             static_cast<const uint16_t*>(dout), ds[0], ds[1], ds[2],
-                                             delta, H, N, rows);
+  return launch_dependent(kern, dim3(blocks), kDeltaThreads, 0, stream, static_cast<const uint16_t*>(o), os[0],
+                          os[1], os[2], static_cast<const uint16_t*>(dout), ds[0], ds[1], ds[2], delta, H, N,
+                          rows);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -232,7 +235,7 @@ static int launch_reorder(const void* in, const int64_t s[4], void* out, const i
 // gather into a second tensor and a copy back move it twice and allocate that tensor.  Registers hold
 // 72 KB a CTA, so that two CTAs share an SM and one's loads run under the other's stores; a cluster of
 // 16 holds 17,550 rows of 64 bytes (the reference's 13 x 30 x 45 grid at D = 64, 16 bit).
-// B200, q, k, v and output of 2 x 48 such heads (1.7 GB to move): 0.69 -> 0.36 ms.
+// B200, q, k, v and output of 2 x 48 such heads (1.7 GB to move): 0.69 -> 0.31 ms.
 constexpr int kPermThreads = 512;
 constexpr int kPermPieces = 9;  // 16-byte pieces a thread holds
 constexpr int kPermTensors = 3;
@@ -262,6 +265,8 @@ __device__ __forceinline__ uint32_t pick3u(int sel, uint32_t v0, uint32_t v1, ui
 
 template <bool kInverse>
 __global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_constant__ PermuteArgs a) {
+  grid_dependents_launch();
+  grid_dependency_wait();
   int unit = blockIdx.y;
   const int chunk = unit % a.chunks;
   unit /= a.chunks;
@@ -335,19 +340,21 @@ static int launch_permute(PermuteArgs& a, int n_tensors, int cluster, cudaStream
   static std::atomic<int> ready[64];  // per device: 0 unknown, 1 clusters of 16 fit, 2 they do not
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BSA_ERR_CUDA;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = static_cast<unsigned>(cluster);
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   const int64_t units = static_cast<int64_t>(n_tensors) * a.B * a.heads * a.chunks;
   if (units > 65535) return BSA_ERR_TOO_LARGE;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(cluster), static_cast<unsigned>(units), 1);
   cfg.blockDim = dim3(kPermThreads, 1, 1);
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   if (cluster > 8) {
     int r = ready[dev].load(std::memory_order_relaxed);
     if (r == 0) {
@@ -379,10 +386,9 @@ extern "C" int bsa_attn_bwd_delta_strided(const void* o, const int64_t o_strides
   if (rows / 128 >= 0x7fffffffLL) return BSA_ERR_TOO_LARGE;
   const bool bf16 = dtype == BSA_BF16;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (D == 64) launch_delta<64>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
-  else if (D == 32) launch_delta<32>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
-  else launch_delta<16>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
-  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+  if (D == 64) return launch_delta<64>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
+  if (D == 32) return launch_delta<32>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
+  return launch_delta<16>(bf16, o, o_strides, dout, do_strides, delta, H, N, rows, st);
 }
 
 extern "C" int bsa_attn_bwd_delta(const void* o, const void* dout, const int64_t s[4], float* delta,

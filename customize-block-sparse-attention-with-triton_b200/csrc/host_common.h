@@ -38,6 +38,25 @@ int cached_qkv_tmap(CUtensorMap* out, const void* base, const int64_t s[4], int 
 // Number of SMs of the current device (cached per device).
 int sm_count(int* out);
 
+// Launches a kernel that may begin while the previous one of the stream is still running (see
+// grid_dependency_wait): its set-up and the launch itself, 2 to 4 us, then cost nothing between kernels
+// that follow one another.
+template <typename... Params, typename... Args>
+int launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                     const Args&... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
+
 // Raises a kernel's dynamic shared-memory limit; done once per (kernel, device) and remembered.
 int ensure_dynamic_smem(const void* kernel, size_t bytes);
 

@@ -55,6 +55,18 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool pred)
   return out != 0;
 }
 
+// Programmatic dependent launch: every kernel of this library is launched so that it may begin while
+// the previous kernel of the stream is still running, does its set-up, and waits here, before it touches
+// memory that another kernel may write or read, until that one has ended and its writes are visible.
+// (Without the attribute on the launch both are no-ops.)
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// The next kernel of the stream may be launched as soon as all CTAs have said so or ended.
+__device__ __forceinline__ void grid_dependents_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ uint64_t global_timer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
