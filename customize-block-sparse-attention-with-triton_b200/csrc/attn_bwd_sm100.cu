@@ -25,22 +25,31 @@
 //
 // Persistent: one CTA per SM starts with block blockIdx.x and draws further blocks from an
 // optional work counter (or walks a fixed stride); long lists first when the mask is causal.
-// Roles (25 warps):
+// Roles (26 warps):
 //   warps 0..15 : compute, two teams of eight warps on alternate supersteps (team = warp / 8, TMEM lane
-//                 quarter = warp % 4, 32 of a tile's 64 columns = (warp / 4) % 2), each team with its
-//                 own S/dP and P/dS columns, so that one team's barrier round trips and products run
-//                 under the other one's arithmetic
+//                 quarter = warp % 4, 32 of a tile's 64 columns = (warp / 4) % 2), so that one team's
+//                 barrier round trips and products run under the other one's arithmetic
 //   warps 16, 19: TMA producers, one for Q and K (and LSE2), one for dO and V (and delta): an SM starts a
 //                 copy only every 190 cycles or so from one warp, and four tiles and four vectors a
 //                 superstep from a single one (1,270 cycles) were what the whole kernel waited for
 //   warps 17, 24: issue the S/dP MMAs, one for each team (a wait, eight MMAs and their commit take an
 //                 issuer longer than the superstep); warp 17 owns TMEM
-//   warp 18     : issues the accumulating MMAs (all issuers run warp-wide with one elected lane issuing)
+//   warps 18, 25: issue the accumulating MMAs (dK/dV: one warp for dV, one for dK; dQ: one for the lanes
+//                 of tile a, one for tile b): a single issuer was at work 1,050 of the 1,370 cycles of a
+//                 superstep, its own waits and commits between batches included.  All issuers run
+//                 warp-wide with one elected lane issuing
 //   warps 20..23: take a block's sums out of tensor memory and store them while the compute warps are
 //                 already at work on the next block
 // A block's own operands are double-buffered: the next block's are loaded while this one is at work.
 // Head dimensions 16 and 32: zero-filled on load by D-wide tensor maps, D / 16 K steps for S and dP,
 // D-wide accumulating products.
+// S and dP of a superstep have one of three slots in TMEM, and P and dS are stored over them: the
+// next superstep but two is what its products must be complete for, not the team's own next one.
+// What bounds it: shared memory.  A dK/dV superstep takes about 1,000 of its port's cycles (S and dP
+// operands 384, accumulating operands 256, copies arriving 256, LSE2 and delta 128) of 1,250 to 1,340
+// in all, a dQ superstep 770 of 1,000; the exponentials take a third of it.  B=2, H=16, N=16384, 25 % of
+// the tiles under a causal mask, both kernels: 1,650 us with M=128 products and one team, 1,430 us with
+// separate S/dP and P/dS columns for each team, 1,347 us with slots and an issuer for each output.
 // Every wait is bounded and every barrier is waited on by warps that see each of its phases.
 #include <math.h>
 
@@ -59,14 +68,18 @@ template <bool kDKDV> constexpr int kRing1 = kRing - kRing0<kDKDV>;
 constexpr int kCW = 16;                    // compute warps: 2 teams x 4 lane quarters x 2 column halves
 constexpr int kTeamW = kCW / 2;
 constexpr int kProdWarp = kCW, kXWarp = kCW + 1, kAccWarp = kCW + 2, kProd2Warp = kCW + 3;
-constexpr int kX2Warp = kCW + 8;           // (warps kCW + 4 .. kCW + 7 write out: lane quarter = warp % 4)
+constexpr int kX2Warp = kCW + 8, kAcc2Warp = kCW + 9;           // (warps kCW + 4 .. kCW + 7 write out: lane quarter = warp % 4)
 constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: three warps at the end only fill one
 constexpr uint32_t kBwdTile = 64 * 64 * 2;
 constexpr uint32_t kBwdTmemCols = 512;
 constexpr int kListIndex = BSA_LIST_PARTIAL_FLAG - 1;  // a list entry without its flag
-// TMEM columns: S (or S^T) of team T at 128 T, its dP (or dP^T) at 128 T + 64; P and dS as 16-bit
-// pairs, 32 columns each, at 256 + 64 T; two fp32 accumulators.
-constexpr uint32_t kTmP = 256, kTmAcc0 = 384, kTmAcc1 = 448;
+// TMEM columns: slot x at 128 x holds S (or S^T) and, 64 further on, dP (or dP^T) of supersteps
+// g % kSlots == x; then P (as 16-bit pairs) over the first half of each 32 columns of S, dS over
+// those of dP: a warp only overwrites what it has read itself.  Two fp32 accumulators.
+constexpr uint32_t kTmAcc0 = 384, kTmAcc1 = 448;
+// The issuers and teams see every second superstep, so the barriers that they wait on come twice for
+// each slot.
+constexpr int kSlots = 3, kXBars = 2 * kSlots;
 
 struct BwdSmem {
   uint8_t stat[2][2][kBwdTile];             // by block parity: the CTA's own K, V (dK/dV) or Q, dO (dQ)
@@ -85,10 +98,12 @@ struct BwdSmem {
   // a place's tiles have landed: one barrier for each place and team, so that the team's issuer and
   // compute warps, which wait on it, see each of its phases
   uint64_t in_full0[2 * kRing0<false>], in_full1[2 * kRing1<true>];
-  uint64_t in_empty0[kRing0<false>];        // accumulating MMAs of the superstep complete
+  uint64_t in_empty0[kRing0<false>];        // accumulating MMAs that read the place complete
   uint64_t in_empty1[kRing1<true>];         // ... (dQ: dP complete)
-  uint64_t x_full[2], x_free[2];            // by team: S/dP complete; S/dP in the compute warps' registers
-  uint64_t d_full[2], d_free[2];            // P/dS stored; accumulating MMAs that read them complete
+  // by superstep modulo kXBars, that is by slot and team:
+  uint64_t x_full[kXBars];                  // S/dP complete (dK/dV: and LSE2 and delta there)
+  uint64_t d_free[kXBars];                  // accumulating MMAs that read P/dS complete: the slot is free
+  uint64_t d_full[kSlots];                  // by slot: P/dS stored
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -204,7 +219,6 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
   constexpr int kR0 = kRing0<kDKDV>, kR1 = kRing1<kDKDV>;
   constexpr uint64_t kTileDesc = kBwdTile >> 4;  // one tile further, in descriptor units
   const int k_steps = p.D >> 4;
-  const uint32_t x_full = smem_u32(&sm->x_full[team]), x_free = smem_u32(&sm->x_free[team]);
   bool ok = true;
   int gs = 0, ni = 0;
   for (int i = 0; ok; ++i) {
@@ -222,28 +236,89 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
       ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, abort_flag) &&
            mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, abort_flag);
       if (!ok) break;
-      // the team must have its previous S/dP in registers (for the first one this asks for the
-      // phase before the first one, which counts as complete)
-      ok = mbar_wait_warp(x_free, ((g >> 1) & 1) ^ 1, abort_flag);
+      // the accumulating products of the slot's previous superstep must be complete
+      if (g >= kSlots)
+        ok = mbar_wait_warp(smem_u32(&sm->d_free[(g - kSlots) % kXBars]), ((g - kSlots) / kXBars) & 1,
+                            abort_flag);
       if (!ok) break;
       tc_fence_after();
       if (leader) {
+        const uint32_t x_at = tmem + 128 * (g % kSlots);
+        const uint32_t x_full = smem_u32(&sm->x_full[g % kXBars]);
         // (a superstep with one tile multiplies with whatever the second tile's place holds: nobody
         // reads those lanes)
         const uint64_t b0 = desc_b0 + static_cast<uint64_t>(2 * (g % kR0)) * kTileDesc;
         const uint64_t b1 = desc_b1 + static_cast<uint64_t>(2 * (g % kR1)) * kTileDesc;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          if (kk < k_steps) umma_ws_ss(tmem + 128 * team, a0 + 2 * kk, b0 + 2 * kk, idesc_x, kk > 0);
+          if (kk < k_steps) umma_ws_ss(x_at, a0 + 2 * kk, b0 + 2 * kk, idesc_x, kk > 0);
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           if (kk < k_steps)
-            umma_ws_ss(tmem + 128 * team + 64, a0 + kTileDesc + 2 * kk, b1 + 2 * kk, idesc_x, kk > 0);
+            umma_ws_ss(x_at + 64, a0 + kTileDesc + 2 * kk, b1 + 2 * kk, idesc_x, kk > 0);
         tc_commit(x_full);
+        if constexpr (kDKDV) mbar_arrive(x_full);  // release: LSE2 and delta have been seen to be there
         if constexpr (!kDKDV) tc_commit(smem_u32(&sm->in_empty1[g % kR1]));  // V is not needed any more
       }
     }
     if (ok && leader) tc_commit(smem_u32(&sm->stat_free[own]));  // this issuer is through with the operands
+    ++ni;
+  }
+  if (!ok) bwd_give_up(sm, p.status, 2);
+}
+
+// The accumulating instructions of one warp.  dK/dV: the first warp's sum dV, the second one's dK (each
+// accumulator has one issuer, which keeps its products in order); dQ: the first warp's write the lanes
+// of tile a, the second one's those of tile b.
+template <bool kBf16, bool kDKDV>
+__device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, uint32_t tmem, bool first,
+                                              int lane, volatile int* abort_flag) {
+  const bool dv = kDKDV && first;
+  const uint32_t idesc = umma_idesc(kBf16, 0, 1, 128, p.D);
+  const bool leader = elect_one();
+  const int places = dv ? kRing1<kDKDV> : kRing0<kDKDV>;
+  const uint64_t desc = smem_desc_sw128(smem_u32(sm->ring[dv ? kRing0<kDKDV> : 0][0]), 8192, 1024);
+  const uint32_t empty = smem_u32(dv ? sm->in_empty1 : sm->in_empty0);
+  const uint32_t acc = tmem + (dv ? kTmAcc0 : kTmAcc1), from = tmem + (dv ? 0 : 64);
+  bool ok = true;
+  int ni = 0, place = 0, slot = 0, x = 0;
+  uint32_t phase = 0;  // of the slot's barrier
+  for (int i = 0; ok; ++i) {
+    int w, w_tiles, w_begin;
+    ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+    if (!ok || w < 0) break;
+    if (w_tiles == 0) continue;
+    // the write-out warps must have read the previous block's accumulators
+    if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1, abort_flag);
+    for (int left = w_tiles; ok && left > 0; left -= 2) {
+      ok = mbar_wait_warp(smem_u32(&sm->d_full[slot]), phase, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      if (leader) {
+        // rows [16 kk, +16) of a streamed tile: column 8 (kk % 2) of the 32 columns of P or dS of warp
+        // column half kk / 2; tile a's in lanes 0..63, tile b's in lanes 64..127; each product writes
+        // the lanes of its tile only
+        const uint32_t cols = from + 128 * slot;
+        const uint64_t b0 = desc + static_cast<uint64_t>(2 * place * (kBwdTile >> 4));
+        const uint32_t more = left != w_tiles;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          if (kDKDV || first)
+            umma_ts_half(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + 128 * kk, idesc, more | (kk > 0), 0);
+        if (left > 1 && (kDKDV || !first)) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_ts_half(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + (kBwdTile >> 4) + 128 * kk, idesc,
+                         more | (kk > 0), 1);
+        }
+        tc_commit(empty + 8 * place);  // place free
+        tc_commit(smem_u32(&sm->d_free[x]));  // P or dS columns free; accumulator updated
+        if (left <= 2) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
+      }
+      if (++place == places) place = 0;
+      if (++x == kXBars) x = 0;
+      if (++slot == kSlots) slot = 0, phase ^= 1;
+    }
     ++ni;
   }
   if (!ok) bwd_give_up(sm, p.status, 2);
@@ -273,19 +348,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->item_full[i]), 1);
-      mbar_init(smem_u32(&sm->item_free[i]), kCW + 8);  // all roles but the first producer
+      mbar_init(smem_u32(&sm->item_free[i]), kCW + 8 + 1);  // all roles but the first producer
       mbar_init(smem_u32(&sm->stat_full[i]), 2);  // two producers
       mbar_init(smem_u32(&sm->stat_free[i]), 2);  // two S/dP issuers
-      mbar_init(smem_u32(&sm->x_full[i]), 1);
-      mbar_init(smem_u32(&sm->x_free[i]), kTeamW);  // one arrival per warp of the team
-      mbar_init(smem_u32(&sm->d_full[i]), kTeamW);
-      mbar_init(smem_u32(&sm->d_free[i]), 1);
+    }
+    for (int i = 0; i < kSlots; ++i) mbar_init(smem_u32(&sm->d_full[i]), kTeamW);  // one arrival per warp
+    for (int i = 0; i < kXBars; ++i) {
+      mbar_init(smem_u32(&sm->x_full[i]), kDKDV ? 2 : 1);
+      mbar_init(smem_u32(&sm->d_free[i]), 2);
     }
     for (int s = 0; s < 2 * kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_full0[s]), 1);
     for (int s = 0; s < 2 * kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_full1[s]), 1);
-    for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), 1);
+    for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), kDKDV ? 1 : 2);
     for (int s = 0; s < kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
-    mbar_init(smem_u32(&sm->acc_done), 1);
+    mbar_init(smem_u32(&sm->acc_done), 2);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
     sm->abort_flag = 0;
     mbar_fence_init();
@@ -309,7 +385,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
 
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
   // issuers do without (56 + 104 + 56 = 3 x 72).
-  if (warp >= kCW && warp < kCW + 4) {
+  if ((warp >= kCW && warp < kCW + 4) || warp >= kCW + 8) {
     give_registers<56>();
     if (warp == kProdWarp) {
       // =========================== TMA producer ===========================
@@ -401,57 +477,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         ++ni;
       }
       if (!ok) bwd_give_up(sm, p.status, 1);
-    } else if (warp == kXWarp) {
-      bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, 0, lane, abort_flag);
-    } else if (warp == kAccWarp) {
-      // =========================== accumulating-MMA issuer ===========================
-      const uint32_t idesc_acc = umma_idesc(kBf16, 0, 1, 128, p.D);
-      const bool leader = elect_one();
-      const uint64_t desc_m0 = smem_desc_sw128(smem_u32(sm->ring[0][0]), 8192, 1024);
-      const uint64_t desc_m1 = smem_desc_sw128(smem_u32(sm->ring[kRing0<kDKDV>][0]), 8192, 1024);
-      bool ok = true;
-      int gs = 0, ni = 0;
-      for (int i = 0; ok; ++i) {
-        int w, w_tiles, w_begin;
-        ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
-        if (!ok || w < 0) break;
-        const int n_super = (w_tiles + 1) >> 1;
-        if (n_super == 0) continue;
-        // the write-out warps must have read the previous block's accumulators
-        if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1, abort_flag);
-        for (int j = 0; ok && j < n_super; ++j, ++gs) {
-          const int s0 = gs % kRing0<kDKDV>, s1 = gs % kRing1<kDKDV>, team = gs & 1;
-          const int nt = min(2, w_tiles - 2 * j);
-          ok = mbar_wait_warp(smem_u32(&sm->d_full[team]), (gs >> 1) & 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          if (leader) {
-            // keys/queries [16 kk, +16) of a tile sit at column 8 kk of the P / dS columns, tile a's in
-            // lanes 0..63, tile b's in lanes 64..127; each product writes the lanes of its tile only
-            const uint32_t p_cols = tmem + kTmP + 64 * team, ds_cols = p_cols + 32;
-            for (int t = 0; t < nt; ++t) {
-              if constexpr (kDKDV) {
-                const uint64_t bmn = desc_m1 + static_cast<uint64_t>((2 * s1 + t) * (kBwdTile >> 4));
-#pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-                  umma_ts_half(tmem + kTmAcc0, p_cols + 8 * kk, bmn + 128 * kk, idesc_acc,
-                               (j > 0) || (kk > 0), t);
-              }
-              const uint64_t bmn = desc_m0 + static_cast<uint64_t>((2 * s0 + t) * (kBwdTile >> 4));
-#pragma unroll
-              for (int kk = 0; kk < 4; ++kk)
-                umma_ts_half(tmem + kTmAcc1, ds_cols + 8 * kk, bmn + 128 * kk, idesc_acc,
-                             (j > 0) || (kk > 0), t);
-            }
-            tc_commit(smem_u32(&sm->in_empty0[s0]));  // places free
-            if constexpr (kDKDV) tc_commit(smem_u32(&sm->in_empty1[s1]));
-            tc_commit(smem_u32(&sm->d_free[team]));  // P/dS columns free; accumulators updated
-            if (j == n_super - 1) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
-          }
-        }
-        ++ni;
-      }
-      if (!ok) bwd_give_up(sm, p.status, 2);
+    } else if (warp == kXWarp || warp == kX2Warp) {
+      bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane, abort_flag);
+    } else if (warp == kAccWarp || warp == kAcc2Warp) {
+      bwd_issue_acc<kBf16, kDKDV>(sm, p, tmem, warp == kAccWarp, lane, abort_flag);
     }
   } else if (warp < kCW) {
     // =========================== compute warps ===========================
@@ -461,8 +490,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     const int t_mine = quarter >> 1;    // lanes 0..63 own tile a of a superstep, 64..127 tile b
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the CTA's block
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t s_at = tmem + lane_base + 128 * team + 32 * ch, dp_at = s_at + 64;
-    const uint32_t p_at = tmem + lane_base + kTmP + 64 * team + 16 * ch, ds_at = p_at + 32;
+    const uint32_t x_base = tmem + lane_base + 32 * ch;
     const float c = p.scale_log2;
     bool ok = true;
     int gs = 0;  // supersteps of earlier items; this team takes those with gs % 2 == team
@@ -497,7 +525,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       gs += n_super;
       for (; ok && j < n_super; j += 2, g += 2) {
         const bool active = 2 * j + t_mine < w_tiles;  // this lane's tile exists (warp-uniform)
-        const uint32_t ph = (g >> 1) & 1;
+        const uint32_t s_at = x_base + 128 * (g % kSlots), dp_at = s_at + 64;
         // A tile with masked elements inside: fetch this lane's 32 mask bytes while S is on its way
         uint32_t mw[8];
         bool partial = false;
@@ -526,36 +554,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
             }
           }
         }
-        if constexpr (kDKDV) {
-          // the LSE2/delta vectors of this stage arrive through the async proxy
-          constexpr int kR0 = kRing0<true>, kR1 = kRing1<true>;
-          ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, abort_flag) &&
-               mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, abort_flag);
-          if (!ok) break;
-        }
-        ok = mbar_wait_warp(smem_u32(&sm->x_full[team]), ph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->x_full[g % kXBars]), (g / kXBars) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (active) {
           const float4* lse4 = reinterpret_cast<const float4*>(&sm->lse[g % kRing0<true>][t_mine][32 * ch]);
           const ulonglong2* del4 = reinterpret_cast<const ulonglong2*>(&sm->delta[g % kRing1<true>][t_mine][32 * ch]);
-          // 16 columns at a time in a loop: half the code, and no more than 32 logits in registers
+          // 8 columns at a time, the next ones on their way from tensor memory meanwhile (straight through
+          // all 32 the registers do not suffice)
+          uint32_t xsb[2][8], xdb[2][8];
+          tmem_ld_32x32b_x8(s_at, xsb[0]);
+          tmem_ld_32x32b_x8(dp_at, xdb[0]);
 #pragma unroll
-          for (int half16 = 0; half16 < 2; ++half16) {
-            uint32_t xs[16], xd[16], pk_p[8], pk_ds[8];
-            tmem_ld_32x32b_x16(s_at + 16 * half16, xs);
-            tmem_ld_32x32b_x16(dp_at + 16 * half16, xd);
+          for (int c8 = 0; c8 < 4; ++c8) {
+            uint32_t *xs = xsb[c8 & 1], *xd = xdb[c8 & 1], pk_p[4], pk_ds[4];
             tc_wait_ld();
-            if (half16 == 1) {  // S/dP are in registers: the team's next ones may be issued
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(smem_u32(&sm->x_free[team]));
-            }
             if (partial) {
               // masked elements: logit -inf, so P = 0 and with it dS = 0
 #pragma unroll
-              for (int q4 = 0; q4 < 4; ++q4) {
-                const uint32_t nz = __vcmpne4(mw[4 * half16 + q4], 0u);
+              for (int q4 = 0; q4 < 2; ++q4) {
+                const uint32_t nz = __vcmpne4(mw[2 * c8 + q4], 0u);
 #pragma unroll
                 for (int bb = 0; bb < 4; ++bb) {
                   const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
@@ -563,16 +581,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
                 }
               }
             }
+            if (c8 < 3) {
+              tmem_ld_32x32b_x8(s_at + 8 * c8 + 8, xsb[(c8 + 1) & 1]);
+              tmem_ld_32x32b_x8(dp_at + 8 * c8 + 8, xdb[(c8 + 1) & 1]);
+            }
 #pragma unroll
-            for (int q = 0; q < 16; q += 4) {
+            for (int q = 0; q < 8; q += 4) {
               // two columns per instruction where the operands allow it
               float pv[4], dsv[4], nl[4];
               uint64_t d2[2];
               if constexpr (kDKDV) {
                 // LSE and delta differ from column to column here
                 // (-inf = a query row with every element masked: see my_lse above)
-                const float4 lv = lse4[4 * half16 + q / 4];
-                const ulonglong2 dv = del4[4 * half16 + q / 4];
+                const float4 lv = lse4[2 * c8 + q / 4];
+                const ulonglong2 dv = del4[2 * c8 + q / 4];
                 nl[0] = lv.x; nl[1] = lv.y; nl[2] = lv.z; nl[3] = lv.w;
                 if constexpr (kElementMask) {
 #pragma unroll
@@ -606,32 +628,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
               pk_ds[q / 2] = pack_2x16<kBf16>(dsv[0], dsv[1]);
               pk_ds[q / 2 + 1] = pack_2x16<kBf16>(dsv[2], dsv[3]);
             }
-            if (half16 == 0) {
-              // the accumulating MMAs of the team's previous superstep must be through with the P/dS
-              // columns
-              ok = mbar_wait_warp(smem_u32(&sm->d_free[team]), ph ^ 1, abort_flag);
-              tc_fence_after();
-            }
-            if (!ok) break;
-            if constexpr (kDKDV) tmem_st_32x32b_x8(p_at + 8 * half16, pk_p);
-            tmem_st_32x32b_x8(ds_at + 8 * half16, pk_ds);
+            if constexpr (kDKDV) tmem_st_32x32b_x4(s_at + 4 * c8, pk_p);
+            tmem_st_32x32b_x4(dp_at + 4 * c8, pk_ds);
           }
           tc_wait_st();
-        } else {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(&sm->x_free[team]));
-          ok = mbar_wait_warp(smem_u32(&sm->d_free[team]), ph ^ 1, abort_flag);
         }
-        if (!ok) break;
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->d_full[team]));
+        if (lane == 0) mbar_arrive(smem_u32(&sm->d_full[g % kSlots]));
       }
       // (the block's sums are merged and stored by the write-out warps; these warps go straight
       // on to the next block, whose first S/dP is usually complete already)
     }
     if (!ok) bwd_give_up(sm, p.status, 3);
-  } else if (warp < kCW + 8) {
+  } else {
     // =========================== write-out ===========================
     // Lane r of an accumulator holds the tile-a sums of row r of the CTA's block, lane r+64 its tile-b
     // sums (unwritten when the list has a single tile).  These four warps (lane quarter = warp % 4)
@@ -735,9 +745,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       if (any_failed) break;
     }
     if (!ok) bwd_give_up(sm, p.status, 3);
-  } else {
-    give_registers<56>();
-    if (warp == kX2Warp) bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, 1, lane, abort_flag);
   }
 
   // (not before: CTAs of the next kernel that wait on free SMs slowed the working ones down by 3 %)

@@ -18,7 +18,6 @@ namespace bsa {
 // Eight lanes own one 128-byte row (64 16-bit values): a warp covers 4 rows per step and a CTA of
 // 8 warps covers 128 rows with 4 independent steps in flight per thread.
 constexpr int kDeltaThreads = 256;
-constexpr int kDeltaRowsPerCta = 128;
 
 template <bool kBf16>
 __device__ __forceinline__ float dot8(const uint4& a, const uint4& b) {

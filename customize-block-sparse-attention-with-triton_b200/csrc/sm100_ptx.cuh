@@ -112,22 +112,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// A look at the barrier that never parks the thread (try_wait may hold it for a system-dependent
-// time, microseconds, when the phase is not complete): for "is it there already?" questions whose
-// answer "no" must not cost anything.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// The same test, but the hardware may park the thread for up to about `hint_ns` until the phase
+// mbar_try_wait, but the hardware may park the thread for up to about `hint_ns` until the phase
 // completes instead of returning at once: a waiting warp then issues next to nothing.
 __device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
   uint32_t ok;
@@ -214,11 +199,6 @@ __device__ __forceinline__ void bulk_load_1d(uint32_t dst_smem, const void* src,
       ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
       : "memory");
 }
-// Makes this thread's earlier ordinary writes to shared memory visible to the async proxy (TMA,
-// tcgen05.mma operand reads); follow it with a barrier before the reader is released.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 
 // ---------------------------------------------------------------------------------------------
 // tcgen05: TMEM allocation
@@ -262,17 +242,7 @@ __device__ __forceinline__ void tc_wait_st() {
 // ---------------------------------------------------------------------------------------------
 // tcgen05.mma.kind::f16 (fp16/bf16 inputs, fp32 accumulate), one CTA
 // ---------------------------------------------------------------------------------------------
-// D[tmem] (+)= A[smem desc] * B[smem desc]
-__device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with M = 64 rows of A in the "weight stationary" form: columns [0, N/2) of the result
+// D[tmem] (+)= A[smem desc] * B[smem desc] with M = 64 rows of A in the "weight stationary" form: columns [0, N/2) of the result
 // go to TMEM lanes 0..63, columns [N/2, N) to lanes 64..127 of the same N/2 TMEM columns, so all
 // lanes are used (the ordinary M = 64 form runs at half rate).
 __device__ __forceinline__ void umma_ws_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
@@ -284,17 +254,6 @@ __device__ __forceinline__ void umma_ws_ss(uint32_t d_tmem, uint64_t a_desc, uin
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc]
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                        uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // D[tmem] (+)= A[tmem] * B[smem desc] for lanes 0..63 (half = 0) or 64..127 (half = 1) only: the other
 // lanes of D keep what they hold, whatever their rows of A are.  Same rate as the full form.
 __device__ __forceinline__ void umma_ts_half(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
@@ -390,25 +349,17 @@ __device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t* r) {
+__device__ __forceinline__ void tmem_st_32x32b_x4(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
-      "r"(r[7])
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr)
       : "memory");
-}
-// n columns (32 or 16 on a load, 16 or 8 on a store) of the warp's 32 lanes
-template <int kCols>
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r) {
-  static_assert(kCols == 32 || kCols == 16, "column count");
-  if constexpr (kCols == 32) tmem_ld_32x32b_x32(taddr, r);
-  else tmem_ld_32x32b_x16(taddr, r);
-}
-template <int kCols>
-__device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t* r) {
-  static_assert(kCols == 16 || kCols == 8, "column count");
-  if constexpr (kCols == 16) tmem_st_32x32b_x16(taddr, r);
-  else tmem_st_32x32b_x8(taddr, r);
 }
 
 // One 32-byte store (a whole sector) instead of two 16-byte ones; the address must be 32-byte
