@@ -28,8 +28,8 @@
 // at the same time, and 2.5 KB more in the softmax loop made everything 10 % slower.  So what is
 // executed per item or per superstep is kept short, waits included.
 // B200, fp16, D = 64, against the form with M = 128 products and both teams on every superstep:
-// N = 17536 with one head, all blocks 136 -> 110 us, a tenth of them 27.0 -> 23.7 us; 8 heads, a
-// tenth 133 -> 110 us; bf16 N = 32000, 32 heads, a tenth 1.53 -> 1.31 ms.
+// N = 17536 with one head, all blocks 136 -> 104 us, a tenth of them 27.0 -> 21.5 us; 8 heads, a
+// tenth 133 -> 103 us; bf16 N = 32000, 32 heads, a tenth 1.53 -> 1.25 ms.
 //
 // Roles (16 warps); every role walks the same item sequence, so set-up of item i+1 and write-out
 // of item i-1 overlap the arithmetic of item i:
@@ -58,11 +58,11 @@
 //
 // Numerics follow the reference's loop (fa2_custom_mask/fa2_fwd.py:150-196): logits scaled by
 // sm_scale*log2(e), exp2 domain, fp32 row sums of the fp32 probabilities, P rounded to the input
-// dtype before P V.  The reference maximum of a row is the maximum of its first tiles and moves only
-// when later logits would make probabilities too large for 16 bit (sum of a superstep above 4096),
-// which leaves O = acc / l unchanged because both use the same reference.  Which partial result a
-// tile goes into depends on its position in the row's list alone, so results do not depend on which
-// CTA computes an item.
+// dtype before P V.  The reference maximum of a row comes from its first 32 logits and moves only
+// when later ones would make probabilities too large for 16 bit (sum of a superstep above 4096), which
+// leaves O = acc / l unchanged because both use the same reference.  Which partial result a tile
+// goes into depends on its position in the row's list alone, so results do not depend on which CTA
+// computes an item.
 //
 // Every wait is bounded; a wait that gives up raises a CTA-wide flag, every role then falls
 // through its loops without touching barriers' data again, and TMEM is always released.  Every
@@ -643,7 +643,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       for (int u = 0; u < n_super && ok; ++u, team ^= 1) {
         const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph, abort_flag);
+        // V first: it is there long before P, whose arrival is what the superstep waits for (each look at
+        // a barrier costs some 50 cycles, and there were two between P and its products: 3 % with
+        // everything listed)
+        const int vs1 = vs + 1 < kVStages ? vs + 1 : 0;
+        ok = mbar_wait_warp(smem_u32(&sm->v_full[vs]), vph, abort_flag) &&
+             (nt <= 2 || mbar_wait_warp(smem_u32(&sm->v_full[vs1]), vs1 > 0 ? vph : vph ^ 1, abort_flag)) &&
+             mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
         // Tiles a and b have their P in columns [0, 32) of the slot, a in lanes 0..63 and b in lanes
@@ -652,9 +658,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t o_acc = tmem + kTmemO + 64 * team;
         for (int pair = 0; pair < 2; ++pair) {
           if (2 * pair >= nt) break;
-          ok = mbar_wait_warp(smem_u32(&sm->v_full[vs]), vph, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
           if (leader) {
             const uint32_t p_cols = tmem + 128 * slot + 32 * pair;
             const uint64_t desc_v = desc_v0 + static_cast<uint64_t>(vs * 2) * (kTileBytes >> 4);
@@ -718,12 +721,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         ok = mbar_wait_warp(smem_u32(&sm->s_full[bar_s]), bar_ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        // The row maximum is looked up only where it is needed: for the item's first superstep of
-        // the team (and when the caller wants it, or with element masks, under which a row may have
-        // nothing yet).  Otherwise the logits are exponentiated against the reference maximum as it
-        // is; a row whose sum shows that this was too low (or not finite) makes the warp do the
-        // superstep again with the maximum.  S is still in tensor memory then: P goes over it last.
-        bool with_max = kElementMask || u < 2 || p.rowmax != nullptr;
+        // The row maximum is looked up only where it is needed: when the caller wants it, and with
+        // element masks as long as one of the warp's rows has nothing yet.  The first superstep of the
+        // team takes the maximum of 32 logits for a reference (all 128 cost 450 cycles more), and
+        // logits are exponentiated against that as it is; a row whose sum shows that it was too low (or
+        // not finite) makes the warp do the superstep again with the maximum of all its logits.  S is
+        // still in tensor memory then: P goes over it last.
+        bool all = p.rowmax != nullptr;
+        if constexpr (kElementMask) all |= u >= 2 && __any_sync(0xffffffffu, m_ref == -INFINITY);
+        bool with_max = all || u < 2;
         if (mine > 0) {
           const bool two = mine > 2;  // both tiles exist (warp-uniform)
           const auto masked = [&](uint32_t* sr, int col) {
@@ -740,13 +746,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (with_max) {
               float zmax = -INFINITY;
 #pragma unroll 1
-              for (int col = 0; col < (two ? 128 : 64); col += 32) {
+              for (int col = 0; col < (!all ? 32 : two ? 128 : 64); col += 32) {
                 tmem_ld_32x32b_x32(s_addr + col, sa);
                 tc_wait_ld();
                 masked(sa, col);
                 zmax = fmaxf(zmax, max_chunk(sa));
               }
               const float alpha = fwd_new_max(zmax * c, m_ref, m_true, l);
+              if (kElementMask && !all && __any_sync(0xffffffffu, m_ref == -INFINITY)) {
+                all = true;  // a row has nothing among those 32
+                m_ref = -INFINITY;
+                continue;
+              }
               if (__any_sync(0xffffffffu, alpha != 1.f)) {
                 // the previous product of this team, two supersteps ago, must be in O
                 const int prev = slot == 2 ? 0 : slot + 1;  // (slot - 2) % 3
@@ -780,8 +791,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             float a0, a1;
             unpack_f32x2(add_f32x2(l0, l1), a0, a1);
             sum = a0 + a1;
-            if (with_max || !__any_sync(0xffffffffu, !(sum <= kMaxRowSum))) break;
-            with_max = true;
+            if (all || !__any_sync(0xffffffffu, !(sum <= kMaxRowSum))) break;
+            all = with_max = true;
+            if (u < 2) m_ref = -INFINITY;  // nothing is summed against it yet
           }
           if (!ok) break;
           l += sum;

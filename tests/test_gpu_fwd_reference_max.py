@@ -26,3 +26,23 @@ def test_logits_that_jump_at_one_block(lib, nb, dtype, tol, D):
         assert (o.float().cpu() - o_ref).abs().max().item() <= tol, (nb, pos)
         err = (lse2.cpu() * 0.6931471805599453 - lse_ref).abs().max().item()
         assert err <= 2e-3 * max(1.0, lse_ref.abs().max().item() / 8), (nb, pos, err)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("nb", [1, 2, 3, 4, 5, 9])
+def test_logits_that_jump_inside_the_first_blocks(lib, nb, dtype):
+    """The reference of a row comes from the first 32 keys of its first tile; here the keys behind
+    them, or the row's second tile, have logits that would not go into 16 bit against it."""
+    from fa2_custom_mask import attention_forward_masked
+    for start in (32, 64, 128):
+        if start >= 64 * nb:
+            continue
+        q, k, v = (t.to(dtype) for t in oracle.make_qkv(1, 2, 64 * nb, 64, seed=nb + start))
+        k[:, :, :start] *= 0.01
+        k[:, :, start:] *= 25
+        mask = torch.ones(1, 1, nb, nb, dtype=torch.bool)
+        o, lse2, rowmax = attention_forward_masked(q.cuda(), k.cuda(), v.cuda(), mask.cuda(), 0.125)
+        o_ref, lse_ref = oracle.attn_forward(q, k, v, mask.expand(1, 2, nb, nb), 0.125)
+        assert (o.float().cpu() - o_ref).abs().max().item() <= 2e-2, (nb, start)
+        err = (lse2.cpu() * 0.6931471805599453 - lse_ref).abs().max().item()
+        assert err <= 2e-3 * max(1.0, lse_ref.abs().max().item() / 8), (nb, start, err)
