@@ -135,13 +135,14 @@ bool run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& 
 }
 
 // ---------------------------------------------------------------------------------------------
-// Errors of the backward: raised by the Python layer's function (fn, status), on whatever thread
+// Errors of the backward: raised by the Python layer's function (fn, status, what a kernel reported), on
+// whatever thread
 // ---------------------------------------------------------------------------------------------
 PyObject* raise_error = nullptr;
 
-[[noreturn]] void raise_in_python(const char* fn, int status) {
+[[noreturn]] void raise_in_python(const char* fn, int status, int code = 0) {
   pybind11::gil_scoped_acquire gil;
-  PyObject* r = PyObject_CallFunction(raise_error, "si", fn, status);
+  PyObject* r = PyObject_CallFunction(raise_error, "sii", fn, status, code);
   Py_XDECREF(r);  // (it always raises)
   python_error err;
   err.persist();
@@ -149,6 +150,14 @@ PyObject* raise_error = nullptr;
 }
 void check(const char* fn, int rc) {
   if (rc != 0) raise_in_python(fn, rc);
+}
+
+// Raises what an earlier kernel reported on this stream, if anything.  The report is taken: the word is
+// zero again, and of several threads that look at the same time one raises.
+void raise_if_reported(StreamState* state) {
+  if (state == nullptr || *state->word == 0) return;
+  const int code = __atomic_exchange_n(state->word, 0, __ATOMIC_RELAXED);
+  if (code != 0) raise_in_python("flash_attention_custom_mask", BSA_ERR_DEVICE_TIMEOUT, code);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -205,7 +214,7 @@ struct AttentionBackward : torch::autograd::Node {
     const c10::cuda::CUDAGuard guard(q.device());
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
     StreamState* state = stream_state(q.device().index(), stream);
-    if (state != nullptr && *state->word != 0) raise_in_python("flash_attention_custom_mask", -9);
+    raise_if_reported(state);
     int32_t* counter = state ? state->counter_ptr : nullptr;
     int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
     // the gradients are laid out like the tensors they belong to, gaps included

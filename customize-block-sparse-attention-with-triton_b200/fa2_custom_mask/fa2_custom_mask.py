@@ -247,9 +247,7 @@ class _StreamState:
         code = int(self.status[0])
         if code != 0:
             self.status.zero_()
-            raise _lib.BsaError("flash_attention_custom_mask", -9,
-                                f"a bounded wait inside an earlier kernel on this stream gave up "
-                                f"(role {code}); its results are incomplete")
+            _raise_native("flash_attention_custom_mask", -9, code)
 
 
 _stream_states = {}
@@ -266,11 +264,12 @@ def _stream_state(device: torch.device, stream: int) -> Optional[_StreamState]:
     return st
 
 
-def _raise_native(fn: str, status: int):
-    """Raises what a step of the native host path reported."""
+def _raise_native(fn: str, status: int, code: int = 0):
+    """Raises what a step of the native host path returned (status) or what an earlier kernel had left in
+    the stream's status word (status -9 and that code)."""
     if status == -9:
-        for st in list(_stream_states.values()):
-            st.raise_if_reported()
+        raise _lib.BsaError(fn, status, f"a bounded wait inside an earlier kernel on this stream gave up "
+                                        f"(role {code}); its results are incomplete")
     raise _lib.BsaError(fn, status, _lib.load().bsa_strerror(status).decode())
 
 
