@@ -245,6 +245,7 @@ struct PermuteArgs {
   const void* plan;       // the axis order of a head, as an index into the six of permute_order()
   int64_t plan_stride;    // in elements
   int plan_is_64;
+  int32_t* status;        // optional
   int B, heads, T, chunks, chunk_bytes, pieces_per_cta;
   int ext[3];             // F, Hh, W
   // floor(n / d) = umulhi(n, m) for n * d < 2^32: m = floor(2^32 / d) + 1
@@ -275,9 +276,12 @@ __global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_c
   int64_t order = a.plan_is_64 ? static_cast<const int64_t*>(a.plan)[h * a.plan_stride]
                                : static_cast<const int32_t*>(a.plan)[h * a.plan_stride];
   if (order < 0) order += 6;
-  // nothing to do for the order (0,1,2); an index that is none leaves the head alone.  The same for
-  // every CTA of the cluster.
-  if (order <= 0 || order > 5) return;
+  // nothing to do for the order (0,1,2); an index that is none leaves the head alone and is reported.
+  // The same for every CTA of the cluster.
+  if (order <= 0 || order > 5) {
+    if (order != 0 && blockIdx.x == 0 && threadIdx.x == 0) report_status(a.status, BSA_REPORT_BAD_ORDER);
+    return;
+  }
   // axis orders 1..5: (0,2,1), (1,2,0), (1,0,2), (2,1,0), (2,0,1)
   const int p0 = order >= 4 ? 2 : (order == 1 ? 0 : 1);
   const int p1 = order == 1 || order == 2 ? 2 : (order == 4 ? 1 : 0);
@@ -399,6 +403,14 @@ extern "C" int bsa_permute_in_place(void* const tensors[], const int64_t* stride
                                     const void* plan, int plan_elem_bytes, int64_t plan_stride,
                                     int inverse, int B, int heads, int T, int D, int F, int Hh, int W,
                                     int elem_bytes, void* stream) {
+  return bsa_permute_in_place_status(tensors, strides, n_tensors, plan, plan_elem_bytes, plan_stride, inverse, B,
+                                     heads, T, D, F, Hh, W, elem_bytes, nullptr, stream);
+}
+
+extern "C" int bsa_permute_in_place_status(void* const tensors[], const int64_t* strides, int n_tensors,
+                                           const void* plan, int plan_elem_bytes, int64_t plan_stride,
+                                           int inverse, int B, int heads, int T, int D, int F, int Hh, int W,
+                                           int elem_bytes, int32_t* status, void* stream) {
   using namespace bsa;
   if (B <= 0 || heads <= 0 || T <= 0 || D <= 0 || F <= 0 || Hh <= 0 || W <= 0 || n_tensors < 1 ||
       n_tensors > kPermTensors || static_cast<int64_t>(F) * Hh * W != T)
@@ -434,6 +446,7 @@ extern "C" int bsa_permute_in_place(void* const tensors[], const int64_t* stride
   a.plan = plan;
   a.plan_stride = plan_stride;
   a.plan_is_64 = plan_elem_bytes == 8;
+  a.status = status;
   a.B = B;
   a.heads = heads;
   a.T = T;

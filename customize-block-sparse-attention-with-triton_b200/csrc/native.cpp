@@ -304,7 +304,8 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
 }
 
 // The image tokens (those behind the first n_text) of one to three tensors [B,heads,tokens,D] reordered in
-// place; false when the tensors, the plan or the grid are nothing that one launch takes.
+// place; false when the tensors, the plan or the grid are nothing that one launch takes, or an earlier
+// kernel has left a report.
 bool permute_tokens(const std::vector<Tensor>& tensors, const Tensor& plan, int64_t F, int64_t Hh, int64_t W,
                     int64_t n_text, bool inverse) {
   const Tensor& t0 = tensors[0];
@@ -329,9 +330,12 @@ bool permute_tokens(const std::vector<Tensor>& tensors, const Tensor& plan, int6
   }
   const c10::cuda::CUDAGuard guard(t0.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream(t0.device().index());
-  if (bsa_permute_in_place(ptrs, strides, tensors.size(), plan.const_data_ptr(), plan.element_size(),
-                           plan.stride(0), inverse ? 1 : 0, t0.size(0), t0.size(1), F * Hh * W, t0.size(3), F,
-                           Hh, W, t0.element_size(), stream) != 0)
+  StreamState* state = stream_state(t0.device().index(), stream);
+  if (state != nullptr && *state->word != 0) return false;
+  if (bsa_permute_in_place_status(ptrs, strides, tensors.size(), plan.const_data_ptr(), plan.element_size(),
+                                  plan.stride(0), inverse ? 1 : 0, t0.size(0), t0.size(1), F * Hh * W, t0.size(3),
+                                  F, Hh, W, t0.element_size(),
+                                  state ? const_cast<int32_t*>(state->word) : nullptr, stream) != 0)
     return false;
   for (const Tensor& t : tensors) t.unsafeGetTensorImpl()->bump_version();
   return true;

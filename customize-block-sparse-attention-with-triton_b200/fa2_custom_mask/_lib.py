@@ -13,6 +13,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libbsattn.so")
 
 BSA_F16, BSA_BF16 = 0, 1
+BSA_REPORT_BAD_ORDER = 64
 
 _lib = None
 
@@ -65,6 +66,8 @@ SIGNATURES = {
     "bsa_inv_reorder_strided": [_vp, _s4, _vp, _s4, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_permute_in_place": [ctypes.POINTER(_vp), _s4, _i, _vp, _i, ctypes.c_int64, _i, _i, _i, _i, _i, _i,
                              _i, _i, _i, _vp],
+    "bsa_permute_in_place_status": [ctypes.POINTER(_vp), _s4, _i, _vp, _i, ctypes.c_int64, _i, _i, _i, _i, _i,
+                                    _i, _i, _i, _i, _vp, _vp],
     "bsa_attn_fwd_block_mask_static": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _s4, _i,
                                        _i, _f, _i, _i, _i, _i, _i, _vp],
     "bsa_static_warmup": [],

@@ -235,7 +235,8 @@ class _StreamState:
     """What the public op keeps per (device, stream), here and in the native host path: the zeroed work
     counter of the persistent kernels (they leave it at zero, also after a bounded wait gave up), and a
     status word in pinned host memory, which the device can write and the host can read without a
-    synchronisation.  The kernels only ever touch the status word when a wait gave up."""
+    synchronisation.  The kernels only ever touch the status word when a wait gave up or a token
+    reorder's plan holds an axis order that is none."""
 
     def __init__(self, counter, status):
         self.counter, self.status = counter, status
@@ -243,7 +244,7 @@ class _StreamState:
     def raise_if_reported(self):
         """Looks at the status word as it is now.  A report means that some earlier call on this
         stream produced incomplete results; it surfaces at the first call after the kernel that
-        gave up has ended."""
+        left it has ended."""
         code = int(self.status[0])
         if code != 0:
             self.status.zero_()
@@ -267,6 +268,9 @@ def _stream_state(device: torch.device, stream: int) -> Optional[_StreamState]:
 def _raise_native(fn: str, status: int, code: int = 0):
     """Raises what a step of the native host path returned (status) or what an earlier kernel had left in
     the stream's status word (status -9 and that code)."""
+    if status == -9 and code == _lib.BSA_REPORT_BAD_ORDER:
+        raise IndexError("the plan of an earlier token reorder on this stream holds an axis-order index "
+                         "outside -6..5; the tokens of that head were left as they are")
     if status == -9:
         raise _lib.BsaError(fn, status, f"a bounded wait inside an earlier kernel on this stream gave up "
                                         f"(role {code}); its results are incomplete")

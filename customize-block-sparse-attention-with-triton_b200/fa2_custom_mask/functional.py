@@ -10,6 +10,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib
+from .fa2_custom_mask import _op_status
 
 # axis orders selectable per head, and their inverses (fa2_custom_mask/functional.py:23-26, 69-76)
 _PERMUTATIONS = ((0, 1, 2), (0, 2, 1), (1, 2, 0), (1, 0, 2), (2, 1, 0), (2, 0, 1))
@@ -25,6 +26,13 @@ def _tables(device):
             torch.tensor(_PERMUTATIONS, dtype=torch.int32, device=device),
             torch.tensor(_PERMUTATIONS_INV, dtype=torch.int32, device=device))
     return _table_cache[key]
+
+
+def _plan_orders(idx, device, table):
+    """The rows of the table (see _tables) that a plan's indexes name.  Indexes held by the host are
+    looked up there, where one that is out of range raises."""
+    on_device = isinstance(idx, torch.Tensor) and idx.is_cuda
+    return _tables(device if on_device else torch.device("cpu"))[table][idx]
 
 
 def _check(tensor, F, H, W):
@@ -82,19 +90,26 @@ def apply_head_wise_reorder(tensor, permute_orders, F, H, W):
 def _in_place(tensors, idx, F, H, W, n_text_tokens, inverse):
     """The reorder of all the tensors in one launch, each byte read and written once; False when the
     tensors are not made for that (a token row that is no multiple of 16 bytes, a grid that the registers
-    of 16 CTAs do not hold, a plan that is not on the device), with nothing done."""
-    return (isinstance(idx, torch.Tensor) and all(isinstance(t, torch.Tensor) and t.is_cuda for t in tensors)
-            and _lib.native().permute_tokens(tensors, idx, F, H, W, n_text_tokens, inverse))
+    of 16 CTAs do not hold, a plan that is not on the device), with nothing done.  Raises what an earlier
+    kernel on the stream has reported."""
+    if not all(isinstance(t, torch.Tensor) and t.is_cuda for t in tensors):
+        return False
+    if (isinstance(idx, torch.Tensor)
+            and _lib.native().permute_tokens(tensors, idx, F, H, W, n_text_tokens, inverse)):
+        return True
+    _op_status(tensors[0].device)
+    return False
 
 
 def permute_qkv_triton(query, key, value, permute_plan, i_block, F=13, H=30, W=45, n_text_tokens=226):
     """Reorders the image tokens of q, k, v in place (text tokens stay) and returns the same three
-    tensors, like the reference (fa2_custom_mask/functional.py:22-43)."""
+    tensors, like the reference (fa2_custom_mask/functional.py:22-43).  An axis-order index outside -6..5
+    raises IndexError: at once from a plan on the host; from one on the device its head is left as it is, and
+    the first call of this package on the stream after the kernel has ended raises."""
     idx = permute_plan['permute'][i_block]  # [N_head]
     if _in_place((query, key, value), idx, F, H, W, n_text_tokens, False):
         return query, key, value
-    permutations, _ = _tables(query.device)
-    permute_orders = permutations[idx]      # [N_head, 3]
+    permute_orders = _plan_orders(idx, query.device, 0)      # [N_head, 3]
     for t in (query, key, value):
         image = t[:, :, n_text_tokens:, :]
         _write_back(image, apply_head_wise_reorder(image, permute_orders, F, H, W), F, H, W)
@@ -119,13 +134,12 @@ def apply_inv_reorder(tensor, permute_orders, inv_permute_orders, F, H, W):
 
 def inv_permute_attn_triton(attn_out, permute_plan, i_block, F=13, H=30, W=45, n_text_tokens=226):
     """Lays the image tokens of the attention output back in place and returns attn_out
-    (fa2_custom_mask/functional.py:64-84)."""
+    (fa2_custom_mask/functional.py:64-84).  Axis-order indexes outside -6..5 as in permute_qkv_triton."""
     idx = permute_plan['permute'][i_block]
     if _in_place((attn_out,), idx, F, H, W, n_text_tokens, True):
         return attn_out
-    permutations, permutations_inv = _tables(attn_out.device)
-    permute_orders = permutations[idx]
-    inv_permute_orders = permutations_inv[idx]
+    permute_orders = _plan_orders(idx, attn_out.device, 0)
+    inv_permute_orders = _plan_orders(idx, attn_out.device, 1)
     attn_image = attn_out[:, :, n_text_tokens:, :]
     _write_back(attn_image, apply_inv_reorder(attn_image, permute_orders, inv_permute_orders, F, H, W),
                 F, H, W)

@@ -47,6 +47,10 @@ typedef enum bsa_status {
   BSA_ERR_DEVICE_TIMEOUT = -9  /* reported by bsa_check_status: a bounded device wait gave up     */
 } bsa_status;
 
+/* What a status word holds beside zero: the role whose bounded wait gave up (1, 2, …), or this: the plan of
+ * a token reorder held an axis order that is none, and the tokens of that head were left as they are. */
+#define BSA_REPORT_BAD_ORDER 64
+
 typedef enum bsa_dtype { BSA_F16 = 0, BSA_BF16 = 1 } bsa_dtype;
 
 /* Library version (BSA_VERSION of the build). No reference counterpart. */
@@ -309,12 +313,18 @@ int bsa_inv_reorder_strided(const void* in, const int64_t in_strides[4], void* o
  *   plan     : device array of the head's axis orders, as indexes (4- or 8-byte integers, plan_stride
  *              elements apart) into (0,1,2), (0,2,1), (1,2,0), (1,0,2), (2,1,0), (2,0,1)
  *   inverse  : 0 lays the tokens out in that order, 1 lays them back
+ * An index may count from the end (-6..-1).  One outside -6..5 leaves its head as it is; the form with a
+ * status word (optional, as in the attention calls) then leaves BSA_REPORT_BAD_ORDER there.
  * BSA_ERR_TOO_LARGE or BSA_ERR_BAD_STRIDE: use the reorder calls above with a second tensor.
  */
 int bsa_permute_in_place(void* const tensors[], const int64_t* strides, int n_tensors,
                          const void* plan, int plan_elem_bytes, int64_t plan_stride, int inverse,
                          int B, int heads, int T, int D, int F, int Hh, int W, int elem_bytes,
                          void* stream);
+int bsa_permute_in_place_status(void* const tensors[], const int64_t* strides, int n_tensors,
+                                const void* plan, int plan_elem_bytes, int64_t plan_stride, int inverse,
+                                int B, int heads, int T, int D, int F, int Hh, int W, int elem_bytes,
+                                int32_t* status, void* stream);
 
 /*
  * Forward attention directly from a block mask, allocating nothing.  It has no counterpart in the

@@ -49,3 +49,51 @@ def test_backward_names_the_role_and_takes_only_its_own_report(lib):
     want = oracle.attn_forward_backward(*(t.detach().cpu() for t in qkv), mask.cpu(), 0.125, do.cpu())[2:]
     for g, w in zip(got, want):
         assert (g.float().cpu() - w).abs().max().item() <= 5e-2
+
+
+def test_an_axis_order_that_is_none_is_reported(lib):
+    """Its head is left as it is, the others are reordered; the first call after the kernel raises, the one
+    after that works.  The same through the next reorder and through the attention op."""
+    from fa2_custom_mask import flash_attention_custom_mask, inv_permute_attn_triton, permute_qkv_triton
+    grid = dict(F=3, H=4, W=5, n_text_tokens=2)
+    x = torch.randn(1, 6, 62, 64).half()
+    good = torch.arange(6)[None]
+    orders = oracle.PERMUTATIONS.copy()
+    orders[[2, 4]] = 0, 1, 2
+    want = x.clone()
+    want[:, :, 2:] = oracle.reorder_by_view(x[:, :, 2:], orders, 3, 4, 5)
+    qkv, mask, _ = _problem(43)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s), torch.no_grad():
+        ts = [x.cuda() for _ in range(3)]
+        permute_qkv_triton(*[t.clone() for t in ts], {"permute": good.cuda()}, 0, **grid)
+        for low, high in ((-7, 6), (-2 ** 31, 2 ** 31 - 1)):
+            bad = good.clone()
+            bad[0, 2], bad[0, 4] = low, high
+            for again in (lambda: permute_qkv_triton(*ts, {"permute": good.cuda()}, 0, **grid),
+                          lambda: inv_permute_attn_triton(ts[0], {"permute": good.cuda().int()}, 0, **grid),
+                          lambda: flash_attention_custom_mask(*qkv, mask, 0.125)):
+                for plan in (bad.cuda(), bad.cuda().int()):
+                    ts = [x.cuda() for _ in range(3)]
+                    permute_qkv_triton(*ts, {"permute": plan}, 0, **grid)
+                    s.synchronize()
+                    assert all(torch.equal(t.cpu(), want) for t in ts)
+                    with pytest.raises(IndexError, match="axis-order"):
+                        again()
+                    assert all(torch.equal(t.cpu(), want) for t in ts)
+                    again()
+                    s.synchronize()
+
+
+def test_an_axis_order_that_is_none_in_a_plan_on_the_host(lib):
+    from fa2_custom_mask import inv_permute_attn_triton, permute_qkv_triton
+    grid = dict(F=3, H=4, W=5, n_text_tokens=2)
+    x = torch.randn(1, 6, 62, 64).half()
+    for bad in (-7, 6):
+        for plan in (torch.tensor([[0, 1, bad, 3, 4, 5]]), [[0, 1, bad, 3, 4, 5]]):
+            ts = [x.cuda() for _ in range(3)]
+            with pytest.raises(IndexError):
+                permute_qkv_triton(*ts, {"permute": plan}, 0, **grid)
+            with pytest.raises(IndexError):
+                inv_permute_attn_triton(ts[0], {"permute": plan}, 0, **grid)
+            assert all(torch.equal(t.cpu(), x) for t in ts)
