@@ -60,6 +60,8 @@ StreamState* stream_state(int device, cudaStream_t stream) {
   if (it == states->end()) {
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
     auto* st = new StreamState;
+    // ordinary tensors whatever the mode of the call that comes first: both layers write to them later
+    const c10::InferenceMode no_inference(false);
     // zeroed on the stream that will use it, so no cross-stream ordering is needed
     st->counter = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
     st->status = at::zeros({1}, at::TensorOptions().dtype(at::kInt)).pin_memory();

@@ -97,3 +97,23 @@ def test_an_axis_order_that_is_none_in_a_plan_on_the_host(lib):
             with pytest.raises(IndexError):
                 inv_permute_attn_triton(ts[0], {"permute": plan}, 0, **grid)
             assert all(torch.equal(t.cpu(), x) for t in ts)
+
+
+def test_report_on_a_stream_first_used_in_inference_mode(lib):
+    """The stream's word belongs to no mode: a report is raised and taken outside inference mode too."""
+    from fa2_custom_mask import _lib, flash_attention_custom_mask
+    s = torch.cuda.Stream(priority=-1)
+    with torch.cuda.stream(s), torch.no_grad():
+        qkv, mask, _ = _problem(42)
+        with torch.inference_mode():
+            want = flash_attention_custom_mask(*qkv, mask, 0.125).clone()
+        word = _word(s)
+        s.synchronize()
+        word.value = 4
+        try:
+            with pytest.raises(_lib.BsaError, match="role 4"):
+                flash_attention_custom_mask(*qkv, mask, 0.125)
+            assert word.value == 0
+            assert torch.equal(flash_attention_custom_mask(*qkv, mask, 0.125), want)
+        finally:
+            word.value = 0
