@@ -287,6 +287,8 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
   if ((type != at::kHalf && type != at::kBFloat16) || k.scalar_type() != type || v.scalar_type() != type ||
       k.device() != q.device() || v.device() != q.device())
     return std::nullopt;
+  // there is no forward derivative: the Python layer's Function says so, where this path would lose the tangent
+  if (q._fw_grad(0).defined() || k._fw_grad(0).defined() || v._fw_grad(0).defined()) return std::nullopt;
   const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
   if ((D != 16 && D != 32 && D != 64) || B == 0 || H == 0 || N == 0 || N % kBlock != 0) return std::nullopt;
   const c10::cuda::CUDAGuard guard(q.device());

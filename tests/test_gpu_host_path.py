@@ -1,0 +1,25 @@
+"""What the native host path of the public op takes, and what it has to leave to the general one."""
+import pytest
+import torch
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(dtype=torch.float16, N=512, D=64, seed=51):
+    q, k, v, do = (t.to(dtype).cuda() for t in oracle.make_qkv(1, 2, N, D, seed=seed, n=4))
+    return q, k, v, do, oracle.make_block_mask(1, 2, N // 64, 0.5, seed=seed).cuda()
+
+
+def test_forward_mode_tangents_are_refused(lib):
+    """The op has no forward derivative; an input with a tangent is refused instead of losing it."""
+    import torch.autograd.forward_ad as fwd
+    from fa2_custom_mask import flash_attention_custom_mask
+    q, k, v, _, mask = _problem()
+    with fwd.dual_level():
+        for i in range(3):
+            args = [fwd.make_dual(t, torch.ones_like(t)) if i == j else t for j, t in enumerate((q, k, v))]
+            for grad in (True, False):
+                with torch.set_grad_enabled(grad), pytest.raises(NotImplementedError):
+                    flash_attention_custom_mask(*args, mask, 0.125)
