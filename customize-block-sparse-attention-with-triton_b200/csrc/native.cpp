@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <mutex>
@@ -287,6 +288,8 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
   if ((type != at::kHalf && type != at::kBFloat16) || k.scalar_type() != type || v.scalar_type() != type ||
       k.device() != q.device() || v.device() != q.device())
     return std::nullopt;
+  // the tracer would see the outputs being allocated and no kernel; the Python layer refuses to be traced
+  if (torch::jit::tracer::isTracing()) return std::nullopt;
   // there is no forward derivative: the Python layer's Function says so, where this path would lose the tangent
   if (q._fw_grad(0).defined() || k._fw_grad(0).defined() || v._fw_grad(0).defined()) return std::nullopt;
   const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);

@@ -23,3 +23,25 @@ def test_forward_mode_tangents_are_refused(lib):
             for grad in (True, False):
                 with torch.set_grad_enabled(grad), pytest.raises(NotImplementedError):
                     flash_attention_custom_mask(*args, mask, 0.125)
+
+
+@pytest.mark.parametrize("byte_mask", [False, True])
+def test_transforms_that_the_op_does_not_have_are_refused(lib, byte_mask):
+    """Tracing, vmap and the functional derivatives: no result rather than one without the kernels."""
+    import torch.func as F
+    from fa2_custom_mask import flash_attention_custom_mask
+    q, k, v, _, mask = _problem()
+    if byte_mask:
+        mask = mask.view(torch.uint8)
+
+    def op(q, mask):
+        return flash_attention_custom_mask(q, k, v, mask, 0.125)
+
+    for call in (lambda: torch.jit.trace(op, (q, mask), check_trace=False),
+                 lambda: torch.jit.trace(op, (q.clone().requires_grad_(True), mask), check_trace=False),
+                 lambda: F.vmap(op, (0, None))(torch.stack([q, q]), mask),
+                 lambda: F.vmap(op, (None, 0))(q, torch.stack([mask, mask])),
+                 lambda: F.grad(lambda q: op(q, mask).sum())(q),
+                 lambda: F.jvp(lambda q: op(q, mask), (q,), (q,))):
+        with pytest.raises((RuntimeError, AssertionError, NotImplementedError)):
+            call()
