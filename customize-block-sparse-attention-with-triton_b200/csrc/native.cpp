@@ -182,8 +182,7 @@ struct Lists {
 // (A node of its own and not torch::autograd::Function: that keeps what is saved in a map of boxed values,
 // which costs a small call another 10 us.)
 struct AttentionBackward : torch::autograd::Node {
-  torch::autograd::SavedVariable q_, k_, v_, o_;
-  Tensor lse2, lists;
+  torch::autograd::SavedVariable q_, k_, v_, o_, lse2_, lists_;
   Tensor dense;  // the caller's mask (or an aligned copy of it): not to be changed before backward
   int64_t Bm, Hm, nb;
   float scale;
@@ -191,9 +190,7 @@ struct AttentionBackward : torch::autograd::Node {
   std::string name() const override { return "AttentionBackward"; }
   void release_variables() override {
     std::lock_guard<std::mutex> lock(mutex_);
-    for (auto* s : {&q_, &k_, &v_, &o_}) s->reset_data();
-    lse2.reset();
-    lists.reset();
+    for (auto* s : {&q_, &k_, &v_, &o_, &lse2_, &lists_}) s->reset_data();
     dense.reset();
   }
 
@@ -201,7 +198,7 @@ struct AttentionBackward : torch::autograd::Node {
     std::lock_guard<std::mutex> lock(mutex_);
     // (unpacking raises when the buffers have been released or an input was modified in place)
     const Tensor q = tma_ready(q_.unpack()), k = tma_ready(k_.unpack()), v = tma_ready(v_.unpack());
-    const Tensor o = o_.unpack(shared_from_this());
+    const Tensor o = o_.unpack(shared_from_this()), lse2 = lse2_.unpack(), lists = lists_.unpack();
     at::AutoDispatchBelowADInplaceOrView no_autograd;
     const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
@@ -254,18 +251,18 @@ Tensor forward_with_grad(const Tensor& q0, const Tensor& k0, const Tensor& v0, c
                          StreamState* state, void* stream) {
   std::shared_ptr<AttentionBackward> node(new AttentionBackward(), torch::autograd::deleteNode);
   node->set_next_edges(torch::autograd::collect_next_edges(q0, k0, v0));
-  Tensor o;
+  Tensor o, lse2, lists;
   {
     at::AutoDispatchBelowADInplaceOrView no_autograd;
-    if (!run_forward(tma_ready(q0), tma_ready(k0), tma_ready(v0), m, scale, state, stream, &o, &node->lse2))
+    if (!run_forward(tma_ready(q0), tma_ready(k0), tma_ready(v0), m, scale, state, stream, &o, &lse2))
       return Tensor();
     // the forward lists each mask row inside the kernel; only the backward needs lists as data
     node->Bm = m.block.size(0);
     node->Hm = m.block.size(1);
     node->nb = m.block.size(2);
     const Lists at(node->Bm, node->Hm, node->nb);
-    node->lists = at::empty({at.words}, q0.options().dtype(at::kInt));
-    int32_t* p = node->lists.mutable_data_ptr<int32_t>();
+    lists = at::empty({at.words}, q0.options().dtype(at::kInt));
+    int32_t* p = lists.mutable_data_ptr<int32_t>();
     if (bsa_tile_lists_places(m.block.const_data_ptr<uint8_t>(), m.block.strides().data(), node->Bm, node->Hm,
                               node->nb, p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, stream) != 0)
       return Tensor();
@@ -275,6 +272,9 @@ Tensor forward_with_grad(const Tensor& q0, const Tensor& k0, const Tensor& v0, c
   node->q_ = torch::autograd::SavedVariable(q0, false);
   node->k_ = torch::autograd::SavedVariable(k0, false);
   node->v_ = torch::autograd::SavedVariable(v0, false);
+  // (saved like the rest, so that offloading and checkpointing hooks get hold of all the memory)
+  node->lse2_ = torch::autograd::SavedVariable(lse2, false);
+  node->lists_ = torch::autograd::SavedVariable(lists, false);
   torch::autograd::set_history(o, node);
   node->o_ = torch::autograd::SavedVariable(o, true);
   return o;

@@ -45,3 +45,24 @@ def test_transforms_that_the_op_does_not_have_are_refused(lib, byte_mask):
                  lambda: F.jvp(lambda q: op(q, mask), (q,), (q,))):
         with pytest.raises((RuntimeError, AssertionError, NotImplementedError)):
             call()
+
+
+def test_saved_tensor_hooks_see_what_the_backward_keeps(lib):
+    """Everything that the op makes for its backward goes through the saved-tensor hooks (offloading,
+    checkpointing): q, k, v, O, the log-sum-exp and the tile lists."""
+    from fa2_custom_mask import flash_attention_custom_mask
+    q, k, v, do, mask = _problem()
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    want = torch.autograd.grad(flash_attention_custom_mask(q, k, v, mask, 0.125), (q, k, v), do)
+    packed = []
+
+    def pack(t):
+        packed.append(t.dtype)
+        return t.cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        o = flash_attention_custom_mask(q, k, v, mask, 0.125)
+    assert sorted(map(str, packed)) == ["torch.float16"] * 4 + ["torch.float32", "torch.int32"]
+    for g, w in zip(torch.autograd.grad(o, (q, k, v), do), want):
+        assert torch.equal(g, w)
