@@ -344,7 +344,8 @@ bool permute_tokens(const std::vector<Tensor>& tensors, const Tensor& plan, int6
                                   F, Hh, W, t0.element_size(),
                                   state ? const_cast<int32_t*>(state->word) : nullptr, stream) != 0)
     return false;
-  for (const Tensor& t : tensors) t.unsafeGetTensorImpl()->bump_version();
+  for (const Tensor& t : tensors)
+    if (!t.is_inference()) t.unsafeGetTensorImpl()->bump_version();  // (inference tensors have no version)
   return true;
 }
 

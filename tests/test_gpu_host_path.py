@@ -66,3 +66,17 @@ def test_saved_tensor_hooks_see_what_the_backward_keeps(lib):
     assert sorted(map(str, packed)) == ["torch.float16"] * 4 + ["torch.float32", "torch.int32"]
     for g, w in zip(torch.autograd.grad(o, (q, k, v), do), want):
         assert torch.equal(g, w)
+
+
+def test_inference_tensors_are_reordered_outside_inference_mode(lib):
+    from fa2_custom_mask import inv_permute_attn_triton, permute_qkv_triton
+    grid = dict(F=3, H=4, W=5, n_text_tokens=2)
+    x = torch.randn(1, 6, 62, 64).half()
+    plan = {"permute": torch.arange(6, device="cuda")[None]}
+    with torch.inference_mode():
+        ts = [x.cuda() for _ in range(3)]
+    want = x.clone()
+    want[:, :, 2:] = oracle.reorder_by_view(x[:, :, 2:], oracle.PERMUTATIONS, 3, 4, 5)
+    for t in permute_qkv_triton(*ts, plan, 0, **grid):
+        assert t.is_inference() and torch.equal(t.cpu(), want)
+        assert torch.equal(inv_permute_attn_triton(t, plan, 0, **grid).cpu(), x)
