@@ -260,9 +260,20 @@ def _stream_state(device: torch.device, stream: int) -> Optional[_StreamState]:
     if st is None:
         tensors = _lib.native().state_tensors(device.index, stream)
         if tensors is None:
-            return None  # inside a graph capture: fixed-stride hand-out, no report
+            return None  # inside a graph capture: no report
         st = _stream_states[key] = _StreamState(*tensors)
     return st
+
+
+def _work_counter(device: torch.device, stream: int, blocks: int) -> Optional[torch.Tensor]:
+    """The work counter for a call on that many blocks (none when a CTA has one of them at most): the
+    stream's, or in a capture, which may be replayed on any stream beside calls on this one, a zeroed word
+    of its own."""
+    if blocks <= torch.cuda.get_device_properties(device).multi_processor_count:
+        return None
+    if not torch.cuda.is_current_stream_capturing():
+        return _stream_state(device, stream).counter
+    return torch.zeros(1, dtype=torch.int32, device=device)
 
 
 def _raise_native(fn: str, status: int, code: int = 0):
@@ -317,13 +328,13 @@ def attention_forward(q, k, v, lists: TileLists, sm_scale: float, want_rowmax: b
     d4, dst = _dense_args(dense, B, H)
     with _on_device(q.device):
         stream = _lib.stream_ptr(q.device)
-        state = _stream_state(q.device, stream.value or 0)
+        counter = _work_counter(q.device, stream.value or 0, B * H * (r1 - r0))
         _lib.check("bsa_attn_fwd_rows", lib.bsa_attn_fwd_rows(
             _lib.ptr(q), _lib.strides4(q), _lib.ptr(k), _lib.strides4(k), _lib.ptr(v),
             _lib.strides4(v), _lib.ptr(o), _lib.strides4(o), _lib.ptr(lse2), _lib.ptr(rowmax),
             _lib.ptr(lists.row_ptr), _lib.ptr(lists.col_idx), sb, sh, float(sm_scale),
             _lib.dtype_code(q.dtype), B, H, N, D, r0, r1, _lib.ptr(d4), dst,
-            _lib.ptr(state.counter if state else None), _lib.ptr(status), stream))
+            _lib.ptr(counter), _lib.ptr(status), stream))
     return o, lse2, rowmax
 
 
@@ -342,13 +353,13 @@ def attention_forward_masked(q, k, v, block_mask: torch.Tensor, sm_scale: float,
     d4, dst = _dense_args(dense, B, H)
     with _on_device(q.device):
         stream = _lib.stream_ptr(q.device)
-        state = _stream_state(q.device, stream.value or 0)
+        counter = _work_counter(q.device, stream.value or 0, B * H * (r1 - r0))
         _lib.check("bsa_attn_fwd_block_mask_rows", lib.bsa_attn_fwd_block_mask_rows(
             _lib.ptr(q), _lib.strides4(q), _lib.ptr(k), _lib.strides4(k), _lib.ptr(v),
             _lib.strides4(v), _lib.ptr(o), _lib.strides4(o), _lib.ptr(lse2), _lib.ptr(rowmax),
             _lib.ptr(m4), _lib.strides4(m4), m4.shape[0], m4.shape[1], float(sm_scale),
             _lib.dtype_code(q.dtype), B, H, N, D, r0, r1, _lib.ptr(d4), dst,
-            _lib.ptr(state.counter if state else None), _lib.ptr(status), stream))
+            _lib.ptr(counter), _lib.ptr(status), stream))
     return o, lse2, rowmax
 
 
@@ -370,8 +381,7 @@ def attention_backward(q, k, v, o, lse2, dout, lists: TileLists, sm_scale: float
     d4, dst = _dense_args(dense, B, H)
     with _on_device(q.device):
         stream = _lib.stream_ptr(q.device)
-        state = _stream_state(q.device, stream.value or 0)
-        counter = state.counter if state else None
+        counter = _work_counter(q.device, stream.value or 0, B * H * (N // BLOCK))
         _lib.check("bsa_attn_bwd_delta_strided", lib.bsa_attn_bwd_delta_strided(
             _lib.ptr(o), _lib.strides4(o), _lib.ptr(dout), ds, _lib.ptr(delta), code, B, H, N, D,
             stream))

@@ -80,3 +80,48 @@ def test_inference_tensors_are_reordered_outside_inference_mode(lib):
     for t in permute_qkv_triton(*ts, plan, 0, **grid):
         assert t.is_inference() and torch.equal(t.cpu(), want)
         assert torch.equal(inv_permute_attn_triton(t, plan, 0, **grid).cpu(), x)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_a_captured_call_does_not_draw_from_its_streams_counter(lib, native):
+    """A graph may be replayed on any stream, beside calls on the one it was captured on.  Seen here with a
+    counter that says that everything has been handed out, and in replays beside such calls."""
+    from fa2_custom_mask import _lib, flash_attention_custom_mask
+    from fa2_custom_mask import fa2_custom_mask as host
+    op = flash_attention_custom_mask if native else host._attention.apply
+    s, other = torch.cuda.Stream(), torch.cuda.Stream()
+    q, k, v, do = (t.cuda() for t in oracle.make_qkv(1, 4, 4096, 64, seed=52, dtype=torch.float16, n=4))
+    mask = oracle.make_block_mask(1, 4, 64, 0.2, seed=52, causal=True).cuda()   # 256 rows of blocks
+    for t in (q, k, v):
+        t.requires_grad_(True)
+
+    def step():
+        o = op(q, k, v, mask, 0.125)
+        return [o.detach(), *torch.autograd.grad(o, (q, k, v), do)]
+
+    with torch.cuda.stream(s):
+        want = step()
+        counter, _ = _lib.native().state_tensors(s.device_index, s.cuda_stream)
+        s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            got = step()
+        for t in got:
+            t.zero_()
+        counter.fill_(1 << 20)
+        graph.replay()
+        s.synchronize()
+        assert int(counter.item()) == 1 << 20
+        counter.zero_()
+        s.synchronize()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
+    eager = []
+    for _ in range(8):
+        with torch.cuda.stream(other):
+            graph.replay()
+        with torch.cuda.stream(s):
+            eager.append(step())
+    torch.cuda.synchronize()
+    for res in (got, *eager):
+        assert all(torch.equal(g, w) for g, w in zip(res, want))
+    assert int(counter.item()) == 0
