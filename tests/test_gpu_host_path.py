@@ -125,3 +125,82 @@ def test_a_captured_call_does_not_draw_from_its_streams_counter(lib, native):
     for res in (got, *eager):
         assert all(torch.equal(g, w) for g, w in zip(res, want))
     assert int(counter.item()) == 0
+
+
+def _layouts(dtype, N, D):
+    """Name -> q, k, v as programs hold them: contiguous, projections, slices of a fused projection, and
+    rows that the copy engine cannot read in place (copied first)."""
+    B, H = 2, 3
+    fused = torch.randn(B, N, 3, H, D, device="cuda", dtype=dtype)
+    return {
+        "bhnd": [torch.randn(B, H, N, D, device="cuda", dtype=dtype) for _ in range(3)],
+        "bnhd": [torch.randn(B, N, H, D, device="cuda", dtype=dtype).transpose(1, 2) for _ in range(3)],
+        "qkv": [fused[:, :, i].transpose(1, 2) for i in range(3)],
+        "odd rows": [torch.randn(B, H, N, D + 1, device="cuda", dtype=dtype)[..., :D] for _ in range(3)],
+    }
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("D", [16, 32, 64])
+def test_ordinary_calls_take_the_native_path(lib, monkeypatch, dtype, D):
+    """Whatever the native path refuses goes through the Python layer without a word and costs six times
+    the host time; here that layer is taken away."""
+    from fa2_custom_mask import flash_attention_custom_mask
+    from fa2_custom_mask import fa2_custom_mask as host
+    monkeypatch.setattr(host, "_attention", None)
+    N, nb = 192, 3
+    block = torch.rand(2, 3, nb, nb, device="cuda") < 0.5
+    dense = torch.rand(N, N, device="cuda") < 0.5
+    masks = [block, block[:1], block[:, :1], block[:1, :1], block[0], block[0, 0], block.view(torch.uint8),
+             block.transpose(2, 3), dense, dense.view(torch.uint8), dense.expand(2, 3, N, N), dense.t()]
+    for name, qkv in _layouts(dtype, N, D).items():
+        for mask in masks if name == "bhnd" else [block, dense]:
+            with torch.no_grad():
+                assert flash_attention_custom_mask(*qkv, mask, 0.125).shape == (2, 3, N, D)
+            for needs in ((True, True, True), (False, True, False)):
+                leaves = [t.detach().requires_grad_(n) for t, n in zip(qkv, needs)]
+                o = flash_attention_custom_mask(*leaves, mask, 0.125)
+                assert o.grad_fn.name() == "AttentionBackward"
+                wanted = [t for t in leaves if t.requires_grad]
+                for g, t in zip(torch.autograd.grad(o, wanted, torch.ones_like(o)), wanted):
+                    assert g.shape == t.shape
+    with pytest.raises(AttributeError):      # what it does not take: no mask
+        flash_attention_custom_mask(*qkv, None, 0.125)
+
+
+def test_reorders_that_take_one_launch(lib, monkeypatch):
+    """Up to 18,432 tokens of rows that split into 64-byte chunks go in one launch, whatever the layout;
+    more, tensors of one storage and plans on the host go through the two-pass form."""
+    from fa2_custom_mask import functional, inv_permute_attn_triton, permute_qkv_triton
+
+    class TwoPass(Exception):
+        pass
+
+    def two_pass(*args):
+        raise TwoPass
+
+    monkeypatch.setattr(functional, "apply_head_wise_reorder", two_pass)
+    monkeypatch.setattr(functional, "apply_inv_reorder", two_pass)
+    plan = {"permute": torch.arange(1, 4, device="cuda")[None]}
+
+    def call(ts, F, H, W, text=0, plan=plan):
+        grid = dict(F=F, H=H, W=W, n_text_tokens=text)
+        permute_qkv_triton(*ts, plan, 0, **grid)
+        inv_permute_attn_triton(ts[0], plan, 0, **grid)
+
+    def tensors(T, D=64, dtype=torch.float16):
+        return [torch.zeros(1, 3, T, D, device="cuda", dtype=dtype) for _ in range(3)]
+
+    call(tensors(226 + 13 * 30 * 45), 13, 30, 45, 226)
+    call(tensors(60, 128, torch.bfloat16), 3, 4, 5)
+    call([t.transpose(1, 2).contiguous().transpose(1, 2) for t in tensors(60)], 3, 4, 5)
+    for D in (64, 128):
+        call(tensors(18432, D), 2, 96, 96)
+        with pytest.raises(TwoPass):
+            call(tensors(18434, D), 2, 13, 709)
+    call(tensors(24576, 24), 4, 64, 96)               # 48-byte rows: one chunk
+    fused = torch.zeros(1, 60, 3, 3, 64, device="cuda", dtype=torch.float16)
+    with pytest.raises(TwoPass):
+        call([fused[:, :, i].transpose(1, 2) for i in range(3)], 3, 4, 5)
+    with pytest.raises(TwoPass):
+        call(tensors(60), 3, 4, 5, plan={"permute": torch.arange(1, 4)[None]})
