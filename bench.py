@@ -14,7 +14,7 @@ steps because the inputs are smaller than L2.  `roofline` times the forward kern
 own CUDA events inside the same steps.  `e2e` runs the public op flash_attention_custom_mask from
 pinned host buffers (H2D of q,k,v,mask and D2H of O inside the timed region).  `cpu_baseline` /
 `--impl reference` time the reference's naive matmul + masked softmax arithmetic
-(kernel-test.py:37-40) on the host cores.  `extra` holds the other BASELINE.json configurations
+(kernel-test.py:37-40) on the host cores.  `extra` holds the other benchmark configurations
 (sharded over the ranks with fa2_custom_mask.sharding when N > 1), the HBM-bound kernels, and the
 reference's own Triton kernel timed on the same GPU from an unmodified copy, if one is present.
 """
@@ -257,7 +257,7 @@ def device_problem(dev, B, H, N, p, dtype, seed, causal=False, n=3):
 
 
 def sharded_measurements(dev, timer, rank, world, peak_tf):
-    """BASELINE.json configurations 3 (row split of the one head), 4 and 5 ((batch, head) split),
+    """Configurations 3 (N = 17536, one head; row split of the one head), 4 and 5 ((batch, head) split),
     partitioned over the ranks by fa2_custom_mask.sharding.plan: strong scaling, no collective on
     the data path.  Every rank times its own share; the job's time is the slowest rank's."""
     import torch.distributed as dist
@@ -274,7 +274,7 @@ def sharded_measurements(dev, timer, rank, world, peak_tf):
         return ms, tiles
 
     out = {}
-    # config 3, one head: fewer (b, h) units than ranks -> query-block rows, balanced by tiles
+    # one head: fewer (b, h) units than ranks -> query-block rows, balanced by tiles
     (q, k, v, mask), _ = make_inputs(seed=2, device=dev)
     row_tiles = mask[0, 0].sum(-1).tolist()
     kind, (r0, r1) = sharding.plan(1, 1, world, rank, row_tiles) if world > 1 else ("rows", (0, len(row_tiles)))
@@ -401,7 +401,7 @@ def single_gpu_measurements(dev, timer, peak_tf, peak_gbs):
         out[name] = {"tiles": tiles, "fwd_ms": ms, "fwd_tflops": tf, "fwd_frac_of_measured_peak": tf / peak_tf}
         del q, k, v, m, lists, o, lse2
     # the forward from a DENSE boolean mask: mask reduction + forward in one public call
-    # (BASELINE.json configs 2 and 3 "including dense-mask -> block preprocessing")
+    # (N = 6400 and 17536, dense-mask -> block preprocessing included)
     for N in (6400, 17536):
         (q, k, v), m = device_problem(dev, 1, 1, N, DENSITY, torch.float16, seed=N)
         dense = m.repeat_interleave(64, dim=-2).repeat_interleave(64, dim=-1)
@@ -439,7 +439,7 @@ def single_gpu_measurements(dev, timer, peak_tf, peak_gbs):
                                      "frac_of_measured_hbm": nbytes / (ms * 1e-3) / 1e9 / peak_gbs,
                                      "note": "three launches over a few MB: launch-latency bound"}
         del m
-    # delta (HBM-bound: O and dO read once, one float per row written), config 5 shape
+    # delta (HBM-bound: O and dO read once, one float per row written), B = 2, H = 16, N = 16384
     B, H, N = 2, 16, 16384
     o, do = (torch.randn(B, H, N, HEAD_DIM, device=dev).to(torch.bfloat16) for _ in range(2))
     delta = torch.empty((B, H, N), dtype=torch.float32, device=dev)
@@ -460,13 +460,14 @@ def single_gpu_measurements(dev, timer, peak_tf, peak_gbs):
     out["reorder_B2_H48_T17550_f16"] = {"ms": ms, "GBps": gbs, "frac_of_measured_hbm": gbs / peak_gbs}
     del x
     # the whole wrapper as a model calls it: q, k, v with 226 text tokens in front, image tokens
-    # gathered out of the slice and copied back in place (two passes per tensor; bytes counted are
-    # those of one pass, so 0.5 of the copy bandwidth is the ceiling)
+    # reordered in place.  Bytes: every moved one read and written once; the heads whose order is
+    # (0,1,2), one in six here, are left alone.
     qkv = [torch.randn(Bv, Hv, 226 + Fv * Yv * Xv, HEAD_DIM, device=dev, dtype=torch.float16)
            for _ in range(3)]
     plan = {"permute": (torch.arange(Hv, device=dev) % 6)[None]}
     ms = timer.median(lambda: permute_qkv_triton(*qkv, plan, 0, Fv, Yv, Xv, 226), 10)
-    gbs = 3 * 2 * Bv * Hv * Fv * Yv * Xv * HEAD_DIM * 2 / (ms * 1e-3) / 1e9
+    moved = 3 * Bv * int((plan["permute"] != 0).sum()) * Fv * Yv * Xv * HEAD_DIM * 2
+    gbs = 2 * moved / (ms * 1e-3) / 1e9
     out["permute_qkv_B2_H48_T226+17550_f16"] = {"ms": ms, "GBps_one_pass": gbs,
                                                 "frac_of_measured_hbm": gbs / peak_gbs}
     del qkv
@@ -620,7 +621,7 @@ def run_ours(args, rank, world, local_rank):
 
 
 PROFILE_CASES = ("fwd_headline", "fwd_dense", "fwd_bwd_causal", "mask_reduce", "tile_lists", "delta",
-                 "reorder")
+                 "reorder", "permute")
 
 
 def run_profile_case(name, iters):
@@ -629,7 +630,7 @@ def run_profile_case(name, iters):
     launches).  Prints nothing that is a benchmark value."""
     from fa2_custom_mask import (_lib, apply_head_wise_reorder, attention_backward,
                                  attention_forward, attention_forward_masked, build_tile_lists,
-                                 reduce_dense_mask)
+                                 permute_qkv_triton, reduce_dense_mask)
     dev = torch.device("cuda", 0)
     torch.cuda.set_device(dev)
     if name in ("fwd_headline", "fwd_dense"):
@@ -637,7 +638,7 @@ def run_profile_case(name, iters):
                                       torch.float16, seed=3)
         fn = lambda: attention_forward_masked(q, k, v, m, SM_SCALE)
     elif name == "fwd_bwd_causal":
-        # BASELINE.json config 5 with 2 x 4 of its 2 x 16 heads
+        # the largest training shape with 2 x 4 of its 2 x 16 heads
         (q, k, v, do), m = device_problem(dev, 2, 4, 16384, 0.25, torch.bfloat16, seed=5, causal=True, n=4)
         lists = build_tile_lists(m)
         o, lse2, _ = attention_forward(q, k, v, lists, SM_SCALE)
@@ -648,7 +649,7 @@ def run_profile_case(name, iters):
         dense = dense.repeat_interleave(64, dim=-2).repeat_interleave(64, dim=-1)   # 307 MB > L2
         fn = lambda: reduce_dense_mask(dense)
     elif name == "tile_lists":
-        m = synth_block_mask(1, 32, 500, DENSITY, seed=1).to(dev)                   # config 4 mask
+        m = synth_block_mask(1, 32, 500, DENSITY, seed=1).to(dev)                   # N = 32000, 32 heads
         fn = lambda: build_tile_lists(m, want_csr=True, want_csc=True)
     elif name == "delta":
         o, do = (torch.randn(2, 16, 16384, HEAD_DIM, device=dev).to(torch.bfloat16) for _ in range(2))
@@ -657,6 +658,10 @@ def run_profile_case(name, iters):
         fn = lambda: lib.bsa_attn_bwd_delta(_lib.ptr(o), _lib.ptr(do), _lib.strides4(o), _lib.ptr(delta),
                                             _lib.dtype_code(o.dtype), 2, 16, 16384, HEAD_DIM,
                                             _lib.stream_ptr(dev))
+    elif name == "permute":
+        ts = [torch.randn(2, 48, 226 + 13 * 30 * 45, HEAD_DIM, device=dev, dtype=torch.float16) for _ in range(3)]
+        plan = {"permute": (torch.arange(48, device=dev) % 6)[None]}                    # 3 x 218 MB > L2
+        fn = lambda: permute_qkv_triton(*ts, plan, 0)
     else:
         x = torch.randn(2, 48, 13 * 30 * 45, HEAD_DIM, device=dev, dtype=torch.float16)  # 216 MB > L2
         orders = torch.tensor([[0, 1, 2], [0, 2, 1], [1, 0, 2], [1, 2, 0], [2, 0, 1], [2, 1, 0]],

@@ -21,15 +21,16 @@
 // the probabilities go over the logits of their slot, which is held from the S product until P V
 // is complete.
 //
-// What bounds it: with everything listed a tile takes about 335 SM cycles, of which the exp2 unit
+// What bounds it: with everything listed a tile takes 346 active SM cycles, of which the exp2 unit
 // is busy 256 (4096 exponentials at 16 per cycle; a loop of nothing but loads, exponentials and
 // stores, two warps per sub-partition, measures 281); what is left are hand-overs between the
 // roles, about 140 cycles each.  With short lists the instruction cache comes first: all roles run
 // at the same time, and 2.5 KB more in the softmax loop made everything 10 % slower.  So what is
 // executed per item or per superstep is kept short, waits included.
-// B200, fp16, D = 64, against the form with M = 128 products and both teams on every superstep:
-// N = 17536 with one head, all blocks 136 -> 104 us, a tenth of them 27.0 -> 21.5 us; 8 heads, a
-// tenth 133 -> 103 us; bf16 N = 32000, 32 heads, a tenth 1.53 -> 1.25 ms.
+// B200, D = 64, public calls back to back on inputs that rotate: fp16 N = 17536 with one head, all blocks
+// 117 us, a tenth of them 19.9 us; 8 heads, a tenth 119 us; bf16 N = 32000, 32 heads, a tenth 1.30 ms.  The
+// form with M = 128 products and both teams on every superstep took 136, 27.0, 133 us and 1.53 ms where
+// this one first took 104, 21.5, 103 us and 1.25 ms (the kernel alone, on the same inputs again and again).
 //
 // Roles (16 warps); every role walks the same item sequence, so set-up of item i+1 and write-out
 // of item i-1 overlap the arithmetic of item i:
@@ -59,8 +60,8 @@
 // Numerics follow the reference's loop (fa2_custom_mask/fa2_fwd.py:150-196): logits scaled by
 // sm_scale*log2(e), exp2 domain, fp32 row sums of the fp32 probabilities, P rounded to the input
 // dtype before P V.  The reference maximum of a row comes from its first 32 logits and moves only
-// when later ones would make probabilities too large for 16 bit (sum of a superstep above 4096), which
-// leaves O = acc / l unchanged because both use the same reference.  Which partial result a tile
+// when later ones would make probabilities too large for 16 bit (sum of a superstep above 4096; then to
+// the maximum of that superstep), which leaves O = acc / l unchanged because both use the same reference.  Which partial result a tile
 // goes into depends on its position in the row's list alone, so results do not depend on which CTA
 // computes an item.
 //

@@ -344,7 +344,7 @@ bool permute_tokens(const std::vector<Tensor>& tensors, const Tensor& plan, int6
         (t.requires_grad() && at::GradMode::is_enabled()))
       return false;
     for (size_t j = 0; j < i; ++j)
-      if (t.is_alias_of(tensors[j])) return false;  // shared storage: one after the other
+      if (t.is_alias_of(tensors[j])) return false;  // they may overlap, or be one tensor given twice
     ptrs[i] = static_cast<char*>(t.mutable_data_ptr()) + n_text * t.stride(2) * t.element_size();
     for (int d = 0; d < 4; ++d) strides[4 * i + d] = t.stride(d);
     // rows that overlap (expanded tensors) cannot be reordered in place

@@ -1,7 +1,7 @@
 """Host side of the block-sparse attention op: same Python surface as the reference's
 fa2_custom_mask/fa2_custom_mask.py, with every device step done by libbsattn (sm_100a CUDA).
 
-    flash_attention_custom_mask(q, k, v, mask, sm_scale)      # torch.autograd.Function.apply
+    flash_attention_custom_mask(q, k, v, mask, sm_scale)      # native host path, else _attention.apply
     build_groups_from_block_mask(mask) -> (groups, n_list) | (None, None)
 
 Differences from the reference that a caller can observe (all are supersets):
