@@ -118,15 +118,13 @@ struct FwdSmem {
   uint64_t list_full[kLists];                 // lister -> everyone: list and header ready
   uint64_t list_free[kLists];                 // producers and issuers are through with list and header
   uint64_t setup_go[2];                       // producer -> lister: time to set up the next item
-  uint64_t q_full[2], q_free[2];
+  uint64_t q_full[2];
   uint64_t k_full[kKStages];
   uint64_t k_empty[kKStages];                 // S of the superstep complete
-  uint64_t v_full[kVStages];
-  uint64_t v_empty[kVStages];                 // P V of the pair complete
   uint64_t s_full[2 * kSlots];                // S of the superstep complete; one per (team, slot), so
                                               // that the team that waits on it sees each phase
-  uint64_t p_full[kSlots];                    // the team's four warps stored P of the superstep
-  uint64_t pv_done[kSlots];                   // P V of the superstep complete: slot free, O current
+  uint64_t p_full[kSlots];                    // the team's four warps stored P of the superstep, its V has landed
+  uint64_t pv_done[kSlots];                   // P V of the superstep complete: slot and V places free, O current
   uint64_t o_full[2];                         // last P V of the item done
   uint64_t stats_full[2];                     // softmax warps published (m, l) of the item
   uint64_t o_free[2];                         // write-out has read accumulators, stats and header
@@ -434,7 +432,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->setup_go[i]), 1);
       mbar_init(smem_u32(&sm->q_full[i]), 1);
-      mbar_init(smem_u32(&sm->q_free[i]), 1);
       mbar_init(smem_u32(&sm->o_full[i]), 1);
       mbar_init(smem_u32(&sm->stats_full[i]), kSoftmaxWarps);
       mbar_init(smem_u32(&sm->o_free[i]), 4);  // one arrival per write-out warp
@@ -443,13 +440,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(smem_u32(&sm->k_full[s]), 1);
       mbar_init(smem_u32(&sm->k_empty[s]), 1);
     }
-    for (int s = 0; s < kVStages; ++s) {
-      mbar_init(smem_u32(&sm->v_full[s]), 1);
-      mbar_init(smem_u32(&sm->v_empty[s]), 1);
-    }
     for (int s = 0; s < 2 * kSlots; ++s) mbar_init(smem_u32(&sm->s_full[s]), 1);
     for (int s = 0; s < kSlots; ++s) {
-      mbar_init(smem_u32(&sm->p_full[s]), kTeamWarps);
+      mbar_init(smem_u32(&sm->p_full[s]), kTeamWarps + 1);
       mbar_init(smem_u32(&sm->pv_done[s]), 1);
     }
     for (int s = 0; s < kLists; ++s) {
@@ -501,9 +494,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint16_t* cols = sm->cols[walk.at];
       const int n_super = (n_tiles + 3) >> 2;
       if (n_super > 0) {
+        // (free: that an item is set up means that the item before the previous one has been written out)
         const int qpar = qi & 1;
-        if (qi >= 2) ok = mbar_wait_warp(smem_u32(&sm->q_free[qpar]), ((qi - 2) >> 1) & 1, abort_flag);
-        if (!ok) break;
         if (lane == 0) {
           const uint32_t bar = smem_u32(&sm->q_full[qpar]);
           mbar_expect_tx(bar, kTileBytes);
@@ -538,26 +530,36 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // =========================== V producer ===========================
     // Loads the V tiles of the listed key blocks, one lane per tile; a warp of its own, so that
     // waiting for a free V stage (P V complete) never holds back the K tiles of a later superstep.
+    // Superstep g has the pairs 2 g and 2 g + 1 of the ring, whether it needs both or not: they were those
+    // of supersteps g - 3 and g - 2.  Its tiles land on the barrier that P arrives on, so that P V has
+    // one wait (a look at a barrier that is long complete costs its issuer 150 cycles and more).
     bool ok = true;
-    int vs = 0, vph = 1;
+    int vs = 0, slot = 0, ph = 1;
     FwdWalk walk;
     for (; ok; walk.next()) {
       ok = walk.wait(sm, abort_flag);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
-      const int n_pairs = (n_tiles + 1) >> 1;
       const uint16_t* cols = sm->cols[walk.at];
-      for (int u = 0; u < n_pairs; ++u) {
-        const int nt = min(2, n_tiles - 2 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->v_empty[vs]), vph, abort_flag);
+      for (int u = 0; 4 * u < n_tiles; ++u) {
+        const int nt = min(4, n_tiles - 4 * u);
+        const int at = lane < 2 ? vs : vs + 1 < kVStages ? vs + 1 : 0;
+        const int row = lane < nt ? static_cast<int>(cols[4 * u + lane] & kColIndex) * 64 : 0;
+        const uint32_t dst = smem_u32(sm->v[at][lane & 1]), bar = smem_u32(&sm->p_full[slot]);
+        // (for the first users these ask for the phase before the first one, which counts as complete)
+        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), ph, abort_flag);
         if (!ok) break;
-        const uint32_t bar = smem_u32(&sm->v_full[vs]);
         if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
         __syncwarp();
-        if (lane < nt)
-          tma_load_4d(smem_u32(sm->v[vs][lane]), &tm_v, bar, 0,
-                      static_cast<int>(cols[2 * u + lane] & kColIndex) * 64, walk.it.y, walk.it.x);
-        if (++vs == kVStages) { vs = 0; vph ^= 1; }
+        if (lane < min(nt, 2)) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
+        const int next = slot + 1 < kSlots ? slot + 1 : 0;
+        ok = mbar_wait_warp(smem_u32(&sm->pv_done[next]), next > 0 ? ph : ph ^ 1, abort_flag);
+        if (!ok) break;
+        if (lane >= 2 && lane < nt) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
+        vs += 2;
+        if (vs >= kVStages) vs -= kVStages;
+        slot = next;
+        if (slot == 0) ph ^= 1;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
@@ -607,7 +609,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (kk < k_steps) umma_ws_ss(d, desc_q + 2 * kk, desc_k + 2 * kk, idesc, kk > 0);
           tc_commit(smem_u32(&sm->s_full[bar_s]));
           tc_commit(smem_u32(&sm->k_empty[ks]));
-          if (u == n_super - 1) tc_commit(smem_u32(&sm->q_free[qpar]));  // Q buffer reusable
         }
         if (++ks == kKStages) { ks = 0; kph ^= 1; }
         if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
@@ -622,8 +623,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const bool leader = elect_one();
     const uint64_t desc_v0 = smem_desc_sw128(smem_u32(sm->v[0][0]), 8192, 1024);
     bool ok = true;
-    int vs = 0, vph = 0;
-    int slot = 0, slot_ph = 0, team = 0;
+    int vs = 0, slot = 0, slot_ph = 0, team = 0;
     FwdWalk walk;
     for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
@@ -644,43 +644,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       for (int u = 0; u < n_super && ok; ++u, team ^= 1) {
         const int nt = min(4, n_tiles - 4 * u);
-        // V first: it is there long before P, whose arrival is what the superstep waits for (each look at
-        // a barrier costs some 50 cycles, and there were two between P and its products: 3 % with
-        // everything listed)
         const int vs1 = vs + 1 < kVStages ? vs + 1 : 0;
-        ok = mbar_wait_warp(smem_u32(&sm->v_full[vs]), vph, abort_flag) &&
-             (nt <= 2 || mbar_wait_warp(smem_u32(&sm->v_full[vs1]), vs1 > 0 ? vph : vph ^ 1, abort_flag)) &&
-             mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph, abort_flag);  // P and V
         if (!ok) break;
         tc_fence_after();
         // Tiles a and b have their P in columns [0, 32) of the slot, a in lanes 0..63 and b in lanes
         // 64..127; c and d in columns [32, 64).  Each product writes the lanes of its tile only.  A
         // lane half's first product of an item starts its accumulator afresh.
         const uint32_t o_acc = tmem + kTmemO + 64 * team;
-        for (int pair = 0; pair < 2; ++pair) {
-          if (2 * pair >= nt) break;
-          if (leader) {
-            const uint32_t p_cols = tmem + 128 * slot + 32 * pair;
-            const uint64_t desc_v = desc_v0 + static_cast<uint64_t>(vs * 2) * (kTileBytes >> 4);
-            const uint32_t started = u > 1 || pair > 0;
+        if (leader) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            if (t >= nt) break;
+            const uint32_t p_cols = tmem + 128 * slot + 32 * (t >> 1);
+            const uint64_t desc_v = desc_v0 + static_cast<uint64_t>((t < 2 ? vs : vs1) * 2 + (t & 1)) * (kTileBytes >> 4);
+            const uint32_t started = u > 1 || t > 1;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              umma_ts_half(o_acc, p_cols + 8 * kk, desc_v + 128 * kk, idesc_pv, started | (kk > 0), 0);
-            if (nt > 2 * pair + 1) {
-#pragma unroll
-              for (int kk = 0; kk < 4; ++kk)
-                umma_ts_half(o_acc, p_cols + 8 * kk, desc_v + (kTileBytes >> 4) + 128 * kk, idesc_pv,
-                             started | (kk > 0), 1);
-            }
-            tc_commit(smem_u32(&sm->v_empty[vs]));
+              umma_ts_half(o_acc, p_cols + 8 * kk, desc_v + 128 * kk, idesc_pv, started | (kk > 0), t & 1);
           }
-          if (++vs == kVStages) { vs = 0; vph ^= 1; }
         }
-        if (!ok) break;
         if (leader) {
           tc_commit(smem_u32(&sm->pv_done[slot]));
           if (u == n_super - 1) tc_commit(smem_u32(&sm->o_full[par]));
         }
+        vs += 2;
+        if (vs >= kVStages) vs -= kVStages;
         if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
       }
     }
