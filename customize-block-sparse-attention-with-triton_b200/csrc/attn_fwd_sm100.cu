@@ -110,7 +110,6 @@ struct FwdSmem {
   alignas(16) int cnt[kMaxSorted];            // sort keys (tile count, item) of the items beyond the first round
   int order[kMaxSorted];                      // those items, longest first
   int4 item[kLists];                          // the item: batch (-1 = no more work), head, query block, tile count
-  int first_team[2];                          // by item parity: the team with the item's first superstep
   float mref[2][2][128];                      // by item parity, softmax team, lane
   float lsum[2][2][128];
   float mtrue[2][2][128];
@@ -685,6 +684,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t o_addr = tmem + lane_base + kTmemO + 64 * team;
     const float c = p.scale_log2;
+    const bool want_max = p.rowmax != nullptr;
     bool ok = true;
     int g = 0;        // supersteps of earlier items; this team takes those with g % 2 == team
     int next = team;  // its next one, with the slot next % kSlots and the barrier next % (2 kSlots)
@@ -713,13 +713,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tc_fence_after();
         // The row maximum is looked up only where it is needed: when the caller wants it, and with
         // element masks as long as one of the warp's rows has nothing yet.  The first superstep of the
-        // team takes the maximum of 32 logits for a reference (all 128 cost 450 cycles more), and
-        // logits are exponentiated against that as it is; a row whose sum shows that it was too low (or
-        // not finite) makes the warp do the superstep again with the maximum of all its logits.  S is
-        // still in tensor memory then: P goes over it last.
-        bool all = p.rowmax != nullptr;
-        if constexpr (kElementMask) all |= u >= 2 && __any_sync(0xffffffffu, m_ref == -INFINITY);
-        bool with_max = all || u < 2;
+        // team takes the maximum of the 32 logits that it holds anyway for a reference, and logits are
+        // exponentiated against that as it is; a row whose sum shows that it was too low (or not finite)
+        // makes the warp do the superstep again with the maximum of all its logits.  S is still in tensor
+        // memory then: P goes over it last.
+        bool with_max = want_max;
+        if constexpr (kElementMask) with_max |= u >= 2 && __any_sync(0xffffffffu, m_ref == -INFINITY);
         if (mine > 0) {
           const bool two = mine > 2;  // both tiles exist (warp-uniform)
           const auto masked = [&](uint32_t* sr, int col) {
@@ -736,18 +735,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (with_max) {
               float zmax = -INFINITY;
 #pragma unroll 1
-              for (int col = 0; col < (!all ? 32 : two ? 128 : 64); col += 32) {
+              for (int col = 0; col < (two ? 128 : 64); col += 32) {
                 tmem_ld_32x32b_x32(s_addr + col, sa);
                 tc_wait_ld();
                 masked(sa, col);
                 zmax = fmaxf(zmax, max_chunk(sa));
               }
               const float alpha = fwd_new_max(zmax * c, slack, m_ref, m_true, l);
-              if (kElementMask && !all && __any_sync(0xffffffffu, m_ref == -INFINITY)) {
-                all = true;  // a row has nothing among those 32
-                m_ref = -INFINITY;
-                continue;
-              }
               if (__any_sync(0xffffffffu, alpha != 1.f)) {
                 // the previous product of this team, two supersteps ago, must be in O
                 const int prev = slot == 2 ? 0 : slot + 1;  // (slot - 2) % 3
@@ -758,13 +752,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 fwd_rescale(o_addr, alpha);
               }
             }
-            const float neg_m = (kElementMask && m_ref == -INFINITY) ? 0.f : -m_ref;
             uint64_t l0 = pack_f32x2(0.f, 0.f), l1 = l0;
             tmem_ld_32x32b_x32(s_addr, sa);
             tmem_ld_32x32b_x32(s_addr + 32, sb);
             tc_wait_ld();
             masked(sa, 0);
             masked(sb, 32);
+            if (u < 2 && !with_max) {
+              m_ref = max_chunk(sa) * c;
+              if (kElementMask && __any_sync(0xffffffffu, m_ref == -INFINITY)) {
+                with_max = true;  // a row has nothing among those 32
+                m_ref = -INFINITY;
+                continue;
+              }
+            }
+            const float neg_m = (kElementMask && m_ref == -INFINITY) ? 0.f : -m_ref;
             exp_chunk<kBf16>(sa, c, neg_m, pk, l0, l1);
             if (two) {
               tmem_ld_32x32b_x32(s_addr + 64, sa);
@@ -781,8 +783,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             float a0, a1;
             unpack_f32x2(add_f32x2(l0, l1), a0, a1);
             sum = a0 + a1;
-            if (all || !__any_sync(0xffffffffu, !(sum <= kMaxRowSum))) break;
-            all = with_max = true;
+            if (with_max || !__any_sync(0xffffffffu, !(sum <= kMaxRowSum))) break;
+            with_max = true;
             // The maximum becomes the reference however little it lies above it: many logits a few units
             // above would fail the test in every later superstep of the row as well (N = 17536, everything
             // listed, keys from the second eighth on 6.3 above: 194 us, 107 with the move; 102 if level).
@@ -804,16 +806,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (bar_s >= 2 * kSlots) { bar_s -= 2 * kSlots; bar_ph ^= 1; }
       }
       if (!ok) break;
-      const int first_team = g & 1;
       g += n_super;
 
-      // publish this item's (m, l) of the warp's lanes; the slots of item i-2 must have been read
-      if (i >= 2) ok = mbar_wait_warp(smem_u32(&sm->o_free[par]), ((i - 2) >> 1) & 1, abort_flag);
-      if (!ok) break;
+      // publish this item's (m, l) of the warp's lanes (that this item was set up means that item i-2,
+      // whose slots these were, has been written out)
       sm->mref[par][team][lane_row] = m_ref;
       sm->lsum[par][team][lane_row] = l;
-      sm->mtrue[par][team][lane_row] = m_true;
-      if (warp == 0 && lane == 0) sm->first_team[par] = first_team;
+      if (want_max) sm->mtrue[par][team][lane_row] = m_true;
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->stats_full[par]));
     }
@@ -842,6 +841,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int lane_row = quarter * 32 + lane;
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the query block
     const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    int g = 0;  // supersteps of earlier items
     FwdWalk walk;
     for (int i = 0;; ++i, walk.next()) {
       const int par = i & 1;
@@ -889,15 +889,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->stats_full[par]), (i >> 1) & 1, abort_flag, 128);
       // The weights of the four partial results need the statistics only, which the softmax warps
       // publish before the item's last P V is complete.
-      int t0 = 0;  // the team with the item's first superstep
+      const int t0 = g & 1;  // the team with the item's first superstep
+      g += (n_tiles + 3) >> 2;
       uint64_t acc[32];  // 64 columns in pairs
       float m_all = -INFINITY, l_all = 0.f, mt = -INFINITY, w0 = 0.f, w1 = 0.f;
       if (ok) {
-        t0 = *const_cast<volatile int*>(&sm->first_team[par]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           m_all = fmaxf(m_all, sm->mref[par][j & 1][r_blk + 64 * (j >> 1)]);
-          mt = fmaxf(mt, sm->mtrue[par][j & 1][r_blk + 64 * (j >> 1)]);
+          if (p.rowmax) mt = fmaxf(mt, sm->mtrue[par][j & 1][r_blk + 64 * (j >> 1)]);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
