@@ -105,7 +105,6 @@ struct BwdSmem {
   uint64_t d_free[kXBars];                  // accumulating MMAs that read P/dS complete: the slot is free
   uint64_t d_full[kSlots];                  // by slot: P/dS stored
   uint32_t tmem_base;
-  int abort_flag;
 };
 
 static_assert(sizeof(BwdSmem) + 1024 <= 232448, "BwdSmem exceeds the shared memory of one CTA");
@@ -131,17 +130,11 @@ struct BwdParams {
   int wide_stores;  // output rows start on 32-byte boundaries
 };
 
-__device__ __forceinline__ void bwd_give_up(BwdSmem* sm, int32_t* status, int code) {
-  sm->abort_flag = 1;
-  report_status(status, code);
-}
-
 // Readers of the item header: wait for item i, read it (the producer looked the list up, so the
 // other roles start an item without a round trip to memory), tell the producer the slot was read.
-__device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, volatile int* abort_flag,
-                                              int* w, int* n_tiles, int* begin) {
+__device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, int* w, int* n_tiles, int* begin) {
   const int par = i & 1;
-  if (!mbar_wait_warp(smem_u32(&sm->item_full[par]), (i >> 1) & 1, abort_flag)) return false;
+  if (!mbar_wait_warp(smem_u32(&sm->item_full[par]), (i >> 1) & 1)) return false;
   *w = *const_cast<volatile int*>(&sm->item[par]);
   *n_tiles = *const_cast<volatile int*>(&sm->item_tiles[par]);
   *begin = *const_cast<volatile int*>(&sm->item_begin[par]);
@@ -190,12 +183,12 @@ template <int kPlaces, bool kVector>
 __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, uint64_t* empty,
                                                const CUtensorMap* map, float* vec_ring, const float* vec,
                                                const BwdItem& it, int n_super, int lane,
-                                               volatile int* abort_flag, int* gs) {
+                                               int* gs) {
   for (int j = 0; j < n_super; ++j, ++*gs) {
     const int s = *gs % kPlaces;
     const int nt = min(2, it.n_tiles - 2 * j), t = lane & 1;
     const int nj = t < nt ? (__ldg(it.ents + 2 * j + t) & kListIndex) : 0;
-    if (!mbar_wait_warp(smem_u32(empty + s), ((*gs / kPlaces) & 1) ^ 1, abort_flag)) return false;
+    if (!mbar_wait_warp(smem_u32(empty + s), ((*gs / kPlaces) & 1) ^ 1)) return false;
     const uint32_t bar = smem_u32(full + *gs % (2 * kPlaces));
     if (lane == 0) mbar_expect_tx(bar, nt * (kBwdTile + (kVector ? 256u : 0u)));
     __syncwarp();
@@ -210,7 +203,7 @@ __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, ui
 // The S/dP instructions of one team's supersteps (one warp).
 template <bool kBf16, bool kDKDV>
 __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uint32_t tmem, int team,
-                                            int lane, volatile int* abort_flag) {
+                                            int lane) {
   constexpr uint32_t idesc_x = umma_idesc(kBf16, 0, 0, 64, 128);
   const bool leader = elect_one();
   const uint64_t desc_a0 = smem_desc_sw128(smem_u32(sm->stat[0][0]), 16, 1024);
@@ -223,23 +216,22 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
   int gs = 0, ni = 0;
   for (int i = 0; ok; ++i) {
     int w, w_tiles, w_begin;
-    ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+    ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
     if (!ok || w < 0) break;
     const int n_super = (w_tiles + 1) >> 1;
     if (n_super == 0) continue;
     const int own = ni & 1;
-    ok = mbar_wait_warp(smem_u32(&sm->stat_full[own]), (ni >> 1) & 1, abort_flag);
+    ok = mbar_wait_warp(smem_u32(&sm->stat_full[own]), (ni >> 1) & 1);
     const uint64_t a0 = desc_a0 + static_cast<uint64_t>(2 * own) * kTileDesc;
     int g = gs + ((gs ^ team) & 1);
     gs += n_super;
     for (; ok && g < gs; g += 2) {
-      ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, abort_flag) &&
-           mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, abort_flag);
+      ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1) &&
+           mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1);
       if (!ok) break;
       // the accumulating products of the slot's previous superstep must be complete
       if (g >= kSlots)
-        ok = mbar_wait_warp(smem_u32(&sm->d_free[(g - kSlots) % kXBars]), ((g - kSlots) / kXBars) & 1,
-                            abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->d_free[(g - kSlots) % kXBars]), ((g - kSlots) / kXBars) & 1);
       if (!ok) break;
       tc_fence_after();
       if (leader) {
@@ -264,7 +256,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
     if (ok && leader) tc_commit(smem_u32(&sm->stat_free[own]));  // this issuer is through with the operands
     ++ni;
   }
-  if (!ok) bwd_give_up(sm, p.status, 2);
+  if (!ok) report_status(p.status, 2);
 }
 
 // The accumulating instructions of one warp.  dK/dV: the first warp's sum dV, the second one's dK (each
@@ -272,7 +264,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
 // of tile a, the second one's those of tile b.
 template <bool kBf16, bool kDKDV>
 __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, uint32_t tmem, bool first,
-                                              int lane, volatile int* abort_flag) {
+                                              int lane) {
   const bool dv = kDKDV && first;
   const uint32_t idesc = umma_idesc(kBf16, 0, 1, 128, p.D);
   const bool leader = elect_one();
@@ -285,13 +277,13 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   uint32_t phase = 0;  // of the slot's barrier
   for (int i = 0; ok; ++i) {
     int w, w_tiles, w_begin;
-    ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+    ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
     if (!ok || w < 0) break;
     if (w_tiles == 0) continue;
     // the write-out warps must have read the previous block's accumulators
-    if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1, abort_flag);
+    if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1);
     for (int left = w_tiles; ok && left > 0; left -= 2) {
-      ok = mbar_wait_warp(smem_u32(&sm->d_full[slot]), phase, abort_flag);
+      ok = mbar_wait_warp(smem_u32(&sm->d_full[slot]), phase);
       if (!ok) break;
       tc_fence_after();
       if (leader) {
@@ -321,7 +313,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
     }
     ++ni;
   }
-  if (!ok) bwd_give_up(sm, p.status, 2);
+  if (!ok) report_status(p.status, 2);
 }
 
 // Persistent: one CTA per SM.  The producer starts with item blockIdx.x and then draws further
@@ -363,7 +355,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     for (int s = 0; s < kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
     mbar_init(smem_u32(&sm->acc_done), 2);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
-    sm->abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == kXWarp) {
@@ -380,7 +371,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
-  volatile int* abort_flag = &sm->abort_flag;
   grid_dependency_wait();
 
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
@@ -411,7 +401,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         }
         // the header slot of item i-2 must have been read by everyone
         if (i >= 2)
-          ok = mbar_wait_warp(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1, abort_flag);
+          ok = mbar_wait_warp(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1);
         if (!ok) break;
         BwdItem it;
         it.n_tiles = 0;
@@ -428,7 +418,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         // the block's own operands: the S/dP instructions of the block before the previous one must
         // be complete
         const int own = ni & 1;
-        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1, abort_flag);
+        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1);
         if (!ok) break;
         {
           const uint32_t bar = smem_u32(&sm->stat_full[own]);
@@ -438,11 +428,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
           }
         }
         ok = bwd_load_tiles<kRing0<kDKDV>, kDKDV>(sm->ring[0][0], sm->in_full0, sm->in_empty0, &tm_str0,
-                                                  sm->lse[0][0], p.lse2, it, n_super, lane, abort_flag,
-                                                  &gs);
+                                                  sm->lse[0][0], p.lse2, it, n_super, lane, &gs);
         ++ni;
       }
-      if (!ok) bwd_give_up(sm, p.status, 1);
+      if (!ok) report_status(p.status, 1);
       if (!terminal && lane == 0) {
         // gave up before the last draw: draw on (without working) until this CTA's first ticket past
         // the end, so that the launch still draws `items` tickets and the counter returns to zero
@@ -458,13 +447,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       int gs = 0, ni = 0;
       for (int i = 0; ok; ++i) {
         int w, w_tiles, w_begin;
-        ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+        ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
         if (!ok || w < 0) break;
         const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
         const int n_super = (w_tiles + 1) >> 1;
         if (n_super == 0) continue;
         const int own = ni & 1;
-        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1, abort_flag);
+        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1);
         if (!ok) break;
         if (lane == 0) {
           const uint32_t bar = smem_u32(&sm->stat_full[own]);
@@ -473,14 +462,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         }
         ok = bwd_load_tiles<kRing1<kDKDV>, kDKDV>(sm->ring[kRing0<kDKDV>][0], sm->in_full1,
                                                   sm->in_empty1, &tm_str1, sm->delta[0][0], p.delta, it,
-                                                  n_super, lane, abort_flag, &gs);
+                                                  n_super, lane, &gs);
         ++ni;
       }
-      if (!ok) bwd_give_up(sm, p.status, 1);
+      if (!ok) report_status(p.status, 1);
     } else if (warp == kXWarp || warp == kX2Warp) {
-      bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane, abort_flag);
+      bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane);
     } else if (warp == kAccWarp || warp == kAcc2Warp) {
-      bwd_issue_acc<kBf16, kDKDV>(sm, p, tmem, warp == kAccWarp, lane, abort_flag);
+      bwd_issue_acc<kBf16, kDKDV>(sm, p, tmem, warp == kAccWarp, lane);
     }
   } else if (warp < kCW) {
     // =========================== compute warps ===========================
@@ -496,7 +485,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     int gs = 0;  // supersteps of earlier items; this team takes those with gs % 2 == team
     for (int i = 0; ok; ++i) {
       int w, w_tiles, w_begin;
-      ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+      ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
       if (!ok || w < 0) break;
       const int n_super = (w_tiles + 1) >> 1;
       if (n_super == 0) continue;  // (the write-out warps store the zero gradients)
@@ -554,7 +543,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
             }
           }
         }
-        ok = mbar_wait_warp(smem_u32(&sm->x_full[g % kXBars]), (g / kXBars) & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->x_full[g % kXBars]), (g / kXBars) & 1);
         if (!ok) break;
         tc_fence_after();
         if (active) {
@@ -640,7 +629,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       // (the block's sums are merged and stored by the write-out warps; these warps go straight
       // on to the next block, whose first S/dP is usually complete already)
     }
-    if (!ok) bwd_give_up(sm, p.status, 3);
+    if (!ok) report_status(p.status, 3);
   } else {
     // =========================== write-out ===========================
     // Lane r of an accumulator holds the tile-a sums of row r of the CTA's block, lane r+64 its tile-b
@@ -667,7 +656,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     int ni = 0;
     for (int i = 0;; ++i) {
       int w = 0, w_tiles = 1, w_begin = 0;
-      if (ok) ok = bwd_next_item(sm, i, lane, abort_flag, &w, &w_tiles, &w_begin);
+      if (ok) ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
       if (ok && w < 0) break;  // no more work: the same for all four warps
       const BwdItem it = bwd_item<kDKDV>(ok ? w : 0, p, ok ? w_tiles : 1, 0);
       const int64_t row = it.blk * 64 + r_blk;
@@ -681,7 +670,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
           *reinterpret_cast<uint4*>(dst + v) = make_uint4(0u, 0u, 0u, 0u);
         continue;
       }
-      if (ok) ok = mbar_wait_warp(smem_u32(&sm->acc_done), ni & 1, abort_flag);
+      if (ok) ok = mbar_wait_warp(smem_u32(&sm->acc_done), ni & 1);
       ++ni;
       const bool live = half == 0 || w_tiles > 1;  // warp-uniform
       bool any_failed = false;
@@ -744,7 +733,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       }
       if (any_failed) break;
     }
-    if (!ok) bwd_give_up(sm, p.status, 3);
+    if (!ok) report_status(p.status, 3);
   }
 
   // (not before: CTAs of the next kernel that wait on free SMs slowed the working ones down by 3 %)

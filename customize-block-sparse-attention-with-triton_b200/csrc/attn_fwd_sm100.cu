@@ -38,19 +38,20 @@
 //                 g % 2's).  A warp loads its tiles' 128 logits, exponentiates them, packs P to 16 bit
 //                 and stores it over the logits (first tile in columns [0, 32) of the slot, second
 //                 one in [32, 64)).
-//   warp 8      : K producer — lists the CTA's first item, then TMA-loads Q and the listed K tiles of
-//                 every item into a 3-deep ring of superstages (4 tiles, held until S is complete),
-//                 one lane per tile, and tells the lister when to set up the next item
+//   warp 8      : K producer — TMA-loads Q and the listed K tiles of every item into a 3-deep ring of
+//                 superstages (4 tiles, held until S is complete), one lane per tile, and tells the lister
+//                 when to set up the next item
 //   warp 9      : S issuer and TMEM owner
 //   warp 10     : P V issuer — O[team] += P_t V_t for the tiles t of the superstep.  P is read from
 //                 TMEM, V is an MN-major shared-memory operand.  Row r of an accumulator sums products
 //                 of tiles a and c, row r+64 of tiles b and d.
 //   warp 11     : V producer — TMA-loads the listed V tiles in pairs into a 5-deep ring (held until
-//                 their P V is complete).  Only listed tiles are ever loaded.
+//                 their P V is complete); they land on the barrier that P arrives on.  Only listed tiles
+//                 are ever loaded.
 //   warps 12..15: write-out — merge the four partial results (m, l, O) of every query row (teams x
 //                 lanes r / r+64), normalise, store O, LSE and the row maximum
-//   warp 15     : also the lister — draws the next item, lists its key blocks (from the mask row, or
-//                 copies the CSR row) into the next of three list buffers and publishes it
+//   warp 15     : also the lister — draws the items, lists their key blocks (from the mask row, or
+//                 copies the CSR row) into the next of three list buffers and publishes them
 // TMEM (512 columns): S/P slots 3 x 128, accumulators 2 x 64.
 //
 // Head dimensions 16 and 32 run on the same 128-byte rows: the tensor maps are D wide, so TMA fills
@@ -85,7 +86,7 @@ constexpr int kTeamWarps = kSoftmaxWarps / 2;
 constexpr int kProducerWarp = 8, kSWarp = 9, kPvWarp = 10, kVProducerWarp = 11;
 constexpr int kListerWarp = 15;      // the last of the write-out warps 12..15: also sets up the items
 constexpr int kFwdThreads = 512;
-constexpr int kGoBefore = 2;         // ordered hand-out: supersteps before an item's end at which the next is drawn
+constexpr int kGoBefore = 2;         // supersteps before an item's end at which the next is set up
 constexpr uint32_t kTileBytes = 64 * 64 * 2;       // one Q, K or V tile
 constexpr uint32_t kFwdTmemCols = 512;
 // TMEM columns: slot r at 128 r; accumulator of softmax team T at 384 + 64 T.
@@ -95,7 +96,6 @@ constexpr float kRescaleThreshold = 8.0f;
 // against a reference maximum that was not checked: far below fp16's 65504.
 constexpr float kMaxRowSum = 4096.0f;
 constexpr int kFwdMaxTiles = 2048;  // key blocks per row that a CTA can list (N <= 131072)
-constexpr int kMaxSorted = 320;     // items beyond the first round that a CTA can put in order
 constexpr uint16_t kColPartial = 0x8000;  // list entry in shared memory: the tile has masked elements
 constexpr uint16_t kColIndex = 0x7fff;
 
@@ -107,13 +107,10 @@ struct FwdSmem {
   // of 20 floats: eight lanes' 16-byte accesses then fall into different banks)
   float xfer[2][64][20];
   uint16_t cols[kLists][kFwdMaxTiles];        // ring over the items: the item's key-block list (| kColPartial)
-  alignas(16) int cnt[kMaxSorted];            // sort keys (tile count, item) of the items beyond the first round
-  int order[kMaxSorted];                      // those items, longest first
   int4 item[kLists];                          // the item: batch (-1 = no more work), head, query block, tile count
   float mref[2][2][128];                      // by item parity, softmax team, lane
   float lsum[2][2][128];
   float mtrue[2][2][128];
-  uint64_t order_full;                        // `order` is ready
   uint64_t list_full[kLists];                 // lister -> everyone: list and header ready
   uint64_t list_free[kLists];                 // producers and issuers are through with list and header
   uint64_t setup_go[2];                       // producer -> lister: time to set up the next item
@@ -270,75 +267,16 @@ __device__ __forceinline__ const uint8_t* fwd_mask_row(const FwdItem& it, const 
          static_cast<int64_t>(it.mb) * p.ms2;
 }
 
-// Number of kept blocks in a contiguous mask row of nb bytes, read by ONE thread: bytes up to the
-// first 4-byte boundary, then words (a word's non-zero bytes are counted with a byte-wise
-// compare), then the tail.
-__device__ __forceinline__ int fwd_count_row(const uint8_t* row, int nb) {
-  int n = 0, c = 0;
-  const int head = static_cast<int>((4u - (reinterpret_cast<uintptr_t>(row) & 3u)) & 3u);
-  for (; c < head && c < nb; ++c) n += __ldg(row + c) != 0 ? 1 : 0;
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(row + c);
-  const int words = (nb - c) >> 2;
-  int k = 0;
-  for (; k + 16 <= words; k += 16) {
-    uint32_t a[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) a[j] = __ldg(w + k + j);
-    int bits = 0;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) bits += __popc(__vcmpne4(a[j], 0u));
-    n += bits >> 3;
-  }
-  for (; k + 4 <= words; k += 4) {
-    const uint32_t a0 = __ldg(w + k), a1 = __ldg(w + k + 1), a2 = __ldg(w + k + 2),
-                   a3 = __ldg(w + k + 3);
-    n += (__popc(__vcmpne4(a0, 0u)) + __popc(__vcmpne4(a1, 0u)) + __popc(__vcmpne4(a2, 0u)) +
-          __popc(__vcmpne4(a3, 0u))) >> 3;
-  }
-  for (; k < words; ++k) n += __popc(__vcmpne4(__ldg(w + k), 0u)) >> 3;
-  for (c += 4 * words; c < nb; ++c) n += __ldg(row + c) != 0 ? 1 : 0;
-  return n;
-}
-
-// When the items are handed out through the work counter and there are at most a few per CTA, it
-// matters who gets which: rows of a random mask differ in length, and the kernel is as slow as
-// the CTA with the largest sum.  The first round is fixed (CTA c takes item c); the remaining
-// items are handed out longest first, so that the CTAs that finish their first item early take
-// the long ones.  Every CTA works the order out for itself (same input, same result) with the
-// four write-out warps, which have nothing to do during the first item: one thread per row counts
-// the row's kept blocks, then every thread ranks its row among all.
-__device__ __forceinline__ void fwd_build_order(FwdSmem* sm, const FwdParams& p, int tid, int first,
-                                                int n2) {
-  for (int j = tid; j < n2; j += 128) {
-    const FwdItem it = fwd_item(first + j, p);
-    int n;
-    if (p.block != nullptr) {
-      n = fwd_count_row(fwd_mask_row(it, p), p.nb);
-    } else {
-      const int64_t li =
-          static_cast<int64_t>(it.b * p.list_b_stride + it.h * p.list_h_stride) * p.nb + it.mb;
-      n = __ldg(p.row_ptr + li + 1) - __ldg(p.row_ptr + li);
-    }
-    // one key per item, all different: longer rows first, equal rows in item order
-    sm->cnt[j] = n * 512 + (511 - j);
-  }
-  const int n4 = (n2 + 3) & ~3;
-  for (int j = n2 + tid; j < n4; j += 128) sm->cnt[j] = -1;  // padding ranks behind every item
-  named_barrier_sync(2, 128);
-  for (int j = tid; j < n2; j += 128) {
-    const int kj = sm->cnt[j];
-    int r0 = 0, r1 = 0, r2 = 0, r3 = 0;
-    for (int k = 0; k < n4; k += 4) {
-      const int4 c = *reinterpret_cast<const int4*>(&sm->cnt[k]);
-      r0 += c.x > kj ? 1 : 0;
-      r1 += c.y > kj ? 1 : 0;
-      r2 += c.z > kj ? 1 : 0;
-      r3 += c.w > kj ? 1 : 0;
-    }
-    sm->order[(r0 + r1) + (r2 + r3)] = j;
-  }
-  named_barrier_sync(2, 128);
-  if (tid == 0) mbar_arrive(smem_u32(&sm->order_full));
+// The bytes of a contiguous mask row of nb bytes as 0xff (kept) or 0, four columns at a time: those of the
+// 4-byte word of memory `word` words behind the one that the row begins in.  Columns that are none give 0,
+// and a word without a column of the row is not read.
+__device__ __forceinline__ uint32_t fwd_row_word(const uint8_t* row, int nb, int word) {
+  const int off = static_cast<int>(reinterpret_cast<uintptr_t>(row) & 3u), c = 4 * word - off;
+  uint32_t v = 0u;
+  if (c < nb) v = __ldg(reinterpret_cast<const uint32_t*>(row - off) + word);
+  if (c < 0) v &= 0xffffffffu << (8 * off);
+  if (c + 4 > nb && c < nb) v &= 0xffffffffu >> (8 * (c + 4 - nb));
+  return v;
 }
 
 // Lists the key blocks of work item w into list buffer `at` (one warp) and publishes list and item.
@@ -349,29 +287,43 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
   uint16_t* cols = sm->cols[at];
   int n_tiles = 0;
   if (p.block != nullptr) {
-    // mask mode: ordered compaction of the kept blocks of mask row (b, h, mb)
+    // mask mode: the kept blocks of mask row (b, h, mb) in order
     const uint8_t* mrow = fwd_mask_row(it, p);
-    // 128 columns per pass, four independent loads per lane; the next pass's loads are issued
-    // before this pass's ballots, so a row costs one round trip to L2 rather than one per pass
-    int byte[4], next[4];
+    if (p.ms3 == 1) {
+      // 128 columns per pass, four per lane; the words of four passes are on their way at a time, so that a
+      // row costs one round trip to memory up to N = 32,000
+      const int off = static_cast<int>(reinterpret_cast<uintptr_t>(mrow) & 3u);
+      uint32_t next[4];
 #pragma unroll
-    for (int jj = 0; jj < 4; ++jj) {
-      const int c = 32 * jj + lane;
-      next[jj] = c < p.nb ? mrow[c * p.ms3] : 0;
-    }
-    for (int c0 = 0; c0 < p.nb; c0 += 128) {
+      for (int j = 0; j < 4; ++j) next[j] = fwd_row_word(mrow, p.nb, 32 * j + lane);
+#pragma unroll 1
+      for (int w = lane; 4 * (w - lane) < p.nb + off; w += 32) {
+        const uint32_t v = next[0];
 #pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        byte[jj] = next[jj];
-        const int c = c0 + 128 + 32 * jj + lane;
-        next[jj] = c < p.nb ? mrow[c * p.ms3] : 0;
+        for (int j = 0; j < 3; ++j) next[j] = next[j + 1];
+        next[3] = fwd_row_word(mrow, p.nb, w + 128);
+        uint16_t* out = cols + n_tiles;
+        uint32_t kept[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          kept[j] = __ballot_sync(0xffffffffu, (v >> (8 * j) & 0xffu) != 0);
+          out += __popc(kept[j] & ((1u << lane) - 1u));
+          n_tiles += __popc(kept[j]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t byte = v >> (8 * j) & 0xffu;
+          if (byte != 0) *out++ = static_cast<uint16_t>((4 * w - off + j) | (kElementMask && byte == 2 ? kColPartial : 0));
+        }
       }
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj) {
-        const unsigned bal = __ballot_sync(0xffffffffu, byte[jj] != 0);
-        if (byte[jj] != 0)
-          cols[n_tiles + __popc(bal & ((1u << lane) - 1u))] = static_cast<uint16_t>(
-              (c0 + 32 * jj + lane) | (kElementMask && byte[jj] == 2 ? kColPartial : 0));
+    } else {
+#pragma unroll 1
+      for (int c0 = 0; c0 < p.nb; c0 += 32) {
+        const int c = c0 + lane, byte = c < p.nb ? mrow[c * p.ms3] : 0;
+        const unsigned bal = __ballot_sync(0xffffffffu, byte != 0);
+        if (byte != 0)
+          cols[n_tiles + __popc(bal & ((1u << lane) - 1u))] =
+              static_cast<uint16_t>(c | (kElementMask && byte == 2 ? kColPartial : 0));
         n_tiles += __popc(bal);
       }
     }
@@ -380,6 +332,7 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
         static_cast<int64_t>(it.b * p.list_b_stride + it.h * p.list_h_stride) * p.nb + it.mb;
     const int beg = __ldg(p.row_ptr + li);
     n_tiles = __ldg(p.row_ptr + li + 1) - beg;
+#pragma unroll 1
     for (int jj = lane; jj < n_tiles; jj += 32) {
       const int e = __ldg(p.col_idx + beg + jj);
       cols[jj] = static_cast<uint16_t>(
@@ -397,8 +350,8 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
 struct FwdWalk {
   int at = 0, ph = 0;  // list buffer, phase of its barrier
   int4 it;             // batch (< 0: no more work), head, query block, tile count
-  __device__ __forceinline__ bool wait(FwdSmem* sm, volatile int* abort_flag) {
-    if (!mbar_wait_warp(smem_u32(&sm->list_full[at]), ph, abort_flag)) return false;
+  __device__ __forceinline__ bool wait(FwdSmem* sm) {
+    if (!mbar_wait_warp(smem_u32(&sm->list_full[at]), ph)) return false;
     it = sm->item[at];
     return true;
   }
@@ -420,14 +373,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x;
-  // items beyond the first round; few enough per CTA for their order to matter?  (mask mode
-  // needs contiguous mask rows for the count)
-  const int n2 = p.items - stride;
-  const bool sorted = p.ticket != nullptr && n2 > 1 && n2 <= kMaxSorted &&
-                      (p.block == nullptr || p.ms3 == 1);
+  const int n2 = p.items - stride;  // items beyond the first round
 
   // ---- set-up ----
   if (threadIdx.x == 0) {
+#pragma unroll 1
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->setup_go[i]), 1);
       mbar_init(smem_u32(&sm->q_full[i]), 1);
@@ -435,20 +385,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(smem_u32(&sm->stats_full[i]), kSoftmaxWarps);
       mbar_init(smem_u32(&sm->o_free[i]), 4);  // one arrival per write-out warp
     }
+#pragma unroll 1
     for (int s = 0; s < kKStages; ++s) {
       mbar_init(smem_u32(&sm->k_full[s]), 1);
       mbar_init(smem_u32(&sm->k_empty[s]), 1);
     }
+#pragma unroll 1
     for (int s = 0; s < 2 * kSlots; ++s) mbar_init(smem_u32(&sm->s_full[s]), 1);
+#pragma unroll 1
     for (int s = 0; s < kSlots; ++s) {
       mbar_init(smem_u32(&sm->p_full[s]), kTeamWarps + 1);
       mbar_init(smem_u32(&sm->pv_done[s]), 1);
     }
+#pragma unroll 1
     for (int s = 0; s < kLists; ++s) {
       mbar_init(smem_u32(&sm->list_full[s]), 1);
       mbar_init(smem_u32(&sm->list_free[s]), 4);  // two producers, two issuers
     }
-    mbar_init(smem_u32(&sm->order_full), 1);
     sm->abort_flag = 0;
     mbar_fence_init();
   }
@@ -468,26 +421,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   volatile int* abort_flag = &sm->abort_flag;
   grid_dependency_wait();
 
-  // 512 threads are launched with 128 registers: the softmax warps, which hold 128 logits each, take
-  // what the others do without (2 x 160 + 80 + 112 = 4 x 128).
+  // 512 threads are launched with 128 registers: the softmax warps, which hold 64 logits and 128
+  // probabilities each, take what the others do without (2 x 168 + 72 + 104 = 4 x 128).  A spill in their
+  // loop (28 bytes at 160) made the kernel 4 to 5 % slower.
   if (warp >= kSoftmaxWarps && warp < kSoftmaxWarps + 4) {
-  give_registers<80>();
+  give_registers<72>();
   if (warp == kProducerWarp) {
     // =========================== K producer ===========================
     bool ok = true;
     // Loads Q and the K tiles of the listed key blocks from the list the lister published, and
-    // tells the lister when to set up the next item.  A set-up takes 3-4 thousand cycles (the draw
-    // from the work counter, the mask row, the ballots in a warp that shares its scheduler with
-    // the softmax warps), about three supersteps.  With many items per CTA it is started as soon as an
-    // item begins; with the few items of the ordered hand-out, where it matters that a CTA draws
-    // its next item only when it is about to need it, kGoBefore supersteps of loads before the end.
+    // tells the lister when to set up the next item: kGoBefore supersteps of loads before the end, so that
+    // a CTA draws its next item when it is about to need it.  (Set up as soon as an item begins: four heads,
+    // N = 6400, causal, a quarter of the blocks 19.3 us against 18.6, the same with many items.  Items
+    // beyond the first round longest first, which every CTA had to work out for itself: 22.0 us; and with
+    // one head, N = 17536, a tenth: 20.2 us against 19.2.)
     int ks = 0, kph = 1;  // ring position, parity to wait for
     int qi = 0;           // non-empty items so far (Q buffer position)
-    fwd_list_item<kElementMask>(sm, p, blockIdx.x, 0, lane);  // the CTA's own first item
     FwdWalk walk;
+#pragma unroll 1
     for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
-      ok = walk.wait(sm, abort_flag);
+      ok = walk.wait(sm);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
       const uint16_t* cols = sm->cols[walk.at];
@@ -502,14 +456,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         ++qi;
       }
-      const int u_go = sorted ? max(n_super - kGoBefore, 0) : 0;
+      const int u_go = max(n_super - kGoBefore, 0);
       if (n_super == 0 && lane == 0) mbar_arrive(smem_u32(&sm->setup_go[par]));
       // One lane per tile issues its load: a single thread can start a tile load only every couple
       // of hundred cycles.
+#pragma unroll 1
       for (int u = 0; u < n_super; ++u) {
         if (u == u_go && lane == 0) mbar_arrive(smem_u32(&sm->setup_go[par]));
         const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->k_empty[ks]), kph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->k_empty[ks]), kph);
         if (!ok) break;
         const uint32_t bar = smem_u32(&sm->k_full[ks]);
         if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
@@ -535,24 +490,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     int vs = 0, slot = 0, ph = 1;
     FwdWalk walk;
+#pragma unroll 1
     for (; ok; walk.next()) {
-      ok = walk.wait(sm, abort_flag);
+      ok = walk.wait(sm);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
       const uint16_t* cols = sm->cols[walk.at];
+#pragma unroll 1
       for (int u = 0; 4 * u < n_tiles; ++u) {
         const int nt = min(4, n_tiles - 4 * u);
         const int at = lane < 2 ? vs : vs + 1 < kVStages ? vs + 1 : 0;
         const int row = lane < nt ? static_cast<int>(cols[4 * u + lane] & kColIndex) * 64 : 0;
         const uint32_t dst = smem_u32(sm->v[at][lane & 1]), bar = smem_u32(&sm->p_full[slot]);
         // (for the first users these ask for the phase before the first one, which counts as complete)
-        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), ph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), ph);
         if (!ok) break;
         if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
         __syncwarp();
         if (lane < min(nt, 2)) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
         const int next = slot + 1 < kSlots ? slot + 1 : 0;
-        ok = mbar_wait_warp(smem_u32(&sm->pv_done[next]), next > 0 ? ph : ph ^ 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->pv_done[next]), next > 0 ? ph : ph ^ 1);
         if (!ok) break;
         if (lane >= 2 && lane < nt) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
         vs += 2;
@@ -577,8 +534,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int ks = 0, kph = 0, qi = 0;
     int slot = 0, slot_ph = 1, bar_s = 0;  // (bar_s: superstep number mod 2 kSlots)
     FwdWalk walk;
+#pragma unroll 1
     for (; ok; walk.next()) {
-      ok = walk.wait(sm, abort_flag);
+      ok = walk.wait(sm);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
       const int n_super = (n_tiles + 3) >> 2;
@@ -586,15 +544,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
       if (n_super == 0) continue;
       const int qpar = qi & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->q_full[qpar]), (qi >> 1) & 1, abort_flag);
+      ok = mbar_wait_warp(smem_u32(&sm->q_full[qpar]), (qi >> 1) & 1);
       if (!ok) break;
       const uint64_t desc_q = desc_q0 + static_cast<uint64_t>(qpar) * kTileDesc;
+#pragma unroll 1
       for (int u = 0; u < n_super; ++u) {
-        ok = mbar_wait_warp(smem_u32(&sm->k_full[ks]), kph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->k_full[ks]), kph);
         if (!ok) break;
         // the slot's previous user, three supersteps ago, must have had its P V completed (for the
         // first users this asks for the phase before the first one, which counts as complete)
-        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), slot_ph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), slot_ph);
         if (!ok) break;
         tc_fence_after();
         if (leader) {
@@ -624,9 +583,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     int vs = 0, slot = 0, slot_ph = 0, team = 0;
     FwdWalk walk;
+#pragma unroll 1
     for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
-      ok = walk.wait(sm, abort_flag);
+      ok = walk.wait(sm);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
       const int n_super = (n_tiles + 3) >> 2;
@@ -635,16 +595,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       // the accumulators are free once the previous item has been read out; the softmax warps
       // meanwhile work ahead
       if (i >= 1)
-        ok = mbar_wait_warp(smem_u32(&sm->o_free[par ^ 1]), ((i - 1) >> 1) & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->o_free[par ^ 1]), ((i - 1) >> 1) & 1);
       if (!ok) break;
       if (n_super == 0) {
         if (leader) mbar_arrive(smem_u32(&sm->o_full[par]));
         continue;
       }
+#pragma unroll 1
       for (int u = 0; u < n_super && ok; ++u, team ^= 1) {
         const int nt = min(4, n_tiles - 4 * u);
         const int vs1 = vs + 1 < kVStages ? vs + 1 : 0;
-        ok = mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph, abort_flag);  // P and V
+        ok = mbar_wait_warp(smem_u32(&sm->p_full[slot]), slot_ph);  // P and V
         if (!ok) break;
         tc_fence_after();
         // Tiles a and b have their P in columns [0, 32) of the slot, a in lanes 0..63 and b in lanes
@@ -676,7 +637,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   } else if (warp < kSoftmaxWarps) {
     // =========================== softmax ===========================
-    take_registers<160>();
+    take_registers<168>();
     const int team = warp >> 2;
     const int quarter = warp & 3;     // TMEM lane quarter this warp may touch
     const int half = quarter >> 1;    // lanes 0..63 own tiles a, c of a superstep, 64..127 b, d
@@ -690,9 +651,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     int next = team;  // its next one, with the slot next % kSlots and the barrier next % (2 kSlots)
     int slot = team, bar_s = team, bar_ph = 0;
     FwdWalk walk;
+#pragma unroll 1
     for (int i = 0; ok; ++i, walk.next()) {
       const int par = i & 1;
-      ok = walk.wait(sm, abort_flag);
+      ok = walk.wait(sm);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
       const int n_super = (n_tiles + 3) >> 2;
@@ -704,11 +666,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         mask_row = p.dense + walk.it.x * p.ds0 + walk.it.y * p.ds1 +
                    static_cast<int64_t>(walk.it.z * 64 + (quarter & 1) * 32 + lane) * p.ds2;
 
+#pragma unroll 1
       for (; next < g + n_super; next += 2) {
         const int u = next - g;
         const uint32_t s_addr = tmem + lane_base + 128 * slot;
         const int mine = n_tiles - 4 * u - half;  // > 0: this lane's first tile exists, > 2: both
-        ok = mbar_wait_warp(smem_u32(&sm->s_full[bar_s]), bar_ph, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sm->s_full[bar_s]), bar_ph);
         if (!ok) break;
         tc_fence_after();
         // The row maximum is looked up only where it is needed: when the caller wants it, and with
@@ -730,6 +693,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           };
           uint32_t pk[64];
           float sum, slack = kRescaleThreshold;
+#pragma unroll 1
           while (true) {
             uint32_t sa[32], sb[32];
             if (with_max) {
@@ -746,7 +710,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 // the previous product of this team, two supersteps ago, must be in O
                 const int prev = slot == 2 ? 0 : slot + 1;  // (slot - 2) % 3
                 ok = mbar_wait_warp(smem_u32(&sm->pv_done[prev]),
-                                    static_cast<uint32_t>((next - 2) / kSlots) & 1u, abort_flag);
+                                    static_cast<uint32_t>((next - 2) / kSlots) & 1u);
                 if (!ok) break;
                 tc_fence_after();
                 fwd_rescale(o_addr, alpha);
@@ -825,58 +789,54 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // barriers of an iteration are always executed, also after a give-up, and the last one carries
     // the give-up vote, so that no warp of this role can be left waiting at one.
     //
-    // One of the four warps is also the lister: it sets up item i+1 when the producer says so
-    // during item i, i.e. between its write-outs of items i-1 and i (the producer lists the
-    // CTA's first item itself, which nothing can overlap).  The draw from the work counter, the mask
-    // row and the ballots take a couple of thousand cycles, which in the producer's own instruction
-    // stream held back the K tiles of the current item.
-    give_registers<112>();
+    // One of the four warps is also the lister: it sets up the CTA's first item, and item i+1 when the
+    // producer says so during item i, i.e. between its write-outs of items i-1 and i.
+    give_registers<104>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
     const bool lister = warp == kListerWarp;
     bool ok = true;
     bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
     int lw = blockIdx.x;
-    if (sorted) fwd_build_order(sm, p, quarter * 32 + lane, stride, n2);
     const int half = quarter >> 1;
     const int lane_row = quarter * 32 + lane;
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the query block
-    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t o_lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kTmemO;
     int g = 0;  // supersteps of earlier items
     FwdWalk walk;
-    for (int i = 0;; ++i, walk.next()) {
+#pragma unroll 1
+    for (int i = -1;; ++i) {
       const int par = i & 1;
-      if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag, 256);
-      walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
-      if (walk.it.x < 0) break;  // no more work: the same for all four warps
-      const int n_tiles = walk.it.w;
+      if (i >= 0) {
+        if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag, 256);
+        walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
+        if (walk.it.x < 0) break;  // no more work: the same for all four warps
+      }
       if (lister && ok) {
         // Sets up the next item, or publishes that there is none; a wait that gives up leaves ok =
         // false and nothing published.  The next ticket when items are handed out dynamically, else
         // a fixed stride.
-        ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1, abort_flag);
-        const int at = walk.at + 1 < kLists ? walk.at + 1 : 0;
-        if (ok && p.ticket != nullptr) {
-          int t = 0;
-          if (lane == 0) {
-            t = atomicAdd(p.ticket, 1);
-            // every CTA draws until its first ticket past the end, so the launch draws exactly
-            // `items` tickets in all; whoever draws the last one leaves the counter at zero
-            if (t == p.items - 1) atomicExch(p.ticket, 0);
+        const int at = i < 0 ? 0 : walk.at + 1 < kLists ? walk.at + 1 : 0;
+        if (i >= 0) {
+          ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1);
+          if (ok && p.ticket != nullptr) {
+            int t = 0;
+            if (lane == 0) {
+              t = atomicAdd(p.ticket, 1);
+              // every CTA draws until its first ticket past the end, so the launch draws exactly
+              // `items` tickets in all; whoever draws the last one leaves the counter at zero
+              if (t == p.items - 1) atomicExch(p.ticket, 0);
+            }
+            t = __shfl_sync(0xffffffffu, t, 0);
+            terminal = t >= n2;
+            lw = stride + t;
+          } else {
+            lw += stride;
           }
-          t = __shfl_sync(0xffffffffu, t, 0);
-          terminal = t >= n2;
-          if (sorted && t < n2) {
-            if (i == 0) ok = mbar_wait_warp(smem_u32(&sm->order_full), 0, abort_flag);
-            t = *const_cast<volatile int*>(&sm->order[t]);
-          }
-          lw = stride + t;
-        } else {
-          lw += stride;
+          // The list buffer was that of item i-2, which these warps have written out (and the softmax
+          // warps with them are through with); the producers and issuers may lag behind.
+          if (ok && i >= 2)
+            ok = mbar_wait_warp_idle(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag, 128);
         }
-        // The list buffer was that of item i-2, which these warps have written out (and the softmax
-        // warps with them are through with); the producers and issuers may lag behind.
-        if (ok && i >= 2)
-          ok = mbar_wait_warp_idle(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag, 128);
         if (ok) {
           if (lw < p.items) {
             fwd_list_item<kElementMask>(sm, p, lw, at, lane);
@@ -886,12 +846,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
       }
+      if (i < 0) continue;
+      const int n_tiles = walk.it.w;
       if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->stats_full[par]), (i >> 1) & 1, abort_flag, 128);
       // The weights of the four partial results need the statistics only, which the softmax warps
       // publish before the item's last P V is complete.
       const int t0 = g & 1;  // the team with the item's first superstep
       g += (n_tiles + 3) >> 2;
-      uint64_t acc[32];  // 64 columns in pairs
       float m_all = -INFINITY, l_all = 0.f, mt = -INFINITY, w0 = 0.f, w1 = 0.f;
       if (ok) {
 #pragma unroll
@@ -911,59 +872,49 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         w0 = m0 == -INFINITY ? 0.f : ex2_approx(m0 - m_all) * inv;
         w1 = m1 == -INFINITY ? 0.f : ex2_approx(m1 - m_all) * inv;
       }
-      if (ok) ok = mbar_wait_warp(smem_u32(&sm->o_full[par]), (i >> 1) & 1, abort_flag);
-      if (ok) {
-        if (n_tiles > 0) {  // warp-uniform
-          // An accumulator holds sums of this item only if the item has a tile for these lanes of it
-          // (warp-uniform).
-          const bool live0 = n_tiles > half, live1 = n_tiles > 4 + half;
-          const uint64_t w0w0 = pack_f32x2(w0, w0), w1w1 = pack_f32x2(w1, w1);
-          tc_fence_after();
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint32_t a0[16], a1[16];
-            const uint32_t o_cols = tmem + lane_base + kTmemO + 16 * q;
-            tmem_ld_32x32b_x16(o_cols + 64 * t0, a0);
-            tmem_ld_32x32b_x16(o_cols + 64 * (t0 ^ 1), a1);
-            tc_wait_ld();
-            if (live1) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                acc[8 * q + j] = fma_f32x2(
-                    pack_f32x2(__uint_as_float(a1[2 * j]), __uint_as_float(a1[2 * j + 1])), w1w1,
-                    mul_f32x2(pack_f32x2(__uint_as_float(a0[2 * j]), __uint_as_float(a0[2 * j + 1])), w0w0));
-            } else {
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                acc[8 * q + j] =
-                    live0 ? mul_f32x2(pack_f32x2(__uint_as_float(a0[2 * j]), __uint_as_float(a0[2 * j + 1])), w0w0)
-                          : 0ull;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) acc[j] = 0ull;
-        }
-        // Accumulators, statistics and the item's header are in registers now: the next item may
-        // use them, while this one is still being merged and stored.
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->o_free[par]));
-      }
-      // Lanes 0..63 finish columns [0, 32) of their rows, lanes 64..127 columns [32, 64) of the same
-      // rows; each hands the other its sums of the other columns.
+      if (ok) ok = mbar_wait_warp(smem_u32(&sm->o_full[par]), (i >> 1) & 1);
+      tc_fence_after();
+      // An accumulator holds sums of this item only if the item has a tile for these lanes of it
+      // (warp-uniform).
+      const bool live0 = n_tiles > half, live1 = n_tiles > 4 + half;
+      const uint64_t w0w0 = pack_f32x2(w0, w0), w1w1 = pack_f32x2(w1, w1);
       const int row = walk.it.z * 64 + r_blk;
-      uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.o) + walk.it.x * p.o_sb +
-                                            walk.it.y * p.o_sh + static_cast<int64_t>(row) * p.o_sn);
+      uint16_t* dst = static_cast<uint16_t*>(p.o) + walk.it.x * p.o_sb + walk.it.y * p.o_sh +
+                      static_cast<int64_t>(row) * p.o_sn;
       bool any_failed = false;
-#pragma unroll
+      // Lanes 0..63 finish columns [0, 32) of their rows, lanes 64..127 columns [32, 64) of the same
+      // rows, 16 columns at a time; each hands the other its sums of the other columns.
+#pragma unroll 1
       for (int part = 0; part < 2; ++part) {
+        uint64_t keep[8];
         if (ok) {
+          uint64_t send[8];
+          const uint32_t at_send = o_lanes + 32 * (half ^ 1) + 16 * part, at_keep = o_lanes + 32 * half + 16 * part;
+          const auto sum = [&](uint32_t cols, uint64_t* acc) {
+            uint32_t a0[16], a1[16];
+            tmem_ld_32x32b_x16(cols + 64 * t0, a0);
+            tmem_ld_32x32b_x16(cols + 64 * (t0 ^ 1), a1);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              acc[j] = live0 ? mul_f32x2(pack_f32x2(__uint_as_float(a0[2 * j]), __uint_as_float(a0[2 * j + 1])), w0w0)
+                             : 0ull;
+              if (live1)
+                acc[j] = fma_f32x2(pack_f32x2(__uint_as_float(a1[2 * j]), __uint_as_float(a1[2 * j + 1])), w1w1, acc[j]);
+            }
+          };
+          sum(at_send, send);
+          sum(at_keep, keep);
           ulonglong2* out = reinterpret_cast<ulonglong2*>(sm->xfer[half][r_blk]);
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            out[j] = half ? make_ulonglong2(acc[8 * part + 2 * j], acc[8 * part + 2 * j + 1])
-                          : make_ulonglong2(acc[16 + 8 * part + 2 * j], acc[16 + 8 * part + 2 * j + 1]);
+          for (int j = 0; j < 4; ++j) out[j] = make_ulonglong2(send[2 * j], send[2 * j + 1]);
+          if (part == 1) {
+            // Accumulators, statistics and the item's header are in registers now: the next item may
+            // use them, while this one is still being merged and stored.
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&sm->o_free[par]));
+          }
         }
         named_barrier_sync(2, 128);
         const int col = 32 * half + 16 * part;
@@ -974,18 +925,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int j = 0; j < 4; ++j) {
             const ulonglong2 x = in[j];
             float f0, f1, f2, f3;
-            unpack_f32x2(add_f32x2(half ? acc[16 + 8 * part + 2 * j] : acc[8 * part + 2 * j], x.x), f0, f1);
-            unpack_f32x2(
-                add_f32x2(half ? acc[16 + 8 * part + 2 * j + 1] : acc[8 * part + 2 * j + 1], x.y), f2, f3);
+            unpack_f32x2(add_f32x2(keep[2 * j], x.x), f0, f1);
+            unpack_f32x2(add_f32x2(keep[2 * j + 1], x.y), f2, f3);
             pkd[2 * j] = pack_2x16<kBf16>(f0, f1);
             pkd[2 * j + 1] = pack_2x16<kBf16>(f2, f3);
           }
           // whole 32-byte sectors when the rows start on such boundaries
           if (p.wide_stores) {
-            st_global_v8(dst + (col >> 3), pkd);
+            st_global_v8(dst + col, pkd);
           } else {
-            dst[col >> 3] = make_uint4(pkd[0], pkd[1], pkd[2], pkd[3]);
-            dst[(col >> 3) + 1] = make_uint4(pkd[4], pkd[5], pkd[6], pkd[7]);
+            *reinterpret_cast<uint4*>(dst + col) = make_uint4(pkd[0], pkd[1], pkd[2], pkd[3]);
+            *reinterpret_cast<uint4*>(dst + col + 8) = make_uint4(pkd[4], pkd[5], pkd[6], pkd[7]);
           }
         }
         // xfer may be overwritten now; all four warps leave together if any gave up
@@ -998,6 +948,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (p.rowmax) p.rowmax[ri] = mt;
       }
       if (any_failed) break;
+      walk.next();
     }
     if (!ok) fwd_give_up(sm, p.status, kFailOut);
     if (lister && !terminal && lane == 0) {
@@ -1009,7 +960,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (t == p.items - 1) atomicExch(p.ticket, 0);
       } while (t < n2);
     }
-
   }
 
   // ---- tear-down: every role arrives here, also after a give-up ----

@@ -112,48 +112,29 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// mbar_try_wait, but the hardware may park the thread for up to about `hint_ns` until the phase
-// completes instead of returning at once: a waiting warp then issues next to nothing.
-__device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait.  Returns false when the wait gave up: either another role of this CTA raised
-// *abort_flag, or about BSA_WAIT_LIMIT_NS passed.  On give-up the caller records the code, raises
-// the flag and leaves through the normal tear-down path so TMEM is always released.
-#ifndef BSA_WAIT_LIMIT_NS
-#define BSA_WAIT_LIMIT_NS 2000000000ull
-#endif
-// (32 bits of the timer and one small loop on purpose: this code is inlined at every wait of every
-// role, and the instruction cache is what the roles of a persistent kernel share most tightly.)
-__device__ __forceinline__ uint32_t global_timer_lo_ns() {
+// Bounded wait.  Returns false when it gave up, which is when the upper half of the SM's cycle counter has
+// moved twice: after 2^32 to 2^33 cycles, 2 to 5 seconds.  On give-up the caller records the code, raises
+// the CTA's flag and leaves through the normal tear-down path so TMEM is always released.
+// (This code is inlined at every wait of every role, and the instruction cache is what the roles of a
+// persistent kernel share most tightly: a loop with a look at the flag, a parked form of the wait and
+// %globaltimer made short lists 3 to 6 % slower.)
+__device__ __forceinline__ uint32_t clock_hi() {
   uint32_t t;
-  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+  asm volatile("mov.u32 %0, %%clock_hi;" : "=r"(t));
   return t;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
-                                          volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t t0 = global_timer_lo_ns();
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
+  const uint32_t t0 = clock_hi();
 #pragma unroll 1
-  while (!mbar_try_wait_parked(bar, parity, 2000u))
-    if (*abort_flag || global_timer_lo_ns() - t0 > static_cast<uint32_t>(BSA_WAIT_LIMIT_NS)) return false;
+  while (!mbar_try_wait(bar, parity))
+    if (clock_hi() - t0 > 1u) return false;
   return true;
 }
 
 // Same wait made by a whole (converged) warp; the verdict is made warp-uniform so that the
 // .sync.aligned instructions that follow are never executed by a partial warp.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
-                                               volatile int* abort_flag) {
-  const bool ok = mbar_wait(bar, parity, abort_flag);
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  const bool ok = mbar_wait(bar, parity);
   return __all_sync(0xffffffffu, ok);
 }
 
@@ -163,11 +144,11 @@ __device__ __forceinline__ bool mbar_wait_warp_idle(uint32_t bar, uint32_t parit
                                                     volatile int* abort_flag, unsigned sleep_ns) {
   bool ok = true;
   if (!mbar_try_wait(bar, parity)) {
-    const uint32_t t0 = global_timer_lo_ns();
+    const uint32_t t0 = clock_hi();
 #pragma unroll 1
     do {
       __nanosleep(sleep_ns);
-      if (*abort_flag || global_timer_lo_ns() - t0 > static_cast<uint32_t>(BSA_WAIT_LIMIT_NS)) {
+      if (*abort_flag || clock_hi() - t0 > 1u) {
         ok = false;
         break;
       }

@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int32_t* status, i
   const uint64_t t0 = global_timer_ns();
   if (warp == 0) {
     // runs out after the wait limit, then raises the CTA's flag like a role of a kernel does
-    const bool ok = mbar_wait_warp(smem_u32(&bar), 0, flag);
+    const bool ok = mbar_wait_warp(smem_u32(&bar), 0);
     if (!ok && lane == 0) {
       abort_flag = 1;
       report_status(status, 99);
