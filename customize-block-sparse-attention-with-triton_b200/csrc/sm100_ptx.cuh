@@ -112,34 +112,34 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait.  Returns false when it gave up, which is when the upper half of the SM's cycle counter has
-// moved twice: after 2^32 to 2^33 cycles, 2 to 5 seconds.  On give-up the caller records the code, raises
-// the CTA's flag and leaves through the normal tear-down path so TMEM is always released.
-// (This code is inlined at every wait of every role, and the instruction cache is what the roles of a
-// persistent kernel share most tightly: a loop with a look at the flag, a parked form of the wait and
-// %globaltimer made short lists 3 to 6 % slower.)
+// Bounded wait of a whole (converged) warp.  Returns false when it gave up: after kWaitTries tries, each of
+// which the hardware suspends for up to 4 us, 2 seconds in all.  On give-up the caller records the code and
+// leaves through the normal tear-down path so TMEM is always released.
+// (This code is inlined at every wait of every role and run through at every superstep, mostly on barriers
+// that are long complete: a loop with a look at a flag, a parked form of the wait and %globaltimer made
+// short lists 3 to 6 % slower, a vote on the verdict the backward 2 to 3 % and the forward 1 to 2 %.)
+constexpr int kWaitTries = 1 << 19;
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  int left = kWaitTries;
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity))
+    if (--left == 0) {
+      __syncwarp();
+      return false;
+    }
+  __syncwarp();  // together again before any .sync.aligned instruction
+  return true;
+}
+
+// Same, for roles that wait for a long time (a whole work item): sleeps between polls so that the
+// waiting warp does not take issue slots from the working warps of its sub-partition.  Also gives up
+// when another role has raised the CTA's flag; its own limit is when the upper half of the SM's cycle
+// counter has moved twice (2^32 to 2^33 cycles, 2 to 5 seconds).
 __device__ __forceinline__ uint32_t clock_hi() {
   uint32_t t;
   asm volatile("mov.u32 %0, %%clock_hi;" : "=r"(t));
   return t;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  const uint32_t t0 = clock_hi();
-#pragma unroll 1
-  while (!mbar_try_wait(bar, parity))
-    if (clock_hi() - t0 > 1u) return false;
-  return true;
-}
-
-// Same wait made by a whole (converged) warp; the verdict is made warp-uniform so that the
-// .sync.aligned instructions that follow are never executed by a partial warp.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
-  const bool ok = mbar_wait(bar, parity);
-  return __all_sync(0xffffffffu, ok);
-}
-
-// Same, for roles that wait for a long time (a whole work item): sleeps between polls so that the
-// waiting warp does not take issue slots from the working warps of its sub-partition.
 __device__ __forceinline__ bool mbar_wait_warp_idle(uint32_t bar, uint32_t parity,
                                                     volatile int* abort_flag, unsigned sleep_ns) {
   bool ok = true;
