@@ -128,6 +128,9 @@ struct BwdParams {
   int32_t* status;
   int32_t* ticket;  // optional work counter (0 at kernel start, left 0): dynamic item hand-out
   int wide_stores;  // output rows start on 32-byte boundaries
+  // dK/dV: dQ of the same call follows in the stream and may begin as soon as SMs are free; dQ: that is
+  // what it does (it reads nothing that dK/dV writes)
+  int together;
 };
 
 // Readers of the item header: wait for item i, read it (the producer looked the list up, so the
@@ -184,11 +187,19 @@ __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, ui
                                                const CUtensorMap* map, float* vec_ring, const float* vec,
                                                const BwdItem& it, int n_super, int lane,
                                                int* gs) {
+#pragma unroll 1
   for (int j = 0; j < n_super; ++j, ++*gs) {
     const int s = *gs % kPlaces;
     const int nt = min(2, it.n_tiles - 2 * j), t = lane & 1;
     const int nj = t < nt ? (__ldg(it.ents + 2 * j + t) & kListIndex) : 0;
-    if (!mbar_wait_warp(smem_u32(empty + s), ((*gs / kPlaces) & 1) ^ 1)) return false;
+    if (kVector) {
+      // dK/dV: the place is free when the products of its previous superstep are (empty: d_free)
+      if (*gs >= kPlaces &&
+          !mbar_wait_warp(smem_u32(empty + (*gs - kPlaces) % kXBars), ((*gs - kPlaces) / kXBars) & 1))
+        return false;
+    } else {
+      if (!mbar_wait_warp(smem_u32(empty + s), ((*gs / kPlaces) & 1) ^ 1)) return false;
+    }
     const uint32_t bar = smem_u32(full + *gs % (2 * kPlaces));
     if (lane == 0) mbar_expect_tx(bar, nt * (kBwdTile + (kVector ? 256u : 0u)));
     __syncwarp();
@@ -214,6 +225,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
   const int k_steps = p.D >> 4;
   bool ok = true;
   int gs = 0, ni = 0;
+#pragma unroll 1
   for (int i = 0; ok; ++i) {
     int w, w_tiles, w_begin;
     ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
@@ -225,6 +237,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
     const uint64_t a0 = desc_a0 + static_cast<uint64_t>(2 * own) * kTileDesc;
     int g = gs + ((gs ^ team) & 1);
     gs += n_super;
+#pragma unroll 1
     for (; ok && g < gs; g += 2) {
       ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1) &&
            mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1);
@@ -275,6 +288,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   bool ok = true;
   int ni = 0, place = 0, slot = 0, x = 0;
   uint32_t phase = 0;  // of the slot's barrier
+#pragma unroll 1
   for (int i = 0; ok; ++i) {
     int w, w_tiles, w_begin;
     ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
@@ -282,6 +296,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
     if (w_tiles == 0) continue;
     // the write-out warps must have read the previous block's accumulators
     if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1);
+#pragma unroll 1
     for (int left = w_tiles; ok && left > 0; left -= 2) {
       ok = mbar_wait_warp(smem_u32(&sm->d_full[slot]), phase);
       if (!ok) break;
@@ -303,7 +318,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
             umma_ts_half(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + (kBwdTile >> 4) + 128 * kk, idesc,
                          more | (kk > 0), 1);
         }
-        tc_commit(empty + 8 * place);  // place free
+        if constexpr (!kDKDV) tc_commit(empty + 8 * place);  // place free
         tc_commit(smem_u32(&sm->d_free[x]));  // P or dS columns free; accumulator updated
         if (left <= 2) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
       }
@@ -338,20 +353,27 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   const int stride = gridDim.x;
 
   if (threadIdx.x == 0) {
+#pragma unroll 1
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->item_full[i]), 1);
       mbar_init(smem_u32(&sm->item_free[i]), kCW + 8 + 1);  // all roles but the first producer
       mbar_init(smem_u32(&sm->stat_full[i]), 2);  // two producers
       mbar_init(smem_u32(&sm->stat_free[i]), 2);  // two S/dP issuers
     }
+#pragma unroll 1
     for (int i = 0; i < kSlots; ++i) mbar_init(smem_u32(&sm->d_full[i]), kTeamW);  // one arrival per warp
+#pragma unroll 1
     for (int i = 0; i < kXBars; ++i) {
       mbar_init(smem_u32(&sm->x_full[i]), kDKDV ? 2 : 1);
       mbar_init(smem_u32(&sm->d_free[i]), 2);
     }
+#pragma unroll 1
     for (int s = 0; s < 2 * kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_full0[s]), 1);
+#pragma unroll 1
     for (int s = 0; s < 2 * kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_full1[s]), 1);
+#pragma unroll 1
     for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), kDKDV ? 1 : 2);
+#pragma unroll 1
     for (int s = 0; s < kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
     mbar_init(smem_u32(&sm->acc_done), 2);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
@@ -371,7 +393,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
-  grid_dependency_wait();
+  // Together, dQ begins while dK/dV is still running: it is launched when all CTAs of dK/dV have passed
+  // this point, so what came before dK/dV has ended and is visible then.  It ends after dK/dV (see the end).
+  if (kDKDV || !p.together) grid_dependency_wait();
+  if (kDKDV && p.together) grid_dependents_launch();
 
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
   // issuers do without (56 + 104 + 56 = 3 x 72).
@@ -382,6 +407,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       bool ok = true;
       bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
       int gs = 0, ni = 0;
+#pragma unroll 1
       for (int i = 0, w = blockIdx.x; ok; ++i) {
         const int par = i & 1;
         if (i > 0) {
@@ -427,7 +453,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
             tma_load_4d(smem_u32(sm->stat[own][0]), &tm_stat0, bar, 0, it.blk * 64, it.h, it.b);
           }
         }
-        ok = bwd_load_tiles<kRing0<kDKDV>, kDKDV>(sm->ring[0][0], sm->in_full0, sm->in_empty0, &tm_str0,
+        ok = bwd_load_tiles<kRing0<kDKDV>, kDKDV>(sm->ring[0][0], sm->in_full0, kDKDV ? sm->d_free : sm->in_empty0, &tm_str0,
                                                   sm->lse[0][0], p.lse2, it, n_super, lane, &gs);
         ++ni;
       }
@@ -445,6 +471,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       // =========================== second TMA producer ===========================
       bool ok = true;
       int gs = 0, ni = 0;
+#pragma unroll 1
       for (int i = 0; ok; ++i) {
         int w, w_tiles, w_begin;
         ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
@@ -461,7 +488,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
           tma_load_4d(smem_u32(sm->stat[own][1]), &tm_stat1, bar, 0, it.blk * 64, it.h, it.b);
         }
         ok = bwd_load_tiles<kRing1<kDKDV>, kDKDV>(sm->ring[kRing0<kDKDV>][0], sm->in_full1,
-                                                  sm->in_empty1, &tm_str1, sm->delta[0][0], p.delta, it,
+                                                  kDKDV ? sm->d_free : sm->in_empty1, &tm_str1, sm->delta[0][0], p.delta, it,
                                                   n_super, lane, &gs);
         ++ni;
       }
@@ -483,6 +510,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     const float c = p.scale_log2;
     bool ok = true;
     int gs = 0;  // supersteps of earlier items; this team takes those with gs % 2 == team
+#pragma unroll 1
     for (int i = 0; ok; ++i) {
       int w, w_tiles, w_begin;
       ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
@@ -512,6 +540,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       int j = (gs ^ team) & 1;
       int g = gs + j;
       gs += n_super;
+#pragma unroll 1
       for (; ok && j < n_super; j += 2, g += 2) {
         const bool active = 2 * j + t_mine < w_tiles;  // this lane's tile exists (warp-uniform)
         const uint32_t s_at = x_base + 128 * (g % kSlots), dp_at = s_at + 64;
@@ -654,6 +683,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     const int col0 = kDKDV ? 0 : 32 * half;
     bool ok = true;
     int ni = 0;
+#pragma unroll 1
     for (int i = 0;; ++i) {
       int w = 0, w_tiles = 1, w_begin = 0;
       if (ok) ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
@@ -745,6 +775,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     tc_fence_after();
     tmem_dealloc(tmem, kBwdTmemCols);
   }
+  // what follows dQ in the stream waits for dQ alone
+  if (!kDKDV && p.together) grid_dependency_wait();
 }
 
 struct BwdOperand {
@@ -759,7 +791,8 @@ static int launch_bwd(BwdOperand q, BwdOperand k, BwdOperand v, BwdOperand dout,
                       const float* delta, BwdOperand out0, BwdOperand out1, const int32_t* list_ptr,
                       const int32_t* list_idx, int list_places, int list_b_stride, int list_h_stride,
                       float sm_scale, int dtype, int B, int H, int N, int D, const uint8_t* dense,
-                      const int64_t* dense_strides, int32_t* ticket, int32_t* status, void* stream) {
+                      const int64_t* dense_strides, int32_t* ticket, int32_t* status, bool together,
+                      void* stream) {
   if (B <= 0 || H <= 0 || N <= 0 || (N % kBlock) != 0 || !head_dim_ok(D)) return BSA_ERR_BAD_SHAPE;
   if (dense != nullptr) {
     if (!dense_strides || !is_aligned(dense, 16)) return BSA_ERR_BAD_POINTER;
@@ -818,6 +851,7 @@ static int launch_bwd(BwdOperand q, BwdOperand k, BwdOperand v, BwdOperand dout,
   prm.sm_scale = sm_scale;
   prm.status = status;
   prm.ticket = ticket;
+  prm.together = together ? 1 : 0;
   {
     // 16 output columns are one 32-byte sector when every row starts on such a boundary
     uintptr_t bits = 0;
@@ -856,7 +890,7 @@ extern "C" int bsa_attn_bwd_dkdv_strided(
   return bsa::launch_bwd<true>({q, q_strides}, {k, k_strides}, {v, v_strides}, {dout, do_strides},
                                lse2, delta, {dv, dv_strides}, {dk, dk_strides}, col_ptr, row_idx,
                                list_places, list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D, dense,
-                               dense_strides, work_counter, status, stream);
+                               dense_strides, work_counter, status, false, stream);
 }
 
 extern "C" int bsa_attn_bwd_dkdv(const void* q, const void* k, const void* v, const void* dout,
@@ -883,7 +917,7 @@ extern "C" int bsa_attn_bwd_dq_strided(
   return bsa::launch_bwd<false>({q, q_strides}, {k, k_strides}, {v, v_strides}, {dout, do_strides},
                                 lse2, delta, {nullptr, nullptr}, {dq, dq_strides}, row_ptr, col_idx,
                                 list_places, list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D, dense,
-                                dense_strides, work_counter, status, stream);
+                                dense_strides, work_counter, status, false, stream);
 }
 
 extern "C" int bsa_attn_bwd_dq(const void* q, const void* k, const void* v, const void* dout,
@@ -896,4 +930,27 @@ extern "C" int bsa_attn_bwd_dq(const void* q, const void* k, const void* v, cons
   return bsa_attn_bwd_dq_strided(q, strides, k, strides, v, strides, dout, strides, lse2, delta, dq,
                                  strides, row_ptr, col_idx, 0, list_b_stride, list_h_stride, sm_scale,
                                  dtype, B, H, N, D, dense, dense_strides, work_counter, status, stream);
+}
+
+extern "C" int bsa_attn_bwd_strided(
+    const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4],
+    const void* v, const int64_t v_strides[4], const void* dout, const int64_t do_strides[4],
+    const float* lse2, const float* delta, void* dq, const int64_t dq_strides[4], void* dk,
+    const int64_t dk_strides[4], void* dv, const int64_t dv_strides[4], const int32_t* row_ptr,
+    const int32_t* col_idx, const int32_t* col_ptr, const int32_t* row_idx, int list_places,
+    int list_b_stride, int list_h_stride, float sm_scale, int dtype, int B, int H, int N, int D,
+    const uint8_t* dense, const int64_t dense_strides[4], int32_t* dkdv_counter, int32_t* dq_counter,
+    int32_t* status, void* stream) {
+  if (!q_strides || !k_strides || !v_strides || !do_strides || !dq_strides || !dk_strides || !dv_strides ||
+      (dkdv_counter != nullptr && dkdv_counter == dq_counter))
+    return BSA_ERR_BAD_POINTER;
+  const int rc = bsa::launch_bwd<true>({q, q_strides}, {k, k_strides}, {v, v_strides}, {dout, do_strides},
+                                       lse2, delta, {dv, dv_strides}, {dk, dk_strides}, col_ptr, row_idx,
+                                       list_places, list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D,
+                                       dense, dense_strides, dkdv_counter, status, true, stream);
+  if (rc != BSA_OK) return rc;
+  return bsa::launch_bwd<false>({q, q_strides}, {k, k_strides}, {v, v_strides}, {dout, do_strides}, lse2, delta,
+                                {nullptr, nullptr}, {dq, dq_strides}, row_ptr, col_idx, list_places,
+                                list_b_stride, list_h_stride, sm_scale, dtype, B, H, N, D, dense, dense_strides,
+                                dq_counter, status, true, stream);
 }

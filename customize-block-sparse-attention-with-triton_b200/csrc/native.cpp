@@ -31,8 +31,8 @@ constexpr int64_t kBlock = 64;
 // and the host can read without a synchronisation.
 // ---------------------------------------------------------------------------------------------
 struct StreamState {
-  Tensor counter, status;
-  int32_t* counter_ptr;
+  Tensor counter, dq_counter, status;
+  int32_t *counter_ptr, *dq_counter_ptr;  // (the dQ kernel runs beside the dK/dV kernel, and has its own)
   volatile int32_t* word;
 };
 
@@ -65,8 +65,10 @@ StreamState* stream_state(int device, cudaStream_t stream) {
     const c10::InferenceMode no_inference(false);
     // zeroed on the stream that will use it, so no cross-stream ordering is needed
     st->counter = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+    st->dq_counter = at::zeros_like(st->counter);
     st->status = at::zeros({1}, at::TensorOptions().dtype(at::kInt)).pin_memory();
     st->counter_ptr = st->counter.data_ptr<int32_t>();
+    st->dq_counter_ptr = st->dq_counter.data_ptr<int32_t>();
     st->word = st->status.data_ptr<int32_t>();
     it = states->emplace(key, st).first;
   }
@@ -79,10 +81,11 @@ StreamState* stream_state(int device, cudaStream_t stream) {
 // it gets a word of its own (*own, out of the graph's memory, zeroed by every replay).  B200, replayed
 // calls with this stream's counter / a zeroed word / none: forward of one head, N = 17536, a tenth of the
 // blocks 21 / 23 / 24 us; forward and backward of 4 heads, N = 6400, causal, a quarter 68 / 72 / 83 us.
-int32_t* work_counter(StreamState* state, int64_t blocks, const at::TensorOptions& options, Tensor* own) {
+int32_t* work_counter(StreamState* state, int64_t blocks, const at::TensorOptions& options, Tensor* own,
+                      bool dq = false) {
   if (blocks <= at::cuda::getDeviceProperties(options.device().index())->multiProcessorCount) return nullptr;
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
-    return state ? state->counter_ptr : nullptr;
+    return !state ? nullptr : dq ? state->dq_counter_ptr : state->counter_ptr;
   *own = at::zeros({1}, options.dtype(at::kInt));
   return own->mutable_data_ptr<int32_t>();
 }
@@ -230,8 +233,9 @@ struct AttentionBackward : torch::autograd::Node {
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
     StreamState* state = stream_state(q.device().index(), stream);
     raise_if_reported(state);
-    Tensor own;
+    Tensor own, dq_own;
     int32_t* counter = work_counter(state, B * H * nb, q.options(), &own);
+    int32_t* dq_counter = work_counter(state, B * H * nb, q.options(), &dq_own, true);
     int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
     // the gradients are laid out like the tensors they belong to, gaps included
     const auto like = [](const Tensor& t) { return at::empty_strided(t.sizes(), t.strides(), t.options()); };
@@ -244,20 +248,13 @@ struct AttentionBackward : torch::autograd::Node {
     check("bsa_attn_bwd_delta_strided",
           bsa_attn_bwd_delta_strided(o.const_data_ptr(), o.strides().data(), dout.const_data_ptr(),
                                      dout.strides().data(), delta_p, code, B, H, N, D, stream));
-    check("bsa_attn_bwd_dkdv_strided",
-          bsa_attn_bwd_dkdv_strided(
+    check("bsa_attn_bwd_strided",
+          bsa_attn_bwd_strided(
               q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
               v.const_data_ptr(), v.strides().data(), dout.const_data_ptr(), dout.strides().data(), lse_p,
-              delta_p, dk.mutable_data_ptr(), dk.strides().data(), dv.mutable_data_ptr(),
-              dv.strides().data(), p + at.col_cnt, p + at.row_idx, nb, sb, sh, scale, code, B, H, N, D,
-              dense_ptr, dense_strides, counter, status, stream));
-    check("bsa_attn_bwd_dq_strided",
-          bsa_attn_bwd_dq_strided(q.const_data_ptr(), q.strides().data(), k.const_data_ptr(),
-                                  k.strides().data(), v.const_data_ptr(), v.strides().data(),
-                                  dout.const_data_ptr(), dout.strides().data(), lse_p, delta_p,
-                                  dq.mutable_data_ptr(), dq.strides().data(), p, p + at.col_idx, nb, sb, sh,
-                                  scale, code, B, H, N, D, dense_ptr, dense_strides, counter, status,
-                                  stream));
+              delta_p, dq.mutable_data_ptr(), dq.strides().data(), dk.mutable_data_ptr(), dk.strides().data(),
+              dv.mutable_data_ptr(), dv.strides().data(), p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, nb, sb,
+              sh, scale, code, B, H, N, D, dense_ptr, dense_strides, counter, dq_counter, status, stream));
     return {dq, dk, dv};
   }
 };

@@ -60,6 +60,8 @@ SIGNATURES = {
                                   _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
     "bsa_attn_bwd_dq_strided": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _s4,
                                 _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
+    "bsa_attn_bwd_strided": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _s4, _vp, _s4, _vp, _s4,
+                             _vp, _vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp, _vp],
     "bsa_reorder": [_vp, _vp, _s4, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_inv_reorder": [_vp, _vp, _s4, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
     "bsa_reorder_strided": [_vp, _s4, _vp, _s4, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],

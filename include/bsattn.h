@@ -268,6 +268,21 @@ int bsa_attn_bwd_dq_strided(const void* q, const int64_t q_strides[4], const voi
                             int D, const uint8_t* dense, const int64_t dense_strides[4],
                             int32_t* work_counter, int32_t* status, void* stream);
 
+/* dK, dV and dQ in one call, with everything as in the two calls above, and faster: the dQ kernel takes the
+ * SMs that the dK/dV kernel has no more work for instead of waiting for its end.  So nothing that the
+ * dK/dV kernel touches may overlap dq, and each kernel has a work counter of its own (both may be NULL).
+ * What follows in the stream waits for both. */
+int bsa_attn_bwd_strided(const void* q, const int64_t q_strides[4], const void* k,
+                         const int64_t k_strides[4], const void* v, const int64_t v_strides[4],
+                         const void* dout, const int64_t do_strides[4], const float* lse2,
+                         const float* delta, void* dq, const int64_t dq_strides[4], void* dk,
+                         const int64_t dk_strides[4], void* dv, const int64_t dv_strides[4],
+                         const int32_t* row_ptr, const int32_t* col_idx, const int32_t* col_ptr,
+                         const int32_t* row_idx, int list_places, int list_b_stride, int list_h_stride,
+                         float sm_scale, int dtype, int B, int H, int N, int D, const uint8_t* dense,
+                         const int64_t dense_strides[4], int32_t* dkdv_counter, int32_t* dq_counter,
+                         int32_t* status, void* stream);
+
 /*
  * Head-wise token reorder; replaces reorder_kernel (fa2_custom_mask/permute.py:5-58, launched from
  * fa2_custom_mask/functional.py:5-20).  For every head h with order (p0,p1,p2) = orders[3h..3h+2],
