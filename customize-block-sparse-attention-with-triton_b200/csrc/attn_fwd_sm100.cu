@@ -148,6 +148,7 @@ struct FwdParams {
   int32_t* status;
   int32_t* ticket;          // optional work counter (0 at kernel start, left 0): dynamic item hand-out
   int wide_stores;          // rows of O start on 32-byte boundaries
+  int successor_early;      // what follows in the stream may begin before this kernel ends, and knows it
 };
 
 enum FwdFail : int { kFailProducer = 1, kFailMma = 2, kFailSoftmax = 3, kFailOut = 4 };
@@ -420,6 +421,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
   grid_dependency_wait();
+  if (p.successor_early) grid_dependents_launch();
 
   // 512 threads are launched with 128 registers: the softmax warps, which hold 64 logits and 128
   // probabilities each, take what the others do without (2 x 168 + 72 + 104 = 4 x 128).  A spill in their
@@ -981,7 +983,7 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
                       const int64_t* block_strides, int list_b_stride, int list_h_stride,
                       float sm_scale, int dtype, int B, int H, int N, int D, int row_begin,
                       int row_end, const uint8_t* dense, const int64_t* dense_strides,
-                      int32_t* status, int32_t* ticket, void* stream) {
+                      int32_t* status, int32_t* ticket, void* stream, bool successor_early = false) {
   if (B <= 0 || H <= 0 || N <= 0 || (N % kBlock) != 0 || !head_dim_ok(D))
     return BSA_ERR_BAD_SHAPE;
   if (!(sm_scale >= 0.f)) return BSA_ERR_BAD_SHAPE;  // the row maximum is taken before scaling
@@ -1046,6 +1048,7 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
   prm.scale_log2 = sm_scale * 1.4426950408889634f;
   prm.status = status;
   prm.ticket = ticket;
+  prm.successor_early = successor_early ? 1 : 0;
   prm.wide_stores =
       ((reinterpret_cast<uintptr_t>(o) |
         static_cast<uintptr_t>((o_strides[0] | o_strides[1] | o_strides[2]) * 2)) & 31u) == 0 ? 1 : 0;
@@ -1121,4 +1124,25 @@ extern "C" int bsa_attn_fwd_block_mask(const void* q, const int64_t q_strides[4]
                                       rowmax, block, block_strides, Bm, Hm, sm_scale, dtype, B, H,
                                       N, D, 0, N > 0 ? N / bsa::kBlock : 0, nullptr, nullptr,
                                       work_counter, status, stream);
+}
+
+extern "C" int bsa_attn_fwd_block_mask_lists(
+    const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4], const void* v,
+    const int64_t v_strides[4], void* o, const int64_t o_strides[4], float* lse2, const uint8_t* block,
+    const int64_t block_strides[4], int Bm, int Hm, float sm_scale, int dtype, int B, int H, int N, int D,
+    const uint8_t* dense, const int64_t dense_strides[4], int32_t* row_cnt, int32_t* col_idx, int32_t* col_cnt,
+    int32_t* row_idx, int32_t* work_counter, int32_t* status, void* stream) {
+  if (!block || !block_strides || !row_cnt || !col_idx || !col_cnt || !row_idx) return BSA_ERR_BAD_POINTER;
+  if ((Bm != 1 && Bm != B) || (Hm != 1 && Hm != H)) return BSA_ERR_BAD_SHAPE;
+  for (int i = 0; i < 4; ++i)
+    if (block_strides[i] < 0) return BSA_ERR_BAD_STRIDE;
+  if (N > 0 && static_cast<int64_t>(Bm) * Hm * (N / bsa::kBlock) * (N / bsa::kBlock) > 0x7fffffffLL)
+    return BSA_ERR_TOO_LARGE;
+  const int rc = bsa::launch_fwd(q, q_strides, k, k_strides, v, v_strides, o, o_strides, lse2, nullptr, nullptr,
+                                 nullptr, block, block_strides, Bm > 1 ? 1 : 0, Hm > 1 ? 1 : 0, sm_scale, dtype,
+                                 B, H, N, D, 0, N > 0 ? N / bsa::kBlock : 0, dense, dense_strides, status,
+                                 work_counter, stream, true);
+  if (rc != BSA_OK) return rc;
+  return bsa::launch_lists_places(block, block_strides, Bm, Hm, N / bsa::kBlock, row_cnt, col_idx, col_cnt, row_idx,
+                                  true, stream);
 }

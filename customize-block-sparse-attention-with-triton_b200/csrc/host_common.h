@@ -57,6 +57,11 @@ int launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, siz
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 
+// bsa_tile_lists_places; together: beside the kernel before it in the stream, which has let it in after it
+// has itself seen the end of everything earlier, the mask included.
+int launch_lists_places(const uint8_t* block, const int64_t s[4], int B, int H, int nb, int32_t* row_cnt,
+                        int32_t* col_idx, int32_t* col_cnt, int32_t* row_idx, bool together, void* stream);
+
 // Raises a kernel's dynamic shared-memory limit; done once per (kernel, device) and remembered.
 int ensure_dynamic_smem(const void* kernel, size_t bytes);
 

@@ -92,6 +92,7 @@ struct ListArgs {
   int32_t* ent[2];
   int32_t* groups;
   int32_t* meta;
+  int together;  // runs beside the kernel before it in the stream, which has seen the mask finished
 };
 
 constexpr int kListThreads = 256;
@@ -222,11 +223,14 @@ __device__ __forceinline__ void lists_along_cols(const ListArgs& a) {
 template <ListMode kMode>
 __global__ void __launch_bounds__(kListThreads) lists_pass_kernel(const ListArgs a) {
   grid_dependents_launch();
-  grid_dependency_wait();
+  if (!a.together) grid_dependency_wait();
   const int kind = blockIdx.y;
-  if (a.ptr[kind] == nullptr) return;
-  if (kind == 0) lists_along_rows<kMode>(a);
-  else lists_along_cols<kMode>(a);
+  if (a.ptr[kind] != nullptr) {
+    if (kind == 0) lists_along_rows<kMode>(a);
+    else lists_along_cols<kMode>(a);
+  }
+  // (what follows in the stream waits for this kernel alone)
+  if (a.together) grid_dependency_wait();
 }
 
 // In-place exclusive scan of the counts of one list kind per CTA; kind 0 also emits the
@@ -478,6 +482,7 @@ extern "C" int bsa_tile_lists_build(const uint8_t* block, const int64_t s[4], in
   a.ent[1] = row_idx;
   a.groups = groups;
   a.meta = meta;
+  a.together = 0;
 
   const int64_t bh = static_cast<int64_t>(B) * H;
   const int64_t warps_per_cta = kListThreads / 32;
@@ -505,10 +510,9 @@ extern "C" int bsa_tile_lists_build(const uint8_t* block, const int64_t s[4], in
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 
-extern "C" int bsa_tile_lists_places(const uint8_t* block, const int64_t s[4], int B, int H, int nb,
-                                     int32_t* row_cnt, int32_t* col_idx, int32_t* col_cnt,
-                                     int32_t* row_idx, void* stream) {
-  using namespace bsa;
+int bsa::launch_lists_places(const uint8_t* block, const int64_t s[4], int B, int H, int nb, int32_t* row_cnt,
+                             int32_t* col_idx, int32_t* col_cnt, int32_t* row_idx, bool together,
+                             void* stream) {
   if (B <= 0 || H <= 0 || nb <= 0) return BSA_ERR_BAD_SHAPE;
   if (!block || !row_cnt || !col_idx || !col_cnt || !row_idx) return BSA_ERR_BAD_POINTER;
   for (int i = 0; i < 4; ++i)
@@ -530,8 +534,15 @@ extern "C" int bsa_tile_lists_places(const uint8_t* block, const int64_t s[4], i
   a.ent[1] = row_idx;
   a.groups = nullptr;
   a.meta = nullptr;
+  a.together = together ? 1 : 0;
   const int64_t rows = (bh * nb + kListThreads / 32 - 1) / (kListThreads / 32), cols = bh * ((nb + 31) / 32);
   const dim3 grid(static_cast<unsigned>(rows > cols ? rows : cols), 2);
   return launch_dependent(lists_pass_kernel<kListPlaces>, grid, kListThreads, 0,
                           static_cast<cudaStream_t>(stream), a);
+}
+
+extern "C" int bsa_tile_lists_places(const uint8_t* block, const int64_t s[4], int B, int H, int nb,
+                                     int32_t* row_cnt, int32_t* col_idx, int32_t* col_cnt,
+                                     int32_t* row_idx, void* stream) {
+  return bsa::launch_lists_places(block, s, B, H, nb, row_cnt, col_idx, col_cnt, row_idx, false, stream);
 }

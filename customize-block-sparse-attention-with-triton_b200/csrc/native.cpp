@@ -137,22 +137,49 @@ bool read_mask(const Tensor& mask, int64_t B, int64_t H, int64_t N, const Tensor
 
 int dtype_code(const Tensor& t) { return t.scalar_type() == at::kHalf ? BSA_F16 : BSA_BF16; }
 
-// Runs the forward; false when the library refused.
+// The tile lists of one call in one buffer of words: counts of the row and column lists, then their
+// entries, every list in a place of nb words.
+struct Lists {
+  int64_t col_cnt, col_idx, row_idx, words;
+  Lists(int64_t Bm, int64_t Hm, int64_t nb) {
+    const int64_t rows = Bm * Hm * nb;
+    col_cnt = rows;
+    col_idx = (2 * rows + 3) & ~int64_t{3};
+    row_idx = col_idx + rows * nb;
+    words = row_idx + rows * nb;
+  }
+};
+
+// Runs the forward, and builds the tile lists that a backward needs if they are wanted; false when the
+// library refused.  (The forward lists each mask row inside the kernel.  The lists are written while it is still
+// running, so their memory has to be allocated before the copies that q, k, v may be are given back.)
 bool run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& m, double scale,
-                 StreamState* state, void* stream, Tensor* o, Tensor* lse2) {
+                 StreamState* state, void* stream, Tensor* o, Tensor* lse2, Tensor* lists) {
   const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
   *o = at::empty({B, H, N, D}, q.options());
   *lse2 = at::empty({B, H, N}, q.options().dtype(at::kFloat));
   Tensor own;
   int32_t* counter = work_counter(state, B * H * (N / kBlock), q.options(), &own);
+  int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
+  const int64_t* dense_strides = m.dense_ptr ? m.dense_strides : nullptr;
+  if (lists != nullptr) {
+    const Lists at(m.block.size(0), m.block.size(1), N / kBlock);
+    *lists = at::empty({at.words}, q.options().dtype(at::kInt));
+    int32_t* p = lists->mutable_data_ptr<int32_t>();
+    return bsa_attn_fwd_block_mask_lists(
+               q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
+               v.const_data_ptr(), v.strides().data(), o->mutable_data_ptr(), o->strides().data(),
+               lse2->mutable_data_ptr<float>(), m.block.const_data_ptr<uint8_t>(), m.block.strides().data(),
+               m.block.size(0), m.block.size(1), static_cast<float>(scale), dtype_code(q), B, H, N, D,
+               m.dense_ptr, dense_strides, p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, counter, status,
+               stream) == 0;
+  }
   return bsa_attn_fwd_block_mask_rows(
              q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
              v.const_data_ptr(), v.strides().data(), o->mutable_data_ptr(), o->strides().data(),
              lse2->mutable_data_ptr<float>(), nullptr, m.block.const_data_ptr<uint8_t>(),
              m.block.strides().data(), m.block.size(0), m.block.size(1), static_cast<float>(scale),
-             dtype_code(q), B, H, N, D, 0, N / kBlock, m.dense_ptr,
-             m.dense_ptr ? m.dense_strides : nullptr, counter,
-             state ? const_cast<int32_t*>(state->word) : nullptr, stream) == 0;
+             dtype_code(q), B, H, N, D, 0, N / kBlock, m.dense_ptr, dense_strides, counter, status, stream) == 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -184,19 +211,6 @@ void raise_if_reported(StreamState* state) {
 // ---------------------------------------------------------------------------------------------
 // Autograd
 // ---------------------------------------------------------------------------------------------
-// The tile lists of one call in one buffer of words: counts of the row and column lists, then their
-// entries, every list in a place of nb words.
-struct Lists {
-  int64_t col_cnt, col_idx, row_idx, words;
-  Lists(int64_t Bm, int64_t Hm, int64_t nb) {
-    const int64_t rows = Bm * Hm * nb;
-    col_cnt = rows;
-    col_idx = (2 * rows + 3) & ~int64_t{3};
-    row_idx = col_idx + rows * nb;
-    words = row_idx + rows * nb;
-  }
-};
-
 // (A node of its own and not torch::autograd::Function: that keeps what is saved in a map of boxed values,
 // which costs a small call another 10 us.)
 struct AttentionBackward : torch::autograd::Node {
@@ -267,18 +281,11 @@ Tensor forward_with_grad(const Tensor& q0, const Tensor& k0, const Tensor& v0, c
   Tensor o, lse2, lists;
   {
     at::AutoDispatchBelowADInplaceOrView no_autograd;
-    if (!run_forward(tma_ready(q0), tma_ready(k0), tma_ready(v0), m, scale, state, stream, &o, &lse2))
+    if (!run_forward(tma_ready(q0), tma_ready(k0), tma_ready(v0), m, scale, state, stream, &o, &lse2, &lists))
       return Tensor();
-    // the forward lists each mask row inside the kernel; only the backward needs lists as data
     node->Bm = m.block.size(0);
     node->Hm = m.block.size(1);
     node->nb = m.block.size(2);
-    const Lists at(node->Bm, node->Hm, node->nb);
-    lists = at::empty({at.words}, q0.options().dtype(at::kInt));
-    int32_t* p = lists.mutable_data_ptr<int32_t>();
-    if (bsa_tile_lists_places(m.block.const_data_ptr<uint8_t>(), m.block.strides().data(), node->Bm, node->Hm,
-                              node->nb, p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, stream) != 0)
-      return Tensor();
   }
   node->dense = m.dense;
   node->scale = static_cast<float>(scale);
@@ -318,7 +325,7 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
     return o.defined() ? std::optional<Tensor>(o) : std::nullopt;
   }
   Tensor o, lse2;
-  if (!run_forward(tma_ready(q), tma_ready(k), tma_ready(v), m, scale, state, stream, &o, &lse2))
+  if (!run_forward(tma_ready(q), tma_ready(k), tma_ready(v), m, scale, state, stream, &o, &lse2, nullptr))
     return std::nullopt;
   return o;
 }
