@@ -267,7 +267,8 @@ __device__ __forceinline__ uint32_t pick3u(int sel, uint32_t v0, uint32_t v1, ui
 }
 
 template <bool kInverse>
-__global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_constant__ PermuteArgs a) {
+__global__ void __launch_bounds__(kPermThreads, 3) permute_kernel(const __grid_constant__ PermuteArgs a) {
+  extern __shared__ __align__(16) uint8_t s_pieces[];  // piece i of thread t at (i * kPermThreads + t) * 16
   grid_dependents_launch();
   grid_dependency_wait();
   int unit = blockIdx.y;
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_c
   const uint32_t vec = static_cast<uint32_t>(a.chunk_bytes) >> 4;
   const uint32_t first = blockIdx.x * a.pieces_per_cta + threadIdx.x;
   const uint32_t end = min(static_cast<uint32_t>(a.T) * vec, (blockIdx.x + 1) * a.pieces_per_cta);
-  uint4 val[kPermPieces];
+  uint4* const mine = reinterpret_cast<uint4*>(s_pieces) + threadIdx.x;
 #pragma unroll
   for (int i = 0; i < kPermPieces; ++i) {
     const uint32_t idx = first + i * kPermThreads;
@@ -325,9 +326,11 @@ __global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_c
       const uint32_t c0 = div_by(t, g1 * g2, m_plane), rem = t - c0 * (g1 * g2);
       const uint32_t c1 = div_by(rem, g2, m_last), c2 = rem - c1 * g2;
       const uint32_t from = c0 * w0 + c1 * w1 + c2 * w2;
-      val[i] = *reinterpret_cast<const uint4*>(base + from * st + piece * 16u);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(mine + i * kPermThreads)),
+                   "l"(base + from * st + piece * 16u) : "memory");
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   // every CTA of the cluster has read its share before any of them stores
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 #pragma unroll
@@ -335,7 +338,7 @@ __global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_c
     const uint32_t idx = first + i * kPermThreads;
     if (idx < end) {
       const uint32_t t = div_by(idx, vec, a.m_vec), piece = idx - t * vec;
-      *reinterpret_cast<uint4*>(base + t * st + piece * 16u) = val[i];
+      *reinterpret_cast<uint4*>(base + t * st + piece * 16u) = mine[i * kPermThreads];
     }
   }
 }
@@ -343,6 +346,9 @@ __global__ void __launch_bounds__(kPermThreads, 2) permute_kernel(const __grid_c
 template <bool kInverse>
 static int launch_permute(PermuteArgs& a, int n_tensors, int cluster, cudaStream_t stream) {
   auto kern = permute_kernel<kInverse>;
+  constexpr size_t kSmem = kPermThreads * kPermPieces * 16;
+  const int smem_rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmem);
+  if (smem_rc != BSA_OK) return smem_rc;
   static std::atomic<int> ready[64];  // per device: 0 unknown, 1 clusters of 16 fit, 2 they do not
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return BSA_ERR_CUDA;
@@ -358,6 +364,7 @@ static int launch_permute(PermuteArgs& a, int n_tensors, int cluster, cudaStream
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(cluster), static_cast<unsigned>(units), 1);
   cfg.blockDim = dim3(kPermThreads, 1, 1);
+  cfg.dynamicSmemBytes = kSmem;
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
