@@ -138,8 +138,8 @@ struct FwdParams {
   int64_t ds0, ds1, ds2;
   void* o;
   int64_t o_sb, o_sh, o_sn;
-  float* lse2;
-  float* rowmax;
+  float* lse2;     // optional
+  float* rowmax;   // optional
   int B, H, N, D, nb;
   int row_begin, nrows;     // the query-block rows [row_begin, row_begin + nrows) of every head
   int list_b_stride, list_h_stride;
@@ -946,7 +946,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (ok && half == 0) {
         const int64_t ri = (static_cast<int64_t>(walk.it.x) * p.H + walk.it.y) * p.N + row;
-        p.lse2[ri] = l_all > 0.f ? m_all + lg2_approx(l_all) : -INFINITY;
+        if (p.lse2) p.lse2[ri] = l_all > 0.f ? m_all + lg2_approx(l_all) : -INFINITY;
         if (p.rowmax) p.rowmax[ri] = mt;
       }
       if (any_failed) break;
@@ -988,7 +988,7 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
     return BSA_ERR_BAD_SHAPE;
   if (!(sm_scale >= 0.f)) return BSA_ERR_BAD_SHAPE;  // the row maximum is taken before scaling
   if (dtype != BSA_F16 && dtype != BSA_BF16) return BSA_ERR_BAD_DTYPE;
-  if (!lse2 || (block == nullptr && (!row_ptr || !col_idx))) return BSA_ERR_BAD_POINTER;
+  if (block == nullptr && (!row_ptr || !col_idx)) return BSA_ERR_BAD_POINTER;
   if (dense != nullptr) {
     // rows of 64 mask bytes are read as four 16-byte words; -inf times a zero scale would be NaN
     if (!dense_strides || !is_aligned(dense, 16)) return BSA_ERR_BAD_POINTER;
@@ -1077,7 +1077,7 @@ extern "C" int bsa_attn_fwd_rows(const void* q, const int64_t q_strides[4], cons
                                  int row_begin, int row_end, const uint8_t* dense,
                                  const int64_t dense_strides[4], int32_t* work_counter,
                                  int32_t* status, void* stream) {
-  if (!row_ptr || !col_idx) return BSA_ERR_BAD_POINTER;
+  if (!row_ptr || !col_idx || !lse2) return BSA_ERR_BAD_POINTER;
   return bsa::launch_fwd(q, q_strides, k, k_strides, v, v_strides, o, o_strides, lse2, rowmax,
                          row_ptr, col_idx, nullptr, nullptr, list_b_stride, list_h_stride, sm_scale,
                          dtype, B, H, N, D, row_begin, row_end, dense, dense_strides, status,
@@ -1102,7 +1102,7 @@ extern "C" int bsa_attn_fwd_block_mask_rows(
     float sm_scale, int dtype, int B, int H, int N, int D, int row_begin, int row_end,
     const uint8_t* dense, const int64_t dense_strides[4], int32_t* work_counter, int32_t* status,
     void* stream) {
-  if (!block || !block_strides) return BSA_ERR_BAD_POINTER;
+  if (!block || !block_strides || !lse2) return BSA_ERR_BAD_POINTER;
   if ((Bm != 1 && Bm != B) || (Hm != 1 && Hm != H)) return BSA_ERR_BAD_SHAPE;
   for (int i = 0; i < 4; ++i)
     if (block_strides[i] < 0) return BSA_ERR_BAD_STRIDE;
@@ -1132,7 +1132,7 @@ extern "C" int bsa_attn_fwd_block_mask_lists(
     const int64_t block_strides[4], int Bm, int Hm, float sm_scale, int dtype, int B, int H, int N, int D,
     const uint8_t* dense, const int64_t dense_strides[4], int32_t* row_cnt, int32_t* col_idx, int32_t* col_cnt,
     int32_t* row_idx, int32_t* work_counter, int32_t* status, void* stream) {
-  if (!block || !block_strides || !row_cnt || !col_idx || !col_cnt || !row_idx) return BSA_ERR_BAD_POINTER;
+  if (!block || !block_strides || !lse2 || !row_cnt || !col_idx || !col_cnt || !row_idx) return BSA_ERR_BAD_POINTER;
   if ((Bm != 1 && Bm != B) || (Hm != 1 && Hm != H)) return BSA_ERR_BAD_SHAPE;
   for (int i = 0; i < 4; ++i)
     if (block_strides[i] < 0) return BSA_ERR_BAD_STRIDE;
@@ -1145,4 +1145,18 @@ extern "C" int bsa_attn_fwd_block_mask_lists(
   if (rc != BSA_OK) return rc;
   return bsa::launch_lists_places(block, block_strides, Bm, Hm, N / bsa::kBlock, row_cnt, col_idx, col_cnt, row_idx,
                                   true, stream);
+}
+
+extern "C" int bsa_attn_fwd_block_mask_output(
+    const void* q, const int64_t q_strides[4], const void* k, const int64_t k_strides[4], const void* v,
+    const int64_t v_strides[4], void* o, const int64_t o_strides[4], const uint8_t* block,
+    const int64_t block_strides[4], int Bm, int Hm, float sm_scale, int dtype, int B, int H, int N, int D,
+    const uint8_t* dense, const int64_t dense_strides[4], int32_t* work_counter, int32_t* status, void* stream) {
+  if (!block || !block_strides) return BSA_ERR_BAD_POINTER;
+  if ((Bm != 1 && Bm != B) || (Hm != 1 && Hm != H)) return BSA_ERR_BAD_SHAPE;
+  for (int i = 0; i < 4; ++i)
+    if (block_strides[i] < 0) return BSA_ERR_BAD_STRIDE;
+  return bsa::launch_fwd(q, q_strides, k, k_strides, v, v_strides, o, o_strides, nullptr, nullptr, nullptr, nullptr,
+                         block, block_strides, Bm > 1 ? 1 : 0, Hm > 1 ? 1 : 0, sm_scale, dtype, B, H, N, D, 0,
+                         N > 0 ? N / bsa::kBlock : 0, dense, dense_strides, status, work_counter, stream);
 }

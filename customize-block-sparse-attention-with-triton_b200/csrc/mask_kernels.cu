@@ -35,6 +35,7 @@ mask_reduce_kernel(const uint8_t* __restrict__ dense, int64_t sb, int64_t sh, in
   const int seg = threadIdx.x & 63;
   const int rg = threadIdx.x >> 6;
   const int col = col0 + seg * 16;
+  grid_dependents_launch();  // (the forward's set-up under this kernel's end: 19.5 -> 19.1 us for both at N = 6400)
   uint32_t any_bits = 0, zero_bits = 0;
   if (col < N) {
     const uint8_t* base = dense + b * sb + h * sh + static_cast<int64_t>(rb) * 64 * sr + col;
@@ -433,8 +434,9 @@ extern "C" int bsa_mask_reduce(const uint8_t* dense, const int64_t s[4], int B, 
   if (partial_tiles && cudaMemsetAsync(partial_tiles, 0, sizeof(int32_t), st) != cudaSuccess)
     return BSA_ERR_CUDA;
   const dim3 grid((N + kReduceCols - 1) / kReduceCols, nb, B * H);
-  // (an ordinary launch: as a dependent one it kept SMs from the forward before and after it, 25 instead
-  // of 20 us for reduction and forward at N = 6400)
+  // (an ordinary launch: the CTAs of a dependent one would all go to the few SMs that happen to be free while
+  // the kernel before it ends, 23.5 instead of 19.5 us for reduction and forward at N = 6400; with an SM held to
+  // its share of them by a request for shared memory 20.5)
   mask_reduce_kernel<<<grid, kReduceThreads, 0, st>>>(dense, s[0], s[1], s[2], H, N, nb, block,
                                                       partial_tiles, mark_partial);
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;

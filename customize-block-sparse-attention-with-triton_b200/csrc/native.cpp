@@ -100,38 +100,57 @@ Tensor tma_ready(const Tensor& t) {
   return ok ? t : t.contiguous();
 }
 
+// (Plain pointers and strides: each view of a tensor costs the host as much as a tenth of a small call.)
 struct Mask {
-  Tensor block;         // bytes [Bm,Hm,nb,nb]
-  Tensor dense;         // bytes [Bm,Hm,N,N], or undefined
-  int64_t dense_strides[4];
+  Tensor owner;                // what the block mask was reduced into, if it was
+  const uint8_t* block;        // bytes [Bm,Hm,nb,nb]
+  int64_t Bm, Hm, block_strides[4];
+  Tensor dense;                // the mask of [Bm,Hm,N,N] elements (or an aligned copy of it), or undefined
   const uint8_t* dense_ptr = nullptr;
+  int64_t dense_strides[4];    // (0 for a broadcast axis)
 };
 
-// The op's mask argument as 4-D bytes; false when it is nothing that this path takes.
+// The op's mask argument; false when it is nothing that this path takes.
 bool read_mask(const Tensor& mask, int64_t B, int64_t H, int64_t N, const Tensor& q, void* stream, Mask* out) {
   const int64_t dims = mask.dim(), nb = N / kBlock;
   if (dims < 2 || dims > 4 || mask.device() != q.device()) return false;
   if (mask.scalar_type() != at::kBool && mask.scalar_type() != at::kByte) return false;
-  Tensor m = mask.scalar_type() == at::kBool ? mask.view(at::kByte) : mask;
-  while (m.dim() < 4) m = m.unsqueeze(0);
-  if ((m.size(0) != 1 && m.size(0) != B) || (m.size(1) != 1 && m.size(1) != H)) return false;
-  if (m.size(2) == nb && m.size(3) == nb) {
-    out->block = m;
+  // axes that are missing in front have size 1
+  int64_t sizes[4], strides[4];
+  const auto look_at = [&](const Tensor& m) {
+    for (int64_t i = 0; i < 4; ++i) {
+      const int64_t d = i - (4 - dims);
+      sizes[i] = d < 0 ? 1 : m.size(d);
+      strides[i] = d < 0 ? m.size(0) * m.stride(0) : m.stride(d);
+    }
+  };
+  look_at(mask);
+  if ((sizes[0] != 1 && sizes[0] != B) || (sizes[1] != 1 && sizes[1] != H)) return false;
+  out->Bm = sizes[0];
+  out->Hm = sizes[1];
+  if (sizes[2] == nb && sizes[3] == nb) {
+    out->block = static_cast<const uint8_t*>(mask.const_data_ptr());
+    for (int i = 0; i < 4; ++i) out->block_strides[i] = strides[i];
     return true;
   }
-  if (m.size(2) != N || m.size(3) != N) return false;
+  if (sizes[2] != N || sizes[3] != N) return false;
   // a dense mask: reduced to blocks, the partly kept ones marked 2, and applied inside those
-  bool ok = m.stride(3) == 1 && reinterpret_cast<uintptr_t>(m.const_data_ptr()) % 16 == 0;
-  for (int i = 0; ok && i < 3; ++i) ok = m.stride(i) % 16 == 0;
-  out->dense = ok ? m : m.contiguous();
-  out->block = at::empty({m.size(0), m.size(1), nb, nb}, m.options());
-  out->dense_ptr = out->dense.const_data_ptr<uint8_t>();
-  for (int i = 0; i < 4; ++i) out->dense_strides[i] = out->dense.stride(i);
-  if (bsa_mask_reduce(out->dense_ptr, out->dense_strides, m.size(0), m.size(1), N,
-                      out->block.mutable_data_ptr<uint8_t>(), nullptr, 1, stream) != 0)
+  bool ok = strides[3] == 1 && reinterpret_cast<uintptr_t>(mask.const_data_ptr()) % 16 == 0;
+  for (int i = 0; ok && i < 3; ++i) ok = strides[i] % 16 == 0;
+  out->dense = ok ? mask : mask.contiguous();
+  if (!ok) look_at(out->dense);
+  out->owner = at::empty({sizes[0], sizes[1], nb, nb}, mask.options().dtype(at::kByte));
+  uint8_t* block = out->owner.mutable_data_ptr<uint8_t>();
+  out->block = block;
+  out->dense_ptr = static_cast<const uint8_t*>(out->dense.const_data_ptr());
+  for (int i = 0; i < 4; ++i) {
+    out->dense_strides[i] = strides[i];
+    out->block_strides[i] = out->owner.stride(i);
+  }
+  if (bsa_mask_reduce(out->dense_ptr, out->dense_strides, sizes[0], sizes[1], N, block, nullptr, 1, stream) != 0)
     return false;
   for (int i = 0; i < 2; ++i)
-    if (m.size(i) == 1) out->dense_strides[i] = 0;  // broadcast
+    if (sizes[i] == 1) out->dense_strides[i] = 0;  // broadcast
   return true;
 }
 
@@ -150,36 +169,33 @@ struct Lists {
   }
 };
 
-// Runs the forward, and builds the tile lists that a backward needs if they are wanted; false when the
-// library refused.  (The forward lists each mask row inside the kernel.  The lists are written while it is still
-// running, so their memory has to be allocated before the copies that q, k, v may be are given back.)
+// Runs the forward; with lse2 and lists also what a backward needs.  False when the library refused.  (The
+// forward lists each mask row inside the kernel.  The lists are written while it is still running, so their
+// memory has to be allocated before the copies that q, k, v may be are given back.)
 bool run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& m, double scale,
                  StreamState* state, void* stream, Tensor* o, Tensor* lse2, Tensor* lists) {
   const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
   *o = at::empty({B, H, N, D}, q.options());
-  *lse2 = at::empty({B, H, N}, q.options().dtype(at::kFloat));
   Tensor own;
   int32_t* counter = work_counter(state, B * H * (N / kBlock), q.options(), &own);
   int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
   const int64_t* dense_strides = m.dense_ptr ? m.dense_strides : nullptr;
-  if (lists != nullptr) {
-    const Lists at(m.block.size(0), m.block.size(1), N / kBlock);
-    *lists = at::empty({at.words}, q.options().dtype(at::kInt));
-    int32_t* p = lists->mutable_data_ptr<int32_t>();
-    return bsa_attn_fwd_block_mask_lists(
+  if (lists == nullptr)
+    return bsa_attn_fwd_block_mask_output(
                q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
-               v.const_data_ptr(), v.strides().data(), o->mutable_data_ptr(), o->strides().data(),
-               lse2->mutable_data_ptr<float>(), m.block.const_data_ptr<uint8_t>(), m.block.strides().data(),
-               m.block.size(0), m.block.size(1), static_cast<float>(scale), dtype_code(q), B, H, N, D,
-               m.dense_ptr, dense_strides, p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, counter, status,
-               stream) == 0;
-  }
-  return bsa_attn_fwd_block_mask_rows(
+               v.const_data_ptr(), v.strides().data(), o->mutable_data_ptr(), o->strides().data(), m.block,
+               m.block_strides, m.Bm, m.Hm, static_cast<float>(scale), dtype_code(q), B, H, N, D, m.dense_ptr,
+               dense_strides, counter, status, stream) == 0;
+  *lse2 = at::empty({B, H, N}, q.options().dtype(at::kFloat));
+  const Lists at(m.Bm, m.Hm, N / kBlock);
+  *lists = at::empty({at.words}, q.options().dtype(at::kInt));
+  int32_t* p = lists->mutable_data_ptr<int32_t>();
+  return bsa_attn_fwd_block_mask_lists(
              q.const_data_ptr(), q.strides().data(), k.const_data_ptr(), k.strides().data(),
              v.const_data_ptr(), v.strides().data(), o->mutable_data_ptr(), o->strides().data(),
-             lse2->mutable_data_ptr<float>(), nullptr, m.block.const_data_ptr<uint8_t>(),
-             m.block.strides().data(), m.block.size(0), m.block.size(1), static_cast<float>(scale),
-             dtype_code(q), B, H, N, D, 0, N / kBlock, m.dense_ptr, dense_strides, counter, status, stream) == 0;
+             lse2->mutable_data_ptr<float>(), m.block, m.block_strides, m.Bm, m.Hm, static_cast<float>(scale),
+             dtype_code(q), B, H, N, D, m.dense_ptr, dense_strides, p, p + at.col_idx, p + at.col_cnt,
+             p + at.row_idx, counter, status, stream) == 0;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -216,7 +232,7 @@ void raise_if_reported(StreamState* state) {
 struct AttentionBackward : torch::autograd::Node {
   torch::autograd::SavedVariable q_, k_, v_, o_, lse2_, lists_;
   Tensor dense;  // the caller's mask (or an aligned copy of it): not to be changed before backward
-  int64_t Bm, Hm, nb;
+  int64_t Bm, Hm, nb, dense_strides[4];
   float scale;
 
   std::string name() const override { return "AttentionBackward"; }
@@ -236,13 +252,7 @@ struct AttentionBackward : torch::autograd::Node {
     if (!grads[0].defined()) return {Tensor(), Tensor(), Tensor()};
     const Tensor dout = tma_ready(grads[0].to(q.scalar_type()));
     const Lists at(Bm, Hm, nb);
-    const uint8_t* dense_ptr = nullptr;
-    int64_t strides[4] = {0, 0, 0, 0};
-    if (dense.defined()) {
-      dense_ptr = dense.const_data_ptr<uint8_t>();
-      for (int i = 0; i < 4; ++i) strides[i] = i < 2 && dense.size(i) == 1 ? 0 : dense.stride(i);
-    }
-    const int64_t* dense_strides = dense_ptr ? strides : nullptr;
+    const uint8_t* dense_ptr = dense.defined() ? static_cast<const uint8_t*>(dense.const_data_ptr()) : nullptr;
     const c10::cuda::CUDAGuard guard(q.device());
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
     StreamState* state = stream_state(q.device().index(), stream);
@@ -268,7 +278,8 @@ struct AttentionBackward : torch::autograd::Node {
               v.const_data_ptr(), v.strides().data(), dout.const_data_ptr(), dout.strides().data(), lse_p,
               delta_p, dq.mutable_data_ptr(), dq.strides().data(), dk.mutable_data_ptr(), dk.strides().data(),
               dv.mutable_data_ptr(), dv.strides().data(), p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, nb, sb,
-              sh, scale, code, B, H, N, D, dense_ptr, dense_strides, counter, dq_counter, status, stream));
+              sh, scale, code, B, H, N, D, dense_ptr, dense_ptr ? dense_strides : nullptr, counter, dq_counter, status,
+              stream));
     return {dq, dk, dv};
   }
 };
@@ -283,11 +294,12 @@ Tensor forward_with_grad(const Tensor& q0, const Tensor& k0, const Tensor& v0, c
     at::AutoDispatchBelowADInplaceOrView no_autograd;
     if (!run_forward(tma_ready(q0), tma_ready(k0), tma_ready(v0), m, scale, state, stream, &o, &lse2, &lists))
       return Tensor();
-    node->Bm = m.block.size(0);
-    node->Hm = m.block.size(1);
-    node->nb = m.block.size(2);
   }
+  node->Bm = m.Bm;
+  node->Hm = m.Hm;
+  node->nb = q0.size(2) / kBlock;
   node->dense = m.dense;
+  for (int i = 0; i < 4; ++i) node->dense_strides[i] = m.dense_strides[i];
   node->scale = static_cast<float>(scale);
   node->q_ = torch::autograd::SavedVariable(q0, false);
   node->k_ = torch::autograd::SavedVariable(k0, false);
@@ -324,8 +336,8 @@ std::optional<Tensor> attention(const Tensor& q, const Tensor& k, const Tensor& 
     Tensor o = forward_with_grad(q, k, v, m, scale, state, stream);
     return o.defined() ? std::optional<Tensor>(o) : std::nullopt;
   }
-  Tensor o, lse2;
-  if (!run_forward(tma_ready(q), tma_ready(k), tma_ready(v), m, scale, state, stream, &o, &lse2, nullptr))
+  Tensor o;
+  if (!run_forward(tma_ready(q), tma_ready(k), tma_ready(v), m, scale, state, stream, &o, nullptr, nullptr))
     return std::nullopt;
   return o;
 }

@@ -50,6 +50,8 @@ SIGNATURES = {
                           _i, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
     "bsa_attn_fwd_block_mask_rows": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _vp, _s4, _i,
                                      _i, _f, _i, _i, _i, _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp],
+    "bsa_attn_fwd_block_mask_output": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _i, _i, _f, _i, _i, _i,
+                                       _i, _i, _vp, _s4, _vp, _vp, _vp],
     "bsa_attn_fwd_block_mask_lists": [_vp, _s4, _vp, _s4, _vp, _s4, _vp, _s4, _vp, _vp, _s4, _i, _i, _f, _i,
                                       _i, _i, _i, _i, _vp, _s4, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "bsa_attn_bwd_delta": [_vp, _vp, _s4, _vp, _i, _i, _i, _i, _i, _vp],

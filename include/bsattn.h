@@ -202,6 +202,15 @@ int bsa_attn_fwd_block_mask_rows(const void* q, const int64_t q_strides[4], cons
                                  const uint8_t* dense, const int64_t dense_strides[4],
                                  int32_t* work_counter, int32_t* status, void* stream);
 
+/* bsa_attn_fwd_block_mask_rows over all rows for callers that only want o. */
+int bsa_attn_fwd_block_mask_output(const void* q, const int64_t q_strides[4], const void* k,
+                                   const int64_t k_strides[4], const void* v, const int64_t v_strides[4],
+                                   void* o, const int64_t o_strides[4], const uint8_t* block,
+                                   const int64_t block_strides[4], int Bm, int Hm, float sm_scale,
+                                   int dtype, int B, int H, int N, int D, const uint8_t* dense,
+                                   const int64_t dense_strides[4], int32_t* work_counter,
+                                   int32_t* status, void* stream);
+
 /* bsa_attn_fwd_block_mask_rows over all rows and bsa_tile_lists_places of the same mask, which a training step
  * needs for its backward: the lists are built on SMs that the forward has no more work for.  So nothing that the
  * forward touches may overlap them.  What follows in the stream waits for both. */
