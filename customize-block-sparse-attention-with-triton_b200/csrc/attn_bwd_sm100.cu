@@ -393,11 +393,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
-  // Together, dQ begins while dK/dV is still running: it is launched when all CTAs of dK/dV have passed
-  // this point, so what came before dK/dV has ended and is visible then.  It ends after dK/dV (see the end).
-  if (kDKDV || !p.together) grid_dependency_wait();
-  if (kDKDV && p.together) grid_dependents_launch();
-
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
   // issuers do without (56 + 104 + 56 = 3 x 72).
   if ((warp >= kCW && warp < kCW + 4) || warp >= kCW + 8) {
@@ -406,6 +401,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       // =========================== TMA producer ===========================
       bool ok = true;
       bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
+      // Whatever touches memory that an earlier kernel may use comes after the first item's header, so one role
+      // waits for the end of that kernel while the others get as far as their first barrier.
+      // Together, dQ begins while dK/dV is still running: it is launched when all CTAs of dK/dV have passed
+      // this point, so what came before dK/dV has ended and is visible then.  It ends after dK/dV (see the end).
+      if (kDKDV || !p.together) grid_dependency_wait();
+      if (kDKDV && p.together) grid_dependents_launch();
       int gs = 0, ni = 0;
 #pragma unroll 1
       for (int i = 0, w = blockIdx.x; ok; ++i) {

@@ -420,8 +420,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
-  grid_dependency_wait();
-  if (p.successor_early) grid_dependents_launch();
 
   // 512 threads are launched with 128 registers: the softmax warps, which hold 64 logits and 128
   // probabilities each, take what the others do without (2 x 168 + 72 + 104 = 4 x 128).  A spill in their
@@ -805,6 +803,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t o_lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kTmemO;
     int g = 0;  // supersteps of earlier items
     FwdWalk walk;
+    if (lister) {
+      // Whatever touches memory that an earlier kernel may use comes after the first list, so one role waits
+      // for the end of that kernel while the others get as far as their first barrier.
+      grid_dependency_wait();
+      if (p.successor_early) grid_dependents_launch();
+    }
 #pragma unroll 1
     for (int i = -1;; ++i) {
       const int par = i & 1;
