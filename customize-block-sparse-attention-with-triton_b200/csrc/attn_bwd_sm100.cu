@@ -767,8 +767,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     if (!ok) report_status(p.status, 3);
   }
 
-  // (not before: CTAs of the next kernel that wait on free SMs slowed the working ones down by 3 %)
-  grid_dependents_launch();
+  // The next kernel may come as soon as a role of every CTA gets here, warps without a role at once: it waits
+  // itself for the end of this one (from the last role on: 1 us later).  Not so when dQ follows that does not
+  // wait: it has been let in above.
+  if (!(kDKDV && p.together)) grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   if (warp == kXWarp) {

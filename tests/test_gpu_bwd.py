@@ -210,3 +210,49 @@ def test_forward_and_backward_in_a_graph(lib):
             assert (out.detach().float().cpu() - o_ref).abs().max() <= 2e-2
             for got, ref in ((q.grad, dq_ref), (k.grad, dk_ref), (v.grad, dv_ref)):
                 assert (got.float().cpu() - ref).abs().max() <= G_TOL
+
+
+@pytest.mark.parametrize("replay", [False, True])
+@pytest.mark.parametrize("B,H,N", [(1, 2, 512), (2, 3, 320), (1, 8, 2048)])
+def test_kernels_that_run_beside_one_another_see_what_they_need(lib, B, H, N, replay):
+    """The tile lists are built beside the forward, and dQ begins beside dK/dV, on SMs that are idle when a
+    sequence is short: neither may begin before what it reads is there.  Steps on new data in the same buffers,
+    called or replayed, against the same kernels one after the other: the same bits."""
+    from fa2_custom_mask import attention_backward, attention_forward, build_tile_lists, flash_attention_custom_mask
+    g = torch.Generator(device="cuda").manual_seed(N)
+    bufs = [torch.randn(B, H, N, 64, device="cuda", generator=g).bfloat16() for _ in range(4)]
+    for t in bufs[:3]:
+        t.requires_grad_(True)
+    nb = N // 64
+    mask = torch.ones(B, H, nb, nb, dtype=torch.bool, device="cuda")
+
+    def step():
+        o = flash_attention_custom_mask(*bufs[:3], mask, 0.125)
+        return [o, *torch.autograd.grad(o, bufs[:3], bufs[3])]
+
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        step()
+        torch.cuda.synchronize()
+        if replay:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=s):
+                outs = step()
+        for _ in range(40):
+            with torch.no_grad():
+                for t in bufs:
+                    t.copy_(torch.randn(B, H, N, 64, device="cuda", generator=g))
+                mask.copy_(torch.rand(B, H, nb, nb, device="cuda", generator=g) < 0.5)
+                mask.logical_or_(torch.eye(nb, dtype=torch.bool, device="cuda"))
+            if replay:
+                graph.replay()
+            else:
+                outs = step()
+            torch.cuda.synchronize()
+            lists = build_tile_lists(mask)
+            q, k, v = (t.detach() for t in bufs[:3])
+            o, lse2, _ = attention_forward(q, k, v, lists, 0.125)
+            torch.cuda.synchronize()
+            for got, ref in zip(outs, [o, *attention_backward(q, k, v, o, lse2, bufs[3], lists, 0.125)]):
+                assert torch.equal(got, ref)
