@@ -281,7 +281,7 @@ __device__ __forceinline__ uint32_t fwd_row_word(const uint8_t* row, int nb, int
 }
 
 // Lists the key blocks of work item w into list buffer `at` (one warp) and publishes list and item.
-template <bool kElementMask>
+template <bool kElementMask, bool kPublish>
 __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, int w, int at,
                                               int lane) {
   const FwdItem it = fwd_item(w, p);
@@ -343,7 +343,7 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
   __syncwarp();
   if (lane == 0) {
     sm->item[at] = make_int4(it.b, it.h, it.mb, n_tiles);
-    mbar_arrive(smem_u32(&sm->list_full[at]));  // release: list and item are visible
+    if constexpr (kPublish) mbar_arrive(smem_u32(&sm->list_full[at]));  // release: list and item are visible
   }
 }
 
@@ -416,7 +416,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_v);
   }
   tc_fence_before();
-  __syncthreads();
+  if (warp == kListerWarp) {
+    // Lists the CTA's first item while the others set up and get as far as their first barrier.  (With the list
+    // from the lister's own loop, behind the jumps to the roles and instructions that no cache held yet, the
+    // first tiles were asked for 2,200 cycles later.)  Everything that touches memory that an earlier
+    // kernel may use comes after this.
+    grid_dependency_wait();
+    if (p.successor_early) grid_dependents_launch();
+    fwd_list_item<kElementMask, false>(sm, p, blockIdx.x, 0, lane);
+    named_barrier_sync(1, kFwdThreads);  // the barriers are there
+    if (lane == 0) mbar_arrive(smem_u32(&sm->list_full[0]));
+  } else {
+    named_barrier_arrive(1, kFwdThreads);
+    named_barrier_sync(3, kFwdThreads - 32);
+  }
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
@@ -789,8 +802,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // barriers of an iteration are always executed, also after a give-up, and the last one carries
     // the give-up vote, so that no warp of this role can be left waiting at one.
     //
-    // One of the four warps is also the lister: it sets up the CTA's first item, and item i+1 when the
-    // producer says so during item i, i.e. between its write-outs of items i-1 and i.
+    // One of the four warps is also the lister: it sets up item i+1 when the producer says so during item i,
+    // i.e. between its write-outs of items i-1 and i (the CTA's first item at the very beginning).
     give_registers<104>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
     const bool lister = warp == kListerWarp;
@@ -803,56 +816,45 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t o_lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kTmemO;
     int g = 0;  // supersteps of earlier items
     FwdWalk walk;
-    if (lister) {
-      // Whatever touches memory that an earlier kernel may use comes after the first list, so one role waits
-      // for the end of that kernel while the others get as far as their first barrier.
-      grid_dependency_wait();
-      if (p.successor_early) grid_dependents_launch();
-    }
 #pragma unroll 1
-    for (int i = -1;; ++i) {
+    for (int i = 0;; ++i) {
       const int par = i & 1;
-      if (i >= 0) {
-        if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag, 256);
-        walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
-        if (walk.it.x < 0) break;  // no more work: the same for all four warps
-      }
+      if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag, 256);
+      walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
+      if (walk.it.x < 0) break;  // no more work: the same for all four warps
       if (lister && ok) {
         // Sets up the next item, or publishes that there is none; a wait that gives up leaves ok =
         // false and nothing published.  The next ticket when items are handed out dynamically, else
         // a fixed stride.
-        const int at = i < 0 ? 0 : walk.at + 1 < kLists ? walk.at + 1 : 0;
-        if (i >= 0) {
-          ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1);
-          if (ok && p.ticket != nullptr) {
-            int t = 0;
-            if (lane == 0) {
-              t = atomicAdd(p.ticket, 1);
-              // every CTA draws until its first ticket past the end, so the launch draws exactly
-              // `items` tickets in all; whoever draws the last one leaves the counter at zero
-              if (t == p.items - 1) atomicExch(p.ticket, 0);
-            }
-            t = __shfl_sync(0xffffffffu, t, 0);
-            terminal = t >= n2;
-            lw = stride + t;
-          } else {
-            lw += stride;
+        const int at = walk.at + 1 < kLists ? walk.at + 1 : 0;
+        ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1);
+        if (ok && p.ticket != nullptr) {
+          int t = 0;
+          if (lane == 0) {
+            t = atomicAdd(p.ticket, 1);
+            // every CTA draws until its first ticket past the end, so the launch draws exactly
+            // `items` tickets in all; whoever draws the last one leaves the counter at zero
+            if (t == p.items - 1) atomicExch(p.ticket, 0);
           }
-          // The list buffer was that of item i-2, which these warps have written out (and the softmax
-          // warps with them are through with); the producers and issuers may lag behind.
-          if (ok && i >= 2)
-            ok = mbar_wait_warp_idle(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag, 128);
+          t = __shfl_sync(0xffffffffu, t, 0);
+          terminal = t >= n2;
+          lw = stride + t;
+        } else {
+          lw += stride;
         }
+        // The list buffer was that of item i-2, which these warps have written out (and the softmax
+        // warps with them are through with); the producers and issuers may lag behind.
+        if (ok && i >= 2)
+          ok = mbar_wait_warp_idle(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag, 128);
         if (ok) {
           if (lw < p.items) {
-            fwd_list_item<kElementMask>(sm, p, lw, at, lane);
+            fwd_list_item<kElementMask, true>(sm, p, lw, at, lane);
           } else if (lane == 0) {
             sm->item[at].x = -1;
             mbar_arrive(smem_u32(&sm->list_full[at]));
           }
         }
       }
-      if (i < 0) continue;
       const int n_tiles = walk.it.w;
       if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->stats_full[par]), (i >> 1) & 1, abort_flag, 128);
       // The weights of the four partial results need the statistics only, which the softmax warps

@@ -30,6 +30,11 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// Counts as one of the threads that named_barrier_sync waits for, without waiting.
+__device__ __forceinline__ void named_barrier_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // Register split between the warpgroups of a block: executed by all four warps of one.  The shares
 // must add up to no more than the registers the block was launched with.
 template <int kRegs>
