@@ -66,3 +66,19 @@ def test_shape_and_dtype_checks_come_before_any_cuda_call(lib):
     assert lib.bsa_reorder_strided(fake, s4, fake, bad_out, fake, 1, 1, 8, 8, 2, 2, 2, 2, None) == -3
     assert lib.bsa_inv_reorder_strided(fake, s4, fake, s4, fake, None, 1, 1, 8, 8, 2, 2, 2, 2,
                                        None) == -4                                     # inv_orders
+
+
+def test_the_two_kernels_of_a_backward_need_work_counters_of_their_own(lib):
+    s4 = (ctypes.c_int64 * 4)(64 * 64, 64 * 64, 64, 1)
+    fake, other = ctypes.c_void_p(0x1000), ctypes.c_void_p(0x2000)
+    args = [fake, s4] * 4 + [fake, fake] + [fake, s4] * 3 + [fake] * 4 + [0, 0, 0, 0.125, 0, 1, 1]
+    assert lib.bsa_attn_bwd_strided(*args, 64, 64, None, None, fake, fake, None, None) == -4
+    assert lib.bsa_attn_bwd_strided(*args, 63, 64, None, None, fake, other, None, None) == -1
+    # the log-sum-exp is optional in one entry point alone
+    args = [fake, s4] * 4
+    assert lib.bsa_attn_fwd_block_mask_rows(*args, None, None, fake, s4, 1, 1, 0.125, 0, 1, 1, 64, 64, 0, 1, None, None,
+                                            None, None, None) == -4
+    assert lib.bsa_attn_fwd_block_mask_output(*args, None, s4, 1, 1, 0.125, 0, 1, 1, 64, 64, None, None, None, None,
+                                              None) == -4
+    assert lib.bsa_attn_fwd_block_mask_output(*args, fake, s4, 1, 1, 0.125, 0, 1, 1, 63, 64, None, None, None, None,
+                                              None) == -1

@@ -434,3 +434,66 @@ def test_output_rows_on_16_byte_boundaries_only(lib):
     torch.cuda.synchronize()
     assert torch.equal(o_view, o_ref) and torch.equal(lse, lse_ref)
     assert not wide[..., :8].any()
+
+
+@pytest.mark.parametrize("nb", [1, 2, 5, 31, 33, 127, 128, 129, 200, 513])
+def test_mask_rows_at_every_alignment(lib, nb):
+    """The kernel lists a mask row four columns a lane from the 4-byte word that it begins in: rows that begin and
+    end at every byte of a word, the last columns of a pass and of the four passes that are fetched together,
+    and masks whose columns are not next to each other, against the lists of the list builder."""
+    from fa2_custom_mask import attention_forward, attention_forward_masked, build_tile_lists
+    q, k, v = (t.cuda() for t in oracle.make_qkv(1, 1, 64 * nb, 16, seed=nb, dtype=torch.float16))
+    g = torch.Generator().manual_seed(nb)
+    mask = (torch.rand(nb, nb, generator=g) < max(0.02, min(0.5, 8 / nb))).to(torch.uint8)
+    mask[0] = 0                       # an empty row, the edges of passes, the last column
+    for c in (0, 3, 4, 127, 128, 511, 512, nb - 1):
+        if c < nb:
+            mask[nb - 1, c] = 1
+    lists = build_tile_lists(mask.cuda().view(1, 1, nb, nb))
+    o_ref, lse_ref, _ = attention_forward(q, k, v, lists, 0.25)
+    wide = torch.full((nb, nb + 9), 7, dtype=torch.uint8, device="cuda")   # (what lies beside a row is not read as kept)
+    for off in range(5):
+        view = wide[:, off:off + nb]
+        view.copy_(mask)
+        o, lse2, _ = attention_forward_masked(q, k, v, view[None, None], 0.25)
+        assert torch.equal(o, o_ref) and torch.equal(lse2, lse_ref), off
+        wide.fill_(7)
+    apart = torch.full((nb, nb, 3), 7, dtype=torch.uint8, device="cuda")
+    apart[..., 1] = mask.cuda()
+    o, lse2, _ = attention_forward_masked(q, k, v, apart[None, None, ..., 1], 0.25)
+    assert torch.equal(o, o_ref) and torch.equal(lse2, lse_ref)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+def test_mask_forms_of_the_public_op(lib, dense):
+    """The op's native path reads the mask through its pointer and strides: masks of two to four axes, bytes and
+    booleans, expanded, transposed and cut out of larger ones give what the same mask as a tensor of its own does."""
+    from fa2_custom_mask import flash_attention_custom_mask
+    B, H, nb = 2, 3, 5
+    n = 64 * nb if dense else nb
+    q, k, v = (t.cuda() for t in oracle.make_qkv(B, H, 64 * nb, 64, seed=5, dtype=torch.float16))
+    g = torch.Generator().manual_seed(6)
+    full = (torch.rand(B, H, n, n, generator=g) < 0.5).cuda()
+    full |= torch.eye(n, dtype=torch.bool, device="cuda")
+
+    def whole(m):                      # the same mask, every axis there and nothing shared
+        while m.dim() < 4:
+            m = m[None]
+        return m.expand(B, H, n, n).contiguous()
+
+    big = torch.zeros(B, H, n + 3, n + 19, dtype=torch.bool, device="cuda")
+    big[:, :, 2:2 + n, 16:16 + n] = full
+    odd = torch.zeros(B, H, n, n + 1, dtype=torch.bool, device="cuda")
+    odd[..., 1:] = full
+    forms = [full[0, 0], full[0], full[:1], full[:, :1], full[0, 0].expand(B, H, n, n), full.transpose(-1, -2),
+             big[:, :, 2:2 + n, 16:16 + n], odd[..., 1:], full[0].transpose(0, 1).contiguous().transpose(0, 1)]
+    for i, m in enumerate(forms):
+        for form in (m, m.view(torch.uint8)):
+            with torch.no_grad():
+                got = flash_attention_custom_mask(q, k, v, form, 0.125)
+                want = flash_attention_custom_mask(q, k, v, whole(m), 0.125)
+            assert torch.equal(got, want), i
+            gq = q.clone().requires_grad_(True)
+            a, = torch.autograd.grad(flash_attention_custom_mask(gq, k, v, form, 0.125).float().sum(), gq)
+            b, = torch.autograd.grad(flash_attention_custom_mask(gq, k, v, whole(m), 0.125).float().sum(), gq)
+            assert torch.equal(a, b), i
