@@ -24,7 +24,8 @@
 // reference's causal loops.  dK and dQ carry the factor sm_scale.
 //
 // Persistent: one CTA per SM starts with block blockIdx.x and draws further blocks from an
-// optional work counter (or walks a fixed stride); long lists first when the mask is causal.
+// optional work counter (or walks a fixed stride); long lists first when the mask is causal.  dQ may run
+// beside dK/dV (see `together`).
 // Roles (26 warps):
 //   warps 0..15 : compute, two teams of eight warps on alternate supersteps (team = warp / 8, TMEM lane
 //                 quarter = warp % 4, 32 of a tile's 64 columns = (warp / 4) % 2), so that one team's
@@ -45,11 +46,12 @@
 // D-wide accumulating products.
 // S and dP of a superstep have one of three slots in TMEM, and P and dS are stored over them: the
 // next superstep but two is what its products must be complete for, not the team's own next one.
-// What bounds it: shared memory.  A dK/dV superstep takes about 1,000 of its port's cycles (S and dP
-// operands 384, accumulating operands 256, copies arriving 256, LSE2 and delta 128) of 1,250 to 1,340
-// in all, a dQ superstep 770 of 1,000; the exponentials take a third of it.  B=2, H=16, N=16384, 25 % of
-// the tiles under a causal mask, both kernels: 1,650 us with M=128 products and one team, 1,430 us with
-// separate S/dP and P/dS columns for each team, 1,347 us with slots and an issuer for each output.
+// What bounds it: the way of a superstep through three slots, with no part of it that is the bound alone.
+// A dK/dV superstep takes 1,200 to 1,290 cycles, of which shared memory's port about 1,000 (S and dP
+// operands 384, accumulating operands 256, copies arriving 256, LSE2 and delta 128), the tensor pipe 900, the
+// exponentials a third; a dQ superstep 960 (port 770).  B=2, H=16, N=16384, 25 % of the tiles under a
+// causal mask, both kernels back to back at the power cap: 1,326 us (1,380 with waits that vote and unrolled
+// loops).  Of 2 x 8 heads, N = 4160, that mask: 38.5 + 29.4 us (40.2 + 31.4).
 // Every wait is bounded and every barrier is waited on by warps that see each of its phases.
 #include <math.h>
 

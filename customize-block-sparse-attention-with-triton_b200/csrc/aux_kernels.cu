@@ -229,15 +229,16 @@ static int launch_reorder(const void* in, const int64_t s[4], void* out, const i
 // head-wise token reorder in place
 // ---------------------------------------------------------------------------------------------
 // One cluster of CTAs reorders one column chunk (64 bytes or more of every row) of one head: every CTA
-// gathers its share of the destination rows into registers, the cluster waits until all of it has been
+// gathers its share of the destination rows into shared memory, the cluster waits until all of it has been
 // read, and every CTA stores its share.  Bound by HBM: each byte is read once and written once, where a
-// gather into a second tensor and a copy back move it twice and allocate that tensor.  Registers hold
-// 72 KB a CTA, so that two CTAs share an SM and one's loads run under the other's stores; a cluster of
-// 16 holds 18,432 rows of 64 bytes, the reference's 13 x 30 x 45 grid among them.  More tokens than that
+// gather into a second tensor and a copy back move it twice and allocate that tensor.  Shared
+// memory holds 72 KB a CTA, so that three CTAs share an SM and one's loads run under the others' stores; a
+// cluster of 16 holds 18,432 rows of 64 bytes, the reference's 13 x 30 x 45 grid among them.  More tokens than that
 // are refused, and the caller goes back to the gather and the copy.
 // B200, D = 64, 16 bit, q, k, v and output of 2 x 48 heads of that grid, orders drawn from all six:
-// 0.69 -> 0.30 ms.  q, k, v alone, 5/6 of the heads with an order to move (1.08 GB read and written):
-// 0.49 -> 0.22 ms, 4.9 TB/s.  A grid of 16 x 33 x 47, too large, stays at 2.2 TB/s by that count.
+// 0.69 ms with the gather and the copy, 0.31 with the rows in registers (two CTAs an SM), 0.28 in shared
+// memory.  q, k, v alone, 5/6 of the heads with an order to move (1.08 GB read and written): 0.49, 0.22 and
+// 0.20 ms, 5.5 TB/s.  A grid of 16 x 33 x 47, too large, stays at 2.2 TB/s by that count.
 constexpr int kPermThreads = 512;
 constexpr int kPermPieces = 9;  // 16-byte pieces a thread holds
 constexpr int kPermTensors = 3;
