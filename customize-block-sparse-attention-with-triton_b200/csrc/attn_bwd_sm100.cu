@@ -52,7 +52,8 @@
 // exponentials a third; a dQ superstep 960 (port 770).  B=2, H=16, N=16384, 25 % of the tiles under a
 // causal mask, both kernels back to back at the power cap: 1,326 us (1,380 with waits that vote and unrolled
 // loops).  Of 2 x 8 heads, N = 4160, that mask: 38.5 + 29.4 us (40.2 + 31.4).
-// Every wait is bounded and every barrier is waited on by warps that see each of its phases.
+// Every wait is bounded, and a role that gives up raises a CTA-wide flag, which the others look at when they wait
+// for an item.  Every barrier is waited on by warps that see each of its phases.
 #include <math.h>
 
 #include "host_common.h"
@@ -107,6 +108,7 @@ struct BwdSmem {
   uint64_t d_free[kXBars];                  // accumulating MMAs that read P/dS complete: the slot is free
   uint64_t d_full[kSlots];                  // by slot: P/dS stored
   uint32_t tmem_base;
+  int abort_flag;                           // a role has given up
 };
 
 static_assert(sizeof(BwdSmem) + 1024 <= 232448, "BwdSmem exceeds the shared memory of one CTA");
@@ -135,11 +137,16 @@ struct BwdParams {
   int together;
 };
 
+__device__ __forceinline__ void bwd_give_up(BwdSmem* sm, int32_t* status, int code) {
+  sm->abort_flag = 1;
+  report_status(status, code);
+}
+
 // Readers of the item header: wait for item i, read it (the producer looked the list up, so the
 // other roles start an item without a round trip to memory), tell the producer the slot was read.
 __device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, int* w, int* n_tiles, int* begin) {
   const int par = i & 1;
-  if (!mbar_wait_warp(smem_u32(&sm->item_full[par]), (i >> 1) & 1)) return false;
+  if (!mbar_wait_warp_item(smem_u32(&sm->item_full[par]), (i >> 1) & 1, &sm->abort_flag)) return false;
   *w = *const_cast<volatile int*>(&sm->item[par]);
   *n_tiles = *const_cast<volatile int*>(&sm->item_tiles[par]);
   *begin = *const_cast<volatile int*>(&sm->item_begin[par]);
@@ -241,12 +248,13 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
     gs += n_super;
 #pragma unroll 1
     for (; ok && g < gs; g += 2) {
-      ok = mbar_wait_warp(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1) &&
-           mbar_wait_warp(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1);
-      if (!ok) break;
+      // (three looks, one vote)
+      bool seen = mbar_poll(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, kWaitTries);
+      seen &= mbar_poll(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, kWaitTries);
       // the accumulating products of the slot's previous superstep must be complete
       if (g >= kSlots)
-        ok = mbar_wait_warp(smem_u32(&sm->d_free[(g - kSlots) % kXBars]), ((g - kSlots) / kXBars) & 1);
+        seen &= mbar_poll(smem_u32(&sm->d_free[(g - kSlots) % kXBars]), ((g - kSlots) / kXBars) & 1, kWaitTries);
+      ok = __all_sync(0xffffffffu, seen);
       if (!ok) break;
       tc_fence_after();
       if (leader) {
@@ -271,7 +279,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
     if (ok && leader) tc_commit(smem_u32(&sm->stat_free[own]));  // this issuer is through with the operands
     ++ni;
   }
-  if (!ok) report_status(p.status, 2);
+  if (!ok) bwd_give_up(sm, p.status, 2);
 }
 
 // The accumulating instructions of one warp.  dK/dV: the first warp's sum dV, the second one's dK (each
@@ -330,7 +338,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
     }
     ++ni;
   }
-  if (!ok) report_status(p.status, 2);
+  if (!ok) bwd_give_up(sm, p.status, 2);
 }
 
 // Persistent: one CTA per SM.  The producer starts with item blockIdx.x and then draws further
@@ -379,6 +387,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     for (int s = 0; s < kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
     mbar_init(smem_u32(&sm->acc_done), 2);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
+    sm->abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == kXWarp) {
@@ -460,7 +469,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
                                                   sm->lse[0][0], p.lse2, it, n_super, lane, &gs);
         ++ni;
       }
-      if (!ok) report_status(p.status, 1);
+      if (!ok) bwd_give_up(sm, p.status, 1);
       if (!terminal && lane == 0) {
         // gave up before the last draw: draw on (without working) until this CTA's first ticket past
         // the end, so that the launch still draws `items` tickets and the counter returns to zero
@@ -495,7 +504,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
                                                   n_super, lane, &gs);
         ++ni;
       }
-      if (!ok) report_status(p.status, 1);
+      if (!ok) bwd_give_up(sm, p.status, 1);
     } else if (warp == kXWarp || warp == kX2Warp) {
       bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane);
     } else if (warp == kAccWarp || warp == kAcc2Warp) {
@@ -661,7 +670,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       // (the block's sums are merged and stored by the write-out warps; these warps go straight
       // on to the next block, whose first S/dP is usually complete already)
     }
-    if (!ok) report_status(p.status, 3);
+    if (!ok) bwd_give_up(sm, p.status, 3);
   } else {
     // =========================== write-out ===========================
     // Lane r of an accumulator holds the tile-a sums of row r of the CTA's block, lane r+64 its tile-b
@@ -766,7 +775,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       }
       if (any_failed) break;
     }
-    if (!ok) report_status(p.status, 3);
+    if (!ok) bwd_give_up(sm, p.status, 3);
   }
 
   // The next kernel may come as soon as a role of every CTA gets here, warps without a role at once: it waits

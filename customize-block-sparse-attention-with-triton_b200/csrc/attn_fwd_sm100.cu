@@ -67,8 +67,9 @@
 // goes into depends on its position in the row's list alone, so results do not depend on which CTA
 // computes an item.
 //
-// Every wait is bounded; a wait that gives up raises a CTA-wide flag, every role then falls
-// through its loops without touching barriers' data again, and TMEM is always released.  Every
+// Every wait is bounded.  A role that gives up leaves its loops and raises a CTA-wide flag, which the sleeping waits
+// and those for an item look at; a role in the middle of an item runs out by itself, within the same
+// 2 seconds or so.  TMEM is always released.  Every
 // barrier is waited on only by warps that see each of its phases, or that know the barrier to be
 // at most one phase behind (a parity wait cannot tell a phase from the one two before it).
 #include <math.h>
@@ -353,7 +354,7 @@ struct FwdWalk {
   int at = 0, ph = 0;  // list buffer, phase of its barrier
   int4 it;             // batch (< 0: no more work), head, query block, tile count
   __device__ __forceinline__ bool wait(FwdSmem* sm) {
-    if (!mbar_wait_warp(smem_u32(&sm->list_full[at]), ph)) return false;
+    if (!mbar_wait_warp_item(smem_u32(&sm->list_full[at]), ph, &sm->abort_flag)) return false;
     it = sm->item[at];
     return true;
   }
@@ -563,11 +564,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint64_t desc_q = desc_q0 + static_cast<uint64_t>(qpar) * kTileDesc;
 #pragma unroll 1
       for (int u = 0; u < n_super; ++u) {
-        ok = mbar_wait_warp(smem_u32(&sm->k_full[ks]), kph);
-        if (!ok) break;
+        // (two looks, one vote)
+        bool seen = mbar_poll(smem_u32(&sm->k_full[ks]), kph, kWaitTries);
         // the slot's previous user, three supersteps ago, must have had its P V completed (for the
         // first users this asks for the phase before the first one, which counts as complete)
-        ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), slot_ph);
+        seen &= mbar_poll(smem_u32(&sm->pv_done[slot]), slot_ph, kWaitTries);
+        ok = __all_sync(0xffffffffu, seen);
         if (!ok) break;
         tc_fence_after();
         if (leader) {
@@ -674,11 +676,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int n_super = (n_tiles + 3) >> 2;
       const uint16_t* cols = sm->cols[walk.at];
       float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
-      // this lane's row of the element-level mask, if there is one
-      const uint8_t* mask_row = nullptr;
-      if constexpr (kElementMask)
-        mask_row = p.dense + walk.it.x * p.ds0 + walk.it.y * p.ds1 +
-                   static_cast<int64_t>(walk.it.z * 64 + (quarter & 1) * 32 + lane) * p.ds2;
 
 #pragma unroll 1
       for (; next < g + n_super; next += 2) {
@@ -701,8 +698,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const auto masked = [&](uint32_t* sr, int col) {
             if constexpr (kElementMask) {
               const uint16_t entry = cols[4 * u + (col >> 6) * 2 + half];
-              if (entry & kColPartial)
+              if (entry & kColPartial) {
+                // (the row's address is worked out here: kept over the item's loop it has no registers)
+                const int4 it = sm->item[walk.at];
+                const uint8_t* mask_row = p.dense + it.x * p.ds0 + it.y * p.ds1 +
+                                          static_cast<int64_t>(it.z * 64 + (quarter & 1) * 32 + lane) * p.ds2;
                 mask_chunk(sr, mask_row + (entry & kColIndex) * 64 + (col & 32));
+              }
             }
           };
           uint32_t pk[64];

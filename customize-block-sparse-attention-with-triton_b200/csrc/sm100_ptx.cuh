@@ -117,23 +117,38 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait of a whole (converged) warp.  Returns false when it gave up: after kWaitTries tries, each of
-// which the hardware suspends for up to 4 us, 2 seconds in all.  On give-up the caller records the code and
-// leaves through the normal tear-down path so TMEM is always released.
-// (This code is inlined at every wait of every role and run through at every superstep, mostly on barriers
-// that are long complete: a loop with a look at a flag, a parked form of the wait and %globaltimer made
-// short lists 3 to 6 % slower, a vote on the verdict the backward 2 to 3 % and the forward 1 to 2 %.)
-constexpr int kWaitTries = 1 << 19;
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
-  int left = kWaitTries;
+// One lane's bounded look-out for the end of a phase.  False: it gave up, after so many tries, each of which the
+// hardware suspends for up to 4 us (75 ns when the lanes of a warp have parted).  Lanes may disagree and come back one by one: the warp has to vote on
+// the verdict before any other .sync.aligned instruction.
+constexpr int kWaitTries = 1 << 19;  // 2 seconds in all
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, int tries) {
 #pragma unroll 1
   while (!mbar_try_wait(bar, parity))
-    if (--left == 0) {
-      __syncwarp();
-      return false;
-    }
-  __syncwarp();  // together again before any .sync.aligned instruction
-  return true;
+    if (--tries == 0) break;
+  return tries != 0;
+}
+
+// Bounded wait of a whole (converged) warp, with one way out and one verdict for all of its lanes.  On give-up
+// the caller records the code, raises the CTA's flag and leaves through the normal tear-down path so TMEM is
+// always released.
+// (This code is inlined at every wait of every role and run through at every superstep, mostly on barriers
+// that are long complete.  Against a way out for each verdict and no vote, which lets lanes go on without
+// the others: forward 0.3 to 1 %, training steps 1 %.  A vote, a look at the flag, a parked form of
+// the wait or %globaltimer in every try cost 2 to 6 %, a look at the flag every 1024 tries 1 to 4 %.)
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int tries = kWaitTries) {
+  return __all_sync(0xffffffffu, mbar_poll(bar, parity, tries));
+}
+
+// The same for the beginning of an item, where a role comes that still had work when another one gave up: it
+// looks at the CTA's flag every quarter of a second.
+constexpr int kItemBatches = 8;
+__device__ __forceinline__ bool mbar_wait_warp_item(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+  for (int batch = 0; batch < kItemBatches; ++batch) {
+    if (mbar_wait_warp(bar, parity, kWaitTries / kItemBatches)) return true;
+    if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+  }
+  return false;
 }
 
 // Same, for roles that wait for a long time (a whole work item): sleeps between polls so that the

@@ -40,7 +40,50 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int32_t* status, i
   }
 }
 
+// What two warps make of a wait when half of their lanes look at a barrier that is complete and the others at
+// one that never will be: the second warp waits as for an item, and the first one raises the flag
+// after 20 ms; the third one makes all of its tries.
+__global__ void __launch_bounds__(96, 1) give_up_selftest_kernel(int32_t* report) {
+  __shared__ uint64_t bar[2];
+  __shared__ int abort_flag;
+  const int warp = uniform_warp_index();
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&bar[0]), 1);
+    mbar_init(smem_u32(&bar[1]), 1);
+    abort_flag = 0;
+    mbar_fence_init();
+    mbar_arrive(smem_u32(&bar[0]));
+  }
+  __syncthreads();
+  volatile int* flag = &abort_flag;
+  const uint64_t t0 = global_timer_ns();
+  if (warp == 0) {
+#pragma unroll 1
+    for (int i = 0; i < 20; ++i) __nanosleep(1000000u);  // (at most a millisecond each)
+    if (lane == 0) *flag = 1;
+  } else {
+    const bool ok = warp == 1 ? mbar_wait_warp_item(smem_u32(&bar[lane & 1]), 0, flag)
+                              : mbar_wait_warp(smem_u32(&bar[lane & 1]), 0);
+    const unsigned went_on = __ballot_sync(0xffffffffu, ok);
+    if (lane == 0) {
+      report[2 * warp - 2] = __popc(went_on);
+      report[2 * warp - 1] = static_cast<int32_t>((global_timer_ns() - t0) / 1000000ull);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) report[4] = 1;
+}
+
 }  // namespace bsa
+
+extern "C" int bsa_selftest_give_up(int32_t* report, void* stream) {
+  if (!report) return BSA_ERR_BAD_POINTER;
+  int rc;
+  if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
+  bsa::give_up_selftest_kernel<<<1, 96, 0, static_cast<cudaStream_t>(stream)>>>(report);
+  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
 
 extern "C" int bsa_selftest_bounded_wait(int32_t* status, int32_t* report, void* stream) {
   if (!report) return BSA_ERR_BAD_POINTER;

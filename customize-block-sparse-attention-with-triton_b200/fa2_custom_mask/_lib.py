@@ -79,6 +79,7 @@ SIGNATURES = {
     "bsa_static_warmup": [],
     "bsa_check_status": [_vp, _vp],
     "bsa_selftest_bounded_wait": [_vp, _vp, _vp],
+    "bsa_selftest_give_up": [_vp, _vp],
 }
 
 

@@ -419,6 +419,16 @@ int bsa_check_status(const int32_t* status, void* stream);
  */
 int bsa_selftest_bounded_wait(int32_t* status, int32_t* report, void* stream);
 
+/*
+ * Self-test of what follows a give-up; no reference counterpart.  Launches one small CTA in which half of the
+ * lanes of two warps wait on a barrier that is complete and half on one that never will be.  The first
+ * warp waits as the kernels' roles wait for their next work item and is released by the CTA's give-up flag,
+ * which is raised some 20 ms after the start; the second one makes all the tries that a wait has.
+ * `report` (device, 5 x int32) receives for each warp how many lanes took the wait for satisfied (none: a
+ * warp goes on or gives up as a whole) and the milliseconds until it had left, and [4] 1 at the end.
+ */
+int bsa_selftest_give_up(int32_t* report, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
