@@ -142,6 +142,15 @@ __device__ __forceinline__ void bwd_give_up(BwdSmem* sm, int32_t* status, int co
   report_status(status, code);
 }
 
+// At the beginning of every role.  The first item is published after the end of the kernel before, which may take
+// any time (one that lets its successor in early and then waits for a peer, say): a role's limited waits
+// begin when that has ended.  Together, dQ begins while dK/dV is still running: it is launched when all CTAs of
+// dK/dV have passed this point, so what came before dK/dV has ended.  It ends after dK/dV (see the end).
+template <bool kDKDV>
+__device__ __forceinline__ void bwd_begin(const BwdParams& p) {
+  if (kDKDV || !p.together) grid_dependency_wait();
+}
+
 // Readers of the item header: wait for item i, read it (the producer looked the list up, so the
 // other roles start an item without a round trip to memory), tell the producer the slot was read.
 __device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, int* w, int* n_tiles, int* begin) {
@@ -234,6 +243,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
   const int k_steps = p.D >> 4;
   bool ok = true;
   int gs = 0, ni = 0;
+  bwd_begin<kDKDV>(p);
 #pragma unroll 1
   for (int i = 0; ok; ++i) {
     int w, w_tiles, w_begin;
@@ -298,6 +308,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   bool ok = true;
   int ni = 0, place = 0, slot = 0, x = 0;
   uint32_t phase = 0;  // of the slot's barrier
+  bwd_begin<kDKDV>(p);
 #pragma unroll 1
   for (int i = 0; ok; ++i) {
     int w, w_tiles, w_begin;
@@ -412,11 +423,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       // =========================== TMA producer ===========================
       bool ok = true;
       bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
-      // Whatever touches memory that an earlier kernel may use comes after the first item's header, so one role
-      // waits for the end of that kernel while the others get as far as their first barrier.
-      // Together, dQ begins while dK/dV is still running: it is launched when all CTAs of dK/dV have passed
-      // this point, so what came before dK/dV has ended and is visible then.  It ends after dK/dV (see the end).
-      if (kDKDV || !p.together) grid_dependency_wait();
+      bwd_begin<kDKDV>(p);
+      // (by the role that has waited, and by no other: a warp without a role must not let dQ in)
       if (kDKDV && p.together) grid_dependents_launch();
       int gs = 0, ni = 0;
 #pragma unroll 1
@@ -483,6 +491,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       // =========================== second TMA producer ===========================
       bool ok = true;
       int gs = 0, ni = 0;
+      bwd_begin<kDKDV>(p);
 #pragma unroll 1
       for (int i = 0; ok; ++i) {
         int w, w_tiles, w_begin;
@@ -522,6 +531,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     const float c = p.scale_log2;
     bool ok = true;
     int gs = 0;  // supersteps of earlier items; this team takes those with gs % 2 == team
+    bwd_begin<kDKDV>(p);
 #pragma unroll 1
     for (int i = 0; ok; ++i) {
       int w, w_tiles, w_begin;
@@ -695,6 +705,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     const int col0 = kDKDV ? 0 : 32 * half;
     bool ok = true;
     int ni = 0;
+    bwd_begin<kDKDV>(p);
 #pragma unroll 1
     for (int i = 0;; ++i) {
       int w = 0, w_tiles = 1, w_begin = 0;

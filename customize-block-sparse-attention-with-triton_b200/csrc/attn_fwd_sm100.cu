@@ -353,6 +353,9 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
 struct FwdWalk {
   int at = 0, ph = 0;  // list buffer, phase of its barrier
   int4 it;             // batch (< 0: no more work), head, query block, tile count
+  // The first item is published after the end of the kernel before, which may take any time (one that lets its
+  // successor in early and then waits for a peer, say): a role's limited waits begin when that has ended.
+  __device__ __forceinline__ FwdWalk() { grid_dependency_wait(); }
   __device__ __forceinline__ bool wait(FwdSmem* sm) {
     if (!mbar_wait_warp_item(smem_u32(&sm->list_full[at]), ph, &sm->abort_flag)) return false;
     it = sm->item[at];

@@ -75,7 +75,24 @@ __global__ void __launch_bounds__(96, 1) give_up_selftest_kernel(int32_t* report
   if (threadIdx.x == 0) report[4] = 1;
 }
 
+// Lets its dependents in at once and ends after so many milliseconds.
+__global__ void __launch_bounds__(32, 1) early_selftest_kernel(int milliseconds) {
+  grid_dependents_launch();
+  const uint64_t t0 = global_timer_ns();
+#pragma unroll 1
+  for (int i = 0; i < 100 * milliseconds && global_timer_ns() - t0 < 1000000ull * milliseconds; ++i)
+    __nanosleep(100000u);
+}
+
 }  // namespace bsa
+
+extern "C" int bsa_selftest_early_kernel(int milliseconds, void* stream) {
+  if (milliseconds < 0 || milliseconds > 10000) return BSA_ERR_BAD_SHAPE;
+  int rc;
+  if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
+  bsa::early_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(milliseconds);
+  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
 
 extern "C" int bsa_selftest_give_up(int32_t* report, void* stream) {
   if (!report) return BSA_ERR_BAD_POINTER;

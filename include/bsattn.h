@@ -429,6 +429,14 @@ int bsa_selftest_bounded_wait(int32_t* status, int32_t* report, void* stream);
  */
 int bsa_selftest_give_up(int32_t* report, void* stream);
 
+/*
+ * For tests; no reference counterpart.  Launches one warp that lets the kernel behind it in the stream begin at
+ * once and sleeps for so many milliseconds (0 to 10,000).  The kernels of this library may begin while the
+ * kernel before them is still running, and their waits are limited (BSA_ERR_DEVICE_TIMEOUT): the limit counts
+ * from the end of that kernel on, however long it takes.
+ */
+int bsa_selftest_early_kernel(int milliseconds, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from oracle import oracle
+
 pytestmark = pytest.mark.gpu
 
 
@@ -15,3 +17,28 @@ def test_a_warp_gives_up_as_a_whole_and_an_items_wait_with_the_flag(lib):
     with_flag, ms_flag, alone, ms_alone, ended = report.cpu().tolist()
     assert with_flag == 0 and alone == 0 and ended == 1
     assert ms_flag < 1000 and ms_alone <= 10000
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_a_long_kernel_ahead_that_lets_us_in_early_is_waited_for(lib, train):
+    """5.5 s, more than any wait's own limit (2^33 cycles for the sleeping ones, 4.4 s at 1.965 GHz): results as
+    without that kernel, and nothing is reported.  Training: ahead of the forward and of the backward."""
+    from fa2_custom_mask import _lib, flash_attention_custom_mask
+    q, k, v, do = (t.cuda() for t in oracle.make_qkv(1, 2, 640, 64, seed=61, dtype=torch.float16, n=4))
+    mask = oracle.make_block_mask(1, 2, 10, 0.5, seed=61).cuda()
+    qkv = [t.requires_grad_(train) for t in (q, k, v)]
+    stream = _lib.stream_ptr(q.device)
+
+    def run(ms):
+        assert lib.bsa_selftest_early_kernel(ms, stream) == 0
+        o = flash_attention_custom_mask(*qkv, mask, 0.125)
+        if not train:
+            return [o]
+        assert lib.bsa_selftest_early_kernel(ms, stream) == 0
+        return [o, *torch.autograd.grad(o, qkv, do)]
+
+    want, got = run(0), run(5500)
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
+    assert all(torch.equal(g, w) for g, w in zip(run(0), want))  # (raises what was reported)
+    torch.cuda.synchronize()
