@@ -97,6 +97,7 @@ constexpr float kRescaleThreshold = 8.0f;
 // Largest sum of a row's probabilities in a superstep (hence largest probability) that may go into P
 // against a reference maximum that was not checked: far below fp16's 65504.
 constexpr float kMaxRowSum = 4096.0f;
+constexpr int kFrontRounds = 4, kFrontRows = 8;  // see fwd_item
 constexpr int kFwdMaxTiles = 2048;  // key blocks per row that a CTA can list (N <= 131072)
 constexpr uint16_t kColPartial = 0x8000;  // list entry in shared memory: the tile has masked elements
 constexpr uint16_t kColIndex = 0x7fff;
@@ -149,6 +150,7 @@ struct FwdParams {
   float scale_log2;
   int32_t* status;
   int32_t* ticket;          // optional work counter (0 at kernel start, left 0): dynamic item hand-out
+  int front, front_items;   // so many first rows of every head come before all others
   int wide_stores;          // rows of O start on 32-byte boundaries
   int successor_early;      // what follows in the stream may begin before this kernel ends, and knows it
 };
@@ -251,14 +253,24 @@ __device__ __forceinline__ void fwd_rescale(uint32_t o_addr, float alpha) {
   }
 }
 
-// Work item w -> (batch, head, query block); late (long, if causal) query blocks of a head first.
+// Work item w -> (batch, head, query block).  Late (long, if causal) query blocks of a head come first, but where a
+// CTA has few items (kFrontRounds at most) the first kFrontRows query blocks of every head come before all
+// others: those of global tokens keep everything, and a kernel ends with the CTA that draws a long item last.
+// Where they are short it makes no difference.  (With many items it matters less, and heads beside one another
+// would share the L2 cache.)  B200, public calls, with / without: two heads, 30 % of the blocks, the first 8 query
+// blocks full, N = 9600 31.8 / 46.8 us, N = 14976 63.1 / 84.0; all rows alike, a tenth, 15.3 / 15.4 and 25.6 / 25.3;
+// N = 6400, 4 heads, causal, a quarter 17.1 / 17.2.  All heads' blocks in turn: 15.8 and 26.4.
+// (An order by length, which every CTA has to work out: 41.3 and 65.5; all rows alike 19.3 and 35.7.  That one
+// also found long rows elsewhere, 8 evenly spread at N = 9600: 41.5, with this order 46.0.  Columns of items, the
+// longest first, read at every draw: 33.3 there, all rows alike 18.5 and 29.0.)
 struct FwdItem {
   int b, h, mb;
 };
 __device__ __forceinline__ FwdItem fwd_item(int w, const FwdParams& p) {
-  const int bh = w / p.nrows;
+  const int late = w - p.front_items;  // >= 0: not one of the front ones
+  const int each = late < 0 ? p.front : p.nrows - p.front, bh = (late < 0 ? w : late) / each;
   FwdItem it;
-  it.mb = p.row_begin + p.nrows - 1 - (w - bh * p.nrows);
+  it.mb = p.row_begin + (late < 0 ? w - bh * each : p.nrows - 1 - (late - bh * each));
   it.b = bh / p.H;
   it.h = bh - it.b * p.H;
   return it;
@@ -1074,6 +1086,9 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
                   : (dtype == BSA_BF16 ? attn_fwd_kernel<true, false> : attn_fwd_kernel<false, false>);
   if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes)) != BSA_OK)
     return rc;
+  // (no more than an eighth of a head's rows: front < nrows)
+  prm.front = prm.items > sms && prm.items <= kFrontRounds * sms ? (nrows / 8 < kFrontRows ? nrows / 8 : kFrontRows) : 0;
+  prm.front_items = B * H * prm.front;
   const dim3 grid(static_cast<unsigned>(prm.items < sms ? prm.items : sms));  // one CTA per SM
   return launch_dependent(kern, grid, kFwdThreads, smem_bytes, static_cast<cudaStream_t>(stream), tm_q, tm_k,
                           tm_v, prm);
