@@ -76,18 +76,24 @@ StreamState* stream_state(int device, cudaStream_t stream) {
   return last = it->second;
 }
 
-// The work counter for a call on `blocks` blocks; none when a CTA has one of them at most.  A captured call
-// may be replayed on any stream, beside calls on this one, and two kernels must not draw from one counter:
-// it gets a word of its own (*own, out of the graph's memory, zeroed by every replay).  B200, replayed
-// calls with this stream's counter / a zeroed word / none: forward of one head, N = 17536, a tenth of the
-// blocks 21 / 23 / 24 us; forward and backward of 4 heads, N = 6400, causal, a quarter 68 / 72 / 83 us.
-int32_t* work_counter(StreamState* state, int64_t blocks, const at::TensorOptions& options, Tensor* own,
-                      bool dq = false) {
-  if (blocks <= at::cuda::getDeviceProperties(options.device().index())->multiProcessorCount) return nullptr;
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
-    return !state ? nullptr : dq ? state->dq_counter_ptr : state->counter_ptr;
-  *own = at::zeros({1}, options.dtype(at::kInt));
-  return own->mutable_data_ptr<int32_t>();
+// The work counters of a call's n kernels (two: dK/dV's and dQ's) for `blocks` blocks; none when a CTA has one of
+// them at most.  A captured call may be replayed on any stream, beside calls on this one, and two kernels must
+// not draw from one counter: it gets words of its own (*own, out of the graph's memory, zeroed by one node of
+// the graph).  B200, replayed calls with this stream's counter / zeroed words / none: forward of one head,
+// N = 17536, a tenth of the blocks 20.5 / 22.0 / 22.5 us; forward and backward of 4 heads, N = 6400, causal, a
+// quarter 65.5 / 67.6 / 67.6 us (67.8 with a node for each word).
+void work_counters(StreamState* state, int64_t blocks, const at::TensorOptions& options, int n, Tensor* own,
+                   int32_t** counters) {
+  for (int i = 0; i < n; ++i) counters[i] = nullptr;
+  if (blocks <= at::cuda::getDeviceProperties(options.device().index())->multiProcessorCount) return;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+    if (state == nullptr) return;
+    counters[0] = state->counter_ptr;
+    if (n > 1) counters[1] = state->dq_counter_ptr;
+    return;
+  }
+  *own = at::zeros({n}, options.dtype(at::kInt));
+  for (int i = 0; i < n; ++i) counters[i] = own->mutable_data_ptr<int32_t>() + i;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -177,7 +183,8 @@ bool run_forward(const Tensor& q, const Tensor& k, const Tensor& v, const Mask& 
   const int64_t B = q.size(0), H = q.size(1), N = q.size(2), D = q.size(3);
   *o = at::empty({B, H, N, D}, q.options());
   Tensor own;
-  int32_t* counter = work_counter(state, B * H * (N / kBlock), q.options(), &own);
+  int32_t* counter;
+  work_counters(state, B * H * (N / kBlock), q.options(), 1, &own, &counter);
   int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
   const int64_t* dense_strides = m.dense_ptr ? m.dense_strides : nullptr;
   if (lists == nullptr)
@@ -257,9 +264,9 @@ struct AttentionBackward : torch::autograd::Node {
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream(q.device().index());
     StreamState* state = stream_state(q.device().index(), stream);
     raise_if_reported(state);
-    Tensor own, dq_own;
-    int32_t* counter = work_counter(state, B * H * nb, q.options(), &own);
-    int32_t* dq_counter = work_counter(state, B * H * nb, q.options(), &dq_own, true);
+    Tensor own;
+    int32_t* counters[2];
+    work_counters(state, B * H * nb, q.options(), 2, &own, counters);
     int32_t* status = state ? const_cast<int32_t*>(state->word) : nullptr;
     // the gradients are laid out like the tensors they belong to, gaps included
     const auto like = [](const Tensor& t) { return at::empty_strided(t.sizes(), t.strides(), t.options()); };
@@ -278,8 +285,8 @@ struct AttentionBackward : torch::autograd::Node {
               v.const_data_ptr(), v.strides().data(), dout.const_data_ptr(), dout.strides().data(), lse_p,
               delta_p, dq.mutable_data_ptr(), dq.strides().data(), dk.mutable_data_ptr(), dk.strides().data(),
               dv.mutable_data_ptr(), dv.strides().data(), p, p + at.col_idx, p + at.col_cnt, p + at.row_idx, nb, sb,
-              sh, scale, code, B, H, N, D, dense_ptr, dense_ptr ? dense_strides : nullptr, counter, dq_counter, status,
-              stream));
+              sh, scale, code, B, H, N, D, dense_ptr, dense_ptr ? dense_strides : nullptr, counters[0], counters[1],
+              status, stream));
     return {dq, dk, dv};
   }
 };

@@ -1,4 +1,6 @@
 """What the native host path of the public op takes, and what it has to leave to the general one."""
+import ctypes
+
 import pytest
 import torch
 
@@ -125,6 +127,36 @@ def test_a_captured_call_does_not_draw_from_its_streams_counter(lib, native):
     for res in (got, *eager):
         assert all(torch.equal(g, w) for g, w in zip(res, want))
     assert int(counter.item()) == 0
+
+
+def test_a_captured_step_zeroes_its_counters_once_for_each_direction(lib):
+    """With more blocks than SMs a graph has two nodes more than with fewer: one for the forward's work counter
+    and one for both of the backward's."""
+    from fa2_custom_mask import flash_attention_custom_mask as op
+
+    def nodes(H):
+        q, k, v, do = (t.cuda() for t in oracle.make_qkv(1, H, 4096, 64, seed=53, dtype=torch.float16, n=4))
+        mask = oracle.make_block_mask(1, H, 64, 0.2, seed=53).cuda()
+        for t in (q, k, v):
+            t.requires_grad_(True)
+
+        def step():
+            o = op(q, k, v, mask, 0.125)
+            return [o.detach(), *torch.autograd.grad(o, (q, k, v), do)]
+
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            step()
+            s.synchronize()
+            graph = torch.cuda.CUDAGraph(keep_graph=True)
+            with torch.cuda.graph(graph, stream=s):
+                step()
+        n = ctypes.c_size_t()
+        assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None,
+                                                           ctypes.byref(n)) == 0
+        return n.value
+
+    assert nodes(4) == nodes(2) + 2      # 256 and 128 blocks for 148 CTAs
 
 
 def _layouts(dtype, N, D):
