@@ -145,7 +145,8 @@ __device__ __forceinline__ void bwd_give_up(BwdSmem* sm, int32_t* status, int co
 // At the beginning of every role.  The first item is published after the end of the kernel before, which may take
 // any time (one that lets its successor in early and then waits for a peer, say): a role's limited waits
 // begin when that has ended.  Together, dQ begins while dK/dV is still running: it is launched when all CTAs of
-// dK/dV have passed this point, so what came before dK/dV has ended.  It ends after dK/dV (see the end).
+// dK/dV have passed this point, so what came before dK/dV has ended.  (That dQ sees it without a wait of its
+// own is observed, not promised: see grid_dependency_wait.)  It ends after dK/dV (see the end).
 template <bool kDKDV>
 __device__ __forceinline__ void bwd_begin(const BwdParams& p) {
   if (kDKDV || !p.together) grid_dependency_wait();

@@ -93,7 +93,8 @@ struct ListArgs {
   int32_t* ent[2];
   int32_t* groups;
   int32_t* meta;
-  int together;  // runs beside the kernel before it in the stream, which has seen the mask finished
+  int together;  // runs beside the kernel before it in the stream, which has seen the mask finished (that this
+                 // one then sees it without a wait of its own is observed, not promised: grid_dependency_wait)
 };
 
 constexpr int kListThreads = 256;

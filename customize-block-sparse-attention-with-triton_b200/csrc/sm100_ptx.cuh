@@ -60,10 +60,15 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool pred)
   return out != 0;
 }
 
-// Programmatic dependent launch: every kernel of this library is launched so that it may begin while
-// the previous kernel of the stream is still running, does its set-up, and waits here, before it touches
-// memory that another kernel may write or read, until that one has ended and its writes are visible.
-// (Without the attribute on the launch both are no-ops.)
+// Programmatic dependent launch: the attention kernels, delta, the lists with places and the in-place reorder are
+// launched so that they may begin while the previous kernel of the stream is still running, do their set-up,
+// and wait here, in every role, before they touch memory that another kernel may write or read, until that one
+// has ended and its writes are visible.  (The mask reduction, the CSR lists and the out-of-place reorder are
+// ordinary launches; without the attribute on the launch both instructions are no-ops.)
+// Two kernels read before they wait: dQ beside dK/dV, and the tile lists of a training forward beside the forward.
+// What they read was written before the kernel that they run beside, which lets them in from a thread that has
+// itself waited for those writes.  That they see them too holds on B200 (steps on new data in the same buffers,
+// called and replayed, are tested bit for bit); the programming model promises it only after a wait of their own.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -256,3 +256,32 @@ def test_kernels_that_run_beside_one_another_see_what_they_need(lib, B, H, N, re
             torch.cuda.synchronize()
             for got, ref in zip(outs, [o, *attention_backward(q, k, v, o, lse2, bufs[3], lists, 0.125)]):
                 assert torch.equal(got, ref)
+
+
+def test_both_work_counters_of_a_backward_are_left_at_zero(lib):
+    """dK/dV and dQ of one call draw from counters of their own (256 blocks for 148 CTAs); a second call on the
+    same words gives the same bits."""
+    import ctypes
+
+    from fa2_custom_mask import _lib, attention_backward, attention_forward, build_tile_lists
+    B, H, N = 1, 4, 4096
+    q, k, v, do = (t.cuda() for t in oracle.make_qkv(B, H, N, 64, seed=37, dtype=torch.float16, n=4))
+    lists = build_tile_lists(oracle.make_block_mask(B, H, N // 64, 0.2, seed=37).cuda())
+    o, lse2, _ = attention_forward(q, k, v, lists, 0.125)
+    want = attention_backward(q, k, v, o, lse2, do, lists, 0.125)
+    delta = torch.empty_like(lse2)
+    counters = torch.zeros(2, dtype=torch.int32, device="cuda")
+    s4, stream = _lib.strides4(q), _lib.stream_ptr(q.device)
+    sb, sh = lists.list_strides(B, H)
+    p = _lib.ptr
+    _lib.check("delta", lib.bsa_attn_bwd_delta_strided(p(o), s4, p(do), s4, p(delta), 0, B, H, N, 64, stream))
+    for _ in range(2):
+        got = [torch.empty_like(q) for _ in range(3)]
+        dq, dk, dv = got
+        _lib.check("backward", lib.bsa_attn_bwd_strided(
+            p(q), s4, p(k), s4, p(v), s4, p(do), s4, p(lse2), p(delta), p(dq), s4, p(dk), s4, p(dv), s4,
+            p(lists.row_ptr), p(lists.col_idx), p(lists.col_ptr), p(lists.row_idx), 0, sb, sh, 0.125, 0, B, H, N, 64,
+            None, None, p(counters), ctypes.c_void_p(counters.data_ptr() + 4), None, stream))
+        torch.cuda.synchronize()
+        assert counters.tolist() == [0, 0]
+        assert all(torch.equal(g, w) for g, w in zip(got, want))
