@@ -101,8 +101,8 @@ struct BwdSmem {
   // a place's tiles have landed: one barrier for each place and team, so that the team's issuer and
   // compute warps, which wait on it, see each of its phases
   uint64_t in_full0[2 * kRing0<false>], in_full1[2 * kRing1<true>];
-  uint64_t in_empty0[kRing0<false>];        // accumulating MMAs that read the place complete
-  uint64_t in_empty1[kRing1<true>];         // ... (dQ: dP complete)
+  uint64_t in_empty0[kRing0<false>];        // dQ: accumulating MMAs that read the place of K complete
+  uint64_t in_empty1[kRing1<false>];        // dQ: dP complete, the place of V is free (dK/dV goes by d_free)
   // by superstep modulo kXBars, that is by slot and team:
   uint64_t x_full[kXBars];                  // S/dP complete (dK/dV: and LSE2 and delta there)
   uint64_t d_free[kXBars];                  // accumulating MMAs that read P/dS complete: the slot is free
@@ -304,7 +304,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   const bool leader = elect_one();
   const int places = dv ? kRing1<kDKDV> : kRing0<kDKDV>;
   const uint64_t desc = smem_desc_sw128(smem_u32(sm->ring[dv ? kRing0<kDKDV> : 0][0]), 8192, 1024);
-  const uint32_t empty = smem_u32(dv ? sm->in_empty1 : sm->in_empty0);
+  const uint32_t empty = smem_u32(sm->in_empty0);  // (dQ)
   const uint32_t acc = tmem + (dv ? kTmAcc0 : kTmAcc1), from = tmem + (dv ? 0 : 64);
   bool ok = true;
   int ni = 0, place = 0, slot = 0, x = 0;
@@ -393,10 +393,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     for (int s = 0; s < 2 * kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_full0[s]), 1);
 #pragma unroll 1
     for (int s = 0; s < 2 * kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_full1[s]), 1);
+    if constexpr (!kDKDV) {
 #pragma unroll 1
-    for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), kDKDV ? 1 : 2);
+      for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), 2);
 #pragma unroll 1
-    for (int s = 0; s < kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
+      for (int s = 0; s < kRing1<false>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
+    }
     mbar_init(smem_u32(&sm->acc_done), 2);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
     sm->abort_flag = 0;

@@ -282,9 +282,10 @@ __device__ __forceinline__ const uint8_t* fwd_mask_row(const FwdItem& it, const 
          static_cast<int64_t>(it.mb) * p.ms2;
 }
 
-// The bytes of a contiguous mask row of nb bytes as 0xff (kept) or 0, four columns at a time: those of the
-// 4-byte word of memory `word` words behind the one that the row begins in.  Columns that are none give 0,
-// and a word without a column of the row is not read.
+// The bytes of a contiguous mask row of nb bytes, four columns at a time: those of the 4-byte word of memory
+// `word` words behind the one that the row begins in.  Columns that are none give 0, and a word without a column of
+// the row is not read.  (So the first and the last word of a row may reach three bytes beyond it, and beyond the
+// caller's mask; an aligned word never reaches beyond what was allocated, and the C interface says so.)
 __device__ __forceinline__ uint32_t fwd_row_word(const uint8_t* row, int nb, int word) {
   const int off = static_cast<int>(reinterpret_cast<uintptr_t>(row) & 3u), c = 4 * word - off;
   uint32_t v = 0u;
@@ -312,11 +313,11 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
 #pragma unroll
       for (int j = 0; j < 4; ++j) next[j] = fwd_row_word(mrow, p.nb, 32 * j + lane);
 #pragma unroll 1
-      for (int w = lane; 4 * (w - lane) < p.nb + off; w += 32) {
+      for (int i = lane; 4 * (i - lane) < p.nb + off; i += 32) {
         const uint32_t v = next[0];
 #pragma unroll
         for (int j = 0; j < 3; ++j) next[j] = next[j + 1];
-        next[3] = fwd_row_word(mrow, p.nb, w + 128);
+        next[3] = fwd_row_word(mrow, p.nb, i + 128);
         uint16_t* out = cols + n_tiles;
         uint32_t kept[4];
 #pragma unroll
@@ -328,7 +329,7 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint32_t byte = v >> (8 * j) & 0xffu;
-          if (byte != 0) *out++ = static_cast<uint16_t>((4 * w - off + j) | (kElementMask && byte == 2 ? kColPartial : 0));
+          if (byte != 0) *out++ = static_cast<uint16_t>((4 * i - off + j) | (kElementMask && byte == 2 ? kColPartial : 0));
         }
       }
     } else {

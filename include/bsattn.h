@@ -184,6 +184,8 @@ int bsa_attn_fwd_block_mask(const void* q, const int64_t q_strides[4], const voi
  *           get o = 0 and lse2 = -inf.  Without it every listed tile is attended in full, as in
  *           the reference kernel.
  * bsa_attn_fwd / bsa_attn_fwd_block_mask are these with the range [0, N/64) and no dense mask.
+ * A block mask with unit inner stride is read in aligned 4-byte words, those that hold a byte of a row: up to three
+ * bytes before and behind a row are read (and ignored), also at the ends of the mask.
  */
 int bsa_attn_fwd_rows(const void* q, const int64_t q_strides[4], const void* k,
                       const int64_t k_strides[4], const void* v, const int64_t v_strides[4], void* o,
