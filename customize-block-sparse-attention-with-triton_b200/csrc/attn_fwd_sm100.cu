@@ -453,10 +453,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   volatile int* abort_flag = &sm->abort_flag;
 
   // 512 threads are launched with 128 registers: the softmax warps, which hold 64 logits and 128
-  // probabilities each, take what the others do without (2 x 168 + 72 + 104 = 4 x 128).  A spill in their
-  // loop (28 bytes at 160) made the kernel 4 to 5 % slower.
+  // probabilities each, take what the others do without (2 x 168 + 72 + 104 = 4 x 128; with an element mask, whose
+  // row and bytes they hold as well, 2 x 184 + 56 + 88).  A spill in their loop (28 bytes at 160; 112 with
+  // an element mask at 168) made the kernel 4 to 5 % slower: causal by element, 10 heads, N = 2048 18.9 / 17.3 us,
+  // a dense mask of whole blocks, one head, N = 6400 19.0 / 18.6.
   if (warp >= kSoftmaxWarps && warp < kSoftmaxWarps + 4) {
-  give_registers<72>();
+  give_registers<kElementMask ? 56 : 72>();
   if (warp == kProducerWarp) {
     // =========================== K producer ===========================
     bool ok = true;
@@ -669,7 +671,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   } else if (warp < kSoftmaxWarps) {
     // =========================== softmax ===========================
-    take_registers<168>();
+    take_registers<kElementMask ? 184 : 168>();
     const int team = warp >> 2;
     const int quarter = warp & 3;     // TMEM lane quarter this warp may touch
     const int half = quarter >> 1;    // lanes 0..63 own tiles a, c of a superstep, 64..127 b, d
@@ -692,6 +694,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int n_super = (n_tiles + 3) >> 2;
       const uint16_t* cols = sm->cols[walk.at];
       float m_ref = -INFINITY, m_true = -INFINITY, l = 0.f;
+      // this lane's row of the element-level mask, if there is one
+      const uint8_t* mask_row = nullptr;
+      if constexpr (kElementMask)
+        mask_row = p.dense + walk.it.x * p.ds0 + walk.it.y * p.ds1 +
+                   static_cast<int64_t>(walk.it.z * 64 + (quarter & 1) * 32 + lane) * p.ds2;
 
 #pragma unroll 1
       for (; next < g + n_super; next += 2) {
@@ -714,13 +721,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const auto masked = [&](uint32_t* sr, int col) {
             if constexpr (kElementMask) {
               const uint16_t entry = cols[4 * u + (col >> 6) * 2 + half];
-              if (entry & kColPartial) {
-                // (the row's address is worked out here: kept over the item's loop it has no registers)
-                const int4 it = sm->item[walk.at];
-                const uint8_t* mask_row = p.dense + it.x * p.ds0 + it.y * p.ds1 +
-                                          static_cast<int64_t>(it.z * 64 + (quarter & 1) * 32 + lane) * p.ds2;
+              if (entry & kColPartial)
                 mask_chunk(sr, mask_row + (entry & kColIndex) * 64 + (col & 32));
-              }
             }
           };
           uint32_t pk[64];
@@ -823,7 +825,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     //
     // One of the four warps is also the lister: it sets up item i+1 when the producer says so during item i,
     // i.e. between its write-outs of items i-1 and i (the CTA's first item at the very beginning).
-    give_registers<104>();
+    give_registers<kElementMask ? 88 : 104>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
     const bool lister = warp == kListerWarp;
     bool ok = true;
