@@ -50,8 +50,9 @@
 // A dK/dV superstep takes 1,200 to 1,290 cycles, of which shared memory's port about 1,000 (S and dP
 // operands 384, accumulating operands 256, copies arriving 256, LSE2 and delta 128), the tensor pipe 900, the
 // exponentials a third; a dQ superstep 960 (port 770).  B=2, H=16, N=16384, 25 % of the tiles under a
-// causal mask, both kernels back to back at the power cap: 1,326 us (1,380 with waits that vote and unrolled
-// loops).  Of 2 x 8 heads, N = 4160, that mask: 38.5 + 29.4 us (40.2 + 31.4).
+// causal mask, both kernels back to back at the power cap: 1,348 us (1,356 with a vote in every try of a wait and
+// unrolled loops; 1,325 with waits that lanes leave one by one, which is not sound).  Of 2 x 8 heads, N = 4160,
+// with such a mask each: 47.7 + 35.9 us (48.2 + 36.8; 46.7 + 35.2).
 // Every wait is bounded, and a role that gives up raises a CTA-wide flag, which the others look at when they wait
 // for an item.  Every barrier is waited on by warps that see each of its phases.
 #include <math.h>

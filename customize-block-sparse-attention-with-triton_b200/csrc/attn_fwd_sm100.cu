@@ -21,7 +21,7 @@
 // the probabilities go over the logits of their slot, which is held from the S product until P V
 // is complete.
 //
-// What bounds it: with everything listed a tile takes 334 active SM cycles, of which the exp2 unit
+// What bounds it: with everything listed a tile takes 336 active SM cycles, of which the exp2 unit
 // is busy 256 (4096 exponentials at 16 per cycle; a loop of nothing but loads, exponentials and
 // stores, two warps per sub-partition, measures 281); what is left are hand-overs between the
 // roles: a look at a barrier that is long complete costs its role 150 to 250 cycles, and the P V
@@ -30,8 +30,8 @@
 // unrolled by the compiler; 55 KB now) the instruction caches of a GPC were 73 % busy.  So what is executed
 // per item or per superstep is kept short, waits included, and no loop is unrolled without a reason.
 // B200, D = 64, public calls back to back on inputs that rotate: fp16 N = 17536 with one head, all blocks
-// 114 us (117 with a P V issuer of three waits and unrolled loops), a tenth of them 18.5 us (19.8); 8 heads, a
-// tenth 110 us (119); bf16 N = 32000, 32 heads, a tenth 1.27 ms (1.29), at the power cap.
+// 116.5 us (118.4 with a P V issuer of three waits and unrolled loops, in turn on one GPU), a tenth of them 18.5 us
+// (19.6); 8 heads, a tenth 112.6 us (118.9); bf16 N = 32000, 32 heads, a tenth 1.295 ms (1.310), at the power cap.
 //
 // Roles (16 warps); every role walks the same item sequence, so set-up of item i+1 and write-out
 // of item i-1 overlap the arithmetic of item i:

@@ -138,7 +138,7 @@ __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, int tri
 // always released.
 // (This code is inlined at every wait of every role and run through at every superstep, mostly on barriers
 // that are long complete.  Against a way out for each verdict and no vote, which lets lanes go on without
-// the others: forward 0.3 to 1 %, training steps 1 %.  A vote, a look at the flag, a parked form of
+// the others: forward 0.3 to 1 %, training steps 1 to 2 %.  A vote, a look at the flag, a parked form of
 // the wait or %globaltimer in every try cost 2 to 6 %, a look at the flag every 1024 tries 1 to 4 %.)
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int tries = kWaitTries) {
   return __all_sync(0xffffffffu, mbar_poll(bar, parity, tries));
