@@ -11,10 +11,11 @@
 // form of the MMA puts columns [0, 128) of its result into lanes 0..63 and columns [128, 256) into
 // lanes 64..127 of the same 128 TMEM columns, which is just the split above.  (An M = 128
 // instruction can only fill the lanes that way with half of its rows multiplied by zeros.)  P V
-// writes the accumulator rows of the lanes that own the tile and leaves the others alone, so the
-// other lanes' P columns need no zeros either.  Measured on one SM, in cycles per tile: S 80 (128
-// with the M = 128 form, both bound by the operand reads from shared memory at 128 B per cycle),
-// P V 128 (any form), S and P V issued together 210 (259).
+// takes tiles a and b, then c and d, in one product each: in the same form every lane half multiplies its own P
+// with its own half of the columns of [V_a | V_b].  A pair whose second tile does not exist has zeros in its place, in P
+// and in V.  Measured on one SM, in cycles per tile: S 80 (128 with the M = 128 form, both bound by the operand
+// reads from shared memory at 128 B per cycle), P V 88 (128 as two M = 128 products with half of the lanes
+// switched off each).
 //
 // The supersteps alternate between two softmax teams of four warps, each with its own accumulator,
 // so that one team exponentiates while the other waits for its products.  Three S slots rotate;
@@ -43,8 +44,8 @@
 //                 superstages (4 tiles, held until S is complete), one lane per tile, and tells the lister
 //                 when to set up the next item
 //   warp 9      : S issuer and TMEM owner
-//   warp 10     : P V issuer — O[team] += P_t V_t for the tiles t of the superstep.  P is read from
-//                 TMEM, V is an MN-major shared-memory operand.  Row r of an accumulator sums products
+//   warp 10     : P V issuer — O[team] += P_t V_t for the tiles t of the superstep, two at a time.  P is read
+//                 from TMEM, V is an MN-major shared-memory operand.  Row r of an accumulator sums products
 //                 of tiles a and c, row r+64 of tiles b and d.
 //   warp 11     : V producer — TMA-loads the listed V tiles in pairs into a 5-deep ring (held until
 //                 their P V is complete); they land on the barrier that P arrives on.  Only listed tiles
@@ -56,8 +57,8 @@
 // TMEM (512 columns): S/P slots 3 x 128, accumulators 2 x 64.
 //
 // Head dimensions 16 and 32 run on the same 128-byte rows: the tensor maps are D wide, so TMA fills
-// the other columns of a tile with zeros without reading them, S takes D / 16 K steps instead of
-// four, and P V is D columns wide.
+// the other columns of a tile with zeros without reading them, and S takes D / 16 K steps instead of
+// four.
 //
 // Numerics follow the reference's loop (fa2_custom_mask/fa2_fwd.py:150-196): logits scaled by
 // sm_scale*log2(e), exp2 domain, fp32 row sums of the fp32 probabilities, P rounded to the input
@@ -533,18 +534,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int u = 0; 4 * u < n_tiles; ++u) {
         const int nt = min(4, n_tiles - 4 * u);
         const int at = lane < 2 ? vs : vs + 1 < kVStages ? vs + 1 : 0;
-        const int row = lane < nt ? static_cast<int>(cols[4 * u + lane] & kColIndex) * 64 : 0;
+        // whole pairs: a tile that does not exist is read behind the last row, which gives zeros
+        const int n_load = (nt + 1) & ~1;
+        const int row = lane < nt ? static_cast<int>(cols[4 * u + lane] & kColIndex) * 64 : p.N;
         const uint32_t dst = smem_u32(sm->v[at][lane & 1]), bar = smem_u32(&sm->p_full[slot]);
         // (for the first users these ask for the phase before the first one, which counts as complete)
         ok = mbar_wait_warp(smem_u32(&sm->pv_done[slot]), ph);
         if (!ok) break;
-        if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
+        if (lane == 0) mbar_expect_tx(bar, kTileBytes * n_load);
         __syncwarp();
-        if (lane < min(nt, 2)) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
+        if (lane < 2) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
         const int next = slot + 1 < kSlots ? slot + 1 : 0;
         ok = mbar_wait_warp(smem_u32(&sm->pv_done[next]), next > 0 ? ph : ph ^ 1);
         if (!ok) break;
-        if (lane >= 2 && lane < nt) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
+        if (lane >= 2 && lane < n_load) tma_load_4d(dst, &tm_v, bar, 0, row, walk.it.y, walk.it.x);
         vs += 2;
         if (vs >= kVStages) vs -= kVStages;
         slot = next;
@@ -611,7 +614,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (!ok) fwd_give_up(sm, p.status, kFailMma);
   } else if (warp == kPvWarp) {
     // =========================== P V issuer ===========================
-    const uint32_t idesc_pv = umma_idesc(kBf16, 0, 1, 128, p.D);  // P (TMEM) x V (MN-major)
+    constexpr uint32_t idesc_pv = umma_idesc(kBf16, 0, 1, 64, 128);  // P (TMEM) x V (MN-major)
     const bool leader = elect_one();
     const uint64_t desc_v0 = smem_desc_sw128(smem_u32(sm->v[0][0]), 8192, 1024);
     bool ok = true;
@@ -643,19 +646,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         // Tiles a and b have their P in columns [0, 32) of the slot, a in lanes 0..63 and b in lanes
-        // 64..127; c and d in columns [32, 64).  Each product writes the lanes of its tile only.  A
-        // lane half's first product of an item starts its accumulator afresh.
+        // 64..127; c and d in columns [32, 64).  The team's first product of an item starts its accumulator
+        // afresh, in all lanes.  (N = 17536, everything listed 114.1 -> 110.8 us, 8 heads, a tenth 111.4 -> 109.1,
+        // bf16 N = 32000, 32 heads, a tenth 1288 -> 1249, against a product for each tile; D = 32, where those are
+        // 32 columns wide, 49.3 -> 49.5.)
         const uint32_t o_acc = tmem + kTmemO + 64 * team;
         if (leader) {
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
+          for (int t = 0; t < 4; t += 2) {
             if (t >= nt) break;
-            const uint32_t p_cols = tmem + 128 * slot + 32 * (t >> 1);
-            const uint64_t desc_v = desc_v0 + static_cast<uint64_t>((t < 2 ? vs : vs1) * 2 + (t & 1)) * (kTileBytes >> 4);
+            const uint32_t p_cols = tmem + 128 * slot + 16 * t;
+            const uint64_t desc_v = desc_v0 + static_cast<uint64_t>((t < 2 ? vs : vs1) * 2) * (kTileBytes >> 4);
             const uint32_t started = u > 1 || t > 1;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              umma_ts_half(o_acc, p_cols + 8 * kk, desc_v + 128 * kk, idesc_pv, started | (kk > 0), t & 1);
+              umma_ws_ts(o_acc, p_cols + 8 * kk, desc_v + 128 * kk, idesc_pv, started | (kk > 0));
           }
         }
         if (leader) {
@@ -777,6 +782,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               exp_chunk<kBf16>(sb, c, neg_m, pk + 48, l0, l1);
             } else {
               exp_chunk<kBf16>(sb, c, neg_m, pk + 16, l0, l1);
+#pragma unroll
+              for (int j = 32; j < 64; ++j) pk[j] = 0u;
             }
             float a0, a1;
             unpack_f32x2(add_f32x2(l0, l1), a0, a1);
@@ -791,9 +798,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
           if (!ok) break;
           l += sum;
-          // this lane's first tile in columns [0, 32) of the slot, its second one in [32, 64)
+          // this lane's first tile in columns [0, 32) of the slot, its second one in [32, 64); zeros for one that
+          // does not exist while the other lane half has it
           tmem_st_32x32b_x32(s_addr, pk);
-          if (two) tmem_st_32x32b_x32(s_addr + 32, pk + 32);
+          if (n_tiles - 4 * u > 2) tmem_st_32x32b_x32(s_addr + 32, pk + 32);
+        } else {
+          uint32_t zero[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) zero[j] = 0u;
+          tmem_st_32x32b_x32(s_addr, zero);
         }
         tc_wait_st();
         tc_fence_before();

@@ -260,6 +260,22 @@ __device__ __forceinline__ void umma_ws_ss(uint32_t d_tmem, uint64_t a_desc, uin
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// D[tmem] (+)= A[tmem] * B[smem desc] in the same form with A in tensor memory: lanes 0..63 of D are their own
+// rows of A times columns [0, N/2) of B, lanes 64..127 their own rows of A times columns [N/2, N).  With two tiles
+// beside one another in B (MN-major, the leading byte offset is the way from one to the other) that is two
+// products of 64 rows at once.  (Ordinary use has the same 64 rows in both lane halves; that each half reads its own
+// is how B200 does it, checked element by element, and every test of the kernels rests on it.)  Two products of 64 x 64
+// with 64 columns: 176 cycles; as two M = 128 products, each with one lane half of the result switched off, 256.
+// Both halves are always written: where there is no second tile, its rows of A and its part of B are zeros.
+__device__ __forceinline__ void umma_ws_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
+                                           uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.ws.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // D[tmem] (+)= A[tmem] * B[smem desc] for lanes 0..63 (half = 0) or 64..127 (half = 1) only: the other
 // lanes of D keep what they hold, whatever their rows of A are.  Same rate as the full form.
 __device__ __forceinline__ void umma_ts_half(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
