@@ -5,8 +5,8 @@
 //       ("supersteps", tiles a and b):
 //         S^T = K [Q_a;Q_b]^T, dP^T = V [dO_a;dO_b]^T                     (SS MMAs, M=64, N=128)
 //         P^T = exp2(S^T c - LSE2[q]), dS^T = P^T (dP^T - delta[q])       (one thread per key row)
-//         dV += P^T_a dO_a + P^T_b dO_b,  dK += dS^T_a Q_a + dS^T_b Q_b   (TS MMAs: A from TMEM, B
-//       MN-major from shared memory).
+//         dV += P^T_a dO_a + P^T_b dO_b,  dK += dS^T_a Q_a + dS^T_b Q_b   (TS MMAs, M=64, N=128: A from
+//       TMEM, B MN-major from shared memory).
 //   dQ    (kDKDV = false): a CTA owns one query block, keeps Q and dO resident and walks the row list
 //       of key blocks two at a time:
 //         S = Q [K_a;K_b]^T, dP = dO [V_a;V_b]^T;  dS = exp2(S c - LSE2[row]) (dP - delta[row]);
@@ -15,9 +15,10 @@
 // The M = 64 "weight stationary" form of the MMA puts the columns of tile a into TMEM lanes 0..63 and
 // those of tile b into lanes 64..127 of the same 64 columns, so every SM sub-partition has
 // exponentials to do whatever the mask is, and no operand is multiplied twice.  The accumulating
-// products write the accumulator rows of the lanes that own the tile and leave the others alone: lane
-// r sums the tile-a products of row r, lane r+64 its tile-b products; the two are added when the block
-// is written out.
+// products take both tiles at once in the same form: lanes 0..63 multiply their P or dS with tile a, lanes 64..127
+// theirs with tile b.  Lane r sums the tile-a products of row r, lane r+64 its tile-b products; the two are
+// added when the block is written out.  A tile b that does not exist is all zeros, in P and dS and in shared
+// memory.
 //
 // Formulas are those of the reference's backward (fa2_custom_mask/fa2_bwd.py:56-74, 116-130) with
 // M replaced by a true base-2 log-sum-exp; the iteration space is the tile lists, not the
@@ -35,15 +36,13 @@
 //                 superstep from a single one (1,270 cycles) were what the whole kernel waited for
 //   warps 17, 24: issue the S/dP MMAs, one for each team (a wait, eight MMAs and their commit take an
 //                 issuer longer than the superstep); warp 17 owns TMEM
-//   warps 18, 25: issue the accumulating MMAs (dK/dV: one warp for dV, one for dK; dQ: one for the lanes
-//                 of tile a, one for tile b): a single issuer was at work 1,050 of the 1,370 cycles of a
-//                 superstep, its own waits and commits between batches included.  All issuers run
-//                 warp-wide with one elected lane issuing
+//   warps 18, 25: issue the accumulating MMAs (dK/dV: one warp for dV, one for dK, since a single issuer of
+//                 both spent most of a superstep on its own waits and commits; dQ has one product and one
+//                 issuer).  All issuers run warp-wide with one elected lane issuing
 //   warps 20..23: take a block's sums out of tensor memory and store them while the compute warps are
 //                 already at work on the next block
 // A block's own operands are double-buffered: the next block's are loaded while this one is at work.
-// Head dimensions 16 and 32: zero-filled on load by D-wide tensor maps, D / 16 K steps for S and dP,
-// D-wide accumulating products.
+// Head dimensions 16 and 32: zero-filled on load by D-wide tensor maps, D / 16 K steps for S and dP.
 // S and dP of a superstep have one of three slots in TMEM, and P and dS are stored over them: the
 // next superstep but two is what its products must be complete for, not the team's own next one.
 // What bounds it: the way of a superstep through three slots, with no part of it that is the bound alone.
@@ -97,7 +96,7 @@ struct BwdSmem {
   int item_tiles[2], item_begin[2];         // ... its list length and where its list begins
   uint64_t item_full[2], item_free[2];      // header published; header read by all its readers
   uint64_t stat_full[2], stat_free[2];      // own operands loaded; their S/dP instructions complete
-  uint64_t acc_done;                        // all accumulating MMAs of the block complete
+  uint64_t acc_done;                        // all accumulating MMAs of the block complete (one arrival per issuer)
   uint64_t acc_free;                        // the write-out warps have read the accumulators
   // a place's tiles have landed: one barrier for each place and team, so that the team's issuer and
   // compute warps, which wait on it, see each of its phases
@@ -201,17 +200,17 @@ __device__ __forceinline__ BwdItem bwd_item(int w, const BwdParams& p, int n_til
 
 // A producer's share of an item's supersteps: the listed tiles a, b of one tensor into its half of the
 // ring (and, dK/dV, the tiles' part of one of the two vectors), one lane per copy, copies of one kind in
-// one instruction.
+// one instruction.  In the place of a tile that does not exist comes block `none`, behind the last one: zeros.
 template <int kPlaces, bool kVector>
 __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, uint64_t* empty,
                                                const CUtensorMap* map, float* vec_ring, const float* vec,
-                                               const BwdItem& it, int n_super, int lane,
+                                               const BwdItem& it, int n_super, int none, int lane,
                                                int* gs) {
 #pragma unroll 1
   for (int j = 0; j < n_super; ++j, ++*gs) {
     const int s = *gs % kPlaces;
     const int nt = min(2, it.n_tiles - 2 * j), t = lane & 1;
-    const int nj = t < nt ? (__ldg(it.ents + 2 * j + t) & kListIndex) : 0;
+    const int nj = t < nt ? (__ldg(it.ents + 2 * j + t) & kListIndex) : none;
     if (kVector) {
       // dK/dV: the place is free when the products of its previous superstep are (empty: d_free)
       if (*gs >= kPlaces &&
@@ -221,9 +220,9 @@ __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, ui
       if (!mbar_wait_warp(smem_u32(empty + s), ((*gs / kPlaces) & 1) ^ 1)) return false;
     }
     const uint32_t bar = smem_u32(full + *gs % (2 * kPlaces));
-    if (lane == 0) mbar_expect_tx(bar, nt * (kBwdTile + (kVector ? 256u : 0u)));
+    if (lane == 0) mbar_expect_tx(bar, 2 * kBwdTile + (kVector ? nt * 256u : 0u));
     __syncwarp();
-    if (lane < 2 && t < nt)
+    if (lane < 2)
       tma_load_4d(smem_u32(ring) + (2 * s + t) * kBwdTile, map, bar, 0, nj * 64, it.h, it.b);
     if (kVector && (lane & 30) == 2 && t < nt)
       bulk_load_1d(smem_u32(vec_ring + (2 * s + t) * 64), vec + it.vec_base + nj * 64, 256, bar);
@@ -272,8 +271,6 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
       if (leader) {
         const uint32_t x_at = tmem + 128 * (g % kSlots);
         const uint32_t x_full = smem_u32(&sm->x_full[g % kXBars]);
-        // (a superstep with one tile multiplies with whatever the second tile's place holds: nobody
-        // reads those lanes)
         const uint64_t b0 = desc_b0 + static_cast<uint64_t>(2 * (g % kR0)) * kTileDesc;
         const uint64_t b1 = desc_b1 + static_cast<uint64_t>(2 * (g % kR1)) * kTileDesc;
 #pragma unroll
@@ -295,13 +292,12 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
 }
 
 // The accumulating instructions of one warp.  dK/dV: the first warp's sum dV, the second one's dK (each
-// accumulator has one issuer, which keeps its products in order); dQ: the first warp's write the lanes
-// of tile a, the second one's those of tile b.
+// accumulator has one issuer, which keeps its products in order); dQ: the first warp's, there is no second one.
 template <bool kBf16, bool kDKDV>
 __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, uint32_t tmem, bool first,
                                               int lane) {
   const bool dv = kDKDV && first;
-  const uint32_t idesc = umma_idesc(kBf16, 0, 1, 128, p.D);
+  constexpr uint32_t idesc = umma_idesc(kBf16, 0, 1, 64, 128);
   const bool leader = elect_one();
   const int places = dv ? kRing1<kDKDV> : kRing0<kDKDV>;
   const uint64_t desc = smem_desc_sw128(smem_u32(sm->ring[dv ? kRing0<kDKDV> : 0][0]), 8192, 1024);
@@ -326,21 +322,15 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
       tc_fence_after();
       if (leader) {
         // rows [16 kk, +16) of a streamed tile: column 8 (kk % 2) of the 32 columns of P or dS of warp
-        // column half kk / 2; tile a's in lanes 0..63, tile b's in lanes 64..127; each product writes
-        // the lanes of its tile only
+        // column half kk / 2; tile a's in lanes 0..63, tile b's in lanes 64..127.  (A product for each
+        // tile, with the other's lanes switched off: bf16 2 x 16 heads, N = 16384, causal, a quarter, forward
+        // and backward 1,835 us, 1,785 so; 2 x 8 heads, N = 4160 97.5 and 96.2.)
         const uint32_t cols = from + 128 * slot;
         const uint64_t b0 = desc + static_cast<uint64_t>(2 * place * (kBwdTile >> 4));
         const uint32_t more = left != w_tiles;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          if (kDKDV || first)
-            umma_ts_half(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + 128 * kk, idesc, more | (kk > 0), 0);
-        if (left > 1 && (kDKDV || !first)) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_ts_half(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + (kBwdTile >> 4) + 128 * kk, idesc,
-                         more | (kk > 0), 1);
-        }
+          umma_ws_ts(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + 128 * kk, idesc, more | (kk > 0));
         if constexpr (!kDKDV) tc_commit(empty + 8 * place);  // place free
         tc_commit(smem_u32(&sm->d_free[x]));  // P or dS columns free; accumulator updated
         if (left <= 2) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
@@ -379,7 +369,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
 #pragma unroll 1
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->item_full[i]), 1);
-      mbar_init(smem_u32(&sm->item_free[i]), kCW + 8 + 1);  // all roles but the first producer
+      mbar_init(smem_u32(&sm->item_free[i]), kCW + 7 + (kDKDV ? 2 : 1));  // all roles but the first producer
       mbar_init(smem_u32(&sm->stat_full[i]), 2);  // two producers
       mbar_init(smem_u32(&sm->stat_free[i]), 2);  // two S/dP issuers
     }
@@ -388,7 +378,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
 #pragma unroll 1
     for (int i = 0; i < kXBars; ++i) {
       mbar_init(smem_u32(&sm->x_full[i]), kDKDV ? 2 : 1);
-      mbar_init(smem_u32(&sm->d_free[i]), 2);
+      mbar_init(smem_u32(&sm->d_free[i]), kDKDV ? 2 : 1);
     }
 #pragma unroll 1
     for (int s = 0; s < 2 * kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_full0[s]), 1);
@@ -396,11 +386,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     for (int s = 0; s < 2 * kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_full1[s]), 1);
     if constexpr (!kDKDV) {
 #pragma unroll 1
-      for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), 2);
+      for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), 1);
 #pragma unroll 1
       for (int s = 0; s < kRing1<false>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
     }
-    mbar_init(smem_u32(&sm->acc_done), 2);
+    mbar_init(smem_u32(&sm->acc_done), kDKDV ? 2 : 1);
     mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
     sm->abort_flag = 0;
     mbar_fence_init();
@@ -478,7 +468,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
           }
         }
         ok = bwd_load_tiles<kRing0<kDKDV>, kDKDV>(sm->ring[0][0], sm->in_full0, kDKDV ? sm->d_free : sm->in_empty0, &tm_str0,
-                                                  sm->lse[0][0], p.lse2, it, n_super, lane, &gs);
+                                                  sm->lse[0][0], p.lse2, it, n_super, p.nb, lane, &gs);
         ++ni;
       }
       if (!ok) bwd_give_up(sm, p.status, 1);
@@ -514,13 +504,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         }
         ok = bwd_load_tiles<kRing1<kDKDV>, kDKDV>(sm->ring[kRing0<kDKDV>][0], sm->in_full1,
                                                   kDKDV ? sm->d_free : sm->in_empty1, &tm_str1, sm->delta[0][0], p.delta, it,
-                                                  n_super, lane, &gs);
+                                                  n_super, p.nb, lane, &gs);
         ++ni;
       }
       if (!ok) bwd_give_up(sm, p.status, 1);
     } else if (warp == kXWarp || warp == kX2Warp) {
       bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane);
-    } else if (warp == kAccWarp || warp == kAcc2Warp) {
+    } else if (warp == kAccWarp || (kDKDV && warp == kAcc2Warp)) {
       bwd_issue_acc<kBf16, kDKDV>(sm, p, tmem, warp == kAccWarp, lane);
     }
   } else if (warp < kCW) {
@@ -675,8 +665,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
             if constexpr (kDKDV) tmem_st_32x32b_x4(s_at + 4 * c8, pk_p);
             tmem_st_32x32b_x4(dp_at + 4 * c8, pk_ds);
           }
-          tc_wait_st();
+        } else {
+          uint32_t zero[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) zero[k] = 0u;
+          if constexpr (kDKDV) tmem_st_32x32b_x16(s_at, zero);
+          tmem_st_32x32b_x16(dp_at, zero);
         }
+        tc_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sm->d_full[g % kSlots]));
@@ -688,7 +684,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   } else {
     // =========================== write-out ===========================
     // Lane r of an accumulator holds the tile-a sums of row r of the CTA's block, lane r+64 its tile-b
-    // sums (unwritten when the list has a single tile).  These four warps (lane quarter = warp % 4)
+    // sums (zeros when the list has a single tile).  These four warps (lane quarter = warp % 4)
     // take the sums out of tensor memory as soon as the block's last MMAs are complete, so that the
     // next block can start accumulating, then add the two halves, scale, round and store, while the
     // compute warps are already at work on the next block.  dK/dV: lanes 0..63 finish dV and hand
@@ -729,28 +725,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       }
       if (ok) ok = mbar_wait_warp(smem_u32(&sm->acc_done), ni & 1);
       ++ni;
-      const bool live = half == 0 || w_tiles > 1;  // warp-uniform
       bool any_failed = false;
 #pragma unroll 1
       for (int q = 0; q < kKeep; q += 32) {
         uint32_t keep[32];
         if (ok) {
           uint4* to = reinterpret_cast<uint4*>(sm->xfer[half][r_blk]);
-          if (live) {
-            uint32_t send[32];
-            tc_fence_after();
-            tmem_ld_32x32b_x32(tm_send + q, send);
-            tmem_ld_32x32b_x32(tm_keep + q, keep);
-            tc_wait_ld();
+          uint32_t send[32];
+          tc_fence_after();
+          tmem_ld_32x32b_x32(tm_send + q, send);
+          tmem_ld_32x32b_x32(tm_keep + q, keep);
+          tc_wait_ld();
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              to[k] = make_uint4(send[4 * k], send[4 * k + 1], send[4 * k + 2], send[4 * k + 3]);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 32; ++k) keep[k] = 0u;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) to[k] = make_uint4(0u, 0u, 0u, 0u);
-          }
+          for (int k = 0; k < 8; ++k)
+            to[k] = make_uint4(send[4 * k], send[4 * k + 1], send[4 * k + 2], send[4 * k + 3]);
           if (q + 32 == kKeep) {
             // the accumulators are out of tensor memory: the next block may start accumulating
             tc_fence_before();

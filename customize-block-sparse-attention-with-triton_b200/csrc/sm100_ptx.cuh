@@ -276,18 +276,6 @@ __device__ __forceinline__ void umma_ws_ts(uint32_t d_tmem, uint32_t a_tmem, uin
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc] for lanes 0..63 (half = 0) or 64..127 (half = 1) only: the other
-// lanes of D keep what they hold, whatever their rows of A are.  Same rate as the full form.
-__device__ __forceinline__ void umma_ts_half(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                             uint32_t idesc, uint32_t accumulate, int half) {
-  const uint32_t off_lo = half != 0 ? 0xffffffffu : 0u, off_hi = ~off_lo;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %6, %6}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(off_lo), "r"(off_hi)
-      : "memory");
-}
 
 // Shared-memory matrix descriptor for a tile stored as rows of 128 bytes with the 128-byte
 // swizzle (what a TMA SWIZZLE_128B load of a [rows][64 x 16-bit] box produces; the tile base must
