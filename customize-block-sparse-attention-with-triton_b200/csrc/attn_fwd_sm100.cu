@@ -131,7 +131,7 @@ struct FwdSmem {
   uint32_t tmem_base;
   int abort_flag;
 };
-static_assert(sizeof(FwdSmem) + 1024 <= 232448, "FwdSmem exceeds the shared memory of one CTA");
+static_assert(sizeof(FwdSmem) <= 232448, "FwdSmem exceeds the shared memory of one CTA");
 
 struct FwdParams {
   const int32_t* row_ptr;   // list mode: CSR row lists
@@ -386,9 +386,11 @@ template <bool kBf16, bool kElementMask>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  FwdSmem* sm = reinterpret_cast<FwdSmem*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  // (Aligned by declaration: every address in it is a constant then.  Rounded up at run time, all roles carried a
+  // base and added to it at every barrier: N = 17536, a tenth, one head 19.15 -> 17.94 us, 8 heads 107.6 -> 102.5;
+  // everything listed 108.9 -> 104.0.)
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  FwdSmem* sm = reinterpret_cast<FwdSmem*>(smem_raw);
 
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
@@ -1096,7 +1098,7 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
   int sms = 0;
   if ((rc = sm_count(&sms)) != BSA_OK) return rc;
 
-  const size_t smem_bytes = sizeof(FwdSmem) + 1024;
+  const size_t smem_bytes = sizeof(FwdSmem);
   auto kern = dense != nullptr
                   ? (dtype == BSA_BF16 ? attn_fwd_kernel<true, true> : attn_fwd_kernel<false, true>)
                   : (dtype == BSA_BF16 ? attn_fwd_kernel<true, false> : attn_fwd_kernel<false, false>);
