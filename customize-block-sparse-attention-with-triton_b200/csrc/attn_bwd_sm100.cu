@@ -27,7 +27,7 @@
 // Persistent: one CTA per SM starts with block blockIdx.x and draws further blocks from an
 // optional work counter (or walks a fixed stride); long lists first when the mask is causal.  dQ may run
 // beside dK/dV (see `together`).
-// Roles (26 warps):
+// Roles (27 warps):
 //   warps 0..15 : compute, two teams of eight warps on alternate supersteps (team = warp / 8, TMEM lane
 //                 quarter = warp % 4, 32 of a tile's 64 columns = (warp / 4) % 2), so that one team's
 //                 barrier round trips and products run under the other one's arithmetic
@@ -39,6 +39,12 @@
 //   warps 18, 25: issue the accumulating MMAs (dK/dV: one warp for dV, one for dK, since a single issuer of
 //                 both spent most of a superstep on its own waits and commits; dQ has one product and one
 //                 issuer).  All issuers run warp-wide with one elected lane issuing
+//   warp 26     : lister: draws the blocks, looks their lists up and publishes them.  It does so while the block
+//                 before is still being loaded.  (By the first producer after its last load, ticket, list and
+//                 first entries were three trips to memory one after the other, 3,000 to 4,000 cycles from one
+//                 block's last copy to the next one's first, with three supersteps of 1,000 in the ring to bridge
+//                 them.  Forward and backward, 2 x 8 heads, N = 4160, causal, a quarter 88.6 -> 84.9 us; 2 x 16
+//                 heads, N = 16384 1,646 -> 1,612.  Set up 2 to 5 supersteps before the last load: the same.)
 //   warps 20..23: take a block's sums out of tensor memory and store them while the compute warps are
 //                 already at work on the next block
 // A block's own operands are double-buffered: the next block's are loaded while this one is at work.
@@ -72,7 +78,9 @@ constexpr int kCW = 16;                    // compute warps: 2 teams x 4 lane qu
 constexpr int kTeamW = kCW / 2;
 constexpr int kProdWarp = kCW, kXWarp = kCW + 1, kAccWarp = kCW + 2, kProd2Warp = kCW + 3;
 constexpr int kX2Warp = kCW + 8, kAcc2Warp = kCW + 9;           // (warps kCW + 4 .. kCW + 7 write out: lane quarter = warp % 4)
-constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: three warps at the end only fill one
+constexpr int kListWarp = kCW + 10;
+constexpr int kGoBefore = 3;                  // supersteps of loads before an item's end at which the next one is set up
+constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: one warp at the end only fills one
 constexpr uint32_t kBwdTile = 64 * 64 * 2;
 constexpr uint32_t kBwdTmemCols = 512;
 constexpr int kListIndex = BSA_LIST_PARTIAL_FLAG - 1;  // a list entry without its flag
@@ -83,6 +91,11 @@ constexpr uint32_t kTmAcc0 = 384, kTmAcc1 = 448;
 // The issuers and teams see every second superstep, so the barriers that they wait on come twice for
 // each slot.
 constexpr int kSlots = 3, kXBars = 2 * kSlots;
+// dQ: places of a block's LSE2 and delta, which are read at each of its supersteps.  Those of block n are fetched when
+// all S/dP of block n-2 are complete, and with that the arithmetic of all but its last kSlots supersteps: what
+// block n-5 has is not read any more, even if all blocks have a single superstep.
+constexpr int kVecPlaces = 5;
+static_assert(kVecPlaces >= kSlots + 2 && kVecPlaces <= kRing0<true> && kVecPlaces <= kRing1<true>);
 
 struct BwdSmem {
   uint8_t stat[2][2][kBwdTile];             // by block parity: the CTA's own K, V (dK/dV) or Q, dO (dQ)
@@ -92,9 +105,12 @@ struct BwdSmem {
   // write-out: what lanes 0..63 and 64..127 hand to each other, 32 columns of 64 rows at a time (rows of
   // 36 floats: eight lanes' 16-byte accesses then fall into different banks)
   float xfer[2][64][36];
-  int item[2];                              // by item parity: the work item, -1 = no more work
-  int item_tiles[2], item_begin[2];         // ... its list length and where its list begins
-  uint64_t item_full[2], item_free[2];      // header published; header read by all its readers
+  // by item parity: the work item
+  int4 item[2];                             // batch (-1 = no more work), head, block, list length
+  int item_begin[2];                        // where its list begins
+  int first[2][32];                         // the first entries of its list
+  uint64_t item_full[2], item_free[2];      // published; read by all its readers
+  uint64_t setup_go[2];                     // first producer -> lister: time to set up the next one
   uint64_t stat_full[2], stat_free[2];      // own operands loaded; their S/dP instructions complete
   uint64_t acc_done;                        // all accumulating MMAs of the block complete (one arrival per issuer)
   uint64_t acc_free;                        // the write-out warps have read the accumulators
@@ -152,65 +168,129 @@ __device__ __forceinline__ void bwd_begin(const BwdParams& p) {
   if (kDKDV || !p.together) grid_dependency_wait();
 }
 
-// Readers of the item header: wait for item i, read it (the producer looked the list up, so the
-// other roles start an item without a round trip to memory), tell the producer the slot was read.
-__device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, int* w, int* n_tiles, int* begin) {
+// A work item as the lister publishes it.
+struct BwdItem {
+  int b, h, blk, n_tiles;  // b < 0: no more work
+  int begin;               // of its list, in list_idx
+  __device__ __forceinline__ int supersteps() const { return (n_tiles + 1) >> 1; }
+  __device__ __forceinline__ int64_t vec_base(const BwdParams& p) const {  // into lse2 / delta
+    return (static_cast<int64_t>(b) * p.H + h) * p.N;
+  }
+};
+
+// Readers of the items: wait for item i, read it, tell the lister that it was read (first: the lane's own of
+// the first 32 entries, for the producers).
+__device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, BwdItem* it, int* first = nullptr) {
   const int par = i & 1;
   if (!mbar_wait_warp_item(smem_u32(&sm->item_full[par]), (i >> 1) & 1, &sm->abort_flag)) return false;
-  *w = *const_cast<volatile int*>(&sm->item[par]);
-  *n_tiles = *const_cast<volatile int*>(&sm->item_tiles[par]);
-  *begin = *const_cast<volatile int*>(&sm->item_begin[par]);
+  const int4 h = sm->item[par];
+  it->b = h.x;
+  it->h = h.y;
+  it->blk = h.z;
+  it->n_tiles = h.w;
+  it->begin = sm->item_begin[par];
+  if (first != nullptr) *first = sm->first[par][lane];
   __syncwarp();
   if (lane == 0) mbar_arrive(smem_u32(&sm->item_free[par]));
   return true;
 }
 
-// Work item w -> (batch, head, block) and the block's list.
-// dQ: long (late) rows first; dK/dV: long (early) key columns first when the mask is causal.
-struct BwdItem {
-  int b, h, blk, n_tiles;
-  const int32_t* ents;
-  int64_t vec_base;  // into lse2 / delta
-};
-// (n_tiles < 0: look the list up; otherwise the caller has its length and beginning already)
+// The lister (one warp): draws the items, looks their lists up and publishes them with the first entries,
+// kGoBefore supersteps of loads before the producers need them.
 template <bool kDKDV>
-__device__ __forceinline__ BwdItem bwd_item(int w, const BwdParams& p, int n_tiles = -1,
-                                            int begin = 0) {
-  BwdItem it;
-  const int bh = w / p.nb;
-  it.blk = kDKDV ? (w - bh * p.nb) : (p.nb - 1 - (w - bh * p.nb));
-  it.b = bh / p.H;
-  it.h = bh - it.b * p.H;
-  if (n_tiles < 0) {
-    const int64_t li =
-        static_cast<int64_t>(it.b * p.list_b_stride + it.h * p.list_h_stride) * p.nb + it.blk;
-    if (p.list_places > 0) {
-      begin = static_cast<int>(li * p.list_places);
-      n_tiles = __ldg(p.list_ptr + li);
-    } else {
-      begin = __ldg(p.list_ptr + li);
-      n_tiles = __ldg(p.list_ptr + li + 1) - begin;
+__device__ __forceinline__ void bwd_list_items(BwdSmem* sm, const BwdParams& p, int lane) {
+  const int stride = gridDim.x;
+  bool ok = true;
+  bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
+  bwd_begin<kDKDV>(p);
+#pragma unroll 1
+  for (int i = 0, w = blockIdx.x;; ++i) {
+    const int par = i & 1;
+    if (i > 0) {
+      ok = mbar_wait_warp_item(smem_u32(&sm->setup_go[par ^ 1]), ((i - 1) >> 1) & 1, &sm->abort_flag);
+      if (!ok) break;
+      if (p.ticket != nullptr) {
+        int t = 0;
+        if (lane == 0) {
+          t = atomicAdd(p.ticket, 1);
+          // every CTA draws until its first ticket past the end, so the launch draws exactly
+          // `items` tickets in all; whoever draws the last one leaves the counter at zero
+          if (t == p.items - 1) atomicExch(p.ticket, 0);
+        }
+        w = stride + __shfl_sync(0xffffffffu, t, 0);
+        terminal = w >= p.items;
+      } else {
+        w += stride;
+      }
     }
+    // Work item w -> (batch, head, block).  dQ: long (late) rows first; dK/dV: long (early) key columns first
+    // when the mask is causal.
+    int4 it = make_int4(-1, 0, 0, 0);
+    int begin = 0, first = 0;
+    if (w < p.items) {
+      const int bh = w / p.nb;
+      it.z = kDKDV ? (w - bh * p.nb) : (p.nb - 1 - (w - bh * p.nb));
+      it.x = bh / p.H;
+      it.y = bh - it.x * p.H;
+      const int64_t li = static_cast<int64_t>(it.x * p.list_b_stride + it.y * p.list_h_stride) * p.nb + it.z;
+      if (p.list_places > 0) {
+        begin = static_cast<int>(li * p.list_places);
+        first = lane < p.list_places ? __ldg(p.list_idx + begin + lane) : 0;
+        it.w = __ldg(p.list_ptr + li);
+      } else {
+        begin = __ldg(p.list_ptr + li);
+        it.w = __ldg(p.list_ptr + li + 1) - begin;
+        if (lane < it.w) first = __ldg(p.list_idx + begin + lane);
+      }
+    }
+    // item i-2 must have been read by everyone
+    if (i >= 2) ok = mbar_wait_warp_item(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1, &sm->abort_flag);
+    if (!ok) break;
+    sm->first[par][lane] = first;
+    if (lane == 0) {
+      sm->item[par] = it;
+      sm->item_begin[par] = begin;
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sm->item_full[par]));  // release: the item is visible
+    if (it.x < 0) break;
   }
-  it.n_tiles = n_tiles;
-  it.ents = p.list_idx + begin;
-  it.vec_base = (static_cast<int64_t>(it.b) * p.H + it.h) * p.N;
-  return it;
+  if (!ok) bwd_give_up(sm, p.status, 1);
+  if (!terminal && lane == 0) {
+    // gave up before the last draw: draw on (without working) until this CTA's first ticket past
+    // the end, so that the launch still draws `items` tickets and the counter returns to zero
+    int t;
+    do {
+      t = atomicAdd(p.ticket, 1);
+      if (t == p.items - 1) atomicExch(p.ticket, 0);
+    } while (stride + t < p.items);
+  }
 }
 
 // A producer's share of an item's supersteps: the listed tiles a, b of one tensor into its half of the
 // ring (and, dK/dV, the tiles' part of one of the two vectors), one lane per copy, copies of one kind in
 // one instruction.  In the place of a tile that does not exist comes block `none`, behind the last one: zeros.
+// (first: the lane's own of the first 32 entries; those behind them are fetched 32 at a time, ahead of need.)
+// go: the barrier on which the lister waits to set up the next item, or 0.
 template <int kPlaces, bool kVector>
 __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, uint64_t* empty,
                                                const CUtensorMap* map, float* vec_ring, const float* vec,
-                                               const BwdItem& it, int n_super, int none, int lane,
-                                               int* gs) {
+                                               const BwdItem& it, const int32_t* ents, int first, int none,
+                                               uint32_t go, int lane, int* gs) {
+  const int n_super = it.supersteps(), j_go = max(n_super - kGoBefore, 0);
+  int mine = first, next = 32 + lane < it.n_tiles ? __ldg(ents + 32 + lane) : 0;
 #pragma unroll 1
   for (int j = 0; j < n_super; ++j, ++*gs) {
+    if (j == j_go && lane == 0 && go != 0) mbar_arrive(go);
     const int s = *gs % kPlaces;
     const int nt = min(2, it.n_tiles - 2 * j), t = lane & 1;
-    const int nj = t < nt ? (__ldg(it.ents + 2 * j + t) & kListIndex) : none;
+    if ((j & 15) == 0 && j > 0) {
+      mine = next;
+      const int at = 2 * j + 32 + lane;
+      if (at < it.n_tiles) next = __ldg(ents + at);
+    }
+    const int entry = __shfl_sync(0xffffffffu, mine, (2 * j + t) & 31);
+    const int nj = t < nt ? (entry & kListIndex) : none;
     if (kVector) {
       // dK/dV: the place is free when the products of its previous superstep are (empty: d_free)
       if (*gs >= kPlaces &&
@@ -225,9 +305,55 @@ __device__ __forceinline__ bool bwd_load_tiles(uint8_t* ring, uint64_t* full, ui
     if (lane < 2)
       tma_load_4d(smem_u32(ring) + (2 * s + t) * kBwdTile, map, bar, 0, nj * 64, it.h, it.b);
     if (kVector && (lane & 30) == 2 && t < nt)
-      bulk_load_1d(smem_u32(vec_ring + (2 * s + t) * 64), vec + it.vec_base + nj * 64, 256, bar);
+      bulk_load_1d(smem_u32(vec_ring + (2 * s + t) * 64), vec + nj * 64, 256, bar);
   }
   return true;
+}
+
+// A producer (one warp): a block's own operand and its share of the streamed tiles.  dQ: the block's part of LSE2
+// or delta comes with the operand, into one of kRing0<true> places.
+template <bool kDKDV, bool kFirst>
+__device__ __forceinline__ void bwd_produce(BwdSmem* sm, const BwdParams& p, const CUtensorMap* own_map,
+                                            const CUtensorMap* map, int lane) {
+  constexpr int kR0 = kRing0<kDKDV>;
+  float* const vec_ring = kFirst ? sm->lse[0][0] : sm->delta[0][0];
+  bool ok = true;
+  int gs = 0, ni = 0;
+  bwd_begin<kDKDV>(p);
+  // (by a role that has waited, and by no other: a warp without a role must not let dQ in)
+  if (kFirst && kDKDV && p.together) grid_dependents_launch();
+#pragma unroll 1
+  for (int i = 0; ok; ++i) {
+    BwdItem it;
+    int first;
+    ok = bwd_next_item(sm, i, lane, &it, &first);
+    if (!ok || it.b < 0) break;
+    const uint32_t go = kFirst ? smem_u32(&sm->setup_go[i & 1]) : 0u;
+    if (it.n_tiles == 0) {
+      if (kFirst && lane == 0) mbar_arrive(go);
+      continue;
+    }
+    // the S/dP instructions of the block before the previous one must be complete
+    const int own = ni & 1;
+    if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1);
+    if (!ok) break;
+    const float* vec = (kFirst ? p.lse2 : p.delta) + it.vec_base(p);
+    if (lane == 0) {
+      const uint32_t bar = smem_u32(&sm->stat_full[own]);
+      mbar_expect_tx(bar, kBwdTile + (kDKDV ? 0u : 256u));
+      tma_load_4d(smem_u32(sm->stat[own][kFirst ? 0 : 1]), own_map, bar, 0, it.blk * 64, it.h, it.b);
+      if constexpr (!kDKDV)
+        bulk_load_1d(smem_u32(vec_ring + (ni % kVecPlaces) * 128), vec + it.blk * 64, 256, bar);
+    }
+    if constexpr (kFirst)
+      ok = bwd_load_tiles<kR0, kDKDV>(sm->ring[0][0], sm->in_full0, kDKDV ? sm->d_free : sm->in_empty0, map, vec_ring,
+                                      vec, it, p.list_idx + it.begin, first, p.nb, go, lane, &gs);
+    else
+      ok = bwd_load_tiles<kRing1<kDKDV>, kDKDV>(sm->ring[kR0][0], sm->in_full1, kDKDV ? sm->d_free : sm->in_empty1, map,
+                                                vec_ring, vec, it, p.list_idx + it.begin, first, p.nb, 0u, lane, &gs);
+    ++ni;
+  }
+  if (!ok) bwd_give_up(sm, p.status, 1);
 }
 
 // The S/dP instructions of one team's supersteps (one warp).
@@ -247,10 +373,10 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
   bwd_begin<kDKDV>(p);
 #pragma unroll 1
   for (int i = 0; ok; ++i) {
-    int w, w_tiles, w_begin;
-    ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
-    if (!ok || w < 0) break;
-    const int n_super = (w_tiles + 1) >> 1;
+    BwdItem it;
+    ok = bwd_next_item(sm, i, lane, &it);
+    if (!ok || it.b < 0) break;
+    const int n_super = it.supersteps();
     if (n_super == 0) continue;
     const int own = ni & 1;
     ok = mbar_wait_warp(smem_u32(&sm->stat_full[own]), (ni >> 1) & 1);
@@ -281,7 +407,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
           if (kk < k_steps)
             umma_ws_ss(x_at + 64, a0 + kTileDesc + 2 * kk, b1 + 2 * kk, idesc_x, kk > 0);
         tc_commit(x_full);
-        if constexpr (kDKDV) mbar_arrive(x_full);  // release: LSE2 and delta have been seen to be there
+        mbar_arrive(x_full);  // release: LSE2 and delta have been seen to be there
         if constexpr (!kDKDV) tc_commit(smem_u32(&sm->in_empty1[g % kR1]));  // V is not needed any more
       }
     }
@@ -309,14 +435,14 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   bwd_begin<kDKDV>(p);
 #pragma unroll 1
   for (int i = 0; ok; ++i) {
-    int w, w_tiles, w_begin;
-    ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
-    if (!ok || w < 0) break;
-    if (w_tiles == 0) continue;
+    BwdItem it;
+    ok = bwd_next_item(sm, i, lane, &it);
+    if (!ok || it.b < 0) break;
+    if (it.n_tiles == 0) continue;
     // the write-out warps must have read the previous block's accumulators
     if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1);
 #pragma unroll 1
-    for (int left = w_tiles; ok && left > 0; left -= 2) {
+    for (int left = it.n_tiles; ok && left > 0; left -= 2) {
       ok = mbar_wait_warp(smem_u32(&sm->d_full[slot]), phase);
       if (!ok) break;
       tc_fence_after();
@@ -327,7 +453,7 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
         // and backward 1,835 us, 1,785 so; 2 x 8 heads, N = 4160 97.5 and 96.2.)
         const uint32_t cols = from + 128 * slot;
         const uint64_t b0 = desc + static_cast<uint64_t>(2 * place * (kBwdTile >> 4));
-        const uint32_t more = left != w_tiles;
+        const uint32_t more = left != it.n_tiles;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
           umma_ws_ts(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + 128 * kk, idesc, more | (kk > 0));
@@ -344,8 +470,8 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   if (!ok) bwd_give_up(sm, p.status, 2);
 }
 
-// Persistent: one CTA per SM.  The producer starts with item blockIdx.x and then draws further
-// items from the optional work counter (or walks a fixed stride), and hands each item's index to
+// Persistent: one CTA per SM.  The lister starts with item blockIdx.x and then draws further
+// items from the optional work counter (or walks a fixed stride), and hands them to
 // the other roles through shared memory; every role walks the same sequence and counts
 // supersteps (gs) and non-empty items (ni) the same way, so barrier phases follow from the counts.
 
@@ -365,13 +491,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
 
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
-  const int stride = gridDim.x;
 
   if (threadIdx.x == 0) {
 #pragma unroll 1
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sm->item_full[i]), 1);
-      mbar_init(smem_u32(&sm->item_free[i]), kCW + 7 + (kDKDV ? 2 : 1));  // all roles but the first producer
+      mbar_init(smem_u32(&sm->item_free[i]), kCW + 8 + (kDKDV ? 2 : 1));  // all other roles
+      mbar_init(smem_u32(&sm->setup_go[i]), 1);
       mbar_init(smem_u32(&sm->stat_full[i]), 2);  // two producers
       mbar_init(smem_u32(&sm->stat_free[i]), 2);  // two S/dP issuers
     }
@@ -379,7 +505,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     for (int i = 0; i < kSlots; ++i) mbar_init(smem_u32(&sm->d_full[i]), kTeamW);  // one arrival per warp
 #pragma unroll 1
     for (int i = 0; i < kXBars; ++i) {
-      mbar_init(smem_u32(&sm->x_full[i]), kDKDV ? 2 : 1);
+      mbar_init(smem_u32(&sm->x_full[i]), 2);  // the commit and the issuer
       mbar_init(smem_u32(&sm->d_free[i]), kDKDV ? 2 : 1);
     }
 #pragma unroll 1
@@ -416,100 +542,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   if ((warp >= kCW && warp < kCW + 4) || warp >= kCW + 8) {
     give_registers<56>();
     if (warp == kProdWarp) {
-      // =========================== TMA producer ===========================
-      bool ok = true;
-      bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
-      bwd_begin<kDKDV>(p);
-      // (by the role that has waited, and by no other: a warp without a role must not let dQ in)
-      if (kDKDV && p.together) grid_dependents_launch();
-      int gs = 0, ni = 0;
-#pragma unroll 1
-      for (int i = 0, w = blockIdx.x; ok; ++i) {
-        const int par = i & 1;
-        if (i > 0) {
-          if (p.ticket != nullptr) {
-            int t = 0;
-            if (lane == 0) {
-              t = atomicAdd(p.ticket, 1);
-              // every CTA draws until its first ticket past the end, so the launch draws exactly
-              // `items` tickets in all; whoever draws the last one leaves the counter at zero
-              if (t == p.items - 1) atomicExch(p.ticket, 0);
-            }
-            w = stride + __shfl_sync(0xffffffffu, t, 0);
-            terminal = w >= p.items;
-          } else {
-            w += stride;
-          }
-        }
-        // the header slot of item i-2 must have been read by everyone
-        if (i >= 2)
-          ok = mbar_wait_warp(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1);
-        if (!ok) break;
-        BwdItem it;
-        it.n_tiles = 0;
-        if (w < p.items) it = bwd_item<kDKDV>(w, p);
-        if (lane == 0) {
-          sm->item[par] = w < p.items ? w : -1;
-          sm->item_tiles[par] = it.n_tiles;
-          sm->item_begin[par] = w < p.items ? static_cast<int>(it.ents - p.list_idx) : 0;
-          mbar_arrive(smem_u32(&sm->item_full[par]));  // release: the header is visible
-        }
-        if (w >= p.items) break;
-        const int n_super = (it.n_tiles + 1) >> 1;
-        if (n_super == 0) continue;
-        // the block's own operands: the S/dP instructions of the block before the previous one must
-        // be complete
-        const int own = ni & 1;
-        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1);
-        if (!ok) break;
-        {
-          const uint32_t bar = smem_u32(&sm->stat_full[own]);
-          if (lane == 0) {
-            mbar_expect_tx(bar, kBwdTile);
-            tma_load_4d(smem_u32(sm->stat[own][0]), &tm_stat0, bar, 0, it.blk * 64, it.h, it.b);
-          }
-        }
-        ok = bwd_load_tiles<kRing0<kDKDV>, kDKDV>(sm->ring[0][0], sm->in_full0, kDKDV ? sm->d_free : sm->in_empty0, &tm_str0,
-                                                  sm->lse[0][0], p.lse2, it, n_super, p.nb, lane, &gs);
-        ++ni;
-      }
-      if (!ok) bwd_give_up(sm, p.status, 1);
-      if (!terminal && lane == 0) {
-        // gave up before the last draw: draw on (without working) until this CTA's first ticket past
-        // the end, so that the launch still draws `items` tickets and the counter returns to zero
-        int t;
-        do {
-          t = atomicAdd(p.ticket, 1);
-          if (t == p.items - 1) atomicExch(p.ticket, 0);
-        } while (stride + t < p.items);
-      }
+      bwd_produce<kDKDV, true>(sm, p, &tm_stat0, &tm_str0, lane);
     } else if (warp == kProd2Warp) {
-      // =========================== second TMA producer ===========================
-      bool ok = true;
-      int gs = 0, ni = 0;
-      bwd_begin<kDKDV>(p);
-#pragma unroll 1
-      for (int i = 0; ok; ++i) {
-        int w, w_tiles, w_begin;
-        ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
-        if (!ok || w < 0) break;
-        const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
-        const int n_super = (w_tiles + 1) >> 1;
-        if (n_super == 0) continue;
-        const int own = ni & 1;
-        if (ni >= 2) ok = mbar_wait_warp(smem_u32(&sm->stat_free[own]), ((ni - 2) >> 1) & 1);
-        if (!ok) break;
-        if (lane == 0) {
-          const uint32_t bar = smem_u32(&sm->stat_full[own]);
-          mbar_expect_tx(bar, kBwdTile);
-          tma_load_4d(smem_u32(sm->stat[own][1]), &tm_stat1, bar, 0, it.blk * 64, it.h, it.b);
-        }
-        ok = bwd_load_tiles<kRing1<kDKDV>, kDKDV>(sm->ring[kRing0<kDKDV>][0], sm->in_full1,
-                                                  kDKDV ? sm->d_free : sm->in_empty1, &tm_str1, sm->delta[0][0], p.delta, it,
-                                                  n_super, p.nb, lane, &gs);
-        ++ni;
-      }
-      if (!ok) bwd_give_up(sm, p.status, 1);
+      bwd_produce<kDKDV, false>(sm, p, &tm_stat1, &tm_str1, lane);
+    } else if (warp == kListWarp) {
+      bwd_list_items<kDKDV>(sm, p, lane);
     } else if (warp == kXWarp || warp == kX2Warp) {
       bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane);
     } else if (warp == kAccWarp || (kDKDV && warp == kAcc2Warp)) {
@@ -526,41 +563,32 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     const uint32_t x_base = tmem + lane_base + 32 * ch;
     const float c = p.scale_log2;
     bool ok = true;
-    int gs = 0;  // supersteps of earlier items; this team takes those with gs % 2 == team
+    int gs = 0, ni = 0;  // supersteps of earlier items (this team takes those with gs % 2 == team), items with any
     bwd_begin<kDKDV>(p);
 #pragma unroll 1
     for (int i = 0; ok; ++i) {
-      int w, w_tiles, w_begin;
-      ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
-      if (!ok || w < 0) break;
-      const int n_super = (w_tiles + 1) >> 1;
+      BwdItem it;
+      ok = bwd_next_item(sm, i, lane, &it);
+      if (!ok || it.b < 0) break;
+      const int n_super = it.supersteps();
       if (n_super == 0) continue;  // (the write-out warps store the zero gradients)
-      float my_lse = 0.f, my_delta = 0.f;
+      const int vec_at = (ni++ % kVecPlaces) * 128 + r_blk;  // (dQ)
       const uint8_t* mask_at = nullptr;
       const int32_t* ents = nullptr;
-      if constexpr (!kDKDV || kElementMask) {
-        const BwdItem it = bwd_item<kDKDV>(w, p, w_tiles, w_begin);
+      if constexpr (kElementMask) {
         const int row = it.blk * 64 + r_blk;
-        ents = it.ents + t_mine;
-        if constexpr (!kDKDV) {
-          // (a row whose elements are all masked has LSE = -inf; every logit it meets is -inf too,
-          // and against a finite stand-in it exponentiates to 0 instead of NaN)
-          my_lse = __ldg(p.lse2 + it.vec_base + row);
-          if constexpr (kElementMask) my_lse = fmaxf(my_lse, -3.0e38f);
-          my_delta = __ldg(p.delta + it.vec_base + row);
-        }
+        ents = p.list_idx + it.begin + t_mine;
         // element-level mask: where this lane's mask bytes of a tile start (dQ: its query row, 32
         // consecutive keys; dK/dV: its key column, 32 consecutive query rows)
-        if constexpr (kElementMask)
-          mask_at = p.dense + it.b * p.ds0 + it.h * p.ds1 +
-                    (kDKDV ? static_cast<int64_t>(row) : static_cast<int64_t>(row) * p.ds2);
+        mask_at = p.dense + it.b * p.ds0 + it.h * p.ds1 +
+                  (kDKDV ? static_cast<int64_t>(row) : static_cast<int64_t>(row) * p.ds2);
       }
       int j = (gs ^ team) & 1;
       int g = gs + j;
       gs += n_super;
 #pragma unroll 1
       for (; ok && j < n_super; j += 2, g += 2) {
-        const bool active = 2 * j + t_mine < w_tiles;  // this lane's tile exists (warp-uniform)
+        const bool active = 2 * j + t_mine < it.n_tiles;  // this lane's tile exists (warp-uniform)
         const uint32_t s_at = x_base + 128 * (g % kSlots), dp_at = s_at + 64;
         // A tile with masked elements inside: fetch this lane's 32 mask bytes while S is on its way
         uint32_t mw[8];
@@ -594,6 +622,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         if (!ok) break;
         tc_fence_after();
         if (active) {
+          float my_lse = 0.f, my_delta = 0.f;
+          if constexpr (!kDKDV) {
+            // (a row whose elements are all masked has LSE = -inf; every logit it meets is -inf too,
+            // and against a finite stand-in it exponentiates to 0 instead of NaN)
+            my_lse = sm->lse[0][0][vec_at];
+            if constexpr (kElementMask) my_lse = fmaxf(my_lse, -3.0e38f);
+            my_delta = sm->delta[0][0][vec_at];
+          }
           const float4* lse4 = reinterpret_cast<const float4*>(&sm->lse[g % kRing0<true>][t_mine][32 * ch]);
           const ulonglong2* del4 = reinterpret_cast<const ulonglong2*>(&sm->delta[g % kRing1<true>][t_mine][32 * ch]);
           // 8 columns at a time, the next ones on their way from tensor memory meanwhile (straight through
@@ -710,15 +746,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     bwd_begin<kDKDV>(p);
 #pragma unroll 1
     for (int i = 0;; ++i) {
-      int w = 0, w_tiles = 1, w_begin = 0;
-      if (ok) ok = bwd_next_item(sm, i, lane, &w, &w_tiles, &w_begin);
-      if (ok && w < 0) break;  // no more work: the same for all four warps
-      const BwdItem it = bwd_item<kDKDV>(ok ? w : 0, p, ok ? w_tiles : 1, 0);
+      BwdItem it{0, 0, 0, 1, 0};
+      if (ok) ok = bwd_next_item(sm, i, lane, &it);
+      if (ok && it.b < 0) break;  // no more work: the same for all four warps
       const int64_t row = it.blk * 64 + r_blk;
       uint16_t* dst = first_out
                           ? static_cast<uint16_t*>(p.out0) + it.b * p.sb0 + it.h * p.sh0 + row * p.sn0
                           : static_cast<uint16_t*>(p.out1) + it.b * p.sb1 + it.h * p.sh1 + row * p.sn1;
-      if (ok && w_tiles == 0) {
+      if (ok && it.n_tiles == 0) {
         // a block with an empty list: zero gradients (the same decision in all four warps)
 #pragma unroll 1
         for (int v = col0; v < min(col0 + kKeep, p.D); v += 8)
