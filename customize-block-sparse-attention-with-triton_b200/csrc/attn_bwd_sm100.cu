@@ -195,14 +195,41 @@ __device__ __forceinline__ bool bwd_next_item(BwdSmem* sm, int i, int lane, BwdI
   return true;
 }
 
+// Work item w -> (batch, head, block) and its list (one warp; first: the lane's own of the first 32 entries).
+// dQ: long (late) rows first; dK/dV: long (early) key columns first when the mask is causal.
+struct BwdFound {
+  int4 it;
+  int begin, first;
+};
+template <bool kDKDV>
+__device__ __forceinline__ BwdFound bwd_look_up(const BwdParams& p, int w, int lane) {
+  BwdFound f{make_int4(-1, 0, 0, 0), 0, 0};
+  if (w < p.items) {
+    const int bh = w / p.nb;
+    f.it.z = kDKDV ? (w - bh * p.nb) : (p.nb - 1 - (w - bh * p.nb));
+    f.it.x = bh / p.H;
+    f.it.y = bh - f.it.x * p.H;
+    const int64_t li = static_cast<int64_t>(f.it.x * p.list_b_stride + f.it.y * p.list_h_stride) * p.nb + f.it.z;
+    if (p.list_places > 0) {
+      f.begin = static_cast<int>(li * p.list_places);
+      if (lane < p.list_places) f.first = __ldg(p.list_idx + f.begin + lane);
+      f.it.w = __ldg(p.list_ptr + li);
+    } else {
+      f.begin = __ldg(p.list_ptr + li);
+      f.it.w = __ldg(p.list_ptr + li + 1) - f.begin;
+      if (lane < f.it.w) f.first = __ldg(p.list_idx + f.begin + lane);
+    }
+  }
+  return f;
+}
+
 // The lister (one warp): draws the items, looks their lists up and publishes them with the first entries,
 // kGoBefore supersteps of loads before the producers need them.
 template <bool kDKDV>
-__device__ __forceinline__ void bwd_list_items(BwdSmem* sm, const BwdParams& p, int lane) {
+__device__ __forceinline__ void bwd_list_items(BwdSmem* sm, const BwdParams& p, BwdFound f, int lane) {
   const int stride = gridDim.x;
   bool ok = true;
   bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
-  bwd_begin<kDKDV>(p);
 #pragma unroll 1
   for (int i = 0, w = blockIdx.x;; ++i) {
     const int par = i & 1;
@@ -223,37 +250,18 @@ __device__ __forceinline__ void bwd_list_items(BwdSmem* sm, const BwdParams& p, 
         w += stride;
       }
     }
-    // Work item w -> (batch, head, block).  dQ: long (late) rows first; dK/dV: long (early) key columns first
-    // when the mask is causal.
-    int4 it = make_int4(-1, 0, 0, 0);
-    int begin = 0, first = 0;
-    if (w < p.items) {
-      const int bh = w / p.nb;
-      it.z = kDKDV ? (w - bh * p.nb) : (p.nb - 1 - (w - bh * p.nb));
-      it.x = bh / p.H;
-      it.y = bh - it.x * p.H;
-      const int64_t li = static_cast<int64_t>(it.x * p.list_b_stride + it.y * p.list_h_stride) * p.nb + it.z;
-      if (p.list_places > 0) {
-        begin = static_cast<int>(li * p.list_places);
-        first = lane < p.list_places ? __ldg(p.list_idx + begin + lane) : 0;
-        it.w = __ldg(p.list_ptr + li);
-      } else {
-        begin = __ldg(p.list_ptr + li);
-        it.w = __ldg(p.list_ptr + li + 1) - begin;
-        if (lane < it.w) first = __ldg(p.list_idx + begin + lane);
-      }
-    }
+    if (i > 0) f = bwd_look_up<kDKDV>(p, w, lane);
     // item i-2 must have been read by everyone
     if (i >= 2) ok = mbar_wait_warp_item(smem_u32(&sm->item_free[par]), ((i - 2) >> 1) & 1, &sm->abort_flag);
     if (!ok) break;
-    sm->first[par][lane] = first;
+    sm->first[par][lane] = f.first;
     if (lane == 0) {
-      sm->item[par] = it;
-      sm->item_begin[par] = begin;
+      sm->item[par] = f.it;
+      sm->item_begin[par] = f.begin;
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(smem_u32(&sm->item_full[par]));  // release: the item is visible
-    if (it.x < 0) break;
+    if (f.it.x < 0) break;
   }
   if (!ok) bwd_give_up(sm, p.status, 1);
   if (!terminal && lane == 0) {
@@ -492,35 +500,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
 
-  if (threadIdx.x == 0) {
-#pragma unroll 1
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sm->item_full[i]), 1);
-      mbar_init(smem_u32(&sm->item_free[i]), kCW + 8 + (kDKDV ? 2 : 1));  // all other roles
-      mbar_init(smem_u32(&sm->setup_go[i]), 1);
-      mbar_init(smem_u32(&sm->stat_full[i]), 2);  // two producers
-      mbar_init(smem_u32(&sm->stat_free[i]), 2);  // two S/dP issuers
-    }
-#pragma unroll 1
-    for (int i = 0; i < kSlots; ++i) mbar_init(smem_u32(&sm->d_full[i]), kTeamW);  // one arrival per warp
-#pragma unroll 1
-    for (int i = 0; i < kXBars; ++i) {
-      mbar_init(smem_u32(&sm->x_full[i]), 2);  // the commit and the issuer
-      mbar_init(smem_u32(&sm->d_free[i]), kDKDV ? 2 : 1);
-    }
-#pragma unroll 1
-    for (int s = 0; s < 2 * kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_full0[s]), 1);
-#pragma unroll 1
-    for (int s = 0; s < 2 * kRing1<true>; ++s) mbar_init(smem_u32(&sm->in_full1[s]), 1);
+  if (warp == 0) {
+    mbar_init_warp(sm->item_full, 2, 1, lane);
+    mbar_init_warp(sm->item_free, 2, kCW + 8 + (kDKDV ? 2 : 1), lane);  // all other roles
+    mbar_init_warp(sm->setup_go, 2, 1, lane);
+    mbar_init_warp(sm->stat_full, 2, 2, lane);        // two producers
+    mbar_init_warp(sm->stat_free, 2, 2, lane);        // two S/dP issuers
+    mbar_init_warp(sm->d_full, kSlots, kTeamW, lane);  // one arrival per warp
+    mbar_init_warp(sm->x_full, kXBars, 2, lane);      // the commit and the issuer
+    mbar_init_warp(sm->d_free, kXBars, kDKDV ? 2 : 1, lane);
+    mbar_init_warp(sm->in_full0, 2 * kRing0<false>, 1, lane);
+    mbar_init_warp(sm->in_full1, 2 * kRing1<true>, 1, lane);
     if constexpr (!kDKDV) {
-#pragma unroll 1
-      for (int s = 0; s < kRing0<false>; ++s) mbar_init(smem_u32(&sm->in_empty0[s]), 1);
-#pragma unroll 1
-      for (int s = 0; s < kRing1<false>; ++s) mbar_init(smem_u32(&sm->in_empty1[s]), 1);
+      mbar_init_warp(sm->in_empty0, kRing0<false>, 1, lane);
+      mbar_init_warp(sm->in_empty1, kRing1<false>, 1, lane);
     }
-    mbar_init(smem_u32(&sm->acc_done), kDKDV ? 2 : 1);
-    mbar_init(smem_u32(&sm->acc_free), 4);  // one arrival per write-out warp
-    sm->abort_flag = 0;
+    mbar_init_warp(&sm->acc_done, 1, kDKDV ? 2 : 1, lane);
+    mbar_init_warp(&sm->acc_free, 1, 4, lane);  // one arrival per write-out warp
+    if (lane == 0) sm->abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == kXWarp) {
@@ -534,7 +531,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     tma_prefetch_desc(&tm_str1);
   }
   tc_fence_before();
-  __syncthreads();
+  BwdFound found;
+  if (warp == kListWarp) {
+    // looks the CTA's first item up while the others set up and get as far as their first wait.  (All of that one after
+    // the other, barriers initialised by one thread: forward and backward, 2 x 8 heads, N = 4160 84.9 us, so 84.0.)
+    bwd_begin<kDKDV>(p);
+    found = bwd_look_up<kDKDV>(p, blockIdx.x, lane);
+    named_barrier_sync(1, kBwdThreads);  // the barriers are there
+  } else {
+    named_barrier_arrive(1, kBwdThreads);
+    named_barrier_sync(3, kBwdThreads - 32);
+  }
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
@@ -546,7 +553,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     } else if (warp == kProd2Warp) {
       bwd_produce<kDKDV, false>(sm, p, &tm_stat1, &tm_str1, lane);
     } else if (warp == kListWarp) {
-      bwd_list_items<kDKDV>(sm, p, lane);
+      bwd_list_items<kDKDV>(sm, p, found, lane);
     } else if (warp == kXWarp || warp == kX2Warp) {
       bwd_issue_x<kBf16, kDKDV>(sm, p, tmem, warp == kX2Warp, lane);
     } else if (warp == kAccWarp || (kDKDV && warp == kAcc2Warp)) {

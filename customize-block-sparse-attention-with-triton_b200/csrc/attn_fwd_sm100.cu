@@ -393,33 +393,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int n2 = p.items - stride;  // items beyond the first round
 
   // ---- set-up ----
-  if (threadIdx.x == 0) {
-#pragma unroll 1
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sm->setup_go[i]), 1);
-      mbar_init(smem_u32(&sm->q_full[i]), 1);
-      mbar_init(smem_u32(&sm->o_full[i]), 1);
-      mbar_init(smem_u32(&sm->stats_full[i]), kSoftmaxWarps);
-      mbar_init(smem_u32(&sm->o_free[i]), 4);  // one arrival per write-out warp
-    }
-#pragma unroll 1
-    for (int s = 0; s < kKStages; ++s) {
-      mbar_init(smem_u32(&sm->k_full[s]), 1);
-      mbar_init(smem_u32(&sm->k_empty[s]), 1);
-    }
-#pragma unroll 1
-    for (int s = 0; s < 2 * kSlots; ++s) mbar_init(smem_u32(&sm->s_full[s]), 1);
-#pragma unroll 1
-    for (int s = 0; s < kSlots; ++s) {
-      mbar_init(smem_u32(&sm->p_full[s]), kTeamWarps + 1);
-      mbar_init(smem_u32(&sm->pv_done[s]), 1);
-    }
-#pragma unroll 1
-    for (int s = 0; s < kLists; ++s) {
-      mbar_init(smem_u32(&sm->list_full[s]), 1);
-      mbar_init(smem_u32(&sm->list_free[s]), 4);  // two producers, two issuers
-    }
-    sm->abort_flag = 0;
+  if (warp == 0) {
+    mbar_init_warp(sm->setup_go, 2, 1, lane);
+    mbar_init_warp(sm->q_full, 2, 1, lane);
+    mbar_init_warp(sm->o_full, 2, 1, lane);
+    mbar_init_warp(sm->stats_full, 2, kSoftmaxWarps, lane);
+    mbar_init_warp(sm->o_free, 2, 4, lane);  // one arrival per write-out warp
+    mbar_init_warp(sm->k_full, kKStages, 1, lane);
+    mbar_init_warp(sm->k_empty, kKStages, 1, lane);
+    mbar_init_warp(sm->s_full, 2 * kSlots, 1, lane);
+    mbar_init_warp(sm->p_full, kSlots, kTeamWarps + 1, lane);
+    mbar_init_warp(sm->pv_done, kSlots, 1, lane);
+    mbar_init_warp(sm->list_full, kLists, 1, lane);
+    mbar_init_warp(sm->list_free, kLists, 4, lane);  // two producers, two issuers
+    if (lane == 0) sm->abort_flag = 0;
     mbar_fence_init();
   }
   if (warp == kSWarp) {

@@ -100,6 +100,10 @@ __device__ __forceinline__ void report_status(int32_t* status, int code) {
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
 }
+// A warp's lanes initialise n <= 32 barriers at once (one after the other takes 30 cycles each).
+__device__ __forceinline__ void mbar_init_warp(uint64_t* bars, int n, uint32_t count, int lane) {
+  if (lane < n) mbar_init(smem_u32(bars + lane), count);
+}
 __device__ __forceinline__ void mbar_fence_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
