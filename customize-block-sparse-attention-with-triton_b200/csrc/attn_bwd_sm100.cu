@@ -606,15 +606,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
           if (partial) {
             const int64_t other = static_cast<int64_t>((e & kListIndex) * 64 + 32 * ch);
             if constexpr (kDKDV) {
+              // this lane's key row as a bit for each of the 32 query rows, then the rows of the lane's elements
               const uint8_t* mp = mask_at + other * p.ds2;
+              uint32_t kept = 0;
 #pragma unroll
-              for (int q4 = 0; q4 < 8; ++q4) {
-                uint32_t w4 = 0;
+              for (int q = 0; q < 32; ++q) kept |= (__ldg(mp + q * p.ds2) != 0 ? 1u : 0u) << q;
 #pragma unroll
-                for (int bb = 0; bb < 4; ++bb)
-                  w4 |= static_cast<uint32_t>(__ldg(mp + (4 * q4 + bb) * p.ds2)) << (8 * bb);
-                mw[q4] = w4;
-              }
+              for (int r = 0; r < 4; ++r) mw[r] = __shfl_sync(0xffffffffu, kept, 8 * r + (lane >> 2)) >> (2 * (lane & 3));
             } else {
               const uint4* mp = reinterpret_cast<const uint4*>(mask_at + other);
 #pragma unroll
@@ -629,86 +627,100 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
         if (!ok) break;
         tc_fence_after();
         if (active) {
-          float my_lse = 0.f, my_delta = 0.f;
-          if constexpr (!kDKDV) {
-            // (a row whose elements are all masked has LSE = -inf; every logit it meets is -inf too,
-            // and against a finite stand-in it exponentiates to 0 instead of NaN)
-            my_lse = sm->lse[0][0][vec_at];
-            if constexpr (kElementMask) my_lse = fmaxf(my_lse, -3.0e38f);
-            my_delta = sm->delta[0][0][vec_at];
-          }
-          const float4* lse4 = reinterpret_cast<const float4*>(&sm->lse[g % kRing0<true>][t_mine][32 * ch]);
-          const ulonglong2* del4 = reinterpret_cast<const ulonglong2*>(&sm->delta[g % kRing1<true>][t_mine][32 * ch]);
-          // 8 columns at a time, the next ones on their way from tensor memory meanwhile (straight through
-          // all 32 the registers do not suffice)
+          // 8 columns of 32 rows (dQ) or 16 of 16 (dK/dV) at a time, the next ones on their way from tensor memory
+          // meanwhile (straight through all of them the registers do not suffice)
           uint32_t xsb[2][8], xdb[2][8];
-          tmem_ld_32x32b_x8(s_at, xsb[0]);
-          tmem_ld_32x32b_x8(dp_at, xdb[0]);
+          if constexpr (kDKDV) {
+            // LSE2 and delta differ from column to column here.  A lane that held all 32 columns of one row read all
+            // of both from shared memory, in 16 loads of 16 bytes that all lanes have in common: 347 cycles of
+            // shared memory's port a superstep of 1,058.  Two columns in eight of four rows need a quarter.
+            const uint64_t* lse2 = reinterpret_cast<const uint64_t*>(&sm->lse[g % kRing0<true>][t_mine][32 * ch + 2 * (lane & 3)]);
+            const uint64_t* del2 = reinterpret_cast<const uint64_t*>(&sm->delta[g % kRing1<true>][t_mine][32 * ch + 2 * (lane & 3)]);
+            const uint64_t c2 = pack_f32x2(c, c);
+            uint64_t neg_l[2], neg_d[2];
+            tmem_ld_16x256b_x2(s_at, xsb[0]);
+            tmem_ld_16x256b_x2(dp_at, xdb[0]);
 #pragma unroll
-          for (int c8 = 0; c8 < 4; ++c8) {
-            uint32_t *xs = xsb[c8 & 1], *xd = xdb[c8 & 1], pk_p[4], pk_ds[4];
-            tc_wait_ld();
-            if (partial) {
-              // masked elements: logit -inf, so P = 0 and with it dS = 0
+            for (int n = 0; n < 4; ++n) {  // columns 16 (n / 2), lanes 16 (n % 2)
+              uint32_t *xs = xsb[n & 1], *xd = xdb[n & 1], pk_p[4], pk_ds[4];
+              if ((n & 1) == 0) {
 #pragma unroll
-              for (int q4 = 0; q4 < 2; ++q4) {
-                const uint32_t nz = __vcmpne4(mw[2 * c8 + q4], 0u);
-#pragma unroll
-                for (int bb = 0; bb < 4; ++bb) {
-                  const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
-                  xs[4 * q4 + bb] = (xs[4 * q4 + bb] & keep) | (0xff800000u & ~keep);
+                for (int k = 0; k < 2; ++k) {
+                  float l0, l1, d0, d1;
+                  unpack_f32x2(lse2[4 * (n + k)], l0, l1);
+                  unpack_f32x2(del2[4 * (n + k)], d0, d1);
+                  // (-inf: a query row with every element masked.  Every logit it meets is -inf too, and against a
+                  // finite stand-in it exponentiates to 0 instead of NaN)
+                  if constexpr (kElementMask) l0 = fmaxf(l0, -3.0e38f), l1 = fmaxf(l1, -3.0e38f);
+                  neg_l[k] = pack_f32x2(-l0, -l1);
+                  neg_d[k] = pack_f32x2(-d0, -d1);
                 }
               }
-            }
-            if (c8 < 3) {
-              tmem_ld_32x32b_x8(s_at + 8 * c8 + 8, xsb[(c8 + 1) & 1]);
-              tmem_ld_32x32b_x8(dp_at + 8 * c8 + 8, xdb[(c8 + 1) & 1]);
-            }
+              tc_wait_ld();
+              if (partial) {
+                // masked elements: logit -inf, so P = 0 and with it dS = 0
 #pragma unroll
-            for (int q = 0; q < 8; q += 4) {
-              // two columns per instruction where the operands allow it
-              float pv[4], dsv[4], nl[4];
-              uint64_t d2[2];
-              if constexpr (kDKDV) {
-                // LSE and delta differ from column to column here
-                // (-inf = a query row with every element masked: see my_lse above)
-                const float4 lv = lse4[2 * c8 + q / 4];
-                const ulonglong2 dv = del4[2 * c8 + q / 4];
-                nl[0] = lv.x; nl[1] = lv.y; nl[2] = lv.z; nl[3] = lv.w;
-                if constexpr (kElementMask) {
-#pragma unroll
-                  for (int t = 0; t < 4; ++t) nl[t] = fmaxf(nl[t], -3.0e38f);
-                }
-                d2[0] = dv.x; d2[1] = dv.y;
+                for (int e = 0; e < 8; ++e)
+                  if ((mw[2 * (n & 1) + ((e >> 1) & 1)] >> (16 * (n >> 1) + 8 * (e >> 2) + (e & 1)) & 1u) == 0) xs[e] = 0xff800000u;
+              }
+              if (n < 3) {
+                const uint32_t next = 16 * ((n + 1) >> 1) + (static_cast<uint32_t>(16 * ((n + 1) & 1)) << 16);
+                tmem_ld_16x256b_x2(s_at + next, xsb[(n + 1) & 1]);
+                tmem_ld_16x256b_x2(dp_at + next, xdb[(n + 1) & 1]);
               }
 #pragma unroll
-              for (int t = 0; t < 4; t += 2) {
-                const uint64_t dp2 =
-                    pack_f32x2(__uint_as_float(xd[q + t]), __uint_as_float(xd[q + t + 1]));
-                uint64_t diff2;
-                if constexpr (kDKDV) {
-                  pv[t] = ex2_approx(fmaf(__uint_as_float(xs[q + t]), c, -nl[t]));
-                  pv[t + 1] = ex2_approx(fmaf(__uint_as_float(xs[q + t + 1]), c, -nl[t + 1]));
-                  diff2 = fma_f32x2(d2[t / 2], pack_f32x2(-1.f, -1.f), dp2);
-                } else {
-                  float z0, z1;
-                  unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(xs[q + t]),
-                                                    __uint_as_float(xs[q + t + 1])),
-                                         pack_f32x2(c, c), pack_f32x2(-my_lse, -my_lse)),
-                               z0, z1);
-                  pv[t] = ex2_approx(z0);
-                  pv[t + 1] = ex2_approx(z1);
-                  diff2 = add_f32x2(dp2, pack_f32x2(-my_delta, -my_delta));
-                }
-                unpack_f32x2(mul_f32x2(pack_f32x2(pv[t], pv[t + 1]), diff2), dsv[t], dsv[t + 1]);
+              for (int e = 0; e < 4; ++e) {  // columns 8 (e / 2), row 8 (e % 2)
+                float z0, z1, ds0, ds1;
+                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(xs[2 * e]), __uint_as_float(xs[2 * e + 1])), c2, neg_l[e >> 1]), z0, z1);
+                const float p0 = ex2_approx(z0), p1 = ex2_approx(z1);
+                const uint64_t diff2 = add_f32x2(pack_f32x2(__uint_as_float(xd[2 * e]), __uint_as_float(xd[2 * e + 1])), neg_d[e >> 1]);
+                unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1), diff2), ds0, ds1);
+                pk_p[e] = pack_2x16<kBf16>(p0, p1);
+                pk_ds[e] = pack_2x16<kBf16>(ds0, ds1);
               }
-              pk_p[q / 2] = pack_2x16<kBf16>(pv[0], pv[1]);
-              pk_p[q / 2 + 1] = pack_2x16<kBf16>(pv[2], pv[3]);
-              pk_ds[q / 2] = pack_2x16<kBf16>(dsv[0], dsv[1]);
-              pk_ds[q / 2 + 1] = pack_2x16<kBf16>(dsv[2], dsv[3]);
+              const uint32_t to = 8 * (n >> 1) + (static_cast<uint32_t>(16 * (n & 1)) << 16);
+              tmem_st_16x128b_x2(s_at + to, pk_p);
+              tmem_st_16x128b_x2(dp_at + to, pk_ds);
             }
-            if constexpr (kDKDV) tmem_st_32x32b_x4(s_at + 4 * c8, pk_p);
-            tmem_st_32x32b_x4(dp_at + 4 * c8, pk_ds);
+          } else {
+            // (a row whose elements are all masked has LSE = -inf: as above)
+            float my_lse = sm->lse[0][0][vec_at];
+            if constexpr (kElementMask) my_lse = fmaxf(my_lse, -3.0e38f);
+            const float my_delta = sm->delta[0][0][vec_at];
+            tmem_ld_32x32b_x8(s_at, xsb[0]);
+            tmem_ld_32x32b_x8(dp_at, xdb[0]);
+#pragma unroll
+            for (int c8 = 0; c8 < 4; ++c8) {
+              uint32_t *xs = xsb[c8 & 1], *xd = xdb[c8 & 1], pk_ds[4];
+              tc_wait_ld();
+              if (partial) {
+#pragma unroll
+                for (int q4 = 0; q4 < 2; ++q4) {
+                  const uint32_t nz = __vcmpne4(mw[2 * c8 + q4], 0u);
+#pragma unroll
+                  for (int bb = 0; bb < 4; ++bb) {
+                    const uint32_t keep = __byte_perm(nz, 0u, 0x1111u * bb);
+                    xs[4 * q4 + bb] = (xs[4 * q4 + bb] & keep) | (0xff800000u & ~keep);
+                  }
+                }
+              }
+              if (c8 < 3) {
+                tmem_ld_32x32b_x8(s_at + 8 * c8 + 8, xsb[(c8 + 1) & 1]);
+                tmem_ld_32x32b_x8(dp_at + 8 * c8 + 8, xdb[(c8 + 1) & 1]);
+              }
+#pragma unroll
+              for (int q = 0; q < 8; q += 2) {
+                float z0, z1, ds0, ds1;
+                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(xs[q]), __uint_as_float(xs[q + 1])),
+                                       pack_f32x2(c, c), pack_f32x2(-my_lse, -my_lse)),
+                             z0, z1);
+                const uint64_t diff2 = add_f32x2(pack_f32x2(__uint_as_float(xd[q]), __uint_as_float(xd[q + 1])),
+                                                 pack_f32x2(-my_delta, -my_delta));
+                unpack_f32x2(mul_f32x2(pack_f32x2(ex2_approx(z0), ex2_approx(z1)), diff2), ds0, ds1);
+                pk_ds[q / 2] = pack_2x16<kBf16>(ds0, ds1);
+              }
+              tmem_st_32x32b_x4(dp_at + 4 * c8, pk_ds);
+            }
           }
         } else {
           uint32_t zero[16];

@@ -376,6 +376,23 @@ __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
+// Shapes 16x256b / 16x128b: 16 lanes (lane_base a multiple of 16 inside the warp's quarter) by 8 / 4 columns, N times
+// beside one another.  Thread i holds, of each 8 columns, columns 2 (i % 4) and 2 (i % 4) + 1 of lanes i / 4
+// (registers 0, 1) and i / 4 + 8 (registers 2, 3); of each 4, column i % 4 of the same two lanes.  So what it has read
+// as two columns of fp32 it can store as one of 16-bit pairs.
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_16x128b_x2(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]),
+               "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
+}
+
 // One 32-byte store (a whole sector) instead of two 16-byte ones; the address must be 32-byte
 // aligned.
 __device__ __forceinline__ void st_global_v8(void* p, const uint32_t* w) {
