@@ -364,6 +364,13 @@ __device__ __forceinline__ void bwd_produce(BwdSmem* sm, const BwdParams& p, con
   if (!ok) bwd_give_up(sm, p.status, 1);
 }
 
+// Write-out: a lane's 32 sums for the lane that finishes their columns.
+__device__ __forceinline__ void bwd_hand_over(float* at, const uint32_t* sums) {
+  uint4* to = reinterpret_cast<uint4*>(at);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) to[k] = make_uint4(sums[4 * k], sums[4 * k + 1], sums[4 * k + 2], sums[4 * k + 3]);
+}
+
 // The S/dP instructions of one team's supersteps (one warp).
 template <bool kBf16, bool kDKDV>
 __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uint32_t tmem, int team,
@@ -545,9 +552,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
-  // issuers do without (56 + 104 + 56 = 3 x 72).
+  // issuers do without (40 + 136 + 40 = 3 x 72).
   if ((warp >= kCW && warp < kCW + 4) || warp >= kCW + 8) {
-    give_registers<56>();
+    give_registers<40>();
     if (warp == kProdWarp) {
       bwd_produce<kDKDV, true>(sm, p, &tm_stat0, &tm_str0, lane);
     } else if (warp == kProd2Warp) {
@@ -749,7 +756,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     // [0, 32), lanes 64..127 columns [32, 64).
     // Both named barriers of an iteration are always executed, also after a give-up, and the
     // last one carries the give-up vote, so that no warp of this role is left waiting at one.
-    take_registers<104>();
+    take_registers<136>();
     const int quarter = warp & 3;
     const int half = quarter >> 1;
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the CTA's block
@@ -782,26 +789,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
       if (ok) ok = mbar_wait_warp(smem_u32(&sm->acc_done), ni & 1);
       ++ni;
       bool any_failed = false;
-#pragma unroll 1
-      for (int q = 0; q < kKeep; q += 32) {
-        uint32_t keep[32];
-        if (ok) {
-          uint4* to = reinterpret_cast<uint4*>(sm->xfer[half][r_blk]);
-          uint32_t send[32];
-          tc_fence_after();
-          tmem_ld_32x32b_x32(tm_send + q, send);
-          tmem_ld_32x32b_x32(tm_keep + q, keep);
-          tc_wait_ld();
+      // All sums are taken out of tensor memory before the first exchange, so that the next block may start
+      // accumulating.
+      uint32_t keep[kKeep], send[32];
+      if (ok) {
+        tc_fence_after();
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            to[k] = make_uint4(send[4 * k], send[4 * k + 1], send[4 * k + 2], send[4 * k + 3]);
-          if (q + 32 == kKeep) {
-            // the accumulators are out of tensor memory: the next block may start accumulating
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sm->acc_free));
-          }
+        for (int q = 0; q < kKeep; q += 32) {
+          if (q > 0) bwd_hand_over(sm->xfer[half][r_blk], send);
+          tmem_ld_32x32b_x32(tm_send + q, send);
+          tmem_ld_32x32b_x32(tm_keep + q, keep + q);
+          tc_wait_ld();
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sm->acc_free));
+        if (kKeep == 32) bwd_hand_over(sm->xfer[half][r_blk], send);
+      }
+#pragma unroll
+      for (int q = 0; q < kKeep; q += 32) {
+        if (q > 0 && ok) bwd_hand_over(sm->xfer[half][r_blk], send);
         named_barrier_sync(2, 128);
         if (ok) {
           const float4* from = reinterpret_cast<const float4*>(sm->xfer[half ^ 1][r_blk]);
@@ -813,10 +820,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
 #pragma unroll
               for (int k = 0; k < 4; ++k) {
                 const float4 x = from[v / 4 + k];
-                o[2 * k] = pack_2x16<kBf16>((__uint_as_float(keep[v + 4 * k]) + x.x) * scale,
-                                            (__uint_as_float(keep[v + 4 * k + 1]) + x.y) * scale);
-                o[2 * k + 1] = pack_2x16<kBf16>((__uint_as_float(keep[v + 4 * k + 2]) + x.z) * scale,
-                                                (__uint_as_float(keep[v + 4 * k + 3]) + x.w) * scale);
+                const uint32_t* mine = keep + q + v + 4 * k;
+                o[2 * k] = pack_2x16<kBf16>((__uint_as_float(mine[0]) + x.x) * scale, (__uint_as_float(mine[1]) + x.y) * scale);
+                o[2 * k + 1] = pack_2x16<kBf16>((__uint_as_float(mine[2]) + x.z) * scale, (__uint_as_float(mine[3]) + x.w) * scale);
               }
               // 16 columns go out as one whole sector when the rows start on such boundaries
               if (p.wide_stores) {
