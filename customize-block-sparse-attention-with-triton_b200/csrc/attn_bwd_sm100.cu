@@ -49,8 +49,8 @@
 //                 already at work on the next block
 // A block's own operands are double-buffered: the next block's are loaded while this one is at work.
 // Head dimensions 16 and 32: zero-filled on load by D-wide tensor maps, D / 16 K steps for S and dP.
-// S and dP of a superstep have one of three slots in TMEM, and P and dS are stored over them: the
-// next superstep but two is what its products must be complete for, not the team's own next one.
+// S and dP of a superstep have slots in TMEM, and P and dS are stored over S: a slot of S is held until their
+// products are complete, one of dP only until the arithmetic is done.
 // What bounds it: the way of a superstep through three slots, with no part of it that is the bound alone.
 // A dK/dV superstep takes 1,200 to 1,290 cycles, of which shared memory's port about 1,000 (S and dP
 // operands 384, accumulating operands 256, copies arriving 256, LSE2 and delta 128), the tensor pipe 900, the
@@ -69,10 +69,10 @@ namespace bsa {
 
 // The streamed tiles: ten places of two tiles (16 KB), split into a ring for Q (dK/dV) or K (dQ) and one
 // for dO or V.  What an accumulating product reads (Q and dO; K) is held from its load to the end of
-// that product, about 5,000 cycles with the arithmetic in between; V only until dP is complete.  With
-// rings too short for that the issuers wait for operands (four places each: a third of the time).
+// that product, about 4,500 cycles with the arithmetic in between; V only until dP is complete.  With
+// rings too short for that the issuers wait for operands (dK/dV, four places each: a third of the time).
 constexpr int kRing = 10;
-template <bool kDKDV> constexpr int kRing0 = kDKDV ? 5 : 7;
+template <bool kDKDV> constexpr int kRing0 = kDKDV ? 5 : 6;
 template <bool kDKDV> constexpr int kRing1 = kRing - kRing0<kDKDV>;
 constexpr int kCW = 16;                    // compute warps: 2 teams x 4 lane quarters x 2 column halves
 constexpr int kTeamW = kCW / 2;
@@ -84,18 +84,27 @@ constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: one warp at t
 constexpr uint32_t kBwdTile = 64 * 64 * 2;
 constexpr uint32_t kBwdTmemCols = 512;
 constexpr int kListIndex = BSA_LIST_PARTIAL_FLAG - 1;  // a list entry without its flag
-// TMEM columns: slot x at 128 x holds S (or S^T) and, 64 further on, dP (or dP^T) of supersteps
-// g % kSlots == x; then P (as 16-bit pairs) over the first half of each 32 columns of S, dS over
-// those of dP: a warp only overwrites what it has read itself.  Two fp32 accumulators.
+// TMEM columns: S (or S^T) of superstep g in slot g % kSlots, 64 columns each, dP (or dP^T) behind them in slot
+// g % kDpSlots; two fp32 accumulators at the end (dQ: one).  P and dS (as 16-bit pairs) go over the 16 columns of S
+// that they come from, P into the first 8 and dS into the last 8 of them (dQ: dS into the first 8): a warp only
+// overwrites what it has read itself.  So a dP slot is free as soon as the arithmetic is done, and where there is one
+// accumulator S can be four supersteps deep: dQ with everything listed, 2 heads, N = 9600, forward and backward 280 us
+// with 3 + 3 slots, 272.5 so, lists of 16 supersteps the same.  (dK/dV with 4 + 2: both teams fall into step, at
+// 1,394 us for 2 x 16 heads, N = 16384 against 1,377.)
+constexpr int kDpSlots = 3;
+template <bool kDKDV> constexpr int kSlots = kDKDV ? 3 : 4;
+template <bool kDKDV> constexpr uint32_t kTmDp = 64 * kSlots<kDKDV>;
 constexpr uint32_t kTmAcc0 = 384, kTmAcc1 = 448;
-// The issuers and teams see every second superstep, so the barriers that they wait on come twice for
-// each slot.
-constexpr int kSlots = 3, kXBars = 2 * kSlots;
+static_assert(kTmDp<true> + 64 * kDpSlots <= kTmAcc0 && kTmDp<false> + 64 * kDpSlots <= kTmAcc1);
+// Barriers by superstep: an even number, so that the issuers and teams, which see every second superstep, see each
+// phase of theirs, and more than there are supersteps between those that look at one and those that complete it.
+constexpr int kXBars = 6;
+static_assert(kXBars % 2 == 0 && kXBars > kSlots<false> && kXBars > kRing0<true> && kXBars > kRing1<true>);
 // dQ: places of a block's LSE2 and delta, which are read at each of its supersteps.  Those of block n are fetched when
-// all S/dP of block n-2 are complete, and with that the arithmetic of all but its last kSlots supersteps: what
+// all S/dP of block n-2 are complete, and with that the arithmetic of all but its last kDpSlots supersteps: what
 // block n-5 has is not read any more, even if all blocks have a single superstep.
 constexpr int kVecPlaces = 5;
-static_assert(kVecPlaces >= kSlots + 2 && kVecPlaces <= kRing0<true> && kVecPlaces <= kRing1<true>);
+static_assert(kVecPlaces >= kDpSlots + 2 && kVecPlaces <= kRing0<true> && kVecPlaces <= kRing1<true>);
 
 struct BwdSmem {
   uint8_t stat[2][2][kBwdTile];             // by block parity: the CTA's own K, V (dK/dV) or Q, dO (dQ)
@@ -119,10 +128,10 @@ struct BwdSmem {
   uint64_t in_full0[2 * kRing0<false>], in_full1[2 * kRing1<true>];
   uint64_t in_empty0[kRing0<false>];        // dQ: accumulating MMAs that read the place of K complete
   uint64_t in_empty1[kRing1<false>];        // dQ: dP complete, the place of V is free (dK/dV goes by d_free)
-  // by superstep modulo kXBars, that is by slot and team:
+  // by superstep modulo kXBars:
   uint64_t x_full[kXBars];                  // S/dP complete (dK/dV: and LSE2 and delta there)
-  uint64_t d_free[kXBars];                  // accumulating MMAs that read P/dS complete: the slot is free
-  uint64_t d_full[kSlots];                  // by slot: P/dS stored
+  uint64_t d_full[kXBars];                  // P/dS stored: the slot of dP is free
+  uint64_t d_free[kXBars];                  // accumulating MMAs that read P/dS complete: the slot of S is free
   uint32_t tmem_base;
   int abort_flag;                           // a role has given up
 };
@@ -380,7 +389,7 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
   const uint64_t desc_a0 = smem_desc_sw128(smem_u32(sm->stat[0][0]), 16, 1024);
   const uint64_t desc_b0 = smem_desc_sw128(smem_u32(sm->ring[0][0]), 16, 1024);
   const uint64_t desc_b1 = smem_desc_sw128(smem_u32(sm->ring[kRing0<kDKDV>][0]), 16, 1024);
-  constexpr int kR0 = kRing0<kDKDV>, kR1 = kRing1<kDKDV>;
+  constexpr int kR0 = kRing0<kDKDV>, kR1 = kRing1<kDKDV>, kDp = kDpSlots, kS = kSlots<kDKDV>;
   constexpr uint64_t kTileDesc = kBwdTile >> 4;  // one tile further, in descriptor units
   const int k_steps = p.D >> 4;
   bool ok = true;
@@ -400,27 +409,31 @@ __device__ __forceinline__ void bwd_issue_x(BwdSmem* sm, const BwdParams& p, uin
     gs += n_super;
 #pragma unroll 1
     for (; ok && g < gs; g += 2) {
-      // (three looks, one vote)
-      bool seen = mbar_poll(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1, kWaitTries);
-      seen &= mbar_poll(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1, kWaitTries);
-      // the accumulating products of the slot's previous superstep must be complete
-      if (g >= kSlots)
-        seen &= mbar_poll(smem_u32(&sm->d_free[(g - kSlots) % kXBars]), ((g - kSlots) / kXBars) & 1, kWaitTries);
-      ok = __all_sync(0xffffffffu, seen);
+      const uint32_t s_tmem = tmem + 64 * (g % kS), dp_tmem = tmem + kTmDp<kDKDV> + 64 * (g % kDp);
+      const uint32_t x_full = smem_u32(&sm->x_full[g % kXBars]);
+      const uint64_t b0 = desc_b0 + static_cast<uint64_t>(2 * (g % kR0)) * kTileDesc;
+      const uint64_t b1 = desc_b1 + static_cast<uint64_t>(2 * (g % kR1)) * kTileDesc;
+      // the tiles, and the accumulating products of the slot's previous superstep must be complete (the first
+      // ones ask for the phase before the first one, which counts as complete)
+      ok = mbar_wait_warp2(smem_u32(&sm->in_full0[g % (2 * kR0)]), (g / (2 * kR0)) & 1,
+                           smem_u32(&sm->d_free[(g + kXBars - kS) % kXBars]), ((g + kXBars - kS) / kXBars + 1) & 1);
       if (!ok) break;
       tc_fence_after();
       if (leader) {
-        const uint32_t x_at = tmem + 128 * (g % kSlots);
-        const uint32_t x_full = smem_u32(&sm->x_full[g % kXBars]);
-        const uint64_t b0 = desc_b0 + static_cast<uint64_t>(2 * (g % kR0)) * kTileDesc;
-        const uint64_t b1 = desc_b1 + static_cast<uint64_t>(2 * (g % kR1)) * kTileDesc;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          if (kk < k_steps) umma_ws_ss(x_at, a0 + 2 * kk, b0 + 2 * kk, idesc_x, kk > 0);
+          if (kk < k_steps) umma_ws_ss(s_tmem, a0 + 2 * kk, b0 + 2 * kk, idesc_x, kk > 0);
+      }
+      __syncwarp();
+      // the arithmetic on the slot's previous superstep must be done
+      ok = mbar_wait_warp2(smem_u32(&sm->in_full1[g % (2 * kR1)]), (g / (2 * kR1)) & 1,
+                           smem_u32(&sm->d_full[(g + kXBars - kDp) % kXBars]), ((g + kXBars - kDp) / kXBars + 1) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      if (leader) {
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          if (kk < k_steps)
-            umma_ws_ss(x_at + 64, a0 + kTileDesc + 2 * kk, b1 + 2 * kk, idesc_x, kk > 0);
+          if (kk < k_steps) umma_ws_ss(dp_tmem, a0 + kTileDesc + 2 * kk, b1 + 2 * kk, idesc_x, kk > 0);
         tc_commit(x_full);
         mbar_arrive(x_full);  // release: LSE2 and delta have been seen to be there
         if constexpr (!kDKDV) tc_commit(smem_u32(&sm->in_empty1[g % kR1]));  // V is not needed any more
@@ -443,10 +456,10 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
   const int places = dv ? kRing1<kDKDV> : kRing0<kDKDV>;
   const uint64_t desc = smem_desc_sw128(smem_u32(sm->ring[dv ? kRing0<kDKDV> : 0][0]), 8192, 1024);
   const uint32_t empty = smem_u32(sm->in_empty0);  // (dQ)
-  const uint32_t acc = tmem + (dv ? kTmAcc0 : kTmAcc1), from = tmem + (dv ? 0 : 64);
+  const uint32_t acc = tmem + (dv ? kTmAcc0 : kTmAcc1), from = tmem + (kDKDV && !dv ? 8 : 0);
   bool ok = true;
   int ni = 0, place = 0, slot = 0, x = 0;
-  uint32_t phase = 0;  // of the slot's barrier
+  uint32_t phase = 0;  // of the superstep's barrier
   bwd_begin<kDKDV>(p);
 #pragma unroll 1
   for (int i = 0; ok; ++i) {
@@ -458,27 +471,27 @@ __device__ __forceinline__ void bwd_issue_acc(BwdSmem* sm, const BwdParams& p, u
     if (ni >= 1) ok = mbar_wait_warp(smem_u32(&sm->acc_free), (ni - 1) & 1);
 #pragma unroll 1
     for (int left = it.n_tiles; ok && left > 0; left -= 2) {
-      ok = mbar_wait_warp(smem_u32(&sm->d_full[slot]), phase);
+      ok = mbar_wait_warp(smem_u32(&sm->d_full[x]), phase);
       if (!ok) break;
       tc_fence_after();
       if (leader) {
-        // rows [16 kk, +16) of a streamed tile: column 8 (kk % 2) of the 32 columns of P or dS of warp
-        // column half kk / 2; tile a's in lanes 0..63, tile b's in lanes 64..127.  (A product for each
+        // rows [16 kk, +16) of a streamed tile: those of P or dS in the first or last 8 of columns [16 kk, +16) of
+        // their slot; tile a's in lanes 0..63, tile b's in lanes 64..127.  (A product for each
         // tile, with the other's lanes switched off: bf16 2 x 16 heads, N = 16384, causal, a quarter, forward
         // and backward 1,835 us, 1,785 so; 2 x 8 heads, N = 4160 97.5 and 96.2.)
-        const uint32_t cols = from + 128 * slot;
+        const uint32_t cols = from + 64 * slot;
         const uint64_t b0 = desc + static_cast<uint64_t>(2 * place * (kBwdTile >> 4));
         const uint32_t more = left != it.n_tiles;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_ws_ts(acc, cols + 32 * (kk >> 1) + 8 * (kk & 1), b0 + 128 * kk, idesc, more | (kk > 0));
+          umma_ws_ts(acc, cols + 16 * kk, b0 + 128 * kk, idesc, more | (kk > 0));
         if constexpr (!kDKDV) tc_commit(empty + 8 * place);  // place free
         tc_commit(smem_u32(&sm->d_free[x]));  // P or dS columns free; accumulator updated
         if (left <= 2) tc_commit(smem_u32(&sm->acc_done));  // the block's sums are final
       }
       if (++place == places) place = 0;
-      if (++x == kXBars) x = 0;
-      if (++slot == kSlots) slot = 0, phase ^= 1;
+      if (++slot == kSlots<kDKDV>) slot = 0;
+      if (++x == kXBars) x = 0, phase ^= 1;
     }
     ++ni;
   }
@@ -513,7 +526,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     mbar_init_warp(sm->setup_go, 2, 1, lane);
     mbar_init_warp(sm->stat_full, 2, 2, lane);        // two producers
     mbar_init_warp(sm->stat_free, 2, 2, lane);        // two S/dP issuers
-    mbar_init_warp(sm->d_full, kSlots, kTeamW, lane);  // one arrival per warp
+    mbar_init_warp(sm->d_full, kXBars, kTeamW, lane);  // one arrival per warp
     mbar_init_warp(sm->x_full, kXBars, 2, lane);      // the commit and the issuer
     mbar_init_warp(sm->d_free, kXBars, kDKDV ? 2 : 1, lane);
     mbar_init_warp(sm->in_full0, 2 * kRing0<false>, 1, lane);
@@ -603,7 +616,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
 #pragma unroll 1
       for (; ok && j < n_super; j += 2, g += 2) {
         const bool active = 2 * j + t_mine < it.n_tiles;  // this lane's tile exists (warp-uniform)
-        const uint32_t s_at = x_base + 128 * (g % kSlots), dp_at = s_at + 64;
+        const uint32_t s_at = x_base + 64 * (g % kSlots<kDKDV>), dp_at = x_base + kTmDp<kDKDV> + 64 * (g % kDpSlots);
         // A tile with masked elements inside: fetch this lane's 32 mask bytes while S is on its way
         uint32_t mw[8];
         bool partial = false;
@@ -685,9 +698,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
                 pk_p[e] = pack_2x16<kBf16>(p0, p1);
                 pk_ds[e] = pack_2x16<kBf16>(ds0, ds1);
               }
-              const uint32_t to = 8 * (n >> 1) + (static_cast<uint32_t>(16 * (n & 1)) << 16);
-              tmem_st_16x128b_x2(s_at + to, pk_p);
-              tmem_st_16x128b_x2(dp_at + to, pk_ds);
+              const uint32_t to = s_at + 16 * (n >> 1) + (static_cast<uint32_t>(16 * (n & 1)) << 16);
+              tmem_st_16x128b_x2(to, pk_p);
+              tmem_st_16x128b_x2(to + 8, pk_ds);
             }
           } else {
             // (a row whose elements are all masked has LSE = -inf: as above)
@@ -726,20 +739,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
                 unpack_f32x2(mul_f32x2(pack_f32x2(ex2_approx(z0), ex2_approx(z1)), diff2), ds0, ds1);
                 pk_ds[q / 2] = pack_2x16<kBf16>(ds0, ds1);
               }
-              tmem_st_32x32b_x4(dp_at + 4 * c8, pk_ds);
+              tmem_st_32x32b_x4(s_at + 16 * (c8 >> 1) + 4 * (c8 & 1), pk_ds);
             }
           }
         } else {
           uint32_t zero[16];
 #pragma unroll
           for (int k = 0; k < 16; ++k) zero[k] = 0u;
-          if constexpr (kDKDV) tmem_st_32x32b_x16(s_at, zero);
-          tmem_st_32x32b_x16(dp_at, zero);
+          tmem_st_32x32b_x16(s_at, zero);
+          tmem_st_32x32b_x16(s_at + 16, zero);
         }
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sm->d_full[g % kSlots]));
+        if (lane == 0) mbar_arrive(smem_u32(&sm->d_full[g % kXBars]));
       }
       // (the block's sums are merged and stored by the write-out warps; these warps go straight
       // on to the next block, whose first S/dP is usually complete already)
