@@ -159,6 +159,16 @@ __device__ __forceinline__ bool mbar_wait_warp2(uint32_t bar0, uint32_t parity0,
   return __all_sync(0xffffffffu, ok);
 }
 
+__device__ __forceinline__ bool mbar_wait_warp3(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
+                                                uint32_t bar2, uint32_t parity2) {
+  const bool seen0 = mbar_try_wait(bar0, parity0), seen1 = mbar_try_wait(bar1, parity1), seen2 = mbar_try_wait(bar2, parity2);
+  bool ok = true;
+  if (!seen0) ok = mbar_poll(bar0, parity0, kWaitTries);
+  if (!seen1) ok &= mbar_poll(bar1, parity1, kWaitTries);
+  if (!seen2) ok &= mbar_poll(bar2, parity2, kWaitTries);
+  return __all_sync(0xffffffffu, ok);
+}
+
 // The same for the beginning of an item, where a role comes that still had work when another one gave up: it
 // looks at the CTA's flag every quarter of a second.
 constexpr int kItemBatches = 8;
