@@ -34,7 +34,7 @@
 // 116.5 us (118.4 with a P V issuer of three waits and unrolled loops, in turn on one GPU), a tenth of them 18.5 us
 // (19.6); 8 heads, a tenth 112.6 us (118.9); bf16 N = 32000, 32 heads, a tenth 1.295 ms (1.310), at the power cap.
 //
-// Roles (16 warps); every role walks the same item sequence, so set-up of item i+1 and write-out
+// Roles (17 warps of 20); every role walks the same item sequence, so set-up of item i+1 and write-out
 // of item i-1 overlap the arithmetic of item i:
 //   warps 0..7  : online softmax (team = warp / 4, TMEM lane quarter = warp % 4; superstep g is team
 //                 g % 2's).  A warp loads its tiles' 128 logits, exponentiates them, packs P to 16 bit
@@ -52,8 +52,15 @@
 //                 are ever loaded.
 //   warps 12..15: write-out — merge the four partial results (m, l, O) of every query row (teams x
 //                 lanes r / r+64), normalise, store O, LSE and the row maximum
-//   warp 15     : also the lister — draws the items, lists their key blocks (from the mask row, or
-//                 copies the CSR row) into the next of three list buffers and publishes them
+//   warp 18     : lister — draws the items, lists their key blocks (from the mask row, or copies the CSR row)
+//                 into the next of three list buffers and publishes them
+// The lister was one of the write-out warps: ticket, list and write-out one after the other took 4,100 cycles an item,
+// more than an item of three supersteps does.  With a warp of its own, and an item there as soon as the one before the
+// one before the previous one has been written out: 24 heads, N = 4160, D = 32, a quarter 46.1 -> 42.6 us; bf16
+// 2 x 16 heads, N = 16384, causal, a quarter 412 -> 390; 8 heads, N = 17536, a tenth 99.2 -> 97.6; lists of one item a CTA the
+// same.  It matters which quarter of the SM it runs in, beside the K producer (warp 16), the S issuer (17), the P V
+// issuer (18) or the V producer (19): 32 heads, N = 32000 1,152 / 1,149 / 1,141 / 1,139 us (1,142 before).  (The K
+// producer as lister: 8 heads 99 -> 103.)
 // TMEM (512 columns): S/P slots 3 x 128, accumulators 2 x 64.
 //
 // Head dimensions 16 and 32 run on the same 128-byte rows: the tensor maps are D wide, so TMA fills
@@ -68,8 +75,8 @@
 // goes into depends on its position in the row's list alone, so results do not depend on which CTA
 // computes an item.
 //
-// Every wait is bounded.  A role that gives up leaves its loops and raises a CTA-wide flag, which the sleeping waits
-// and those for an item look at; a role in the middle of an item runs out by itself, within the same
+// Every wait is bounded.  A role that gives up leaves its loops and raises a CTA-wide flag, which the waits for an
+// item and of the write-out look at; a role in the middle of an item runs out by itself, within the same
 // 2 seconds or so.  TMEM is always released.  Every
 // barrier is waited on only by warps that see each of its phases, or that know the barrier to be
 // at most one phase behind (a parity wait cannot tell a phase from the one two before it).
@@ -87,8 +94,8 @@ constexpr int kLists = 3;       // items set up at a time: one being worked on, 
 constexpr int kSoftmaxWarps = 8;
 constexpr int kTeamWarps = kSoftmaxWarps / 2;
 constexpr int kProducerWarp = 8, kSWarp = 9, kPvWarp = 10, kVProducerWarp = 11;
-constexpr int kListerWarp = 15;      // the last of the write-out warps 12..15: also sets up the items
-constexpr int kFwdThreads = 512;
+constexpr int kListerWarp = 18;
+constexpr int kFwdThreads = 32 * 20;  // whole warpgroups: one warp at the end fills one
 constexpr int kGoBefore = 2;         // supersteps before an item's end at which the next is set up
 constexpr uint32_t kTileBytes = 64 * 64 * 2;       // one Q, K or V tile
 constexpr uint32_t kFwdTmemCols = 512;
@@ -112,21 +119,21 @@ struct FwdSmem {
   float xfer[2][64][20];
   uint16_t cols[kLists][kFwdMaxTiles];        // ring over the items: the item's key-block list (| kColPartial)
   int4 item[kLists];                          // the item: batch (-1 = no more work), head, query block, tile count
-  float mref[2][2][128];                      // by item parity, softmax team, lane
-  float lsum[2][2][128];
-  float mtrue[2][2][128];
+  float mref[kLists][2][128];                 // by list buffer of the item, softmax team, lane
+  float lsum[kLists][2][128];
+  float mtrue[kLists][2][128];
   uint64_t list_full[kLists];                 // lister -> everyone: list and header ready
-  uint64_t list_free[kLists];                 // producers and issuers are through with list and header
+  uint64_t list_free[kLists];                 // everyone is through with list, header and statistics
   uint64_t setup_go[2];                       // producer -> lister: time to set up the next item
-  uint64_t q_full[2];
-  uint64_t k_full[kKStages];
+  uint64_t q_free[2];                         // S of the item complete
+  uint64_t k_full[kKStages];                  // the superstep's K tiles (and, with an item's first, its Q) are there
   uint64_t k_empty[kKStages];                 // S of the superstep complete
   uint64_t s_full[2 * kSlots];                // S of the superstep complete; one per (team, slot), so
                                               // that the team that waits on it sees each phase
   uint64_t p_full[kSlots];                    // the team's four warps stored P of the superstep, its V has landed
   uint64_t pv_done[kSlots];                   // P V of the superstep complete: slot and V places free, O current
   uint64_t o_full[2];                         // last P V of the item done
-  uint64_t stats_full[2];                     // softmax warps published (m, l) of the item
+  uint64_t stats_full[kLists];                // softmax warps published (m, l) of the item
   uint64_t o_free[2];                         // write-out has read accumulators, stats and header
   uint32_t tmem_base;
   int abort_flag;
@@ -283,8 +290,8 @@ __device__ __forceinline__ const uint8_t* fwd_mask_row(const FwdItem& it, const 
          static_cast<int64_t>(it.mb) * p.ms2;
 }
 
-// Lists the key blocks of work item w into list buffer `at` (one warp) and publishes list and item.
-template <bool kElementMask, bool kPublish>
+// Lists the key blocks of work item w into list buffer `at` (one warp), with the item itself.
+template <bool kElementMask>
 __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, int w, int at,
                                               int lane) {
   const FwdItem it = fwd_item(w, p);
@@ -351,11 +358,7 @@ __device__ __forceinline__ void fwd_list_item(FwdSmem* sm, const FwdParams& p, i
           (e & kColIndex) | (kElementMask && (e & BSA_LIST_PARTIAL_FLAG) ? kColPartial : 0));
     }
   }
-  __syncwarp();
-  if (lane == 0) {
-    sm->item[at] = make_int4(it.b, it.h, it.mb, n_tiles);
-    if constexpr (kPublish) mbar_arrive(smem_u32(&sm->list_full[at]));  // release: list and item are visible
-  }
+  if (lane == 0) sm->item[at] = make_int4(it.b, it.h, it.mb, n_tiles);
 }
 
 // A role's walk over the items: waits for the next one to be published and reads its header.
@@ -387,7 +390,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   FwdSmem* sm = reinterpret_cast<FwdSmem*>(smem_raw);
 
-  const int warp = uniform_warp_index();
+  // (the lister's warps come first: the first list is what all others wait for)
+  const int hw_warp = uniform_warp_index(), warp = hw_warp >= 4 ? hw_warp - 4 : hw_warp + 16;
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x;
   const int n2 = p.items - stride;  // items beyond the first round
@@ -395,9 +399,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // ---- set-up ----
   if (warp == 0) {
     mbar_init_warp(sm->setup_go, 2, 1, lane);
-    mbar_init_warp(sm->q_full, 2, 1, lane);
+    mbar_init_warp(sm->q_free, 2, 1, lane);
     mbar_init_warp(sm->o_full, 2, 1, lane);
-    mbar_init_warp(sm->stats_full, 2, kSoftmaxWarps, lane);
+    mbar_init_warp(sm->stats_full, kLists, kSoftmaxWarps, lane);
     mbar_init_warp(sm->o_free, 2, 4, lane);  // one arrival per write-out warp
     mbar_init_warp(sm->k_full, kKStages, 1, lane);
     mbar_init_warp(sm->k_empty, kKStages, 1, lane);
@@ -405,7 +409,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     mbar_init_warp(sm->p_full, kSlots, kTeamWarps + 1, lane);
     mbar_init_warp(sm->pv_done, kSlots, 1, lane);
     mbar_init_warp(sm->list_full, kLists, 1, lane);
-    mbar_init_warp(sm->list_free, kLists, 4, lane);  // two producers, two issuers
+    mbar_init_warp(sm->list_free, kLists, 8, lane);  // two producers, two issuers, four write-out warps
     if (lane == 0) sm->abort_flag = 0;
     mbar_fence_init();
   }
@@ -426,7 +430,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // kernel may use comes after this.
     grid_dependency_wait();
     if (p.successor_early) grid_dependents_launch();
-    fwd_list_item<kElementMask, false>(sm, p, blockIdx.x, 0, lane);
+    fwd_list_item<kElementMask>(sm, p, blockIdx.x, 0, lane);
     named_barrier_sync(1, kFwdThreads);  // the barriers are there
     if (lane == 0) mbar_arrive(smem_u32(&sm->list_full[0]));
   } else {
@@ -437,13 +441,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const uint32_t tmem = sm->tmem_base;
   volatile int* abort_flag = &sm->abort_flag;
 
-  // 512 threads are launched with 128 registers: the softmax warps, which hold 64 logits and 128
-  // probabilities each, take what the others do without (2 x 168 + 72 + 104 = 4 x 128; with an element mask, whose
-  // row and bytes they hold as well, 2 x 184 + 56 + 88).  A spill in their loop (28 bytes at 160; 112 with
-  // an element mask at 168) made the kernel 4 to 5 % slower: causal by element, 10 heads, N = 2048 18.9 / 17.3 us,
-  // a dense mask of whole blocks, one head, N = 6400 19.0 / 18.6.
+  // 640 threads are launched with 96 registers: the softmax warps, which hold 64 logits and 128 probabilities each,
+  // take what the others do without (2 x 160 + 40 + 88 + 32 = 5 x 96).  The write-out needs its 88: with 80 or 72 short
+  // lists are 1 or 2 % slower.
   if (warp >= kSoftmaxWarps && warp < kSoftmaxWarps + 4) {
-  give_registers<kElementMask ? 56 : 72>();
+  give_registers<40>();
   if (warp == kProducerWarp) {
     // =========================== K producer ===========================
     bool ok = true;
@@ -464,16 +466,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int n_tiles = walk.it.w;
       const uint16_t* cols = sm->cols[walk.at];
       const int n_super = (n_tiles + 3) >> 2;
-      if (n_super > 0) {
-        // (free: that an item is set up means that the item before the previous one has been written out)
-        const int qpar = qi & 1;
-        if (lane == 0) {
-          const uint32_t bar = smem_u32(&sm->q_full[qpar]);
-          mbar_expect_tx(bar, kTileBytes);
-          tma_load_4d(smem_u32(sm->q[qpar]), &tm_q, bar, 0, walk.it.z * 64, walk.it.y, walk.it.x);
-        }
-        ++qi;
-      }
       const int u_go = max(n_super - kGoBefore, 0);
       if (n_super == 0 && lane == 0) mbar_arrive(smem_u32(&sm->setup_go[par]));
       // One lane per tile issues its load: a single thread can start a tile load only every couple
@@ -482,10 +474,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int u = 0; u < n_super; ++u) {
         if (u == u_go && lane == 0) mbar_arrive(smem_u32(&sm->setup_go[par]));
         const int nt = min(4, n_tiles - 4 * u);
-        ok = mbar_wait_warp(smem_u32(&sm->k_empty[ks]), kph);
+        const int qpar = qi & 1;
+        // (the item before the previous one is through with its Q as long as this one lasts)
+        ok = mbar_wait_warp2(smem_u32(&sm->k_empty[ks]), kph, smem_u32(&sm->q_free[qpar]), ((qi >> 1) & 1) ^ 1);
         if (!ok) break;
         const uint32_t bar = smem_u32(&sm->k_full[ks]);
-        if (lane == 0) mbar_expect_tx(bar, kTileBytes * nt);
+        if (lane == 0) {
+          mbar_expect_tx(bar, kTileBytes * (nt + (u == 0)));
+          if (u == 0) tma_load_4d(smem_u32(sm->q[qpar]), &tm_q, bar, 0, walk.it.z * 64, walk.it.y, walk.it.x);
+        }
         __syncwarp();
         if (lane < nt) {  // in shared memory a, c, b, d; only a, b: next to each other
           const int at = nt > 2 ? ((lane & 1) << 1) | (lane >> 1) : lane;
@@ -494,6 +491,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         if (++ks == kKStages) { ks = 0; kph ^= 1; }
       }
+      if (n_super > 0) ++qi;
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
     }
@@ -564,8 +562,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (lane == 0) mbar_arrive(smem_u32(&sm->list_free[walk.at]));
       if (n_super == 0) continue;
       const int qpar = qi & 1;
-      ok = mbar_wait_warp(smem_u32(&sm->q_full[qpar]), (qi >> 1) & 1);
-      if (!ok) break;
       const uint64_t desc_q = desc_q0 + static_cast<uint64_t>(qpar) * kTileDesc;
 #pragma unroll 1
       for (int u = 0; u < n_super; ++u) {
@@ -588,6 +584,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (kk < k_steps) umma_ws_ss(d, desc_q + 2 * kk, desc_k + 2 * kk, idesc, kk > 0);
           tc_commit(smem_u32(&sm->s_full[bar_s]));
           tc_commit(smem_u32(&sm->k_empty[ks]));
+          if (u == n_super - 1) tc_commit(smem_u32(&sm->q_free[qpar]));
         }
         if (++ks == kKStages) { ks = 0; kph ^= 1; }
         if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
@@ -660,7 +657,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   } else if (warp < kSoftmaxWarps) {
     // =========================== softmax ===========================
-    take_registers<kElementMask ? 184 : 168>();
+    take_registers<160>();
     const int team = warp >> 2;
     const int quarter = warp & 3;     // TMEM lane quarter this warp may touch
     const int half = quarter >> 1;    // lanes 0..63 own tiles a, c of a superstep, 64..127 b, d
@@ -676,7 +673,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     FwdWalk walk;
 #pragma unroll 1
     for (int i = 0; ok; ++i, walk.next()) {
-      const int par = i & 1;
       ok = walk.wait(sm);
       if (!ok || walk.it.x < 0) break;  // (no more work)
       const int n_tiles = walk.it.w;
@@ -803,33 +799,26 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if (!ok) break;
       g += n_super;
 
-      // publish this item's (m, l) of the warp's lanes (that this item was set up means that item i-2,
-      // whose slots these were, has been written out)
-      sm->mref[par][team][lane_row] = m_ref;
-      sm->lsum[par][team][lane_row] = l;
-      if (want_max) sm->mtrue[par][team][lane_row] = m_true;
+      // publish this item's (m, l) of the warp's lanes (that this item is there means that the one that had its list
+      // buffer has been written out)
+      sm->mref[walk.at][team][lane_row] = m_ref;
+      sm->lsum[walk.at][team][lane_row] = l;
+      if (want_max) sm->mtrue[walk.at][team][lane_row] = m_true;
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sm->stats_full[par]));
+      if (lane == 0) mbar_arrive(smem_u32(&sm->stats_full[walk.at]));
     }
     if (!ok) fwd_give_up(sm, p.status, kFailSoftmax);
-  } else {
+  } else if (warp < kSoftmaxWarps + 8) {
     // =========================== write-out ===========================
     // Merges the four partial results of every query row (first / second team of the item x lanes
     // r / r+64).  A warp reads both accumulators of its own lanes from TMEM; lanes 64..127 hand
     // their weighted rows to each other through shared memory, 16 columns at a time.  All named
     // barriers of an iteration are always executed, also after a give-up, and the last one carries
     // the give-up vote, so that no warp of this role can be left waiting at one.
-    //
-    // One of the four warps is also the lister: it sets up item i+1 when the producer says so during item i,
-    // i.e. between its write-outs of items i-1 and i (the CTA's first item at the very beginning).
-    give_registers<kElementMask ? 88 : 104>();
+    give_registers<88>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
-    const bool lister = warp == kListerWarp;
     bool ok = true;
-    bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
-    int lw = blockIdx.x;
     const int half = quarter >> 1;
-    const int lane_row = quarter * 32 + lane;
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the query block
     const uint32_t o_lanes = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + kTmemO;
     int g = 0;  // supersteps of earlier items
@@ -837,44 +826,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll 1
     for (int i = 0;; ++i) {
       const int par = i & 1;
-      if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag, 256);
+      if (ok) ok = mbar_wait_warp_item(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag);
       walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
       if (walk.it.x < 0) break;  // no more work: the same for all four warps
-      if (lister && ok) {
-        // Sets up the next item, or publishes that there is none; a wait that gives up leaves ok =
-        // false and nothing published.  The next ticket when items are handed out dynamically, else
-        // a fixed stride.
-        const int at = walk.at + 1 < kLists ? walk.at + 1 : 0;
-        ok = mbar_wait_warp(smem_u32(&sm->setup_go[par]), (i >> 1) & 1);
-        if (ok && p.ticket != nullptr) {
-          int t = 0;
-          if (lane == 0) {
-            t = atomicAdd(p.ticket, 1);
-            // every CTA draws until its first ticket past the end, so the launch draws exactly
-            // `items` tickets in all; whoever draws the last one leaves the counter at zero
-            if (t == p.items - 1) atomicExch(p.ticket, 0);
-          }
-          t = __shfl_sync(0xffffffffu, t, 0);
-          terminal = t >= n2;
-          lw = stride + t;
-        } else {
-          lw += stride;
-        }
-        // The list buffer was that of item i-2, which these warps have written out (and the softmax
-        // warps with them are through with); the producers and issuers may lag behind.
-        if (ok && i >= 2)
-          ok = mbar_wait_warp_idle(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag, 128);
-        if (ok) {
-          if (lw < p.items) {
-            fwd_list_item<kElementMask, true>(sm, p, lw, at, lane);
-          } else if (lane == 0) {
-            sm->item[at].x = -1;
-            mbar_arrive(smem_u32(&sm->list_full[at]));
-          }
-        }
-      }
       const int n_tiles = walk.it.w;
-      if (ok) ok = mbar_wait_warp_idle(smem_u32(&sm->stats_full[par]), (i >> 1) & 1, abort_flag, 128);
+      if (ok) ok = mbar_wait_warp_item(smem_u32(&sm->stats_full[walk.at]), walk.ph, abort_flag);
       // The weights of the four partial results need the statistics only, which the softmax warps
       // publish before the item's last P V is complete.
       const int t0 = g & 1;  // the team with the item's first superstep
@@ -885,7 +841,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         // zero in place of the maximum.  Everything between two items is kept short: 50 KB of code against an
         // instruction cache of 32 KB on an SM.  With a select at every use here, and masks at every word of a row in
         // the lister: N = 17536, a tenth 17.87 / 17.70 us, 24 heads of N = 4160, D = 32 45.4 / 44.9.)
-        const float *m_at = &sm->mref[par][t0][r_blk], *l_at = &sm->lsum[par][t0][r_blk];
+        const float *m_at = &sm->mref[walk.at][t0][r_blk], *l_at = &sm->lsum[walk.at][t0][r_blk];
         const int other = t0 ? -128 : 128;  // the other team's
         const float m0 = m_at[0], m1 = m_at[other], m2 = m_at[64], m3 = m_at[other + 64];
         m_all = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
@@ -896,7 +852,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         l_all += e2 * l_at[64];
         l_all += e3 * l_at[other + 64];
         if (p.rowmax) {
-          const float* t_at = &sm->mtrue[par][0][r_blk];
+          const float* t_at = &sm->mtrue[walk.at][0][r_blk];
           mt = fmaxf(fmaxf(t_at[0], t_at[64]), fmaxf(t_at[128], t_at[192]));
         }
         const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
@@ -947,7 +903,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             // use them, while this one is still being merged and stored.
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sm->o_free[par]));
+            if (lane == 0) {
+              mbar_arrive(smem_u32(&sm->o_free[par]));
+              mbar_arrive(smem_u32(&sm->list_free[walk.at]));
+            }
           }
         }
         named_barrier_sync(2, 128);
@@ -985,7 +944,47 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       walk.next();
     }
     if (!ok) fwd_give_up(sm, p.status, kFailOut);
-    if (lister && !terminal && lane == 0) {
+  } else {
+  give_registers<32>();
+  if (warp == kListerWarp) {
+    // =========================== lister ===========================
+    // Sets up item i+1 when the K producer says so during item i, or publishes that there is none; a wait that gives
+    // up leaves ok = false and nothing published.
+    bool ok = true;
+    bool terminal = p.ticket == nullptr;  // drew a ticket past the end (or draws none)
+    int w = blockIdx.x, at = 0;
+#pragma unroll 1
+    for (int i = 0; w < p.items; ++i) {
+      ok = mbar_wait_warp_item(smem_u32(&sm->setup_go[i & 1]), (i >> 1) & 1, abort_flag);
+      if (!ok) break;
+      // the next ticket when items are handed out dynamically, else a fixed stride
+      if (p.ticket != nullptr) {
+        int t = 0;
+        if (lane == 0) {
+          t = atomicAdd(p.ticket, 1);
+          // every CTA draws until its first ticket past the end, so the launch draws exactly
+          // `items` tickets in all; whoever draws the last one leaves the counter at zero
+          if (t == p.items - 1) atomicExch(p.ticket, 0);
+        }
+        t = __shfl_sync(0xffffffffu, t, 0);
+        terminal = t >= n2;
+        w = stride + t;
+      } else {
+        w += stride;
+      }
+      if (++at == kLists) at = 0;
+      // the list buffer was that of item i-2
+      if (i >= 2) ok = mbar_wait_warp_item(smem_u32(&sm->list_free[at]), ((i - 2) / kLists) & 1, abort_flag);
+      if (!ok) break;
+      if (w < p.items)
+        fwd_list_item<kElementMask>(sm, p, w, at, lane);
+      else if (lane == 0)
+        sm->item[at].x = -1;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sm->list_full[at]));  // release: list and item are visible
+    }
+    if (!ok) fwd_give_up(sm, p.status, kFailOut);
+    if (!terminal && lane == 0) {
       // gave up before the last draw: draw on (without working) until this CTA's first ticket past
       // the end, so that the launch still draws `items` tickets and the counter returns to zero
       int t;
@@ -995,11 +994,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       } while (t < n2);
     }
   }
+  }
 
   // ---- tear-down: every role arrives here, also after a give-up ----
-  // (by the first role that is through with its work; let in at the beginning, CTAs of the next kernel that wait
+  // (by the first role that is through with its work, not by warps without one; let in at the beginning, CTAs of the next kernel that wait
   // on free SMs slowed the working ones down by 3 %, let in by the last role they come 0.5 us late)
-  grid_dependents_launch();
+  if (warp < kSoftmaxWarps + 8 || warp == kListerWarp) grid_dependents_launch();
   tc_fence_before();
   __syncthreads();
   if (warp == kSWarp) {

@@ -28,9 +28,9 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int32_t* status, i
     }
     if (lane == 0) report[0] = ok ? 1 : 0;
   } else {
-    // the sleeping form of the wait: leaves because the other warp raised the flag (or by its own
-    // limit, whichever comes first)
-    const bool ok = mbar_wait_warp_idle(smem_u32(&bar), 0, flag, 256);
+    // the wait for an item: leaves because the other warp raised the flag (or by its own limit, whichever comes
+    // first)
+    const bool ok = mbar_wait_warp_item(smem_u32(&bar), 0, flag);
     if (lane == 0) report[1] = ok ? 1 : 0;
   }
   __syncthreads();
