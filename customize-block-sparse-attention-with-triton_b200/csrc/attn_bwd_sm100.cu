@@ -77,8 +77,8 @@ template <bool kDKDV> constexpr int kRing1 = kRing - kRing0<kDKDV>;
 constexpr int kCW = 16;                    // compute warps: 2 teams x 4 lane quarters x 2 column halves
 constexpr int kTeamW = kCW / 2;
 constexpr int kProdWarp = kCW, kXWarp = kCW + 1, kAccWarp = kCW + 2, kProd2Warp = kCW + 3;
-constexpr int kX2Warp = kCW + 8, kAcc2Warp = kCW + 9;           // (warps kCW + 4 .. kCW + 7 write out: lane quarter = warp % 4)
-constexpr int kListWarp = kCW + 10;
+constexpr int kX2Warp = 26, kAcc2Warp = 24;           // (warps kCW + 4 .. kCW + 7 write out: lane quarter = warp % 4)
+constexpr int kListWarp = 27;
 constexpr int kGoBefore = 3;                  // supersteps of loads before an item's end at which the next one is set up
 constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: one warp at the end only fills one
 constexpr uint32_t kBwdTile = 64 * 64 * 2;
