@@ -51,13 +51,15 @@
 // Head dimensions 16 and 32: zero-filled on load by D-wide tensor maps, D / 16 K steps for S and dP.
 // S and dP of a superstep have slots in TMEM, and P and dS are stored over S: a slot of S is held until their
 // products are complete, one of dP only until the arithmetic is done.
-// What bounds it: the way of a superstep through three slots, with no part of it that is the bound alone.
-// A dK/dV superstep takes 1,200 to 1,290 cycles, of which shared memory's port about 1,000 (S and dP
-// operands 384, accumulating operands 256, copies arriving 256, LSE2 and delta 128), the tensor pipe 900, the
-// exponentials a third; a dQ superstep 960 (port 770).  B=2, H=16, N=16384, 25 % of the tiles under a
-// causal mask, both kernels back to back at the power cap: 1,348 us (1,356 with a vote in every try of a wait and
-// unrolled loops; 1,325 with waits that lanes leave one by one, which is not sound).  Of 2 x 8 heads, N = 4160,
-// with such a mask each: 47.7 + 35.9 us (48.2 + 36.8; 46.7 + 35.2).
+// What bounds it: the way of a superstep through its slots, with no part of it that is the bound alone.
+// A dK/dV superstep takes 950 cycles (900 to 1,000 more at a block's end), of which the tensor pipe 756, shared memory's
+// port about 1,000 (operands of S and dP 384, of the accumulating products 256, copies arriving 256, LSE2 and delta and the
+// looks at barriers 200; part of it at once), the exponentials 512; a dQ superstep 790, of which the tensor pipe 585.  One
+// superstep's way is 750 cycles to the logits, 850 for the arithmetic, 220 to the accumulating products, 550 until
+// they are complete.  B=2, H=16, N=16384, 25 % of the tiles under a causal mask, forward and backward at the power
+// cap: 1,528 us (1,845 with products of one tile each, shared memory not aligned, no lister and the steps below).
+// (With S and dP multiplied from tensor memory, which has no room for K and V, the port and the tensor pipe would have
+// 128 cycles a superstep less: 3 %.)
 // Every wait is bounded, and a role that gives up raises a CTA-wide flag, which the others look at when they wait
 // for an item.  Every barrier is waited on by warps that see each of its phases.
 #include <math.h>

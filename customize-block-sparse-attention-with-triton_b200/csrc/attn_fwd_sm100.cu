@@ -22,17 +22,19 @@
 // the probabilities go over the logits of their slot, which is held from the S product until P V
 // is complete.
 //
-// What bounds it: with everything listed a tile takes 336 active SM cycles, of which the exp2 unit
-// is busy 256 (4096 exponentials at 16 per cycle; a loop of nothing but loads, exponentials and
-// stores, two warps per sub-partition, measures 281); what is left are hand-overs between the
-// roles: a look at a barrier that is long complete costs its role 150 to 250 cycles, and the P V
-// issuer, when it had three of them a superstep, was slower than the softmax warps.  With short lists
-// the instruction cache comes first: all roles run at the same time, and with 86 KB of code (most of it
-// unrolled by the compiler; 55 KB now) the instruction caches of a GPC were 73 % busy.  So what is executed
-// per item or per superstep is kept short, waits included, and no loop is unrolled without a reason.
+// What bounds it: with everything listed a tile takes 320 active SM cycles, of which the exp2 unit
+// is busy 256 (4096 exponentials at 16 per cycle).  The softmax warps wait for nothing: of a team's 2,600 cycles a superstep
+// 2,000 lie between its logits and its last exponential (64 columns take a warp 730 cycles alone and 1,160 beside
+// the other team's, 512 being the unit's limit), the rest are a look at a barrier, two loads, a store and an
+// arrival, 60 to 120 cycles each.  MMA operand reads (144 cycles a tile) and arriving tiles (128) take most of shared
+// memory's port.  With short lists the way of an item comes first: ticket and list 2,000 cycles, first tiles 1,600, from the
+// last product to the last store 2,300; and the instruction cache: all roles run at the same time, and with 86 KB of
+// code (most of it unrolled by the compiler; 50 KB now) the instruction caches of a GPC were 73 % busy.  So what is
+// executed per item or per superstep is kept short, waits included, and no loop is unrolled without a reason.
 // B200, D = 64, public calls back to back on inputs that rotate: fp16 N = 17536 with one head, all blocks
-// 116.5 us (118.4 with a P V issuer of three waits and unrolled loops, in turn on one GPU), a tenth of them 18.5 us
-// (19.6); 8 heads, a tenth 112.6 us (118.9); bf16 N = 32000, 32 heads, a tenth 1.295 ms (1.310), at the power cap.
+// 106 us (115 with products of one tile each, shared memory not aligned and a write-out warp for lister, in turn on one
+// GPU), a tenth of them 17.1 us (18.5); 8 heads, a tenth 100 us (111); bf16 N = 32000, 32 heads, a tenth 1.180 ms
+// (1.280), at the power cap.
 //
 // Roles (17 warps of 20); every role walks the same item sequence, so set-up of item i+1 and write-out
 // of item i-1 overlap the arithmetic of item i:
