@@ -98,6 +98,11 @@ constexpr int kTeamWarps = kSoftmaxWarps / 2;
 constexpr int kProducerWarp = 8, kSWarp = 9, kPvWarp = 10, kVProducerWarp = 11;
 constexpr int kListerWarp = 18;
 constexpr int kFwdThreads = 32 * 20;  // whole warpgroups: one warp at the end fills one
+// Registers by warpgroup: 2 softmax, producers and issuers, write-out, lister.  All waits are bounded but the one for
+// registers that the block was not launched with; and a share above what a warp has is taken, not given.
+constexpr int kLaunchRegs = 96, kSoftmaxRegs = 160, kIssuerRegs = 40, kWriteRegs = 88, kListerRegs = 32;
+static_assert(2 * kSoftmaxRegs + kIssuerRegs + kWriteRegs + kListerRegs <= kLaunchRegs * kFwdThreads / 128);
+static_assert(kSoftmaxRegs >= kLaunchRegs && kIssuerRegs <= kLaunchRegs && kWriteRegs <= kLaunchRegs);
 constexpr int kGoBefore = 2;         // supersteps before an item's end at which the next is set up
 constexpr uint32_t kTileBytes = 64 * 64 * 2;       // one Q, K or V tile
 constexpr uint32_t kFwdTmemCols = 512;
@@ -447,7 +452,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   // take what the others do without (2 x 160 + 40 + 88 + 32 = 5 x 96).  The write-out needs its 88: with 80 or 72 short
   // lists are 1 or 2 % slower.
   if (warp >= kSoftmaxWarps && warp < kSoftmaxWarps + 4) {
-  give_registers<40>();
+  give_registers<kIssuerRegs>();
   if (warp == kProducerWarp) {
     // =========================== K producer ===========================
     bool ok = true;
@@ -659,7 +664,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
   } else if (warp < kSoftmaxWarps) {
     // =========================== softmax ===========================
-    take_registers<160>();
+    take_registers<kSoftmaxRegs>();
     const int team = warp >> 2;
     const int quarter = warp & 3;     // TMEM lane quarter this warp may touch
     const int half = quarter >> 1;    // lanes 0..63 own tiles a, c of a superstep, 64..127 b, d
@@ -817,7 +822,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // their weighted rows to each other through shared memory, 16 columns at a time.  All named
     // barriers of an iteration are always executed, also after a give-up, and the last one carries
     // the give-up vote, so that no warp of this role can be left waiting at one.
-    give_registers<88>();
+    give_registers<kWriteRegs>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
     bool ok = true;
     const int half = quarter >> 1;
@@ -947,7 +952,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
     if (!ok) fwd_give_up(sm, p.status, kFailOut);
   } else {
-  give_registers<32>();
+  give_registers<kListerRegs>();
   if (warp == kListerWarp) {
     // =========================== lister ===========================
     // Sets up item i+1 when the K producer says so during item i, or publishes that there is none; a wait that gives
