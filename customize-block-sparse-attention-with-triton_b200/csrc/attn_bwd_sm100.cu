@@ -773,8 +773,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     // compute warps are already at work on the next block.  dK/dV: lanes 0..63 finish dV and hand
     // over their sums of dK, lanes 64..127 the other way round; dQ: lanes 0..63 finish columns
     // [0, 32), lanes 64..127 columns [32, 64).
-    // Both named barriers of an iteration are always executed, also after a give-up, and the
-    // last one carries the give-up vote, so that no warp of this role is left waiting at one.
+    // Each 32 columns take two named barriers, also after a give-up, the second one with the give-up vote
+    // (role_leaves); a warp that is told that there is no more work comes to both before it leaves.
     take_registers<136>();
     const int quarter = warp & 3;
     const int half = quarter >> 1;
@@ -793,7 +793,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     for (int i = 0;; ++i) {
       BwdItem it{0, 0, 0, 1, 0};
       if (ok) ok = bwd_next_item(sm, i, lane, &it);
-      if (ok && it.b < 0) break;  // no more work: the same for all four warps
+      if (ok && it.b < 0) {  // no more work
+        named_barrier_sync(2, 128);
+        role_leaves(2, 128, false);
+        break;
+      }
       const int64_t row = it.blk * 64 + r_blk;
       uint16_t* dst = first_out
                           ? static_cast<uint16_t*>(p.out0) + it.b * p.sb0 + it.h * p.sh0 + row * p.sn0
@@ -854,7 +858,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
           }
         }
         // xfer may be overwritten now; all four warps leave together on a give-up
-        any_failed = named_barrier_or(2, 128, !ok);
+        any_failed = role_leaves(2, 128, !ok);
         if (any_failed) break;
       }
       if (any_failed) break;

@@ -819,9 +819,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // =========================== write-out ===========================
     // Merges the four partial results of every query row (first / second team of the item x lanes
     // r / r+64).  A warp reads both accumulators of its own lanes from TMEM; lanes 64..127 hand
-    // their weighted rows to each other through shared memory, 16 columns at a time.  All named
-    // barriers of an iteration are always executed, also after a give-up, and the last one carries
-    // the give-up vote, so that no warp of this role can be left waiting at one.
+    // their weighted rows to each other through shared memory, 16 columns at a time.  Each time
+    // takes two named barriers, also after a give-up, the second one with the give-up vote (role_leaves); a warp
+    // that is told that there is no more work comes to both before it leaves.
     give_registers<kWriteRegs>();
     const int quarter = warp & 3;  // lane quarter a warp may touch = its index mod 4
     bool ok = true;
@@ -835,7 +835,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int par = i & 1;
       if (ok) ok = mbar_wait_warp_item(smem_u32(&sm->list_full[walk.at]), walk.ph, abort_flag);
       walk.it = ok ? sm->item[walk.at] : make_int4(0, 0, 0, 0);
-      if (walk.it.x < 0) break;  // no more work: the same for all four warps
+      if (walk.it.x < 0) {  // no more work
+        named_barrier_sync(2, 128);
+        role_leaves(2, 128, false);
+        break;
+      }
       const int n_tiles = walk.it.w;
       if (ok) ok = mbar_wait_warp_item(smem_u32(&sm->stats_full[walk.at]), walk.ph, abort_flag);
       // The weights of the four partial results need the statistics only, which the softmax warps
@@ -939,7 +943,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
         }
         // xfer may be overwritten now; all four warps leave together if any gave up
-        any_failed = named_barrier_or(2, 128, !ok);
+        any_failed = role_leaves(2, 128, !ok);
         if (any_failed) break;
       }
       if (ok && half == 0) {

@@ -60,6 +60,14 @@ __device__ __forceinline__ bool named_barrier_or(int id, int threads, bool pred)
   return out != 0;
 }
 
+// The vote of a role of several warps that meet at a named barrier in their items.  Each of them waits for the item by
+// itself, and a wait may run out in one warp while the others still see what it waited for: an item, one that
+// needs no barrier, or the end of the work.  So whenever they have met, for an item, because a wait has run out, or
+// at the end of the work, they vote: all of them go on, or none does.
+__device__ __forceinline__ bool role_leaves(int id, int threads, bool gave_up) {
+  return named_barrier_or(id, threads, gave_up);
+}
+
 // Programmatic dependent launch: the attention kernels, delta, the lists with places and the in-place reorder are
 // launched so that they may begin while the previous kernel of the stream is still running, do their set-up,
 // and wait here, in every role, before they touch memory that another kernel may write or read, until that one

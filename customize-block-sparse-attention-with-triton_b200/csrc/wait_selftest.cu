@@ -75,6 +75,29 @@ __global__ void __launch_bounds__(96, 1) give_up_selftest_kernel(int32_t* report
   if (threadIdx.x == 0) report[4] = 1;
 }
 
+// The loop of a role of four warps that wait for their items one by one, as the attention kernels' write-out does:
+// items 0, 2, 3 and 6 have work, 1, 4 and 5 have none, 7 is the end, and the wait of warp w for item run_out[w] runs out
+// (not at all if there is no such item).  report[w]: after how many items with work the warp went on, 100 more once it has left.
+__global__ void __launch_bounds__(128, 1) role_vote_selftest_kernel(int4 run_out, int32_t* report) {
+  const int warp = uniform_warp_index();
+  const int mine = warp == 0 ? run_out.x : warp == 1 ? run_out.y : warp == 2 ? run_out.z : run_out.w;
+  int done = 0;
+#pragma unroll 1
+  for (int i = 0;; ++i) {
+    const bool ok = i != mine;
+    if (ok && i == 7) {
+      named_barrier_sync(2, 128);
+      role_leaves(2, 128, false);
+      break;
+    }
+    if (ok && (i == 1 || i == 4 || i == 5)) continue;
+    named_barrier_sync(2, 128);
+    if (role_leaves(2, 128, !ok)) break;
+    ++done;
+  }
+  if ((threadIdx.x & 31) == 0) report[warp] = done + 100;
+}
+
 // Lets its dependents in at once and ends after so many milliseconds.
 __global__ void __launch_bounds__(32, 1) early_selftest_kernel(int milliseconds) {
   grid_dependents_launch();
@@ -91,6 +114,15 @@ extern "C" int bsa_selftest_early_kernel(int milliseconds, void* stream) {
   int rc;
   if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
   bsa::early_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(milliseconds);
+  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
+
+extern "C" int bsa_selftest_role_vote(int item0, int item1, int item2, int item3, int32_t* report, void* stream) {
+  if (!report) return BSA_ERR_BAD_POINTER;
+  int rc;
+  if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
+  bsa::role_vote_selftest_kernel<<<1, 128, 0, static_cast<cudaStream_t>(stream)>>>(make_int4(item0, item1, item2, item3),
+                                                                                   report);
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 

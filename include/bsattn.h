@@ -432,6 +432,15 @@ int bsa_selftest_bounded_wait(int32_t* status, int32_t* report, void* stream);
 int bsa_selftest_give_up(int32_t* report, void* stream);
 
 /*
+ * Self-test of how a role of four warps leaves its loop over work items when the wait of one of them runs out; no
+ * reference counterpart.  Eight items: 0, 2, 3 and 6 with work, 1, 4 and 5 without, 7 is the end of the work.  The
+ * wait of warp w for item `item`w is taken to run out (-1 or more than 7: none does).  `report` (device, 4 x int32)
+ * receives for each warp after how many items with work it went on, plus 100 once it has left: no warp goes on
+ * without the others, and all of them leave.
+ */
+int bsa_selftest_role_vote(int item0, int item1, int item2, int item3, int32_t* report, void* stream);
+
+/*
  * For tests; no reference counterpart.  Launches one warp that lets the kernel behind it in the stream begin at
  * once and sleeps for so many milliseconds (0 to 10,000).  The kernels of this library may begin while the
  * kernel before them is still running, and their waits are limited (BSA_ERR_DEVICE_TIMEOUT): the limit counts
