@@ -572,12 +572,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const uint64_t desc_q = desc_q0 + static_cast<uint64_t>(qpar) * kTileDesc;
 #pragma unroll 1
       for (int u = 0; u < n_super; ++u) {
-        // (two looks, one vote)
-        bool seen = mbar_poll(smem_u32(&sm->k_full[ks]), kph, kWaitTries);
         // the slot's previous user, three supersteps ago, must have had its P V completed (for the
         // first users this asks for the phase before the first one, which counts as complete)
-        seen &= mbar_poll(smem_u32(&sm->pv_done[slot]), slot_ph, kWaitTries);
-        ok = __all_sync(0xffffffffu, seen);
+        ok = mbar_wait_warp2(smem_u32(&sm->k_full[ks]), kph, smem_u32(&sm->pv_done[slot]), slot_ph);
         if (!ok) break;
         tc_fence_after();
         if (leader) {

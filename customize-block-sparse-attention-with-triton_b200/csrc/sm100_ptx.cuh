@@ -158,23 +158,32 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
 
 // Two barriers at once: both looks are on their way together.  (A look takes 150 to 250 cycles while the tensor cores
 // read their operands from shared memory, and one after the other cost the backward's S/dP issuers 450 cycles a
-// superstep of 950: 2 x 16 heads, N = 16384, causal, a quarter, forward and backward 1,402 -> 1,378 us.)
+// superstep of 950: 2 x 16 heads, N = 16384, causal, a quarter, forward and backward 1,402 -> 1,378 us.)  The barriers
+// share one limit, and the warp is together when it looks at one again: its limit would be 0.04 s otherwise.
+__device__ __forceinline__ void mbar_poll_shared(uint32_t bar, uint32_t parity, int* tries) {
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity))
+    if (--*tries <= 0) break;
+  __syncwarp();
+}
 __device__ __forceinline__ bool mbar_wait_warp2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
   const bool seen0 = mbar_try_wait(bar0, parity0), seen1 = mbar_try_wait(bar1, parity1);
-  bool ok = true;
-  if (!seen0) ok = mbar_poll(bar0, parity0, kWaitTries);
-  if (!seen1) ok &= mbar_poll(bar1, parity1, kWaitTries);
-  return __all_sync(0xffffffffu, ok);
+  if (__all_sync(0xffffffffu, seen0 && seen1)) return true;
+  int tries = kWaitTries;
+  mbar_poll_shared(bar0, parity0, &tries);
+  mbar_poll_shared(bar1, parity1, &tries);
+  return __all_sync(0xffffffffu, tries > 0);
 }
 
 __device__ __forceinline__ bool mbar_wait_warp3(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
                                                 uint32_t bar2, uint32_t parity2) {
   const bool seen0 = mbar_try_wait(bar0, parity0), seen1 = mbar_try_wait(bar1, parity1), seen2 = mbar_try_wait(bar2, parity2);
-  bool ok = true;
-  if (!seen0) ok = mbar_poll(bar0, parity0, kWaitTries);
-  if (!seen1) ok &= mbar_poll(bar1, parity1, kWaitTries);
-  if (!seen2) ok &= mbar_poll(bar2, parity2, kWaitTries);
-  return __all_sync(0xffffffffu, ok);
+  if (__all_sync(0xffffffffu, seen0 && seen1 && seen2)) return true;
+  int tries = kWaitTries;
+  mbar_poll_shared(bar0, parity0, &tries);
+  mbar_poll_shared(bar1, parity1, &tries);
+  mbar_poll_shared(bar2, parity2, &tries);
+  return __all_sync(0xffffffffu, tries > 0);
 }
 
 // The same for the beginning of an item, where a role comes that still had work when another one gave up: it

@@ -75,6 +75,27 @@ __global__ void __launch_bounds__(96, 1) give_up_selftest_kernel(int32_t* report
   if (threadIdx.x == 0) report[4] = 1;
 }
 
+// How long the forms of a wait last on barriers that nothing ever completes, one warp each: on one barrier, on two at
+// once, on three at once.
+__global__ void __launch_bounds__(96, 1) wait_limits_selftest_kernel(int32_t* report) {
+  __shared__ uint64_t bar[3];
+  const int warp = uniform_warp_index();
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 3; ++i) mbar_init(smem_u32(&bar[i]), 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  const uint32_t b0 = smem_u32(&bar[0]), b1 = smem_u32(&bar[1]), b2 = smem_u32(&bar[2]);
+  const uint64_t t0 = global_timer_ns();
+  const bool ok = warp == 0 ? mbar_wait_warp(b0, 0) : warp == 1 ? mbar_wait_warp2(b0, 0, b1, 0) : mbar_wait_warp3(b0, 0, b1, 0, b2, 0);
+  const unsigned went_on = __ballot_sync(0xffffffffu, ok);
+  if (lane == 0) {
+    report[2 * warp] = __popc(went_on);
+    report[2 * warp + 1] = static_cast<int32_t>((global_timer_ns() - t0) / 1000000ull);
+  }
+}
+
 // The loop of a role of four warps that wait for their items one by one, as the attention kernels' write-out does:
 // items 0, 2, 3 and 6 have work, 1, 4 and 5 have none, 7 is the end, and the wait of warp w for item run_out[w] runs out
 // (not at all if there is no such item).  report[w]: after how many items with work the warp went on, 100 more once it has left.
@@ -114,6 +135,14 @@ extern "C" int bsa_selftest_early_kernel(int milliseconds, void* stream) {
   int rc;
   if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
   bsa::early_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(milliseconds);
+  return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
+}
+
+extern "C" int bsa_selftest_wait_limits(int32_t* report, void* stream) {
+  if (!report) return BSA_ERR_BAD_POINTER;
+  int rc;
+  if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
+  bsa::wait_limits_selftest_kernel<<<1, 96, 0, static_cast<cudaStream_t>(stream)>>>(report);
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 

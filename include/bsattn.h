@@ -432,6 +432,14 @@ int bsa_selftest_bounded_wait(int32_t* status, int32_t* report, void* stream);
 int bsa_selftest_give_up(int32_t* report, void* stream);
 
 /*
+ * Self-test of the limit of the kernels' waits; no reference counterpart.  Launches one small CTA whose warps wait on
+ * barriers that nothing completes: the first on one, the second on two at once, the third on three at once.
+ * `report` (device, 6 x int32) receives for each warp how many lanes took the wait for satisfied (none) and the
+ * milliseconds until it had left (the same for all, about two seconds).
+ */
+int bsa_selftest_wait_limits(int32_t* report, void* stream);
+
+/*
  * Self-test of how a role of four warps leaves its loop over work items when the wait of one of them runs out; no
  * reference counterpart.  Eight items: 0, 2, 3 and 6 with work, 1, 4 and 5 without, 7 is the end of the work.  The
  * wait of warp w for item `item`w is taken to run out (-1 or more than 7: none does).  `report` (device, 4 x int32)
