@@ -28,8 +28,10 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int32_t* status, i
     }
     if (lane == 0) report[0] = ok ? 1 : 0;
   } else {
-    // the wait for an item: leaves because the other warp raised the flag (or by its own limit, whichever comes
-    // first)
+    // the wait for an item, begun a second later, so that it leaves because the other warp raised the flag and not by its
+    // own limit
+#pragma unroll 1
+    for (int i = 0; i < 2000 && global_timer_ns() - t0 < 1000000000ull; ++i) __nanosleep(1000000u);
     const bool ok = mbar_wait_warp_item(smem_u32(&bar), 0, flag);
     if (lane == 0) report[1] = ok ? 1 : 0;
   }
@@ -76,19 +78,35 @@ __global__ void __launch_bounds__(96, 1) give_up_selftest_kernel(int32_t* report
 }
 
 // How long the forms of a wait last on barriers that nothing ever completes, one warp each: on one barrier, on two at
-// once, on three at once.
-__global__ void __launch_bounds__(96, 1) wait_limits_selftest_kernel(int32_t* report) {
+// once, on three at once, for an item, and for an item when the sixth warp raises the flag after 100 ms.
+__global__ void __launch_bounds__(192, 1) wait_limits_selftest_kernel(int32_t* report) {
   __shared__ uint64_t bar[3];
+  __shared__ int flags[2];
   const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 3; ++i) mbar_init(smem_u32(&bar[i]), 1);
+    flags[0] = flags[1] = 0;
     mbar_fence_init();
   }
   __syncthreads();
+  volatile int* flag = flags;
   const uint32_t b0 = smem_u32(&bar[0]), b1 = smem_u32(&bar[1]), b2 = smem_u32(&bar[2]);
   const uint64_t t0 = global_timer_ns();
-  const bool ok = warp == 0 ? mbar_wait_warp(b0, 0) : warp == 1 ? mbar_wait_warp2(b0, 0, b1, 0) : mbar_wait_warp3(b0, 0, b1, 0, b2, 0);
+  bool ok = false;
+  if (warp == 0) {
+    ok = mbar_wait_warp(b0, 0);
+  } else if (warp == 1) {
+    ok = mbar_wait_warp2(b0, 0, b1, 0);
+  } else if (warp == 2) {
+    ok = mbar_wait_warp3(b0, 0, b1, 0, b2, 0);
+  } else if (warp < 5) {
+    ok = mbar_wait_warp_item(b0, 0, flag + (warp - 3));
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < 100; ++i) __nanosleep(1000000u);  // (at most a millisecond each)
+    if (lane == 0) flag[1] = 1;
+  }
   const unsigned went_on = __ballot_sync(0xffffffffu, ok);
   if (lane == 0) {
     report[2 * warp] = __popc(went_on);
@@ -142,7 +160,7 @@ extern "C" int bsa_selftest_wait_limits(int32_t* report, void* stream) {
   if (!report) return BSA_ERR_BAD_POINTER;
   int rc;
   if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
-  bsa::wait_limits_selftest_kernel<<<1, 96, 0, static_cast<cudaStream_t>(stream)>>>(report);
+  bsa::wait_limits_selftest_kernel<<<1, 192, 0, static_cast<cudaStream_t>(stream)>>>(report);
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 

@@ -411,8 +411,8 @@ int bsa_check_status(const int32_t* status, void* stream);
 
 /*
  * Self-test of the kernels' bounded waits; no reference counterpart.  Launches one small CTA in
- * which one warp waits on a barrier that nothing ever completes and a second warp waits beside
- * it.  The first wait runs out after the library's wait limit (about two seconds), records 99 in
+ * which one warp waits on a barrier that nothing ever completes and a second warp begins to do so
+ * a second later.  The first wait runs out after the library's wait limit (about two seconds), records 99 in
  * `status` (optional) and raises the CTA's give-up flag, which releases the second warp; both
  * leave through the end of the kernel.  `report` (device, 4 x int32) receives: [0] 1 if the first
  * wait was satisfied (never), [1] the same for the second, [2] 1 once both warps reached the end
@@ -433,9 +433,11 @@ int bsa_selftest_give_up(int32_t* report, void* stream);
 
 /*
  * Self-test of the limit of the kernels' waits; no reference counterpart.  Launches one small CTA whose warps wait on
- * barriers that nothing completes: the first on one, the second on two at once, the third on three at once.
- * `report` (device, 6 x int32) receives for each warp how many lanes took the wait for satisfied (none) and the
- * milliseconds until it had left (the same for all, about two seconds).
+ * barriers that nothing completes: the first on one, the second on two at once, the third on three at once, the
+ * fourth as the kernels' roles wait for their next work item, the fifth likewise, with a give-up flag that the sixth
+ * raises after some 100 ms.  `report` (device, 12 x int32) receives for each warp how many lanes took the wait for
+ * satisfied (none) and the milliseconds until it had left: about two seconds for the first four, which have the same
+ * limit, less than half a second for the fifth.
  */
 int bsa_selftest_wait_limits(int32_t* report, void* stream);
 
