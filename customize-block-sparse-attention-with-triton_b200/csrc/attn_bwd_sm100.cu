@@ -83,6 +83,12 @@ constexpr int kX2Warp = 26, kAcc2Warp = 24;           // (warps kCW + 4 .. kCW +
 constexpr int kListWarp = 27;
 constexpr int kGoBefore = 3;                  // supersteps of loads before an item's end at which the next one is set up
 constexpr int kBwdThreads = 32 * (kCW + 12);  // whole warpgroups: one warp at the end only fills one
+// Registers by warpgroup: 4 compute, which keep what they are launched with, producers and first issuers, write-out,
+// second issuers and lister.  All waits are bounded but the one for registers that the block was not launched
+// with.  (kBwdLaunchRegs is what the compiler makes of the launch bounds; the host compares before the first launch.)
+constexpr int kBwdLaunchRegs = 72, kBwdIssuerRegs = 40, kBwdWriteRegs = 136;
+static_assert((kCW / 4) * kBwdLaunchRegs + 2 * kBwdIssuerRegs + kBwdWriteRegs <= kBwdLaunchRegs * kBwdThreads / 128);
+static_assert(kBwdWriteRegs >= kBwdLaunchRegs && kBwdIssuerRegs <= kBwdLaunchRegs);
 constexpr uint32_t kBwdTile = 64 * 64 * 2;
 constexpr uint32_t kBwdTmemCols = 512;
 constexpr int kListIndex = BSA_LIST_PARTIAL_FLAG - 1;  // a list entry without its flag
@@ -573,7 +579,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
   // 896 threads are launched with 72 registers: the write-out warps take what the producers and the
   // issuers do without (40 + 136 + 40 = 3 x 72).
   if ((warp >= kCW && warp < kCW + 4) || warp >= kCW + 8) {
-    give_registers<40>();
+    give_registers<kBwdIssuerRegs>();
     if (warp == kProdWarp) {
       bwd_produce<kDKDV, true>(sm, p, &tm_stat0, &tm_str0, lane);
     } else if (warp == kProd2Warp) {
@@ -775,7 +781,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_stat0,
     // [0, 32), lanes 64..127 columns [32, 64).
     // Each 32 columns take two named barriers, also after a give-up, the second one with the give-up vote
     // (role_leaves); a warp that is told that there is no more work comes to both before it leaves.
-    take_registers<136>();
+    take_registers<kBwdWriteRegs>();
     const int quarter = warp & 3;
     const int half = quarter >> 1;
     const int r_blk = (quarter & 1) * 32 + lane;  // row of the CTA's block
@@ -968,7 +974,7 @@ static int launch_bwd(BwdOperand q, BwdOperand k, BwdOperand v, BwdOperand dout,
                                                     : attn_bwd_kernel<false, kDKDV, true>)
                                : (dtype == BSA_BF16 ? attn_bwd_kernel<true, kDKDV, false>
                                                     : attn_bwd_kernel<false, kDKDV, false>);
-  if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes)) != BSA_OK)
+  if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, kBwdLaunchRegs)) != BSA_OK)
     return rc;
   int sms = 0;
   if ((rc = sm_count(&sms)) != BSA_OK) return rc;

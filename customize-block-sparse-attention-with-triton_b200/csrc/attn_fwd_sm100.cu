@@ -99,10 +99,12 @@ constexpr int kProducerWarp = 8, kSWarp = 9, kPvWarp = 10, kVProducerWarp = 11;
 constexpr int kListerWarp = 18;
 constexpr int kFwdThreads = 32 * 20;  // whole warpgroups: one warp at the end fills one
 // Registers by warpgroup: 2 softmax, producers and issuers, write-out, lister.  All waits are bounded but the one for
-// registers that the block was not launched with; and a share above what a warp has is taken, not given.
+// registers that the block was not launched with; and a share above what a warp has is taken, not given.  (kLaunchRegs
+// is what the compiler makes of the launch bounds; the host compares before the first launch.)
 constexpr int kLaunchRegs = 96, kSoftmaxRegs = 160, kIssuerRegs = 40, kWriteRegs = 88, kListerRegs = 32;
 static_assert(2 * kSoftmaxRegs + kIssuerRegs + kWriteRegs + kListerRegs <= kLaunchRegs * kFwdThreads / 128);
-static_assert(kSoftmaxRegs >= kLaunchRegs && kIssuerRegs <= kLaunchRegs && kWriteRegs <= kLaunchRegs);
+static_assert(kSoftmaxRegs >= kLaunchRegs && kIssuerRegs <= kLaunchRegs && kWriteRegs <= kLaunchRegs &&
+              kListerRegs <= kLaunchRegs);
 constexpr int kGoBefore = 2;         // supersteps before an item's end at which the next is set up
 constexpr uint32_t kTileBytes = 64 * 64 * 2;       // one Q, K or V tile
 constexpr uint32_t kFwdTmemCols = 512;
@@ -1100,7 +1102,7 @@ static int launch_fwd(const void* q, const int64_t q_strides[4], const void* k,
   auto kern = dense != nullptr
                   ? (dtype == BSA_BF16 ? attn_fwd_kernel<true, true> : attn_fwd_kernel<false, true>)
                   : (dtype == BSA_BF16 ? attn_fwd_kernel<true, false> : attn_fwd_kernel<false, false>);
-  if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes)) != BSA_OK)
+  if ((rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem_bytes, kLaunchRegs)) != BSA_OK)
     return rc;
   // (no more than an eighth of a head's rows: front < nrows)
   prm.front = prm.items > sms && prm.items <= kFrontRounds * sms ? (nrows / 8 < kFrontRows ? nrows / 8 : kFrontRows) : 0;

@@ -43,7 +43,16 @@ int sm_count(int* out) {
   return BSA_OK;
 }
 
-int ensure_dynamic_smem(const void* kernel, size_t bytes) {
+int check_launch_registers(const void* kernel, int launch_regs) {
+  cudaFuncAttributes attr;
+  if (cudaFuncGetAttributes(&attr, kernel) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return BSA_ERR_CUDA;
+  }
+  return attr.numRegs == launch_regs ? BSA_OK : BSA_ERR_REGISTERS;
+}
+
+int ensure_dynamic_smem(const void* kernel, size_t bytes, int launch_regs) {
   // a handful of kernels x devices: a small fixed table guarded by a spin flag is enough
   struct Entry { const void* k; int dev; };
   static Entry table[128];
@@ -54,6 +63,10 @@ int ensure_dynamic_smem(const void* kernel, size_t bytes) {
   const int n = count.load(std::memory_order_acquire);
   for (int i = 0; i < n; ++i)
     if (table[i].k == kernel && table[i].dev == dev) return BSA_OK;
+  if (launch_regs != 0) {
+    const int rc = check_launch_registers(kernel, launch_regs);
+    if (rc != BSA_OK) return rc;
+  }
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(bytes)) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -160,6 +173,7 @@ extern "C" const char* bsa_strerror(int status) {
     case BSA_ERR_UNSUPPORTED_ARCH: return "current device is not compute capability 10.x (B200)";
     case BSA_ERR_TOO_LARGE: return "problem exceeds a fixed capacity of this entry point";
     case BSA_ERR_DEVICE_TIMEOUT: return "a bounded wait inside a kernel gave up";
+    case BSA_ERR_REGISTERS: return "the kernel was built with another number of registers than its roles share out";
     default: return "unknown status";
   }
 }

@@ -62,7 +62,13 @@ int launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, siz
 int launch_lists_places(const uint8_t* block, const int64_t s[4], int B, int H, int nb, int32_t* row_cnt,
                         int32_t* col_idx, int32_t* col_cnt, int32_t* row_idx, bool together, void* stream);
 
-// Raises a kernel's dynamic shared-memory limit; done once per (kernel, device) and remembered.
-int ensure_dynamic_smem(const void* kernel, size_t bytes);
+// Raises a kernel's dynamic shared-memory limit; done once per (kernel, device) and remembered.  launch_regs: what
+// its roles share out a thread, 0 if they share out nothing; see check_launch_registers.
+int ensure_dynamic_smem(const void* kernel, size_t bytes, int launch_regs = 0);
+
+// BSA_OK if the kernel is launched with just so many registers a thread, else BSA_ERR_REGISTERS.  The shares of a
+// kernel whose roles exchange registers are constants, the number at launch is the compiler's: with fewer than they
+// add up to, the roles that take some would wait for them, and that wait has no limit.
+int check_launch_registers(const void* kernel, int launch_regs);
 
 }  // namespace bsa

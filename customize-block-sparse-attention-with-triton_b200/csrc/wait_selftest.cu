@@ -164,6 +164,15 @@ extern "C" int bsa_selftest_wait_limits(int32_t* report, void* stream) {
   return cudaGetLastError() == cudaSuccess ? BSA_OK : BSA_ERR_CUDA;
 }
 
+extern "C" int bsa_selftest_launch_registers(int more) {
+  int rc;
+  if ((rc = bsa::check_device_sm100()) != BSA_OK) return rc;
+  const void* kernel = reinterpret_cast<const void*>(bsa::role_vote_selftest_kernel);
+  cudaFuncAttributes attr;
+  if (cudaFuncGetAttributes(&attr, kernel) != cudaSuccess) return BSA_ERR_CUDA;
+  return bsa::check_launch_registers(kernel, attr.numRegs + more);
+}
+
 extern "C" int bsa_selftest_role_vote(int item0, int item1, int item2, int item3, int32_t* report, void* stream) {
   if (!report) return BSA_ERR_BAD_POINTER;
   int rc;

@@ -44,7 +44,8 @@ typedef enum bsa_status {
   BSA_ERR_NO_DRIVER = -6,      /* cuTensorMapEncodeTiled could not be resolved                    */
   BSA_ERR_UNSUPPORTED_ARCH = -7, /* current device is not compute capability 10.x                 */
   BSA_ERR_TOO_LARGE = -8,      /* problem exceeds a documented fixed capacity                     */
-  BSA_ERR_DEVICE_TIMEOUT = -9  /* reported by bsa_check_status: a bounded device wait gave up     */
+  BSA_ERR_DEVICE_TIMEOUT = -9, /* reported by bsa_check_status: a bounded device wait gave up     */
+  BSA_ERR_REGISTERS = -10      /* built with another number of registers than the kernel's roles share out */
 } bsa_status;
 
 /* What a status word holds beside zero: the role whose bounded wait gave up (1, 2, …), or this: the plan of
@@ -449,6 +450,14 @@ int bsa_selftest_wait_limits(int32_t* report, void* stream);
  * without the others, and all of them leave.
  */
 int bsa_selftest_role_vote(int item0, int item1, int item2, int item3, int32_t* report, void* stream);
+
+/*
+ * Self-test of the check that goes before the attention kernels' launches; no reference counterpart.  Their roles
+ * share out the registers that a block is launched with, and would wait without a limit for more.  Compares a small
+ * kernel with `more` registers a thread more than it was built with: BSA_OK for 0, BSA_ERR_REGISTERS for any other.
+ * Launches nothing.
+ */
+int bsa_selftest_launch_registers(int more);
 
 /*
  * For tests; no reference counterpart.  Launches one warp that lets the kernel behind it in the stream begin at
