@@ -255,6 +255,10 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
                    bar)
                : "memory");
 }
+// What this thread has written to shared memory may be read by MMAs and bulk copies after the next barrier.
+__device__ __forceinline__ void async_proxy_fence() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
 __device__ __forceinline__ void tc_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -280,8 +284,8 @@ __device__ __forceinline__ void umma_ws_ss(uint32_t d_tmem, uint64_t a_desc, uin
 // D[tmem] (+)= A[tmem] * B[smem desc] in the same form with A in tensor memory: lanes 0..63 of D are their own
 // rows of A times columns [0, N/2) of B, lanes 64..127 their own rows of A times columns [N/2, N).  With two tiles
 // beside one another in B (MN-major, the leading byte offset is the way from one to the other) that is two
-// products of 64 rows at once.  (Ordinary use has the same 64 rows in both lane halves; that each half reads its own
-// is how B200 does it, checked element by element, and every test of the kernels rests on it.)  Two products of 64 x 64
+// products of 64 rows at once.  (Ordinary use has the same 64 rows in both lane halves.  That each half reads its own
+// is how B200 does it and not promised anywhere; product_selftest.cu checks it element by element.)  Two products of 64 x 64
 // with 64 columns: 176 cycles; as two M = 128 products, each with one lane half of the result switched off, 256.
 // Both halves are always written: where there is no second tile, its rows of A and its part of B are zeros.
 __device__ __forceinline__ void umma_ws_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,

@@ -81,6 +81,7 @@ SIGNATURES = {
     "bsa_selftest_bounded_wait": [_vp, _vp, _vp],
     "bsa_selftest_give_up": [_vp, _vp],
     "bsa_selftest_wait_limits": [_vp, _vp],
+    "bsa_selftest_half_products": [_vp, _vp, _vp, _i, _vp, _vp],
     "bsa_selftest_launch_registers": [_i],
     "bsa_selftest_role_vote": [_i, _i, _i, _i, _vp, _vp],
     "bsa_selftest_early_kernel": [_i, _vp],
