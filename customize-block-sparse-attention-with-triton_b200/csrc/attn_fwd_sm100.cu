@@ -576,7 +576,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int u = 0; u < n_super; ++u) {
         // the slot's previous user, three supersteps ago, must have had its P V completed (for the
         // first users this asks for the phase before the first one, which counts as complete)
-        ok = mbar_wait_warp2(smem_u32(&sm->k_full[ks]), kph, smem_u32(&sm->pv_done[slot]), slot_ph);
+        ok = mbar_wait_warp_in_turn(smem_u32(&sm->k_full[ks]), kph, smem_u32(&sm->pv_done[slot]), slot_ph);
         if (!ok) break;
         tc_fence_after();
         if (leader) {

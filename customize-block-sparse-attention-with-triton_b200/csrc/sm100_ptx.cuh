@@ -156,23 +156,29 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, in
   return __all_sync(0xffffffffu, mbar_poll(bar, parity, tries));
 }
 
-// Two barriers at once: both looks are on their way together.  (A look takes 150 to 250 cycles while the tensor cores
-// read their operands from shared memory, and one after the other cost the backward's S/dP issuers 450 cycles a
-// superstep of 950: 2 x 16 heads, N = 16384, causal, a quarter, forward and backward 1,402 -> 1,378 us.)  The barriers
-// share one limit, and the warp is together when it looks at one again: its limit would be 0.04 s otherwise.
+// Several barriers, one after the other, which share one limit.  The warp is together whenever it begins to look at one:
+// its limit would be 0.04 s otherwise.
 __device__ __forceinline__ void mbar_poll_shared(uint32_t bar, uint32_t parity, int* tries) {
 #pragma unroll 1
   while (!mbar_try_wait(bar, parity))
     if (--*tries <= 0) break;
   __syncwarp();
 }
-__device__ __forceinline__ bool mbar_wait_warp2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
-  const bool seen0 = mbar_try_wait(bar0, parity0), seen1 = mbar_try_wait(bar1, parity1);
-  if (__all_sync(0xffffffffu, seen0 && seen1)) return true;
+__device__ __forceinline__ bool mbar_wait_warp_in_turn(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
   int tries = kWaitTries;
   mbar_poll_shared(bar0, parity0, &tries);
   mbar_poll_shared(bar1, parity1, &tries);
   return __all_sync(0xffffffffu, tries > 0);
+}
+
+// Two barriers at once: both looks are on their way together.  (A look takes 150 to 250 cycles while the tensor cores
+// read their operands from shared memory, and one after the other cost the backward's S/dP issuers 450 cycles a
+// superstep of 950: 2 x 16 heads, N = 16384, causal, a quarter, forward and backward 1,402 -> 1,378 us.  The forward's S
+// issuer, which has time for them, takes them in turn: N = 17536, everything listed 107.2 us so, 106.5 in turn.)
+__device__ __forceinline__ bool mbar_wait_warp2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+  const bool seen0 = mbar_try_wait(bar0, parity0), seen1 = mbar_try_wait(bar1, parity1);
+  if (__all_sync(0xffffffffu, seen0 && seen1)) return true;
+  return mbar_wait_warp_in_turn(bar0, parity0, bar1, parity1);
 }
 
 __device__ __forceinline__ bool mbar_wait_warp3(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,
