@@ -27,19 +27,19 @@
 // Persistent: one CTA per SM starts with block blockIdx.x and draws further blocks from an
 // optional work counter (or walks a fixed stride); long lists first when the mask is causal.  dQ may run
 // beside dK/dV (see `together`).
-// Roles (27 warps):
+// Roles (28 warps; warp 25 has none):
 //   warps 0..15 : compute, two teams of eight warps on alternate supersteps (team = warp / 8, TMEM lane
 //                 quarter = warp % 4, 32 of a tile's 64 columns = (warp / 4) % 2), so that one team's
 //                 barrier round trips and products run under the other one's arithmetic
 //   warps 16, 19: TMA producers, one for Q and K (and LSE2), one for dO and V (and delta): an SM starts a
 //                 copy only every 190 cycles or so from one warp, and four tiles and four vectors a
 //                 superstep from a single one (1,270 cycles) were what the whole kernel waited for
-//   warps 17, 24: issue the S/dP MMAs, one for each team (a wait, eight MMAs and their commit take an
+//   warps 17, 26: issue the S/dP MMAs, one for each team (a wait, eight MMAs and their commit take an
 //                 issuer longer than the superstep); warp 17 owns TMEM
-//   warps 18, 25: issue the accumulating MMAs (dK/dV: one warp for dV, one for dK, since a single issuer of
+//   warps 18, 24: issue the accumulating MMAs (dK/dV: one warp for dV, one for dK, since a single issuer of
 //                 both spent most of a superstep on its own waits and commits; dQ has one product and one
 //                 issuer).  All issuers run warp-wide with one elected lane issuing
-//   warp 26     : lister: draws the blocks, looks their lists up and publishes them.  It does so while the block
+//   warp 27     : lister: draws the blocks, looks their lists up and publishes them.  It does so while the block
 //                 before is still being loaded.  (By the first producer after its last load, ticket, list and
 //                 first entries were three trips to memory one after the other, 3,000 to 4,000 cycles from one
 //                 block's last copy to the next one's first, with three supersteps of 1,000 in the ring to bridge
@@ -57,7 +57,7 @@
 // looks at barriers 200; part of it at once), the exponentials 512; a dQ superstep 790, of which the tensor pipe 585.  One
 // superstep's way is 750 cycles to the logits, 850 for the arithmetic, 220 to the accumulating products, 550 until
 // they are complete.  B=2, H=16, N=16384, 25 % of the tiles under a causal mask, forward and backward at the power
-// cap: 1,528 us (1,845 with products of one tile each, shared memory not aligned, no lister and the steps below).
+// cap: 1,578 us (1,904 with products of one tile each, shared memory not aligned, no lister and the steps below).
 // (With S and dP multiplied from tensor memory, which has no room for K and V, the port and the tensor pipe would have
 // 128 cycles a superstep less: 3 %.)
 // Every wait is bounded, and a role that gives up raises a CTA-wide flag, which the others look at when they wait

@@ -313,8 +313,8 @@ __device__ __forceinline__ void umma_ws_ts(uint32_t d_tmem, uint32_t a_tmem, uin
 //    1024 bytes apart (stride byte offset).
 //  * MN-major use (the 64 contiguous elements are the M/N axis, rows are the contraction axis):
 //    one MMA consumes 16 rows = 2 groups of 8 rows, groups 1024 bytes apart (stride byte offset);
-//    the next k-step starts 2048 bytes further.  The leading byte offset would step to a second
-//    64-element chunk of the M/N axis, which never happens for N = 64.
+//    the next k-step starts 2048 bytes further.  The leading byte offset is the way to the second
+//    64-element chunk of the M/N axis: all accumulating products have N = 128, two tiles 8192 bytes apart.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes,
                                                     uint32_t sbo_bytes) {
   uint64_t d = 0;
